@@ -146,11 +146,12 @@ cudaError_t launch_herk_plain(const void* v, const int* count, int nsrc_max, int
 // partial + slice * slice_stride, source count counts[tl]): sum the valid
 // chunks (ceil(count / chunk) of them) in order and write the full Hermitian
 // matrix (nant x nant complex R, row-major) to
-// out + ((f * ntimes_out) + t0 + tl) * nant * nant.
+// out + ((f * ntimes_out) + t0 + tl) * nant * nant.  max_chunks: the most
+// chunks a slice can have (it picks the split of the work only).
 template <typename R>
 cudaError_t launch_reduce(const R* partial, size_t slice_stride, const int* counts, int nt,
-                          int nf, int t0, int ntimes_out, int chunk, int Np, int nant, void* out,
-                          cudaStream_t st);
+                          int nf, int t0, int ntimes_out, int chunk, int max_chunks, int Np,
+                          int nant, void* out, cudaStream_t st);
 
 // --- hv_tc.cu --------------------------------------------------------------
 // Launch shape of the fused kernel; 0 everywhere = the defaults.

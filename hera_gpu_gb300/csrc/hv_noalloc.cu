@@ -23,6 +23,7 @@
 //    call left behind does not matter.
 //  - Requests whose working memory exceeds the array are rejected with
 //    HV_ERR_ARG and a message naming the bytes needed.
+#include <algorithm>
 #include <cuda_runtime.h>
 
 #include <cstdarg>
@@ -150,7 +151,8 @@ extern "C" int hv_vis_gpu_noalloc(const void* d_antpos, int nant, double freq,
                                        static_cast<const Ucoef32*>(U) + (size_t)t * Np, beamT,
                                        Np, nant, beam_px, v, st));
     HV_NA_CK(launch_herk_plain<float>(v, counts + t, nsrc, Np, partial, st));
-    HV_NA_CK(launch_reduce<float>(partial, 0, counts + t, 1, 1, 0, 1, kPlainChunk, Np, nant,
+    HV_NA_CK(launch_reduce<float>(partial, 0, counts + t, 1, 1, 0, 1, kPlainChunk,
+                                  ceil_div(std::max(nsrc, 1), kPlainChunk), Np, nant,
                                   static_cast<float2*>(d_vis_out) + (size_t)t * NN, st));
   }
 #undef HV_NA_CK

@@ -198,19 +198,36 @@ template <typename R> struct Acc;
 template <> struct Acc<float> { using type = KahanF; };
 template <> struct Acc<double> { using type = SumD; };
 
-// Upper 32 x 32 output tile `tile` of slice sl (block of 256 threads).
-template <typename R>
-__device__ __forceinline__ void reduce_tile(const R* __restrict__ partial_base,
+// A slice's upper triangle is reduced in 32 x 32 tiles (row tile A <= column
+// tile B) by blocks of 256 threads: block `part` of a tile takes kCols of its
+// columns b and every row, kCols / 8 elements a thread.  An element is a
+// serial compensated sum over the slice's chunks, so the kernel is bound by
+// memory latency until enough loads are in flight: a thread loads
+// kReduceAhead chunks (both planes) before it adds any of them.  With many
+// chunks (single calls: tens to hundreds) a block takes a quarter of a tile,
+// which spreads small arrays (one to a few tiles a slice) over the SMs; with
+// few chunks a block takes a whole tile, since finding its place costs more
+// than its loads.  Measured on GB300: 30 antennas x 25 slices x 204 chunks
+// 437 us before (whole tiles, one chunk at a time), 29 us now; 350 antennas x
+// 60 slices x 34 chunks 325 us and 176 us (1 GB of partial sums: 5.7 TB/s).
+constexpr int kReduceAhead = 8;
+// Chunks from which a tile is split over four blocks (at 512 antennas x 10
+// slices x 2 chunks splitting it costs 10 us; from 34 chunks on it pays).
+constexpr int kReduceSplitChunks = 8;
+template <typename R, int kCols>
+__device__ __forceinline__ void reduce_part(const R* __restrict__ partial_base,
                                             size_t slice_stride, const int* __restrict__ counts,
                                             int nf, int t0, int ntimes_out, int chunk, int Np,
                                             int nant,
                                             typename Traits<R>::C* __restrict__ out_base,
-                                            int tile, int sl,
+                                            int tile, int part, int sl,
                                             typename Traits<R>::C (*T)[33]) {
   using C = typename Traits<R>::C;
   const int nbt = ceil_div(nant, 32);
   int A, B;
   decode_upper(tile, nbt, A, B);
+  const int b0 = B * 32 + part * kCols;
+  if (b0 >= nant) return;
   const int tl = sl / nf, f = sl % nf;
   const R* partial = partial_base + (size_t)sl * slice_stride;
   C* out = out_base + ((size_t)f * ntimes_out + t0 + tl) * (size_t)nant * nant;
@@ -218,55 +235,61 @@ __device__ __forceinline__ void reduce_tile(const R* __restrict__ partial_base,
   const int nk = n > 0 ? ceil_div(n, chunk) : 0;
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
   const size_t plane = (size_t)Np * Np;
-  for (int bb = ty; bb < 32; bb += 8) {
-    const int a = A * 32 + tx, b = B * 32 + bb;
+  const int a = A * 32 + tx;
+#pragma unroll 1
+  for (int bb = ty; bb < kCols; bb += 8) {
+    const int b = b0 + bb;
     typename Acc<R>::type re, im;
-    if (a < nant && b < nant) {
-      const R* p = partial + (size_t)b * Np + a;
-      for (int k = 0; k < nk; ++k) {
-        re.add(p[(size_t)k * 2 * plane]);
-        im.add(p[(size_t)k * 2 * plane + plane]);
+    // rows and columns past nant lie in the padding (Np is a multiple of
+    // 128), so every lane loads and the loop's conditions are uniform
+    const R* p = partial + (size_t)b * Np + a;
+    int k = 0;
+    for (; k + kReduceAhead <= nk; k += kReduceAhead) {
+      R x[kReduceAhead], y[kReduceAhead];
+#pragma unroll
+      for (int q = 0; q < kReduceAhead; ++q) {
+        x[q] = p[(size_t)(k + q) * 2 * plane];
+        y[q] = p[(size_t)(k + q) * 2 * plane + plane];
+      }
+#pragma unroll
+      for (int q = 0; q < kReduceAhead; ++q) {
+        re.add(x[q]);
+        im.add(y[q]);
       }
     }
-    C val;
-    val.x = re.s; val.y = im.s;
-    T[bb][tx] = val;
-  }
-  __syncthreads();
-  // out[a][b], b contiguous across the warp
-  for (int aa = ty; aa < 32; aa += 8) {
-    const int a = A * 32 + aa, b = B * 32 + tx;
-    if (a >= nant || b >= nant) continue;
-    C val;
-    if (A < B || aa <= tx) {
-      val = T[tx][aa];
-    } else {
-      val = T[aa][tx];
-      val.y = -val.y;
+    for (; k < nk; ++k) {
+      re.add(p[(size_t)k * 2 * plane]);
+      im.add(p[(size_t)k * 2 * plane + plane]);
     }
-    if (a == b) val.y = R(0);
-    out[(size_t)a * nant + b] = val;
-  }
-  if (A < B) {
-    // mirrored block: out[b][a] = conj(V[a][b]), a contiguous across the warp
-    for (int bb = ty; bb < 32; bb += 8) {
-      const int a = A * 32 + tx, b = B * 32 + bb;
-      if (a >= nant || b >= nant) continue;
-      C val = T[bb][tx];
-      val.y = -val.y;
+    C val;
+    val.x = re.s;
+    val.y = a == b ? R(0) : im.s;
+    T[bb][tx] = val;
+    if (a <= b && b < nant) {
+      // below the diagonal: out[b][a] = conj(V[a][b]), a contiguous
+      val.y = a == b ? R(0) : -val.y;
       out[(size_t)b * nant + a] = val;
     }
   }
+  __syncthreads();
+  // above the diagonal: out[a][b], kCols consecutive b a row
+#pragma unroll
+  for (int i = threadIdx.x; i < 32 * kCols; i += 256) {
+    const int aa = i / kCols, bb = i % kCols;
+    const int ao = A * 32 + aa, bo = b0 + bb;
+    if (ao < bo && bo < nant) out[(size_t)ao * nant + bo] = T[bb][aa];
+  }
 }
 
-template <typename R>
+template <typename R, int kCols>
 __global__ void __launch_bounds__(256)
 reduce_kernel(const R* __restrict__ partial_base, size_t slice_stride,
               const int* __restrict__ counts, int nf, int t0, int ntimes_out, int chunk, int Np,
               int nant, typename Traits<R>::C* __restrict__ out_base) {
-  __shared__ typename Traits<R>::C T[32][33];
-  reduce_tile<R>(partial_base, slice_stride, counts, nf, t0, ntimes_out, chunk, Np, nant,
-                 out_base, blockIdx.x, blockIdx.y, T);
+  __shared__ typename Traits<R>::C T[kCols][33];
+  constexpr int kParts = 32 / kCols;
+  reduce_part<R, kCols>(partial_base, slice_stride, counts, nf, t0, ntimes_out, chunk, Np, nant,
+                        out_base, blockIdx.x / kParts, blockIdx.x % kParts, blockIdx.y, T);
 }
 
 // Every simulation of a batch: its split-K chunks reduced into its output.
@@ -280,8 +303,8 @@ reduce_batch_kernel(const PrepSim* __restrict__ sims, int nsims,
   const int tiles = nbt * (nbt + 1) / 2;
   const int local = (int)(blockIdx.x - __ldg(pre + si));
   const size_t slice = (size_t)ceil_div(sm.S > 0 ? sm.S : 1, sm.chunk) * 2 * sm.Np * sm.Np;
-  reduce_tile<float>(sm.partial, slice, sm.counts, sm.F, 0, sm.T, sm.chunk, sm.Np, sm.nant,
-                     static_cast<float2*>(sm.out), local % tiles, local / tiles, T);
+  reduce_part<float, 32>(sm.partial, slice, sm.counts, sm.F, 0, sm.T, sm.chunk, sm.Np, sm.nant,
+                         static_cast<float2*>(sm.out), local % tiles, 0, local / tiles, T);
 }
 
 cudaError_t launch_reduce_batch(const PrepSim* sims, int nsims, const PrepPre& pre,
@@ -293,13 +316,19 @@ cudaError_t launch_reduce_batch(const PrepSim* sims, int nsims, const PrepPre& p
 
 template <typename R>
 cudaError_t launch_reduce(const R* partial, size_t slice_stride, const int* counts, int nt,
-                          int nf, int t0, int ntimes_out, int chunk, int Np, int nant, void* out,
-                          cudaStream_t st) {
+                          int nf, int t0, int ntimes_out, int chunk, int max_chunks, int Np,
+                          int nant, void* out, cudaStream_t st) {
+  using C = typename Traits<R>::C;
   const int nbt = ceil_div(nant, 32);
-  dim3 grid(nbt * (nbt + 1) / 2, nt * nf);
-  reduce_kernel<R><<<grid, 256, 0, st>>>(partial, slice_stride, counts, nf, t0, ntimes_out,
-                                         chunk, Np, nant,
-                                         reinterpret_cast<typename Traits<R>::C*>(out));
+  const int tiles = nbt * (nbt + 1) / 2;
+  if (max_chunks >= kReduceSplitChunks)
+    reduce_kernel<R, 8><<<dim3(tiles * 4, nt * nf), 256, 0, st>>>(
+        partial, slice_stride, counts, nf, t0, ntimes_out, chunk, Np, nant,
+        reinterpret_cast<C*>(out));
+  else
+    reduce_kernel<R, 32><<<dim3(tiles, nt * nf), 256, 0, st>>>(
+        partial, slice_stride, counts, nf, t0, ntimes_out, chunk, Np, nant,
+        reinterpret_cast<C*>(out));
   return cudaGetLastError();
 }
 
@@ -307,7 +336,7 @@ template cudaError_t launch_gen_phasors<float>(const void*, const int*, int, con
 template cudaError_t launch_gen_phasors<double>(const void*, const int*, int, const void*, const double*, int, int, int, void*, cudaStream_t);
 template cudaError_t launch_herk_plain<float>(const void*, const int*, int, int, float*, cudaStream_t);
 template cudaError_t launch_herk_plain<double>(const void*, const int*, int, int, double*, cudaStream_t);
-template cudaError_t launch_reduce<float>(const float*, size_t, const int*, int, int, int, int, int, int, int, void*, cudaStream_t);
-template cudaError_t launch_reduce<double>(const double*, size_t, const int*, int, int, int, int, int, int, int, void*, cudaStream_t);
+template cudaError_t launch_reduce<float>(const float*, size_t, const int*, int, int, int, int, int, int, int, int, void*, cudaStream_t);
+template cudaError_t launch_reduce<double>(const double*, size_t, const int*, int, int, int, int, int, int, int, int, void*, cudaStream_t);
 
 }  // namespace hv
