@@ -127,8 +127,9 @@ def tc_chunk(nsrc, nslices, ngroups, num_sms):
     """Split-K chunk the library picks (hv_tc.cu tc_chunk_sources)."""
     nchunk = max(1, -(-40 * num_sms // (nslices * ngroups)))
     c = -(-max(nsrc // 2, 1) // nchunk)
-    c = min(16384, max(1024, c))
-    return (c + 31) // 32 * 32
+    c = min(32768, max(1024, c))
+    unit = 2048 if c > 2048 else 32
+    return (c + unit // 2) // unit * unit
 
 
 def tc_groups(nant):

@@ -1496,7 +1496,11 @@ int tc_chunk_sources(int nsrc, int nslices, int ngroups, int num_sms) {
   const long long up = std::max(nsrc / 2, 1);
   long long c = (up + nchunk - 1) / nchunk;
   c = std::min<long long>(32768, std::max<long long>(1024, c));
-  c = (c + 31) / 32 * 32;
+  // whole stages; above one accumulator flush, whole flushes: a chunk a few
+  // stages longer than that pays another epilogue for them (350 antennas x
+  // 1M sources x 16 slices: 4128 sources took three flushes, 4096 take two)
+  const long long unit = c > TC_FLUSH_SOURCES ? TC_FLUSH_SOURCES : 32;
+  c = (c + unit / 2) / unit * unit;
   return (int)c;
 }
 
