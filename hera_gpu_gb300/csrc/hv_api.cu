@@ -267,12 +267,17 @@ int run_device(hv_context* ctx, int method, const R* antpos, int nant, const dou
       const R* crd_use = crd_eq;
       const R* I_use = I_sky;
       if (nsrc > 0) {
-        HV_ENSURE(ctx->sortkv, sizeof(unsigned long long) * (size_t)sort_pad(nsrc));
+        HV_ENSURE(ctx->sortkv, sizeof(unsigned long long) * (size_t)nsrc);
         HV_ENSURE(ctx->crd_sorted, sizeof(float) * 3 * (size_t)nsrc);
         HV_ENSURE(ctx->I_sorted, sizeof(float) * (size_t)nsrc);
+        // the sort's digit tables (half a byte a source) use the partial sums'
+        // buffer (at least 4 bytes a source and 128 KB), not yet in use
+        if (sort_table_bytes(nsrc) > ctx->partial.cap)
+          return fail(ctx, HV_ERR_OOM, "no room for the sort's digit tables");
         int nl = 0;
         HV_CK(launch_sort_sources(reinterpret_cast<const float*>(crd_eq),
                                   reinterpret_cast<const float*>(I_sky), nsrc, ctx->sortkv.p,
+                                  ctx->partial.p,
                                   static_cast<float*>(ctx->crd_sorted.p),
                                   static_cast<float*>(ctx->I_sorted.p), &nl, st));
         ctx->launches += nl;

@@ -96,13 +96,16 @@ cudaError_t launch_prep(const R* crd_eq, const R* I_sky, int nsrc, const R* eq2t
 cudaError_t launch_ubound(const void* U, int nslices, int Np, float* umax, cudaStream_t st);
 
 // --- hv_sort.cu ------------------------------------------------------------
-// Spatial (Morton) order of the sources: kv_buf needs sort_pad(nsrc) 64-bit
-// words; writes the permuted crd_eq (3 x nsrc) and I_sky.  *launches is set
-// to the number of kernels launched.
-int sort_pad(int nsrc);
+// Spatial (Morton) order of the sources: kv_buf needs nsrc 64-bit words and
+// table_buf sort_table_bytes(nsrc); writes the permuted crd_eq (3 x nsrc, at
+// an 8-byte aligned address: it holds sort words in between) and I_sky.
+// *launches is set to the number of kernels launched.
+size_t sort_table_bytes(int nsrc);
 cudaError_t launch_sort_sources(const float* crd_eq, const float* I_sky, int nsrc, void* kv_buf,
-                                float* crd_sorted, float* I_sorted, int* launches,
-                                cudaStream_t st);
+                                void* table_buf, float* crd_sorted, float* I_sorted,
+                                int* launches, cudaStream_t st);
+// Words of a batch's segment of nsrc sources: a power of two, at least 2048.
+int sort_pad(int nsrc);
 
 // launch_prep with records of time tt at rec + tt * rec_stride.
 template <typename R>

@@ -34,3 +34,16 @@ def test_split_k_reduction(nant, nsrc, method, tol):
     check_hermitian(v)
     ref = vis_oracle(*[a.astype(np.float64) if isinstance(a, np.ndarray) else a for a in args])
     assert rel_frobenius(v, ref).max() <= tol
+
+
+# spatial sort: one block up to 4096 sources (rows of 512), the radix passes
+# beyond (tiles of 2048); any order gives the same sum up to rounding, so a
+# lost or doubled source shows as an error far above the tolerance
+@gpu
+@pytest.mark.parametrize("nsrc", [1, 31, 512, 513, 4095, 4096, 4097, 6144, 6145])
+def test_spatial_sort_keeps_every_source(nsrc):
+    args = sim(5, nsrc, seed=nsrc)
+    args[3][:, : nsrc // 3] = args[3][:, :1]      # ties: many sources in one direction
+    v = vis_gpu(*args, precision=1, method="tc")
+    ref = vis_oracle(*[a.astype(np.float64) if isinstance(a, np.ndarray) else a for a in args])
+    np.testing.assert_allclose(v, ref, rtol=1e-4, atol=1e-4 * max(1e-30, np.abs(ref).max()))
