@@ -16,6 +16,7 @@
 #include <cstdio>
 #include <algorithm>
 #include <cstring>
+#include <iterator>
 #include <string>
 #include <utility>
 #include <vector>
@@ -68,6 +69,9 @@ struct hv_context {
   // workspace
   DevBuf freqs, beamT, ucoef, rec, counts, blkcounts, v, partial, tcgroups;
   DevBuf umax, sortkv, crd_sorted, I_sorted, tctable, pixmax, sbound;
+  // tensor-core FP64 product: given back when another path finds no room
+  DevBuf f64_v, f64_digits, f64_words, f64_small;
+  bool f64_running = false;
   HostBuf tctable_h;  // page-locked staging of the fused kernel's simulation table
   // page-locked blocks given back by destroyed batches, kept for the next
   // ones: freeing page-locked memory waits for the whole device
@@ -115,6 +119,25 @@ int fail(hv_context* c, int code, const char* fmt, ...) {
     }                                                               \
   } while (0)
 
+void release(hv_context* ctx, DevBuf& b) {
+  if (b.p) cudaFree(b.p);
+  ctx->held -= b.cap;
+  b.p = nullptr;
+  b.cap = 0;
+}
+
+// Gives the FP64 product's workspace back (unless it is in use); false if
+// there was none.  The device is idle: ensure() has waited for it.
+bool release_f64(hv_context* ctx) {
+  if (ctx->f64_running) return false;
+  bool any = false;
+  for (DevBuf* b : {&ctx->f64_v, &ctx->f64_digits, &ctx->f64_words, &ctx->f64_small}) {
+    any = any || b->p;
+    release(ctx, *b);
+  }
+  return any;
+}
+
 int ensure(hv_context* ctx, DevBuf& b, size_t bytes) {
   if (bytes == 0) bytes = 256;
   if (b.cap >= bytes) return HV_OK;
@@ -128,10 +151,15 @@ int ensure(hv_context* ctx, DevBuf& b, size_t bytes) {
   }
   size_t want = bytes + bytes / 8;  // slack against regrowth
   if (ctx->budget && ctx->held + want > ctx->budget) want = bytes;
+  if (ctx->budget && ctx->held + want > ctx->budget) release_f64(ctx);
   if (ctx->budget && ctx->held + want > ctx->budget)
     return fail(ctx, HV_ERR_OOM, "workspace of %zu bytes exceeds the HBM budget (%zu held of %zu)",
                 want, ctx->held, ctx->budget);
   cudaError_t e = cudaMalloc(&b.p, want);
+  if (e == cudaErrorMemoryAllocation && release_f64(ctx)) {
+    cudaGetLastError();
+    e = cudaMalloc(&b.p, want);
+  }
   if (e != cudaSuccess) {
     cudaGetLastError();
     b.p = nullptr;
@@ -166,13 +194,6 @@ int ensure_host(hv_context* ctx, HostBuf& b, size_t bytes) {
     if (r_ != HV_OK) return r_;               \
   } while (0)
 
-void release(hv_context* ctx, DevBuf& b) {
-  if (b.p) cudaFree(b.p);
-  ctx->held -= b.cap;
-  b.p = nullptr;
-  b.cap = 0;
-}
-
 int check_shapes(hv_context* ctx, int precision, int method, int nant, int nfreq,
                  int ntimes, int nsrc, int P) {
   if (precision != 1 && precision != 2)
@@ -200,6 +221,113 @@ int check_shapes(hv_context* ctx, int precision, int method, int nant, int nfreq
 // records of one batch of times.
 constexpr size_t kTcPartialCap = size_t(6) << 30;
 constexpr size_t kTcRecCap = size_t(4) << 30;
+
+// FP64 product on the tensor cores (hv_f64.cu) for every slice; HV_OK, an
+// error, or -1: the SIMT product is to be used (arrays whose class sums would
+// not fit, or no room for the workspace within the budget or on the device).
+// Measured at 350 antennas x 100k sources x 3 times: SIMT 102.7 ms a call;
+// at 25 antennas x 1008 sources x 35 times SIMT 75 ms (few tiles a slice, one
+// slice at a time).
+constexpr int kF64MaxNp = 2048;             // 96 bytes of class sums an element: 400 MB
+constexpr int kF64Window = 65536;           // sources per window (40 bytes a phasor)
+constexpr size_t kF64Cap = size_t(4) << 30; // workspace of the slices of one launch
+
+int run_f64(hv_context* ctx, const double* eq2tops, const double* crd_eq, const double* I_sky,
+            int nsrc, int nant, int Np, int nfreq, int ntimes, int P, int* counts, void* out,
+            cudaStream_t st) {
+  using namespace hv;
+  if (Np > kF64MaxNp) return -1;
+  const int S1 = std::max(nsrc, 1);
+  const int S = std::min(kF64Window, (S1 + 31) / 32 * 32);
+  const size_t b_v = sizeof(double2) * (size_t)S * Np, b_dig = f64_digit_bytes(Np, S),
+               b_w = f64_word_bytes(Np), b_rec = sizeof(SrcRec64) * (size_t)S1,
+               b_small = sizeof(uint32_t) * Np + sizeof(int);
+  const size_t per = b_v + b_dig + b_w;
+  // slices a launch: whole times, or some frequencies of one time; as many
+  // (half as many after each failure) as the budget and the device hold
+  long long nz = std::max<long long>(1, std::min<long long>(
+      std::min<long long>(32768, (long long)ntimes * nfreq), (long long)(kF64Cap / per)));
+  int ntb = 0, nfb = 0;
+  struct Running {
+    hv_context* c;
+    ~Running() { c->f64_running = false; }
+  } running{ctx};
+  for (;; nz /= 2) {
+    ctx->f64_running = nz > 0;
+    if (nz == 0) {
+      cudaDeviceSynchronize();
+      release_f64(ctx);
+      return -1;
+    }
+    nfb = (int)std::min<long long>(nfreq, nz);
+    ntb = nfb == nfreq ? (int)std::max<long long>(1, std::min<long long>(ntimes, nz / nfreq)) : 1;
+    const size_t n = (size_t)ntb * nfb;
+    const std::pair<DevBuf*, size_t> want[] = {
+        {&ctx->f64_v, b_v * n},
+        {&ctx->f64_digits, b_dig * n},
+        {&ctx->f64_words, b_w * n},
+        {&ctx->f64_small, f64_table_bytes() + b_small * n},
+        {&ctx->rec, b_rec * ntb},
+        {&ctx->blkcounts, sizeof(int) * (size_t)prep_blocks(nsrc) * ntb}};
+    // before any buffer grows: a buffer grown for more slices than fit would
+    // leave less room for the others
+    size_t grow = 0;
+    for (auto& w : want) grow += w.second > w.first->cap ? w.second - w.first->cap : 0;
+    grow += grow / 8 + 256 * std::size(want);  // ensure()'s slack
+    if (ctx->budget && ctx->held + grow > ctx->budget) continue;
+    int r = HV_OK;
+    for (auto& w : want)
+      if (r == HV_OK) r = ensure(ctx, *w.first, w.second);
+    if (r == HV_OK) break;
+    if (r != HV_ERR_OOM) return r;
+    ctx->err.clear();
+  }
+  const size_t nmax = (size_t)ntb * nfb;
+  char* small = static_cast<char*>(ctx->f64_small.p);
+  uint32_t* rowmax = reinterpret_cast<uint32_t*>(small + f64_table_bytes());
+  int* flags = reinterpret_cast<int*>(rowmax + nmax * Np);
+  long long* words = static_cast<long long*>(ctx->f64_words.p);
+  HV_LAUNCH(1, launch_f64_table(small, st));
+  F64Dims d{};
+  d.u_nf = nfreq;
+  d.nant = nant;
+  d.Np = Np;
+  d.S = S;
+  d.nks = S / 32;
+  d.v_stride = (size_t)S * Np;
+  d.dig_stride = b_dig;
+  d.w_stride = b_w / sizeof(long long);
+  for (int t0 = 0; t0 < ntimes; t0 += ntb) {
+    const int nt = std::min(ntb, ntimes - t0);
+    HV_LAUNCH(2, launch_prep_strided<double>(crd_eq, I_sky, nsrc, eq2tops, t0, nt, P,
+                                             static_cast<int*>(ctx->blkcounts.p), ctx->rec.p,
+                                             (size_t)S1, counts + t0, st));
+    d.counts = counts + t0;
+    for (int f0 = 0; f0 < nfreq; f0 += nfb) {
+      d.nf = std::min(nfb, nfreq - f0);
+      const int n = nt * d.nf;
+      const Ucoef64* U = static_cast<const Ucoef64*>(ctx->ucoef.p) +
+                         ((size_t)t0 * nfreq + f0) * Np;
+      const double* beam = static_cast<const double*>(ctx->beamT.p) + (size_t)f0 * P * P * Np;
+      for (d.s0 = 0; d.s0 < S1; d.s0 += S) {
+        HV_CK(cudaMemsetAsync(rowmax, 0, (char*)(flags + nmax) - (char*)rowmax, st));
+        HV_CK(cudaMemsetAsync(words, 0, b_w * n, st));
+        HV_LAUNCH(1, launch_f64_phasors(d, n, ctx->rec.p, (size_t)S1, U, beam, P, small,
+                                        ctx->f64_v.p, rowmax, st));
+        // digits and class sums; the SIMT product of the flagged slices
+        HV_LAUNCH_TIMED(launch_f64_product(d, n, ctx->f64_v.p, rowmax, ctx->f64_digits.p, flags,
+                                           words, ctx->num_sms, ctx->d_err, ctx->wait_ns, st),
+                        st);
+        HV_LAUNCH(2, launch_herk_flagged(d, n, ctx->f64_v.p, flags,
+                                         static_cast<double*>(ctx->f64_digits.p),
+                                         b_dig / sizeof(double), st));
+        HV_LAUNCH(1, launch_f64_final(d, n, words, rowmax, flags, ctx->f64_digits.p, t0, f0,
+                                      ntimes, out, st));
+      }
+    }
+  }
+  return HV_OK;
+}
 
 template <typename R>
 int run_device(hv_context* ctx, int method, const R* antpos, int nant, const double* freqs,
@@ -333,6 +461,12 @@ int run_device(hv_context* ctx, int method, const R* antpos, int nant, const dou
       }
     }
     return HV_OK;
+  }
+
+  if constexpr (sizeof(R) == 8) {
+    const int r = run_f64(ctx, eq2tops, crd_eq, I_sky, nsrc, nant, Np, nfreq, ntimes, P, counts,
+                          out, st);
+    if (r >= 0) return r;
   }
 
   // plain form: one time at a time, one frequency at a time
@@ -504,7 +638,8 @@ int hv_destroy(hv_context* ctx) {
                     &ctx->out_vis, &ctx->freqs, &ctx->beamT, &ctx->ucoef, &ctx->rec,
                     &ctx->counts, &ctx->blkcounts, &ctx->v, &ctx->partial, &ctx->tcgroups,
                     &ctx->umax, &ctx->sortkv, &ctx->crd_sorted, &ctx->I_sorted, &ctx->tctable,
-                    &ctx->pixmax, &ctx->sbound};
+                    &ctx->pixmax, &ctx->sbound, &ctx->f64_v, &ctx->f64_digits,
+                    &ctx->f64_words, &ctx->f64_small};
   for (DevBuf* b : bufs) release(ctx, *b);
   if (ctx->tctable_h.p) cudaFreeHost(ctx->tctable_h.p);
   for (auto& hp : ctx->host_pool) cudaFreeHost(hp.first);

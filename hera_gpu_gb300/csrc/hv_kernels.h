@@ -145,6 +145,13 @@ template <typename R>
 cudaError_t launch_herk_plain(const void* v, const int* count, int nsrc_max, int Np,
                               R* partial, cudaStream_t st);
 
+// The same for nz slices in FP64, only those with flags[z] set (hv_f64.cu):
+// the sources of window d, their chunks' sums at partial + z *
+// partial_stride.
+struct F64Dims;
+cudaError_t launch_herk_flagged(const F64Dims& d, int nz, const void* v, const int* flags,
+                                double* partial, size_t partial_stride, cudaStream_t st);
+
 // For each of nt * nf slices (slice = tl * nf + f, partial sums at
 // partial + slice * slice_stride, source count counts[tl]): sum the valid
 // chunks (ceil(count / chunk) of them) in order and write the full Hermitian
@@ -155,6 +162,39 @@ template <typename R>
 cudaError_t launch_reduce(const R* partial, size_t slice_stride, const int* counts, int nt,
                           int nf, int t0, int ntimes_out, int chunk, int max_chunks, int Np,
                           int nant, void* out, cudaStream_t st);
+
+// --- hv_f64.cu -------------------------------------------------------------
+// FP64 product on the tensor cores.  Slices z = tl * nf + fl (nf of the
+// launch's frequencies), sources in windows of up to S (a multiple of 32)
+// from s0 on of each time's records; buffers with a stride a slice.
+struct F64Dims {
+  const int* counts;  // sources above the horizon per time
+  int nf, u_nf;       // frequencies of the launch, and of U
+  int nant, Np;
+  int s0, S, nks;     // window of sources; S / 32
+  size_t v_stride;    // phasors (complex128) a slice: S * Np
+  size_t dig_stride;  // bytes of digits a slice: f64_digit_bytes
+  size_t w_stride;    // words a slice: f64_word_bytes / 8
+};
+size_t f64_digit_bytes(int Np, int S);
+size_t f64_word_bytes(int Np);
+size_t f64_table_bytes();
+cudaError_t launch_f64_table(void* table, cudaStream_t st);
+// Phasors v[z][s][a] and the largest component per antenna, rowmax[z][Np]
+// (high words; zeroed beforehand).  U, beamT: of the launch's first slice.
+cudaError_t launch_f64_phasors(const F64Dims& d, int nz, const void* rec, size_t rec_stride,
+                               const void* U, const double* beamT, int P, const void* table,
+                               void* v, uint32_t* rowmax, cudaStream_t st);
+// Digits of v and their class sums, added to W (zeroed beforehand); flags[z]
+// (zeroed beforehand) is set for slices that need launch_herk_flagged.
+cudaError_t launch_f64_product(const F64Dims& d, int nz, const void* v, const uint32_t* rowmax,
+                               void* dig, int* flags, long long* W, int num_sms, int* err,
+                               unsigned long long wait_ns, cudaStream_t st);
+// The window's visibilities, stored to (s0 = 0) or added to the output
+// (nfreq, ntimes, nant, nant) at times t0 + tl, frequencies f0 + fl.
+cudaError_t launch_f64_final(const F64Dims& d, int nz, const long long* W,
+                             const uint32_t* rowmax, const int* flags, const void* partial,
+                             int t0, int f0, int ntimes, void* out, cudaStream_t st);
 
 // --- hv_tc.cu --------------------------------------------------------------
 // Launch shape of the fused kernel; 0 everywhere = the defaults.

@@ -4,7 +4,8 @@
 //   gen_phasors : v[s][a] = A_a(l_s, m_s) sqrt(I_s) exp(2 pi i U_a . s)
 //                 (InterpolateBeam + MeasEq, vis.py:46-110) written to HBM.
 //   herk_plain  : V[a][b] = sum_s v[a,s] conj(v[b,s]) on the upper triangle
-//                 only, FP32 (precision 1) or FP64 (precision 2) FMA on the
+//                 only, FP32 (precision 1) or FP64 (precision 2, where the
+//                 tensor-core product of hv_f64.cu does not apply) FMA on the
 //                 CUDA cores; the reference runs a full CGEMM/ZGEMM
 //                 (vis.py:246-249).  Sources are split into chunks of
 //                 kPlainChunk; each chunk's partial sum is stored.
@@ -72,11 +73,9 @@ __device__ __forceinline__ void decode_upper(int t, int nb, int& I, int& J) {
 }
 
 template <typename R>
-__global__ void __launch_bounds__(256)
-herk_plain_kernel(const typename Traits<R>::C* __restrict__ v, const int* __restrict__ count,
-                  int Np, R* __restrict__ partial) {
+__device__ __forceinline__ void herk_tile(const typename Traits<R>::C* __restrict__ v, int n,
+                                          int Np, R* __restrict__ partial) {
   using C = typename Traits<R>::C;
-  const int n = *count;
   const int s0 = blockIdx.y * kPlainChunk;
   if (s0 >= n) return;
   const int s1 = min(s0 + kPlainChunk, n);
@@ -166,6 +165,32 @@ herk_plain_kernel(const typename Traits<R>::C* __restrict__ v, const int* __rest
       pim[(size_t)b * Np + a] = acc_im[i][j];
     }
   }
+}
+
+template <typename R>
+__global__ void __launch_bounds__(256)
+herk_plain_kernel(const typename Traits<R>::C* __restrict__ v, const int* __restrict__ count,
+                  int Np, R* __restrict__ partial) {
+  herk_tile<R>(v, *count, Np, partial);
+}
+
+__global__ void __launch_bounds__(256)
+herk_flagged_kernel(const F64Dims d, const double2* __restrict__ v,
+                    const int* __restrict__ flags, double* __restrict__ partial,
+                    size_t partial_stride) {
+  const int z = blockIdx.z;
+  if (!flags[z]) return;
+  const int n = max(0, min(d.counts[z / d.nf] - d.s0, d.S));
+  herk_tile<double>(v + (size_t)z * d.v_stride, n, d.Np, partial + (size_t)z * partial_stride);
+}
+
+cudaError_t launch_herk_flagged(const F64Dims& d, int nz, const void* v, const int* flags,
+                                double* partial, size_t partial_stride, cudaStream_t st) {
+  const int nb = d.Np / kHT;
+  const dim3 grid(nb * (nb + 1) / 2, ceil_div(d.S, kPlainChunk), nz);
+  herk_flagged_kernel<<<grid, 256, 0, st>>>(d, static_cast<const double2*>(v), flags, partial,
+                                            partial_stride);
+  return cudaGetLastError();
 }
 
 template <typename R>

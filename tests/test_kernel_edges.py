@@ -47,3 +47,91 @@ def test_spatial_sort_keeps_every_source(nsrc):
     v = vis_gpu(*args, precision=1, method="tc")
     ref = vis_oracle(*[a.astype(np.float64) if isinstance(a, np.ndarray) else a for a in args])
     np.testing.assert_allclose(v, ref, rtol=1e-4, atol=1e-4 * max(1e-30, np.abs(ref).max()))
+
+
+# FP64 product on the tensor cores.  Each entry is compared relative to
+# sqrt(V_aa V_bb), the scale FP64 rounding acts on, so that an antenna with a
+# faint beam is held to the same relative error.  1e-11 is the FP64 path's
+# bound (phases of up to ~1e3 cycles rounded in FP64: 1e3 * 2^-53 * 2 pi).
+F64_TOL = 1e-11
+
+
+def oracle64(args):
+    return vis_oracle(*[a.astype(np.float64) if isinstance(a, np.ndarray) else a for a in args])
+
+
+def check64(v, ref):
+    p = np.sqrt(np.abs(np.einsum("taa->ta", ref)))
+    scale = p[:, :, None] * p[:, None, :]
+    assert np.all(np.abs(v - ref) <= F64_TOL * scale + 1e-300)
+
+
+# one to three antenna blocks; sources around the 32-source steps
+@gpu
+@pytest.mark.parametrize("nant,nsrc", [(1, 1), (2, 63), (32, 65), (33, 500), (127, 4200),
+                                       (128, 130), (129, 1000), (300, 700), (7, 0)])
+def test_fp64_product(nant, nsrc):
+    args = sim(nant, nsrc, ntimes=2, seed=nant + nsrc, dtype=np.float64)
+    v = vis_gpu(*args, precision=2)
+    check_hermitian(v)
+    check64(v, oracle64(args))
+
+
+# more than one window of 65536 sources above the horizon
+@gpu
+def test_fp64_product_source_windows():
+    args = sim(5, 150_000, ntimes=1, seed=3, dtype=np.float64)
+    v = vis_gpu(*args, precision=2)
+    check_hermitian(v)
+    check64(v, oracle64(args))
+
+
+# several launches of whole times, and of some frequencies of one time, must
+# give the bits of one launch: a budget leaves room for fewer slices, or for
+# none (the SIMT product: other rounding)
+@gpu
+def test_fp64_product_under_a_budget():
+    from hera_gpu_gb300 import vis_gpu_multifreq
+    from hera_gpu_gb300._native import Context
+    c = synth.config_array(seed=4, nant=130, nsrc=3000, ntimes=3, nfreq=3, fmin=1e8, fmax=2e8, P=9)
+    bm = synth.beams_for(c, dtype=np.float64)
+    args = (c["antpos"], c["freqs"], c["eq2tops"], c["crd_eq"], c["I_sky"], bm)
+    full = vis_gpu_multifreq(*args, precision=2)
+    for mb, same in ((120, True), (60, True), (33, False)):
+        v = vis_gpu_multifreq(*args, precision=2, context=Context(0, hbm_budget_bytes=mb << 20))
+        if same:
+            np.testing.assert_array_equal(v, full)
+        else:
+            assert np.abs(v - full).max() <= F64_TOL * np.abs(full).max()
+
+
+# antennas of very different scale, a dark antenna, and scales outside the
+# digit form's range (2^-400): the slice takes the SIMT product
+@gpu
+@pytest.mark.parametrize("small", [1e-30, 1e-100, 1e-140])
+def test_fp64_product_antenna_scales(small):
+    args = list(sim(40, 900, ntimes=1, seed=5, dtype=np.float64))
+    bm = args[5].copy()
+    bm[3] *= small
+    bm[17] = 0.0
+    bm[21] *= -1.0
+    args[5] = bm
+    v = vis_gpu(*args, precision=2)
+    check64(v, oracle64(args))
+    np.testing.assert_array_equal(v[0, 17], 0)
+
+
+# infinities and NaN reach the entries they reach in the SIMT product
+@gpu
+@pytest.mark.parametrize("bad", [np.nan, np.inf])
+def test_fp64_product_not_finite(bad):
+    args = list(sim(35, 400, ntimes=2, seed=6, dtype=np.float64))
+    clean = vis_gpu(*args, precision=2)
+    bm = args[5].copy()
+    bm[4] = bad
+    args[5] = bm
+    v = vis_gpu(*args, precision=2)
+    others = [a for a in range(35) if a != 4]
+    assert not np.isfinite(v[:, 4]).any() and not np.isfinite(v[:, :, 4]).any()
+    np.testing.assert_allclose(v[:, others][:, :, others], clean[:, others][:, :, others],
+                               rtol=0, atol=F64_TOL * np.abs(clean).max())
