@@ -135,3 +135,30 @@ def test_fp64_product_not_finite(bad):
     assert not np.isfinite(v[:, 4]).any() and not np.isfinite(v[:, :, 4]).any()
     np.testing.assert_allclose(v[:, others][:, :, others], clean[:, others][:, :, others],
                                rtol=0, atol=F64_TOL * np.abs(clean).max())
+
+
+# median strip kernels: every window shape they take (and the nearest they do
+# not), images narrower than a window, at the edges of the strips (128 columns
+# for 3 x 3, 52 to 62 otherwise) and of their 16 rows, with signed zeros,
+# infinities, NaN and ties
+@gpu
+@pytest.mark.parametrize("ks", [(h, w) for h in (1, 3, 5, 7, 9) for w in (1, 3, 5, 7, 9)]
+                         + [(1, 11), (11, 1), (11, 3), (2, 3)])
+def test_median_strips(ks):
+    from hera_gpu_gb300 import MedianFilter
+    from oracle import median_filter_oracle
+    rng = np.random.default_rng(ks[0] * 16 + ks[1])
+    for shape in ((1, 1), (2, 3), (15, 52), (16, 54), (17, 63), (33, 129), (40, 260)):
+        img = rng.normal(size=shape).astype(np.float32)
+        img[rng.random(shape) < 0.2] = 0.0
+        img[rng.random(shape) < 0.1] = -0.0
+        img[rng.random(shape) < 0.1] = 1.0
+        img[rng.random(shape) < 0.03] = np.inf
+        img[rng.random(shape) < 0.03] = -np.inf
+        out = MedianFilter(input=img, kernel_size=ks)[0]
+        ref = median_filter_oracle(img, *ks)
+        np.testing.assert_array_equal(out, ref)          # zeros compare equal whatever their sign
+    # keys order -0.0 below 0.0 and NaN by its bits: a window of NaN is NaN
+    img[:] = np.nan
+    inner = MedianFilter(input=img, kernel_size=ks)[0][8:-8, 8:-8]
+    assert np.isnan(inner).all()
