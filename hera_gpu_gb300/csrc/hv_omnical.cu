@@ -25,7 +25,9 @@
 // needed.  The sums over each antenna's and each unique baseline's
 // baselines are gathers over a fixed incidence list (CSR), each segment
 // summed by a fixed group of lanes in a fixed order, so the result does not
-// depend on scheduling and repeats bit for bit.
+// depend on scheduling and repeats bit for bit.  In float32, arrays of 17 to
+// 256 antennas whose baselines are distinct antenna pairs take a kernel of
+// their own (omnical_dense_kernel).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -247,7 +249,15 @@ __device__ __forceinline__ R chisq_part(const C* sol, int nants, const uint2* __
 // |m_b|^2 = |g_i|^2 |g_j|^2 |u_k|^2, so the factor is taken as
 // w_b ra_i ra_j ru_k with ra = |g0|^2 / |g|^2 per antenna and ru per unique
 // baseline: nants + nubls divisions an iteration instead of nbls.
-template <typename R, bool kDataShared>
+//
+// kFactored (float64, which is bound by the FP64 pipe): the ratios are kept
+// multiplied into the factors, p_a = conj(g_a) ra_a and c_k = conj(u_k) ru_k,
+// so that d_b = data_b w_b p_i conj(p_j) c_k takes 14 operations instead of 17;
+// the weights come from the factors' magnitudes (3 instead of 11), and a step
+// divides once a segment instead of twice: 12 iterations of 1000 problems of 54
+// antennas 1.72 and 1.52 ms, of 200 of 180 antennas 5.05 and 4.41 ms.  It takes 8 bytes more of shared
+// memory a segment; problems that only fit without it go without.
+template <typename R, bool kDataShared, bool kFactored>
 __global__ void __launch_bounds__(kOmMaxThreads, OM_MINB) omnical_kernel(const OmParams<R> p) {
   using C = typename Cx<R>::T;
   constexpr int U = Unroll<R>::n;
@@ -259,7 +269,8 @@ __global__ void __launch_bounds__(kOmMaxThreads, OM_MINB) omnical_kernel(const O
   R* const gw = reinterpret_cast<R*>(solB + nseg);  // gwgt | uwgt
   R* const mg0 = gw + nseg;                         // |g0|^2 | |u0|^2
   R* const ra = mg0 + nseg;                         // ratios
-  R* const red = ra + nseg;                         // 96 values
+  R* const red = ra + (kFactored ? 2 : 1) * nseg;   // 96 values
+  C* const pc = reinterpret_cast<C*>(ra);           // kFactored: p | c instead of the ratios
   unsigned char* next = reinterpret_cast<unsigned char*>(red + 96);
   next = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(next) + 15) & ~uintptr_t(15));
   C* const d = reinterpret_cast<C*>(next);
@@ -305,11 +316,19 @@ __global__ void __launch_bounds__(kOmMaxThreads, OM_MINB) omnical_kernel(const O
         // weights from the current model (calc_dwgts, calc_gu_wgt)
         for (int s = tid; s < nseg; s += nt) {
           mg0[s] = mag2(sol[s]);
-          ra[s] = 1;
+          if constexpr (kFactored) pc[s] = conjc(sol[s]);
+          else ra[s] = 1;
         }
+        if (kFactored) __syncthreads();  // the magnitudes are read below
         for (int pn = 0; pn < np; ++pn) {
           const int b0 = pn * PB, nb = min(PB, nbls - b0);
-          for (int b = tid; b < nb; b += nt) dw[b] = mag2(model(sol, nants, bl[b0 + b])) * wgt[b0 + b];
+          for (int b = tid; b < nb; b += nt) {
+            const uint2 e = bl[b0 + b];
+            if constexpr (kFactored)
+              dw[b] = mg0[e.x & 0xffffu] * mg0[e.x >> 16] * (mg0[nants + e.y] * wgt[b0 + b]);
+            else
+              dw[b] = mag2(model(sol, nants, e)) * wgt[b0 + b];
+          }
           __syncthreads();
           seg_gather<Unroll<R>::gather, RealV<R>>(
               p.seg_off + (size_t)pn * (nseg + 1), p.seg_ent, nseg, p.group,
@@ -318,7 +337,17 @@ __global__ void __launch_bounds__(kOmMaxThreads, OM_MINB) omnical_kernel(const O
           __syncthreads();  // dw is overwritten below
         }
       } else {
-        for (int s = tid; s < nseg; s += nt) ra[s] = mg0[s] / mag2(sol[s]);
+        for (int s = tid; s < nseg; s += nt) {
+          const R q = mg0[s] / mag2(sol[s]);
+          if constexpr (kFactored) {
+            C c = conjc(sol[s]);
+            c.x *= q;
+            c.y *= q;
+            pc[s] = c;
+          } else {
+            ra[s] = q;
+          }
+        }
         __syncthreads();
       }
       // d_b = data_b conj(m_b) dwgts_b / |m_b|^2 (calc_gu_buf), summed per
@@ -340,11 +369,18 @@ __global__ void __launch_bounds__(kOmMaxThreads, OM_MINB) omnical_kernel(const O
           for (int q = 0; q < U; ++q)
             if (c0 + q * nt < nb) {
               const int i = e[q].x & 0xffffu, j = e[q].x >> 16;
-              const C m = model(sol, nants, e[q]);
-              const R t = w[q] * ra[i] * ra[j] * ra[nants + e[q].y];
-              C z = cmul(x[q], conjc(m));
-              z.x *= t;
-              z.y *= t;
+              C z;
+              if constexpr (kFactored) {
+                x[q].x *= w[q];
+                x[q].y *= w[q];
+                z = cmul(cmul(x[q], cmul(pc[i], conjc(pc[j]))), pc[nants + e[q].y]);
+              } else {
+                const C m = model(sol, nants, e[q]);
+                const R t = w[q] * ra[i] * ra[j] * ra[nants + e[q].y];
+                z = cmul(x[q], conjc(m));
+                z.x *= t;
+                z.y *= t;
+              }
               d[c0 + q * nt] = z;
             }
         }
@@ -368,8 +404,14 @@ __global__ void __launch_bounds__(kOmMaxThreads, OM_MINB) omnical_kernel(const O
                 nsol[s] = f;  // partial sum
                 return;
               }
-              f.x = one_m + gs * v.x / gw[s];
-              f.y = gs * v.y / gw[s];
+              if constexpr (kFactored) {
+                const R q = gs / gw[s];
+                f.x = one_m + q * v.x;
+                f.y = q * v.y;
+              } else {
+                f.x = one_m + gs * v.x / gw[s];
+                f.y = gs * v.y / gw[s];
+              }
               nsol[s] = cmul(sol[s], f);
             });
         __syncthreads();
@@ -406,9 +448,409 @@ __global__ void __launch_bounds__(kOmMaxThreads, OM_MINB) omnical_kernel(const O
   }
 }
 
+// ------------------------------------------------------- dense kernel ----
+// Arrays whose baselines are antenna pairs, each pair at most once (the usual
+// case), seen as the lower triangle of the antenna matrix: a group of GL lanes
+// takes a row r, lane l its columns l, l + GL, ... below r, the same ones in
+// every row.  The column antennas' factors and sums so stay in registers, the
+// row antenna's factor is one broadcast, its sum a register until the row's
+// butterfly, and a baseline costs one gather (its unique baseline's factor)
+// and one read-modify-write (its sum) in shared memory.  The general kernel
+// below gathers six solution values, stores d and reads it back three times
+// through incidence lists, a panel of baselines at a time.
+//
+// Sums of unique baselines: every group has two private copies (one for pairs
+// stored as (row, column), one for (column, row)), added up in a fixed order
+// after the pass; the plan makes sure that no unique baseline occurs twice
+// among the lanes that write a copy at the same time.  So the result does not
+// depend on scheduling.
+//
+// With p_a = conj(g_a) |g0_a|^2 / |g_a|^2 and c_k likewise for u_k,
+//   d_b = data_b w_b p_i conj(p_j) c_k
+// (see the general kernel); for a pair stored as (column, row) the conjugate
+// is formed, from the conjugates of data and c_k.
+//
+// float32 only: float64 is bound by the FP64 pipe, where adding up the private
+// copies costs more than the gathers (54 antennas, 1000 problems, 12
+// iterations: 2.1 ms, general kernel 1.7 ms).
+//
+// Bound by issue slots (67% busy at 180 antennas) and the shared-memory pipe
+// (81%: gathers and updates at the unique baselines' scattered places).
+// Measured on GB300, 12 iterations of 2000 problems, general kernel and this
+// one: 180 antennas 3.70 and 2.48 ms, 128 antennas 2.84 and 1.64 ms, 54
+// antennas 0.44 and 0.36 ms; 12 antennas (4000 problems) 94 and 103 us, so it
+// starts at kDenseMinAnts.
+constexpr int kDenseMinAnts = 17, kDenseMaxAnts = 256;
+constexpr int kDenseThreads = 256;
+constexpr uint32_t kNoPair = 0x7fffu;  // slot without a baseline (256 antennas: < 32640 pairs)
+
+struct DenseParams {
+  int ndata, nants, nubls, nbls;
+  const int* row_off;    // [nants] first slot of each row
+  const uint32_t* slots; // baseline | (column, row) order << 15 | unique baseline << 16
+  const float2* data;
+  const float* wgts;
+  float2* gains;
+  float2* ubls;
+  float* chisq;
+  float* conv;
+  uint32_t* iters;
+  float conv_crit;
+  float gstep;
+  int maxiter, check_every, check_after;
+  int* counter;
+};
+
+size_t dense_smem(int nants, int nubls, int groups) {
+  const size_t nseg = (size_t)nants + nubls;
+  return sizeof(float2) * (3 * nseg + 2 * (size_t)groups * nubls + (size_t)groups * nants + nants) +
+         sizeof(float) * (2 * nseg + 96) + 16;
+}
+
+template <int GL, int NB>
+__global__ void __launch_bounds__(kDenseThreads, NB <= 6 ? 3 : 2)
+omnical_dense_kernel(const DenseParams p) {
+  using R = float;
+  using C = float2;
+  constexpr int GW = 32 / GL;  // groups a warp
+  extern __shared__ __align__(16) unsigned char smem[];
+  const int nants = p.nants, nubls = p.nubls, nbls = p.nbls, nseg = nants + nubls;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int nwarps = blockDim.x >> 5, ngroups = nwarps * GW;
+  const int grp = warp * GW + lane / GL, gl = lane & (GL - 1);
+  const int tid = threadIdx.x, nt = blockDim.x;
+  C* const solA = reinterpret_cast<C*>(smem);
+  C* const solB = solA + nseg;
+  C* const pc = solB + nseg;                  // p | c
+  C* const ucopy = pc + nseg;                 // [group][order][nubls]
+  C* const colsum = ucopy + 2 * ngroups * nubls;  // [group][nants]
+  C* const rowsum = colsum + ngroups * nants;     // [nants]
+  R* const gw = reinterpret_cast<R*>(rowsum + nants);  // gwgt | uwgt
+  R* const mg0 = gw + nseg;                   // |g0|^2 | |u0|^2
+  R* const red = mg0 + nseg;                  // 96 values
+  __shared__ int s_prob;
+  const R one_m = (R)(1.0f - p.gstep);  // formed in float, as the reference
+  const R gs = (R)p.gstep;
+
+  for (;;) {
+    __syncthreads();
+    if (tid == 0) s_prob = atomicAdd(p.counter, 1);
+    __syncthreads();
+    const int prob = s_prob;
+    if (prob >= p.ndata) return;
+    const C* const __restrict__ data = p.data + (size_t)prob * nbls;
+    const R* const __restrict__ wgt = p.wgts + (size_t)prob * nbls;
+    for (int s = tid; s < nseg; s += nt) {
+      const C x = s < nants ? p.gains[(size_t)prob * nants + s]
+                            : p.ubls[(size_t)prob * nubls + (s - nants)];
+      solA[s] = x;
+      pc[s] = conjc(x);
+      mg0[s] = mag2(x);
+    }
+    for (int i = tid; i < 2 * ngroups * nubls; i += nt) ucopy[i] = C{};
+    if (tid == 0) rowsum[0] = C{};
+    __syncthreads();
+    C *sol = solA, *nsol = solB;
+
+    // Every pair of this group, a row at a time: the data and weights of the
+    // whole row are loaded together (its slots were while the row before was
+    // worked on), then row_begin(row), pair(chunk, valid, swapped, unique
+    // baseline, data, weight) for each chunk (converged: the chunk loop is
+    // uniform across the warp) and row_end(row).  A chunk's column antenna is
+    // chunk * GL + gl (past nants where the pair is not valid: a read within
+    // the shared arrays, unused).
+    auto rows = [&](auto&& row_begin, auto&& pair, auto&& row_end) {
+      auto load_slots = [&](int rw, uint32_t (&e)[NB]) {
+        const uint32_t* slot = p.slots + __ldg(p.row_off + max(rw - lane / GL, 0)) + gl;
+#pragma unroll
+        for (int cb = 0; cb < NB; ++cb) e[cb] = cb * GL < rw ? __ldg(slot + cb * GL) : kNoPair;
+      };
+      uint32_t e[NB];
+      int rw = nants - 1 - warp * GW;
+      load_slots(rw, e);
+#pragma unroll 1
+      for (; rw >= 1; rw -= ngroups) {
+        C d[NB];
+        R w[NB];
+        uint32_t en[NB];
+#pragma unroll
+        for (int cb = 0; cb < NB; ++cb) {
+          const uint32_t b = e[cb] & kNoPair;
+          d[cb] = b != kNoPair ? __ldg(data + b) : C{};
+          w[cb] = b != kNoPair ? __ldg(wgt + b) : R(0);
+        }
+        load_slots(rw - ngroups, en);
+        const int r = max(rw - lane / GL, 0);
+        row_begin(r);
+#pragma unroll
+        for (int cb = 0; cb < NB; ++cb)
+          if (cb * GL < rw)
+            pair(cb, (e[cb] & kNoPair) != kNoPair, (int)((e[cb] >> 15) & 1u), (int)(e[cb] >> 16),
+                 d[cb], w[cb]);
+        row_end(r);
+#pragma unroll
+        for (int cb = 0; cb < NB; ++cb) e[cb] = en[cb];
+      }
+    };
+    auto group_sum = [&](R v) {
+#pragma unroll
+      for (int o = GL / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+      return v;
+    };
+    C* const my_u = ucopy + 2 * grp * nubls;
+    // sum |data - model|^2 w of a solution over this thread's pairs
+    auto chisq_part = [&](const C* x) {
+      R acc = 0;
+      C gr{};
+      rows([&](int r) { gr = x[r]; },
+           [&](int cb, bool ok, int sw, int k, C d, R w) {
+             if (!ok) return;
+             C u = x[nants + k];
+             if (sw) {
+               u = conjc(u);
+               d = conjc(d);
+             }
+             const C m = cmul(cmul(gr, conjc(x[cb * GL + gl])), u);
+             const R dx = d.x - m.x, dy = d.y - m.y;
+             acc += (dx * dx + dy * dy) * w;
+           },
+           [&](int) {});
+      return acc;
+    };
+
+    // chi^2 of the starting solution (redcal.py:566-577)
+    R chisq = chisq_part(sol), z1 = 0, z2 = 0;
+    block_sum3(chisq, z1, z2, red);
+    R conv = 0;
+    uint32_t iters = 0;
+
+    for (int it = 1; it <= p.maxiter; ++it) {
+      if (it % p.check_every == 1) {
+        // weights from the current model (calc_dwgts, calc_gu_wgt): |m|^2 w
+        R col[NB];
+#pragma unroll
+        for (int cb = 0; cb < NB; ++cb) col[cb] = 0;
+        C gr{};
+        R row = 0;
+        rows([&](int r) {
+               row = 0;
+               gr = sol[r];
+             },
+             [&](int cb, bool ok, int sw, int k, C, R w) {
+               R dw = 0;
+               if (ok) {
+                 const C u = sol[nants + k];
+                 dw = mag2(cmul(cmul(gr, conjc(sol[cb * GL + gl])), sw ? conjc(u) : u)) * w;
+                 my_u[sw * nubls + k].x += dw;
+               }
+               row += dw;
+               col[cb] += dw;
+               __syncwarp();
+             },
+             [&](int r) {
+               const R v = group_sum(row);
+               if (gl == 0) rowsum[r].x = v;
+             });
+#pragma unroll
+        for (int cb = 0; cb < NB; ++cb)
+          if (cb * GL + gl < nants) colsum[grp * nants + cb * GL + gl].x = col[cb];
+        __syncthreads();
+        for (int s = tid; s < nseg; s += nt) {
+          R v = 0;
+          if (s < nants) {
+            v = s ? rowsum[s].x : R(0);
+            for (int g = 0; g < ngroups; ++g) v += colsum[g * nants + s].x;
+          } else {
+            for (int c = 0; c < 2 * ngroups; ++c) {
+              C& u = ucopy[c * nubls + (s - nants)];
+              v += u.x;
+              u.x = 0;
+            }
+          }
+          gw[s] = v;
+        }
+        __syncthreads();
+      }
+      // d_b of every pair (calc_gu_buf), summed per antenna and unique
+      // baseline, then the step (update_gains/_ubls)
+      {
+        C col[NB];
+#pragma unroll
+        for (int cb = 0; cb < NB; ++cb) col[cb] = C{};
+        C gr{}, row{};
+        rows([&](int r) {
+               row = C{};
+               gr = pc[r];
+             },
+             [&](int cb, bool ok, int sw, int k, C d, R w) {
+               if (ok) {
+                 C c = pc[nants + k];
+                 if (sw) {
+                   c = conjc(c);
+                   d = conjc(d);
+                 }
+                 d.x *= w;
+                 d.y *= w;
+                 const C z = cmul(cmul(d, cmul(gr, conjc(pc[cb * GL + gl]))), c);
+                 row.x += z.x;
+                 row.y += z.y;
+                 col[cb].x += z.x;
+                 col[cb].y -= z.y;
+                 C& u = my_u[sw * nubls + k];
+                 C t = u;
+                 t.x += z.x;
+                 t.y += sw ? -z.y : z.y;
+                 u = t;
+               }
+               __syncwarp();
+             },
+             [&](int r) {
+               const R x = group_sum(row.x), y = group_sum(row.y);
+               if (gl == 0) {
+                 C t;
+                 t.x = x;
+                 t.y = y;
+                 rowsum[r] = t;
+               }
+             });
+#pragma unroll
+        for (int cb = 0; cb < NB; ++cb)
+          if (cb * GL + gl < nants) colsum[grp * nants + cb * GL + gl] = col[cb];
+      }
+      __syncthreads();
+      const bool rebase = (it + 1) % p.check_every == 1;
+      for (int s = tid; s < nseg; s += nt) {
+        C v{};
+        if (s < nants) {
+          if (s) v = rowsum[s];
+          for (int g = 0; g < ngroups; ++g) {
+            const C t = colsum[g * nants + s];
+            v.x += t.x;
+            v.y += t.y;
+          }
+        } else {
+          for (int c = 0; c < 2 * ngroups; ++c) {
+            C& u = ucopy[c * nubls + (s - nants)];
+            v.x += u.x;
+            v.y += u.y;
+            u = C{};
+          }
+        }
+        C f;
+        f.x = one_m + gs * v.x / gw[s];
+        f.y = gs * v.y / gw[s];
+        const C x = cmul(sol[s], f);
+        nsol[s] = x;
+        // the next iteration's factor: its weights are formed anew from x, or
+        // those at hand go on
+        C c = conjc(x);
+        if (rebase) {
+          mg0[s] = mag2(x);
+        } else {
+          const R q = mg0[s] / mag2(x);
+          c.x *= q;
+          c.y *= q;
+        }
+        pc[s] = c;
+      }
+      __syncthreads();
+      const bool check = !(it < p.maxiter && (it < p.check_after || it % p.check_every != 0));
+      if (check) {
+        // convergence and chi^2 of the stepped solution (calc_conv,
+        // calc_chisq, update_active)
+        R nchisq = chisq_part(nsol), csum = 0, cwgt = 0;
+        for (int s = tid; s < nseg; s += nt) {
+          const C x = nsol[s], y = sol[s];
+          const R dx = x.x - y.x, dy = x.y - y.y;
+          csum += dx * dx + dy * dy;
+          cwgt += mag2(x);
+        }
+        block_sum3(nchisq, csum, cwgt, red);
+        conv = sqrt(csum / cwgt);
+        if (conv < p.conv_crit || nchisq > chisq) break;
+        chisq = nchisq;
+        iters = (uint32_t)it;
+      }
+      C* t = sol; sol = nsol; nsol = t;
+    }
+    __syncthreads();
+    for (int s = tid; s < nseg; s += nt) {
+      if (s < nants) p.gains[(size_t)prob * nants + s] = sol[s];
+      else p.ubls[(size_t)prob * nubls + (s - nants)] = sol[s];
+    }
+    if (tid == 0) {
+      p.chisq[prob] = chisq;
+      p.conv[prob] = conv;
+      p.iters[prob] = iters;
+    }
+  }
+}
+
+// Launch shape of the dense kernel: lanes a row, chunks of columns a lane, and
+// the table of pairs by row.
+struct DensePlan {
+  int gl = 0, nb = 0, threads = 0;
+  std::vector<int> row_off;
+  std::vector<uint32_t> slots;
+};
+
+// Rows of up to 128 antennas take half a warp: fewer idle lanes at the row's
+// end (54 antennas: 77% busy, 61% with whole warps).
+bool make_dense_plan(const uint32_t* ggu, int nbls, int nants, int nubls, DensePlan* pl) {
+  if (nants < kDenseMinAnts || nants > kDenseMaxAnts || nbls < 1 || nubls < 1 || nubls > 65535 ||
+      nbls > nants * (nants - 1) / 2)
+    return false;
+  pl->gl = nants <= 128 ? 16 : 32;
+  const int need = (nants + pl->gl - 1) / pl->gl;
+  pl->nb = pl->gl == 32 ? (need <= 6 ? 6 : 8) : need <= 2 ? 2 : need <= 4 ? 4 : 8;
+  // a few rows a group: small arrays take few warps, so that more problems
+  // share an SM
+  const int gw = 32 / pl->gl;
+  const int warps = std::max(1, std::min(kDenseThreads / 32, (nants + 3 * gw - 1) / (3 * gw)));
+  pl->threads = 32 * warps;
+  if (dense_smem(nants, nubls, warps * gw) > (size_t)kOmSmemLimit) return false;
+  // rows padded to whole chunks of the longest row of their warp's groups
+  pl->row_off.resize(nants);
+  int n = 0;
+  for (int r = 0; r < nants; ++r) {
+    pl->row_off[r] = n;
+    n += (r + gw - 1 + pl->gl - 1) / pl->gl * pl->gl + (r + gw - 1 == 0 ? pl->gl : 0);
+  }
+  pl->slots.assign(n, kNoPair);
+  for (int b = 0; b < nbls; ++b) {
+    const uint32_t i = ggu[3 * b], j = ggu[3 * b + 1], k = ggu[3 * b + 2];
+    if (i == j) return false;
+    const uint32_t r = std::max(i, j), c = std::min(i, j);
+    uint32_t& s = pl->slots[pl->row_off[r] + c];
+    if (s != kNoPair) return false;  // the pair again
+    s = (uint32_t)b | (i == r ? 0u : 0x8000u) | (k << 16);
+  }
+  // no unique baseline twice among the lanes that add to one copy at a time
+  std::vector<int> seen(2 * (size_t)nubls, -1);
+  int stamp = 0;
+  for (int r = 1; r < nants; ++r)
+    for (int c0 = 0; c0 < r; c0 += pl->gl, ++stamp)
+      for (int c = c0; c < std::min(r, c0 + pl->gl); ++c) {
+        const uint32_t s = pl->slots[pl->row_off[r] + c];
+        if ((s & kNoPair) == kNoPair) continue;
+        int& q = seen[(size_t)((s >> 15) & 1u) * nubls + (s >> 16)];
+        if (q == stamp) return false;
+        q = stamp;
+      }
+  return true;
+}
+
+using DenseFn = void (*)(DenseParams);
+DenseFn dense_kernel(int gl, int nb) {
+  if (gl == 32) return nb == 6 ? omnical_dense_kernel<32, 6> : omnical_dense_kernel<32, 8>;
+  return nb == 2   ? omnical_dense_kernel<16, 2>
+         : nb == 4 ? omnical_dense_kernel<16, 4>
+                   : omnical_dense_kernel<16, 8>;
+}
+
 struct Plan {
   int threads = 64, group = 1, blocks_per_sm = 1, panel = 0, npanels = 1;
-  bool data_shared = false;
+  bool data_shared = false, factored = false;
   size_t smem = 0;
 };
 
@@ -416,13 +858,15 @@ struct Plan {
 // in shared memory when that leaves 16 warps an SM, else panels of
 // baselines sized for two CTAs (or the thread limit) an SM.
 template <typename R>
-int make_plan(int nants, int nubls, int nbls, Plan* out) {
+int make_plan(int nants, int nubls, int nbls, bool factored, Plan* out) {
   using C = typename Cx<R>::T;
   Plan pl;
   const int t = ((nbls / 2 + 31) / 32) * 32;
   pl.threads = std::max(64, std::min(kOmMaxThreads, t));
   const size_t nseg = (size_t)nants + nubls;
-  const size_t fixed = (2 * sizeof(C) + 3 * sizeof(R)) * nseg + 96 * sizeof(R) + 16;
+  pl.factored = factored;
+  const size_t fixed =
+      (2 * sizeof(C) + (factored ? 4 : 3) * sizeof(R)) * nseg + 96 * sizeof(R) + 16;
   auto per_sm = [&](size_t s) {
     return std::min(32, std::min(kOmThreadsPerSm / pl.threads, (int)((228 * 1024) / (s + 1024))));
   };
@@ -523,6 +967,66 @@ int check_sizes(hv_context* ctx, int precision, int nbls, int nants, int nubls, 
   return HV_OK;
 }
 
+int run_dense(hv_context* ctx, const DensePlan& dp, int nbls, void* d_gains, int nants,
+              void* d_ubls, int nubls, const void* d_data, const void* d_wgts, int ndata,
+              double conv_crit, int maxiter, int check_every, int check_after, double gain,
+              void* d_chisq, uint32_t* d_iters, void* d_conv, cudaStream_t st) {
+  const DenseFn fn = dense_kernel(dp.gl, dp.nb);
+  const size_t smem = dense_smem(nants, nubls, dp.threads / dp.gl);
+  int per_sm = 0;
+  if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, kOmSmemLimit) !=
+          cudaSuccess ||
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, dp.threads, smem) != cudaSuccess)
+    return HV_ERR_CUDA;
+  const int grid = std::min(ndata, std::max(1, per_sm) * std::max(1, hv_context_num_sms(ctx)));
+  const size_t n_off = sizeof(int) * dp.row_off.size(), n_slot = sizeof(uint32_t) * dp.slots.size();
+  const size_t o_slot = (n_off + 255) & ~size_t(255), o_cnt = (o_slot + n_slot + 255) & ~size_t(255);
+  void* buf = nullptr;
+  if (cudaMallocAsync(&buf, o_cnt + 256, st) != cudaSuccess) {
+    cudaGetLastError();
+    return fail(ctx, HV_ERR_OOM, "omnical: device allocation failed");
+  }
+  char* b8 = static_cast<char*>(buf);
+  int r = HV_OK;
+  if (cudaMemcpyAsync(b8, dp.row_off.data(), n_off, cudaMemcpyHostToDevice, st) != cudaSuccess ||
+      cudaMemcpyAsync(b8 + o_slot, dp.slots.data(), n_slot, cudaMemcpyHostToDevice, st) !=
+          cudaSuccess ||
+      cudaMemsetAsync(b8 + o_cnt, 0, sizeof(int), st) != cudaSuccess)
+    r = HV_ERR_CUDA;
+  if (r == HV_OK) {
+    DenseParams p;
+    p.ndata = ndata;
+    p.nants = nants;
+    p.nubls = nubls;
+    p.nbls = nbls;
+    p.row_off = reinterpret_cast<const int*>(b8);
+    p.slots = reinterpret_cast<const uint32_t*>(b8 + o_slot);
+    p.data = static_cast<const float2*>(d_data);
+    p.wgts = static_cast<const float*>(d_wgts);
+    p.gains = static_cast<float2*>(d_gains);
+    p.ubls = static_cast<float2*>(d_ubls);
+    p.chisq = static_cast<float*>(d_chisq);
+    p.conv = static_cast<float*>(d_conv);
+    p.iters = d_iters;
+    p.conv_crit = (float)conv_crit;
+    p.gstep = (float)gain;
+    p.maxiter = maxiter;
+    p.check_every = check_every;
+    p.check_after = check_after;
+    p.counter = reinterpret_cast<int*>(b8 + o_cnt);
+    fn<<<grid, dp.threads, smem, st>>>(p);
+    const cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) {
+      hv_context_set_error(ctx, cudaGetErrorString(e));
+      r = HV_ERR_CUDA;
+    } else {
+      hv_context_add_launches(ctx, 1);
+    }
+  }
+  cudaFreeAsync(buf, st);
+  return r;
+}
+
 template <typename R>
 int run_typed(hv_context* ctx, const uint32_t* ggu, int nbls, void* d_gains, int nants,
               void* d_ubls, int nubls, const void* d_data, const void* d_wgts, int ndata,
@@ -531,8 +1035,16 @@ int run_typed(hv_context* ctx, const uint32_t* ggu, int nbls, void* d_gains, int
   int r = check_indices(ctx, ggu, nbls, nants, nubls);
   if (r != HV_OK) return r;
   if (ndata == 0) return HV_OK;
+  if (sizeof(R) == 4) {
+    DensePlan dp;
+    if (make_dense_plan(ggu, nbls, nants, nubls, &dp))
+      return run_dense(ctx, dp, nbls, d_gains, nants, d_ubls, nubls, d_data, d_wgts, ndata,
+                       conv_crit, maxiter, check_every, check_after, gain, d_chisq, d_iters,
+                       d_conv, st);
+  }
   Plan pl;
-  if (make_plan<R>(nants, nubls, nbls, &pl) != HV_OK)
+  if ((sizeof(R) == 4 || make_plan<R>(nants, nubls, nbls, true, &pl) != HV_OK) &&
+      make_plan<R>(nants, nubls, nbls, false, &pl) != HV_OK)
     return fail(ctx, HV_ERR_ARG, "omnical: too many antennas and unique baselines for one CTA");
   std::vector<uint2> bl;
   std::vector<int> off;
@@ -562,8 +1074,11 @@ int run_typed(hv_context* ctx, const uint32_t* ggu, int nbls, void* d_gains, int
   if (r == HV_OK) {
     static bool configured[2] = {false, false};
     if (!configured[sizeof(R) == 8]) {
-      for (const void* k : {reinterpret_cast<const void*>(omnical_kernel<R, false>),
-                            reinterpret_cast<const void*>(omnical_kernel<R, true>)})
+      constexpr bool kF = sizeof(R) == 8;
+      for (const void* k : {reinterpret_cast<const void*>(omnical_kernel<R, false, false>),
+                            reinterpret_cast<const void*>(omnical_kernel<R, true, false>),
+                            reinterpret_cast<const void*>(omnical_kernel<R, false, kF>),
+                            reinterpret_cast<const void*>(omnical_kernel<R, true, kF>)})
         if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kOmSmemLimit) !=
             cudaSuccess)
           r = HV_ERR_CUDA;
@@ -596,10 +1111,13 @@ int run_typed(hv_context* ctx, const uint32_t* ggu, int nbls, void* d_gains, int
     p.check_after = check_after;
     p.group = pl.group;
     p.counter = reinterpret_cast<int*>(b8 + o_cnt);
-    if (pl.data_shared)
-      omnical_kernel<R, true><<<grid, pl.threads, pl.smem, st>>>(p);
+    constexpr bool kF = sizeof(R) == 8;
+    if (pl.factored)
+      (pl.data_shared ? omnical_kernel<R, true, kF>
+                      : omnical_kernel<R, false, kF>)<<<grid, pl.threads, pl.smem, st>>>(p);
     else
-      omnical_kernel<R, false><<<grid, pl.threads, pl.smem, st>>>(p);
+      (pl.data_shared ? omnical_kernel<R, true, false>
+                      : omnical_kernel<R, false, false>)<<<grid, pl.threads, pl.smem, st>>>(p);
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) {
       hv_context_set_error(ctx, cudaGetErrorString(e));

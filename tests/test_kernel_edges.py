@@ -162,3 +162,51 @@ def test_median_strips(ks):
     img[:] = np.nan
     inner = MedianFilter(input=img, kernel_size=ks)[0][8:-8, 8:-8]
     assert np.isnan(inner).all()
+
+
+# omnical in float32: the antenna-matrix kernel (17 to 256 antennas, distinct
+# pairs) at the edges of its rows and column chunks, with pairs in both orders,
+# baselines in any order and some missing; and layouts it must leave to the
+# general kernel (16 and 257 antennas, a pair twice, one unique baseline for
+# all).  A dozen iterations: float32 rounding (6e-8 a step and term) stays far
+# below 1e-5 of the largest gain, and no problem is near a stop.
+@gpu
+@pytest.mark.parametrize("nants", [16, 17, 31, 32, 33, 64, 65, 128, 129, 192, 193, 256, 257])
+@pytest.mark.parametrize("kind", ["plain", "shuffled", "twice", "one"])
+def test_omnical_layouts(nants, kind):
+    from hera_gpu_gb300 import omnical
+    from oracle import omnical_oracle
+    if kind != "plain" and nants not in (17, 64, 129, 193):
+        pytest.skip("the other layouts at one size of each launch shape")
+    ggu, nubls = synth.hex_redundant_layout(nants)
+    rng = np.random.default_rng(nants)
+    if kind == "one":       # the same unique baseline many times in a row
+        ggu = ggu.copy()
+        ggu[:, 2] = 0
+        nubls = 1
+    g0, u0, d, w = synth.redundant_data(ggu, nubls, 3, seed=nants, noise=0.05)
+    if kind == "shuffled":
+        keep = rng.permutation(len(ggu))[: len(ggu) * 9 // 10]
+        keep = np.unique(np.concatenate([keep, [np.flatnonzero(ggu[:, 2] == k)[0] for k in range(nubls)]]))
+        keep = rng.permutation(keep)
+        ggu, d, w = ggu[keep], d[:, keep], w[:, keep]
+        swap = rng.random(len(ggu)) < 0.5
+        ggu = ggu.copy()
+        ggu[swap] = ggu[swap][:, [1, 0, 2]]
+        d[:, swap] = np.conj(d[:, swap])     # the model of (j, i) with the same unique baseline:
+        # conj(g_i) g_j u differs from conj(g_i conj(g_j) u) by u's phase, so give the pair its own
+        # consistent data
+        d[:, swap] = d[:, swap] * np.exp(2j * np.angle(u0[:, ggu[swap, 2]]))
+    if kind == "twice":
+        ggu = np.concatenate([ggu, ggu[:1]])
+        d, w = np.concatenate([d, d[:, :1]], 1), np.concatenate([w, w[:, :1]], 1)
+    a = [x.astype(t) for x, t in ((g0, np.complex64), (u0, np.complex64), (d, np.complex64),
+                                  (w, np.float32))]
+    got = omnical(ggu, *a, 1e-10, 12, precision=1)
+    ref = omnical_oracle(ggu, *a, 1e-10, 12, precision=1)
+    assert np.abs(got["gains"] - ref["gains"]).max() <= 1e-5 * np.abs(ref["gains"]).max()
+    assert np.abs(got["ubls"] - ref["ubls"]).max() <= 1e-5 * np.abs(ref["ubls"]).max()
+    np.testing.assert_allclose(got["chisq"], ref["chisq"], rtol=1e-3)
+    np.testing.assert_array_equal(got["iters"], ref["iters"])
+    again = omnical(ggu, *[x[1:] for x in a], 1e-10, 12, precision=1)
+    np.testing.assert_array_equal(again["gains"], got["gains"][1:])
