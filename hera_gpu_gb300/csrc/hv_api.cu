@@ -457,7 +457,7 @@ int run_device(hv_context* ctx, int method, const R* antpos, int nant, const dou
         if (nsrc > 0 && ctx->share.launched > 1) ctx->launches += ctx->share.launched - 1;
         HV_LAUNCH(1, launch_reduce<float>(static_cast<float*>(ctx->partial.p), slice_floats,
                                           counts + t0, nt, nfreq, t0, ntimes, chunk,
-                                          ceil_div(S1, chunk), Np, nant, out, st));
+                                          ceil_div(S1, chunk), Np, nant, true, out, st));
       }
     }
     return HV_OK;
@@ -487,7 +487,7 @@ int run_device(hv_context* ctx, int method, const R* antpos, int nant, const dou
                                            static_cast<R*>(ctx->partial.p), st),
                       st);
       HV_LAUNCH(1, launch_reduce<R>(static_cast<R*>(ctx->partial.p), 0, counts + t, 1, 1, 0, 1,
-                                    kPlainChunk, chunks, Np, nant, o, st));
+                                    kPlainChunk, chunks, Np, nant, false, o, st));
     }
   }
   return HV_OK;

@@ -157,11 +157,13 @@ cudaError_t launch_herk_flagged(const F64Dims& d, int nz, const void* v, const i
 // chunks (ceil(count / chunk) of them) in order and write the full Hermitian
 // matrix (nant x nant complex R, row-major) to
 // out + ((f * ntimes_out) + t0 + tl) * nant * nant.  max_chunks: the most
-// chunks a slice can have (it picks the split of the work only).
+// chunks a slice can have (it picks the split of the work only).  antisym:
+// the partial sums of the fused kernel, whose diagonal 128 x 128 blocks hold M
+// in the imaginary plane, Im V = M - M^T.
 template <typename R>
 cudaError_t launch_reduce(const R* partial, size_t slice_stride, const int* counts, int nt,
                           int nf, int t0, int ntimes_out, int chunk, int max_chunks, int Np,
-                          int nant, void* out, cudaStream_t st);
+                          int nant, bool antisym, void* out, cudaStream_t st);
 
 // --- hv_f64.cu -------------------------------------------------------------
 // FP64 product on the tensor cores.  Slices z = tl * nf + fl (nf of the

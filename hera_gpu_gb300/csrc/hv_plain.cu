@@ -239,14 +239,18 @@ constexpr int kReduceAhead = 8;
 // Chunks from which a tile is split over four blocks (at 512 antennas x 10
 // slices x 2 chunks splitting it costs 10 us; from 34 chunks on it pays).
 constexpr int kReduceSplitChunks = 8;
-template <typename R, int kCols>
+//
+// kAntisym (the fused kernel's partial sums): in the 128 x 128 blocks on the
+// diagonal the imaginary plane holds M with Im V = M - M^T, so their blocks sum
+// M's transposed part as well (read along its rows, handed over through TM).
+template <typename R, int kCols, bool kAntisym>
 __device__ __forceinline__ void reduce_part(const R* __restrict__ partial_base,
                                             size_t slice_stride, const int* __restrict__ counts,
                                             int nf, int t0, int ntimes_out, int chunk, int Np,
                                             int nant,
                                             typename Traits<R>::C* __restrict__ out_base,
                                             int tile, int part, int sl,
-                                            typename Traits<R>::C (*T)[33]) {
+                                            typename Traits<R>::C (*T)[33], R (*TM)[33]) {
   using C = typename Traits<R>::C;
   const int nbt = ceil_div(nant, 32);
   int A, B;
@@ -261,6 +265,26 @@ __device__ __forceinline__ void reduce_part(const R* __restrict__ partial_base,
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
   const size_t plane = (size_t)Np * Np;
   const int a = A * 32 + tx;
+  const bool antisym = kAntisym && A / (kAntPad / 32) == B / (kAntPad / 32);
+  if (antisym) {
+#pragma unroll 1
+    for (int i = threadIdx.x; i < 32 * kCols; i += 256) {
+      const int aa = i / kCols, bb = i % kCols;
+      const R* p = partial + plane + (size_t)(A * 32 + aa) * Np + b0 + bb;
+      typename Acc<R>::type m;
+      int k = 0;
+      for (; k + kReduceAhead <= nk; k += kReduceAhead) {
+        R x[kReduceAhead];
+#pragma unroll
+        for (int q = 0; q < kReduceAhead; ++q) x[q] = p[(size_t)(k + q) * 2 * plane];
+#pragma unroll
+        for (int q = 0; q < kReduceAhead; ++q) m.add(x[q]);
+      }
+      for (; k < nk; ++k) m.add(p[(size_t)k * 2 * plane]);
+      TM[bb][aa] = m.s;
+    }
+    __syncthreads();
+  }
 #pragma unroll 1
   for (int bb = ty; bb < kCols; bb += 8) {
     const int b = b0 + bb;
@@ -288,7 +312,7 @@ __device__ __forceinline__ void reduce_part(const R* __restrict__ partial_base,
     }
     C val;
     val.x = re.s;
-    val.y = a == b ? R(0) : im.s;
+    val.y = a == b ? R(0) : antisym ? im.s - TM[bb][tx] : im.s;
     T[bb][tx] = val;
     if (a <= b && b < nant) {
       // below the diagonal: out[b][a] = conj(V[a][b]), a contiguous
@@ -306,15 +330,17 @@ __device__ __forceinline__ void reduce_part(const R* __restrict__ partial_base,
   }
 }
 
-template <typename R, int kCols>
+template <typename R, int kCols, bool kAntisym>
 __global__ void __launch_bounds__(256)
 reduce_kernel(const R* __restrict__ partial_base, size_t slice_stride,
               const int* __restrict__ counts, int nf, int t0, int ntimes_out, int chunk, int Np,
               int nant, typename Traits<R>::C* __restrict__ out_base) {
   __shared__ typename Traits<R>::C T[kCols][33];
+  __shared__ R TM[kAntisym ? kCols : 1][33];
   constexpr int kParts = 32 / kCols;
-  reduce_part<R, kCols>(partial_base, slice_stride, counts, nf, t0, ntimes_out, chunk, Np, nant,
-                        out_base, blockIdx.x / kParts, blockIdx.x % kParts, blockIdx.y, T);
+  reduce_part<R, kCols, kAntisym>(partial_base, slice_stride, counts, nf, t0, ntimes_out, chunk,
+                                  Np, nant, out_base, blockIdx.x / kParts, blockIdx.x % kParts,
+                                  blockIdx.y, T, TM);
 }
 
 // Every simulation of a batch: its split-K chunks reduced into its output.
@@ -322,14 +348,16 @@ __global__ void __launch_bounds__(256)
 reduce_batch_kernel(const PrepSim* __restrict__ sims, int nsims,
                     const long long* __restrict__ pre) {
   __shared__ float2 T[32][33];
+  __shared__ float TM[32][33];
   const int si = find_segment(pre, nsims, blockIdx.x);
   const PrepSim& sm = sims[si];
   const int nbt = ceil_div(sm.nant, 32);
   const int tiles = nbt * (nbt + 1) / 2;
   const int local = (int)(blockIdx.x - __ldg(pre + si));
   const size_t slice = (size_t)ceil_div(sm.S > 0 ? sm.S : 1, sm.chunk) * 2 * sm.Np * sm.Np;
-  reduce_part<float, 32>(sm.partial, slice, sm.counts, sm.F, 0, sm.T, sm.chunk, sm.Np, sm.nant,
-                         static_cast<float2*>(sm.out), local % tiles, 0, local / tiles, T);
+  reduce_part<float, 32, true>(sm.partial, slice, sm.counts, sm.F, 0, sm.T, sm.chunk, sm.Np,
+                               sm.nant, static_cast<float2*>(sm.out), local % tiles, 0,
+                               local / tiles, T, TM);
 }
 
 cudaError_t launch_reduce_batch(const PrepSim* sims, int nsims, const PrepPre& pre,
@@ -342,18 +370,15 @@ cudaError_t launch_reduce_batch(const PrepSim* sims, int nsims, const PrepPre& p
 template <typename R>
 cudaError_t launch_reduce(const R* partial, size_t slice_stride, const int* counts, int nt,
                           int nf, int t0, int ntimes_out, int chunk, int max_chunks, int Np,
-                          int nant, void* out, cudaStream_t st) {
+                          int nant, bool antisym, void* out, cudaStream_t st) {
   using C = typename Traits<R>::C;
   const int nbt = ceil_div(nant, 32);
-  const int tiles = nbt * (nbt + 1) / 2;
-  if (max_chunks >= kReduceSplitChunks)
-    reduce_kernel<R, 8><<<dim3(tiles * 4, nt * nf), 256, 0, st>>>(
-        partial, slice_stride, counts, nf, t0, ntimes_out, chunk, Np, nant,
-        reinterpret_cast<C*>(out));
-  else
-    reduce_kernel<R, 32><<<dim3(tiles, nt * nf), 256, 0, st>>>(
-        partial, slice_stride, counts, nf, t0, ntimes_out, chunk, Np, nant,
-        reinterpret_cast<C*>(out));
+  const bool split = max_chunks >= kReduceSplitChunks;
+  const dim3 grid(nbt * (nbt + 1) / 2 * (split ? 4 : 1), nt * nf);
+  auto* kernel = split ? (antisym ? reduce_kernel<R, 8, true> : reduce_kernel<R, 8, false>)
+                       : (antisym ? reduce_kernel<R, 32, true> : reduce_kernel<R, 32, false>);
+  kernel<<<grid, 256, 0, st>>>(partial, slice_stride, counts, nf, t0, ntimes_out, chunk, Np, nant,
+                               reinterpret_cast<C*>(out));
   return cudaGetLastError();
 }
 
@@ -361,7 +386,7 @@ template cudaError_t launch_gen_phasors<float>(const void*, const int*, int, con
 template cudaError_t launch_gen_phasors<double>(const void*, const int*, int, const void*, const double*, int, int, int, void*, cudaStream_t);
 template cudaError_t launch_herk_plain<float>(const void*, const int*, int, int, float*, cudaStream_t);
 template cudaError_t launch_herk_plain<double>(const void*, const int*, int, int, double*, cudaStream_t);
-template cudaError_t launch_reduce<float>(const float*, size_t, const int*, int, int, int, int, int, int, int, int, void*, cudaStream_t);
-template cudaError_t launch_reduce<double>(const double*, size_t, const int*, int, int, int, int, int, int, int, int, void*, cudaStream_t);
+template cudaError_t launch_reduce<float>(const float*, size_t, const int*, int, int, int, int, int, int, int, int, bool, void*, cudaStream_t);
+template cudaError_t launch_reduce<double>(const double*, size_t, const int*, int, int, int, int, int, int, int, int, bool, void*, cudaStream_t);
 
 }  // namespace hv

@@ -54,6 +54,10 @@
 //     ReV += ReA ReB^T + ImA ImB^T,   ImV += ImA ReB^T - ReA ImB^T
 //   (V[a,b] = sum_s v_a conj(v_b)); the minus sign is the instruction
 //   descriptor's negate-A bit.  Split BF16 keeps hi*hi + hi*lo + lo*hi.
+//   A block with itself (a diagonal pair) takes M = ImA ReA^T alone: its ImV
+//   is M - M^T, which the reduction over the source chunks forms.  At 350
+//   antennas each of the three groups has a diagonal block, so this takes 1/8
+//   of the MMA work away: @NEG@.
 //
 // Second form (kForm = 1, HV_METHOD_TC_FP16): FP16 hi parts and FP8 (E4M3)
 // cross terms.  Per (time, frequency) slice the phasors are scaled by a power
@@ -166,6 +170,10 @@ struct TcGroup {
   int slot_rows[3];  // valid antenna rows of each slot's block
   int sa;            // slot of the row block (A operand); the column blocks (B) are slots 0, 1
   int n_mma;         // MMA N: 128 + the columns of slot 1 for two pairs, else those of slot 0
+  // columns [neg_col, neg_col + neg_n) of the off-diagonal pairs (neg_n = 0:
+  // none): the ones that take the -Re Im products (a diagonal pair's
+  // imaginary part is M - M^T with M = Im Re^T, formed by the reduction)
+  int neg_col, neg_n;
   int pI[2], pJ[2];  // row and column block of each pair; pI > pJ: computed below the diagonal
   int pN[2];         // valid columns of block pJ, rounded up to 16
   // Cluster mode (one CTA per group, cluster rank = group index): every
@@ -330,10 +338,13 @@ __device__ __forceinline__ void mma_bf16(uint32_t d_tmem, uint32_t a_lo, uint32_
 // with B the group's column blocks side by side (N up to 256).  a, b:
 // descriptor low words of the row block's tile and of the first column
 // block's tile; along K, Re hi, Im hi, Re lo, Im lo are 32 bytes (2
-// descriptor units) apart.  first: the stage opens the item.
+// descriptor units) apart.  first: the stage opens the item.  The last
+// product only runs on the columns of off-diagonal pairs (idn: their number
+// as N; noff: their first column and b_neg their block's tile; idn = 0: none).
 __device__ __forceinline__ void issue_group(uint32_t d_re, uint32_t a, uint32_t b, uint32_t idp,
-                                            uint32_t idn, bool first) {
-  const uint32_t d_im = d_re + 256;
+                                            uint32_t idn, uint32_t noff, uint32_t b_neg,
+                                            bool first) {
+  const uint32_t d_im = d_re + 256, d_neg = d_im + noff;
 #pragma unroll
   for (int pr = 0; pr < 3; ++pr) {
     const uint32_t aa = a + (pr == 2 ? 4u : 0u), bb = b + (pr == 1 ? 4u : 0u);  // lo: 64 B on
@@ -341,7 +352,7 @@ __device__ __forceinline__ void issue_group(uint32_t d_re, uint32_t a, uint32_t 
     mma_bf16(d_re, aa, bb, idp, acc);            // Re Re
     mma_bf16(d_re, aa + 2u, bb + 2u, idp, 1u);   // Im Im
     mma_bf16(d_im, aa + 2u, bb, idp, acc);       // Im Re
-    mma_bf16(d_im, aa, bb + 2u, idn, 1u);        // -Re Im
+    if (idn) mma_bf16(d_neg, aa, b_neg + (pr == 1 ? 4u : 0u) + 2u, idn, 1u);  // -Re Im
   }
 }
 
@@ -363,15 +374,18 @@ __device__ __forceinline__ void mma_e4m3(uint32_t d_tmem, uint32_t a_lo, uint32_
 // +0, +2, +4, +6).  The FP16 and E4M3 instruction descriptors coincide.
 __device__ __forceinline__ void issue_group_f16f8(uint32_t d_re, uint32_t a16, uint32_t b16,
                                                   uint32_t a8, uint32_t b8, uint32_t idp,
-                                                  uint32_t idn, bool first) {
-  const uint32_t d_im = d_re + 256;
+                                                  uint32_t idn, uint32_t noff, uint32_t b_neg,
+                                                  bool first) {
+  const uint32_t d_im = d_re + 256, d_neg = d_im + noff;
+  const uint32_t b8_neg = b8 + b_neg;
+  b_neg += b16;
 #pragma unroll
   for (uint32_t h = 0; h < 4; h += 2) {  // source halves s0-15, s16-31
     const uint32_t acc = (first && h == 0) ? 0u : 1u;
     mma_bf16(d_re, a16 + h, b16 + h, idp, acc);              // Re Re
     mma_bf16(d_re, a16 + 4u + h, b16 + 4u + h, idp, 1u);     // Im Im
     mma_bf16(d_im, a16 + 4u + h, b16 + h, idp, acc);         // Im Re
-    mma_bf16(d_im, a16 + h, b16 + 4u + h, idn, 1u);          // -Re Im
+    if (idn) mma_bf16(d_neg, a16 + h, b_neg + 4u + h, idn, 1u);  // -Re Im
   }
 #pragma unroll
   for (int pr = 0; pr < 2; ++pr) {  // X8 (a) x L8 (b), then L8 (a) x X8 (b)
@@ -379,7 +393,7 @@ __device__ __forceinline__ void issue_group_f16f8(uint32_t d_re, uint32_t a16, u
     mma_e4m3(d_re, a8 + xa, b8 + yb, idp, 1u);               // Re Re
     mma_e4m3(d_re, a8 + xa + 2u, b8 + yb + 2u, idp, 1u);     // Im Im
     mma_e4m3(d_im, a8 + xa + 2u, b8 + yb, idp, 1u);          // Im Re
-    mma_e4m3(d_im, a8 + xa, b8 + yb + 2u, idn, 1u);          // -Re Im
+    if (idn) mma_e4m3(d_neg, a8 + xa, b8_neg + yb + 2u, idn, 1u);  // -Re Im
   }
 }
 
@@ -1103,7 +1117,11 @@ tc_vis_kernel(const __grid_constant__ CUtensorMap rec_map, const __grid_constant
         const TcGroup* gp = SIM_P(d, groups) + d.g;
         const int nm = __ldg(&gp->n_mma);
         const uint32_t abt = kForm == 0 ? 1u : 0u;  // BF16, or FP16 / E4M3
-        const uint32_t idp = idesc_mma(nm, false, abt), idn = idesc_mma(nm, true, abt);
+        const int neg_n = __ldg(&gp->neg_n);
+        const uint32_t noff = (uint32_t)__ldg(&gp->neg_col);
+        const uint32_t b_neg = noff ? (uint32_t)(TC_SLOT >> 4) : 0u;  // slot 1's tile
+        const uint32_t idp = idesc_mma(nm, false, abt);
+        const uint32_t idn = neg_n ? idesc_mma(neg_n, true, abt) : 0u;
         const uint32_t a0 = desc_lo(op_base + (uint32_t)__ldg(&gp->sa) * TC_SLOT);
         const uint32_t b0 = desc_lo(op_base);
         for (int j0 = 0; j0 < d.nst && ok; j0 += FLUSH) {
@@ -1121,11 +1139,11 @@ tc_vis_kernel(const __grid_constant__ CUtensorMap rec_map, const __grid_constant
             tc_fence_after();
             const uint32_t so = ((uint32_t)s * stage_bytes) >> 4;
             if constexpr (kForm == 0) {
-              issue_group(tmem, a0 + so, b0 + so, idp, idn, j == j0);
+              issue_group(tmem, a0 + so, b0 + so, idp, idn, noff, b0 + so + b_neg, j == j0);
             } else {
               const uint32_t o8 = tile8_off >> 4;
               issue_group_f16f8(tmem, a0 + so, b0 + so, a0 + so + o8, b0 + so + o8, idp, idn,
-                                j == j0);
+                                noff, b_neg, j == j0);
             }
             // the stage's slots may be refilled -- here and, in cluster mode,
             // by the CTAs that wrote them -- once these MMAs have read them
@@ -1235,6 +1253,14 @@ std::vector<TcGroup> make_groups(int nant) {
     }
     g.sa = slot_of(prs[0].first);
     g.n_mma = g.npairs == 2 ? TC_ROWS + g.pN[1] : g.pN[0];
+    g.neg_col = 0;
+    g.neg_n = g.n_mma;
+    if (g.pI[0] == g.pJ[0]) {  // the first pair is diagonal
+      g.neg_col = TC_ROWS;
+      g.neg_n = g.npairs == 2 ? g.pN[1] : 0;
+    } else if (g.npairs == 2 && g.pI[1] == g.pJ[1]) {
+      g.neg_n = TC_ROWS;
+    }
     out.push_back(g);
   }
   return out;
