@@ -508,13 +508,23 @@ __device__ __forceinline__ void tc_relative_span(SrcRec32* __restrict__ rec, siz
     // over the 8 lanes of the unit: largest spread, and whether every
     // source sits on the reference's beam pixel (padding counts as same)
     for (int o = 4; o > 0; o >>= 1) d1 = fmaxf(d1, __shfl_xor_sync(0xffffffffu, d1, o));
-    const unsigned differ = __ballot_sync(0xffffffffu, i < n && pix != ref_pix);
-    const bool same_pix = ((differ >> (threadIdx.x & 24)) & 0xffu) == 0;
+    // ... and, from the ends (padding counts as the last pixel), how many
+    // records lie on the first and on the last record's pixel
+    const int last_pix = __shfl_sync(0xffffffffu, pix, (threadIdx.x & 24) | min(7, n - 1 - (i & ~7)) & 31);
+    const unsigned u = threadIdx.x & 24;
+    const unsigned differ = (__ballot_sync(0xffffffffu, i < n && pix != ref_pix) >> u) & 0xffu;
+    const unsigned not_last = (__ballot_sync(0xffffffffu, i < n && pix != last_pix) >> u) & 0xffu;
+    const bool same_pix = differ == 0;
+    // records on the first pixel before any other; all the rest on the last
+    const int first_run = differ ? __ffs(differ) - 1 : 8;
+    const bool two_pix = !same_pix && n - (i & ~7) >= 8 && (not_last >> first_run) == 0;
     __syncwarp();
     if (i < n) {
       // pad word of the unit's first record: the spread as a float, with the
-      // sign bit set when all eight sources share one beam pixel
+      // sign bit set when all eight sources share one beam pixel; of its
+      // second: where the second of two pixels starts (0: not two pixels)
       if ((i & 7) == 0) r[i].pad = __float_as_int(d1) | (same_pix ? (int)0x80000000u : 0);
+      if ((i & 7) == 1) r[i].pad = two_pix ? first_run : 0;
     } else if (i < npad) {
       r[i] = SrcRec32{};
     }

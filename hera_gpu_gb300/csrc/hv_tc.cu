@@ -57,7 +57,8 @@
 //   A block with itself (a diagonal pair) takes M = ImA ReA^T alone: its ImV
 //   is M - M^T, which the reduction over the source chunks forms.  At 350
 //   antennas each of the three groups has a diagonal block, so this takes 1/8
-//   of the MMA work away: @NEG@.
+//   of the MMA work away (FP16 + FP8 at 203 antennas 4% faster, split BF16 at 350
+//   antennas 0.8%: the generators set its pace).
 //
 // Second form (kForm = 1, HV_METHOD_TC_FP16): FP16 hi parts and FP8 (E4M3)
 // cross terms.  Per (time, frequency) slice the phasors are scaled by a power
@@ -509,31 +510,43 @@ __device__ __forceinline__ void slice_scale(float bound, float& c, float& inv_c2
 // All lanes read the same records, so the branch does not diverge.  Padding
 // records have zero amplitude.  beam_a: the antenna's column of the
 // transposed beam.
-template <bool kNear, bool kOnePixel>
+// A beam pixel for one antenna: its corners as c00 + fx d1 + fy (d2 + fx d3),
+// the bilinear interpolant with the differences formed once.
+struct PixelBeam {
+  float c00, d1, d2, d3;
+};
+__device__ __forceinline__ PixelBeam load_pixel(const float* beam_a, float pix, int Np, int dx,
+                                                int dy) {
+  const float* bp = beam_a + (size_t)__float_as_int(pix) * Np;
+  PixelBeam b;
+  b.c00 = __ldg(bp);
+  const float c01 = __ldg(bp + (size_t)dx * Np);
+  const float c10 = __ldg(bp + (size_t)dy * Np);
+  const float c11 = __ldg(bp + (size_t)(dx + dy) * Np);
+  b.d1 = c01 - b.c00;
+  b.d2 = c10 - b.c00;
+  b.d3 = (c11 - c10) - b.d1;
+  return b;
+}
+
+// kPixels: 1 or 2, the beam pixels the unit covers (2: the records from
+// `second` on lie on the other one), or 0: any.
+template <bool kNear, int kPixels>
 __device__ __forceinline__ void gen_unit_path(const SrcRec32* rec, const Ucoef32& uc,
                                               const float* beam_a, int Np, int dx, int dy,
-                                              float4 ref, float ph_ref, float csc, float* rv,
-                                              float* iv) {
-  // one pixel for the unit: its corners as c00 + fx d1 + fy (d2 + fx d3),
-  // the bilinear interpolant with the differences formed once per unit
-  float c00 = 0.f, d1 = 0.f, d2 = 0.f, d3 = 0.f;
-  if (kOnePixel) {
-    const float* bp = beam_a + (size_t)__float_as_int(reinterpret_cast<const float4*>(rec)[1].x) * Np;
-    c00 = __ldg(bp);
-    const float c01 = __ldg(bp + (size_t)dx * Np);
-    const float c10 = __ldg(bp + (size_t)dy * Np);
-    const float c11 = __ldg(bp + (size_t)(dx + dy) * Np);
-    d1 = c01 - c00;
-    d2 = c10 - c00;
-    d3 = (c11 - c10) - d1;
-  }
+                                              float4 ref, float ph_ref, int second, float csc,
+                                              float* rv, float* iv) {
+  PixelBeam b{}, b2{};
+  if (kPixels) b = load_pixel(beam_a, reinterpret_cast<const float4*>(rec)[1].x, Np, dx, dy);
+  if (kPixels == 2) b2 = load_pixel(beam_a, reinterpret_cast<const float4*>(rec + 7)[1].x, Np, dx, dy);
 #pragma unroll
   for (int q = 0; q < 8; ++q) {
     const float4* rp = reinterpret_cast<const float4*>(rec + q);
     const float4 ra = rp[0], rb = rp[1];  // sx sy sz amp | pix fx fy -
     float A;
-    if (kOnePixel) {
-      A = fmaf(rb.z, fmaf(rb.y, d3, d2), fmaf(rb.y, d1, c00));
+    if (kPixels) {
+      if (kPixels == 2 && q == second) b = b2;
+      A = fmaf(rb.z, fmaf(rb.y, b.d3, b.d2), fmaf(rb.y, b.d1, b.c00));
     } else {
       const float* bp = beam_a + (size_t)__float_as_int(rb.x) * Np;
       const float b00 = __ldg(bp);
@@ -570,14 +583,19 @@ __device__ __forceinline__ void gen_unit(const SrcRec32* rec, const Ucoef32& uc,
   const float4* rp0 = reinterpret_cast<const float4*>(rec);
   const float4 q0a = rp0[0], q0b = rp0[1];
   const int flags = __float_as_int(q0b.w);
+  const int second = __float_as_int(reinterpret_cast<const float4*>(rec + 1)[1].w);
   const bool one_pixel = flags < 0;
   const bool near = __int_as_float(flags & 0x7fffffff) <= dlim;
   if (near) {
     const float ph_ref = phase_exact(uc, q0a.x, q0a.y, q0a.z);
-    if (one_pixel) gen_unit_path<true, true>(rec, uc, beam_a, Np, dx, dy, q0a, ph_ref, csc, rv, iv);
-    else gen_unit_path<true, false>(rec, uc, beam_a, Np, dx, dy, q0a, ph_ref, csc, rv, iv);
+    if (one_pixel)
+      gen_unit_path<true, 1>(rec, uc, beam_a, Np, dx, dy, q0a, ph_ref, 0, csc, rv, iv);
+    else if (second)
+      gen_unit_path<true, 2>(rec, uc, beam_a, Np, dx, dy, q0a, ph_ref, second, csc, rv, iv);
+    else
+      gen_unit_path<true, 0>(rec, uc, beam_a, Np, dx, dy, q0a, ph_ref, 0, csc, rv, iv);
   } else {
-    gen_unit_path<false, false>(rec, uc, beam_a, Np, dx, dy, q0a, 0.f, csc, rv, iv);
+    gen_unit_path<false, 0>(rec, uc, beam_a, Np, dx, dy, q0a, 0.f, 0, csc, rv, iv);
   }
 }
 
