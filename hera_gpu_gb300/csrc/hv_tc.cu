@@ -101,15 +101,16 @@ constexpr int TC_ROWS = 128;          // antennas per block = MMA M
 constexpr int TC_SLOT = 16384;        // one operand tile: 128 rows x 128 B
 // Sources per stage: 16 for split BF16 (one tile per slot: hi and lo of 16
 // sources), 32 for FP16 + FP8 (two tiles per slot, see above).
-// Record stages: at least the operand stages (TC_MAX_STAGES), which makes
-// every phase-parity wait on a record barrier exact (see the generators).
-constexpr int TC_NREC_ALL = 8;
+// Record stages: at least the operand stages (and, for split BF16, whose
+// generators may wait for records first, plus the generator teams), which
+// makes every phase-parity wait on a record barrier exact (see the
+// generators).
 template <int kForm> struct TcForm;
 template <> struct TcForm<0> {
-  static constexpr int KS = 16, TILES = 1, NREC = TC_NREC_ALL;
+  static constexpr int KS = 16, TILES = 1, NREC = 16;
 };
 template <> struct TcForm<1> {
-  static constexpr int KS = 32, TILES = 2, NREC = TC_NREC_ALL;
+  static constexpr int KS = 32, TILES = 2, NREC = 8;
 };
 constexpr int TC_KS_MAX = 32;
 // Record stages: more than operand stages (they are small), so the TMA
@@ -154,7 +155,8 @@ constexpr int TC_MAX_STAGES = 8;
 #ifndef TC_FLUSH_SOURCES
 #define TC_FLUSH_SOURCES 2048
 #endif
-static_assert(TC_MAX_STAGES <= TC_NREC_ALL, "record stages >= operand stages");
+static_assert(2 * TC_MAX_STAGES <= TcForm<0>::NREC && TC_MAX_STAGES <= TcForm<1>::NREC,
+              "record stages >= operand stages (+ teams)");
 static_assert(TC_FLUSH_SOURCES % TC_KS_MAX == 0, "flush interval: whole stages of every form");
 constexpr int TC_TMEM_COLS = 512;
 constexpr int TC_SMEM_LIMIT = 227 * 1024;
@@ -529,14 +531,34 @@ __device__ __forceinline__ PixelBeam load_pixel(const float* beam_a, float pix, 
   return b;
 }
 
+// A read-only load kept in program order with its like.
+__device__ __forceinline__ void ldg_early(float& v, const float* p) {
+  asm volatile("ld.global.nc.f32 %0, [%1];" : "=f"(v) : "l"(p));
+}
+
 // kPixels: 1 or 2, the beam pixels the unit covers (2: the records from
-// `second` on lie on the other one), or 0: any.
-template <bool kNear, int kPixels>
+// `second` on lie on the other one), or 0: any.  kEarly (split BF16, whose
+// threads have the registers): with any pixels, every corner of the unit is in
+// flight before the first is used (1% on sparse catalogues; 1% slower with the
+// 96 registers of the FP16 + FP8 form).
+template <bool kNear, int kPixels, bool kEarly>
 __device__ __forceinline__ void gen_unit_path(const SrcRec32* rec, const Ucoef32& uc,
                                               const float* beam_a, int Np, int dx, int dy,
                                               float4 ref, float ph_ref, int second, float csc,
                                               float* rv, float* iv) {
   PixelBeam b{}, b2{};
+  float g[8][4];
+  if (!kPixels && kEarly) {
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      const float* bp =
+          beam_a + (size_t)__float_as_int(reinterpret_cast<const float4*>(rec + q)[1].x) * Np;
+      ldg_early(g[q][0], bp);
+      ldg_early(g[q][1], bp + (size_t)dx * Np);
+      ldg_early(g[q][2], bp + (size_t)dy * Np);
+      ldg_early(g[q][3], bp + (size_t)(dx + dy) * Np);
+    }
+  }
   if (kPixels) b = load_pixel(beam_a, reinterpret_cast<const float4*>(rec)[1].x, Np, dx, dy);
   if (kPixels == 2) b2 = load_pixel(beam_a, reinterpret_cast<const float4*>(rec + 7)[1].x, Np, dx, dy);
 #pragma unroll
@@ -547,6 +569,8 @@ __device__ __forceinline__ void gen_unit_path(const SrcRec32* rec, const Ucoef32
     if (kPixels) {
       if (kPixels == 2 && q == second) b = b2;
       A = fmaf(rb.z, fmaf(rb.y, b.d3, b.d2), fmaf(rb.y, b.d1, b.c00));
+    } else if (kEarly) {
+      A = lerp(lerp(g[q][0], g[q][1], rb.y), lerp(g[q][2], g[q][3], rb.y), rb.z);
     } else {
       const float* bp = beam_a + (size_t)__float_as_int(rb.x) * Np;
       const float b00 = __ldg(bp);
@@ -577,6 +601,7 @@ __device__ __forceinline__ void gen_unit_path(const SrcRec32* rec, const Ucoef32
 }
 
 // csc: the slice's scale (1 for split BF16; a power of two, so exact).
+template <bool kEarly>
 __device__ __forceinline__ void gen_unit(const SrcRec32* rec, const Ucoef32& uc,
                                          const float* beam_a, int Np, int dx, int dy, float dlim,
                                          float csc, float* rv, float* iv) {
@@ -589,13 +614,13 @@ __device__ __forceinline__ void gen_unit(const SrcRec32* rec, const Ucoef32& uc,
   if (near) {
     const float ph_ref = phase_exact(uc, q0a.x, q0a.y, q0a.z);
     if (one_pixel)
-      gen_unit_path<true, 1>(rec, uc, beam_a, Np, dx, dy, q0a, ph_ref, 0, csc, rv, iv);
+      gen_unit_path<true, 1, kEarly>(rec, uc, beam_a, Np, dx, dy, q0a, ph_ref, 0, csc, rv, iv);
     else if (second)
-      gen_unit_path<true, 2>(rec, uc, beam_a, Np, dx, dy, q0a, ph_ref, second, csc, rv, iv);
+      gen_unit_path<true, 2, kEarly>(rec, uc, beam_a, Np, dx, dy, q0a, ph_ref, second, csc, rv, iv);
     else
-      gen_unit_path<true, 0>(rec, uc, beam_a, Np, dx, dy, q0a, ph_ref, 0, csc, rv, iv);
+      gen_unit_path<true, 0, kEarly>(rec, uc, beam_a, Np, dx, dy, q0a, ph_ref, 0, csc, rv, iv);
   } else {
-    gen_unit_path<false, 0>(rec, uc, beam_a, Np, dx, dy, q0a, 0.f, 0, csc, rv, iv);
+    gen_unit_path<false, 0, kEarly>(rec, uc, beam_a, Np, dx, dy, q0a, 0.f, 0, csc, rv, iv);
   }
 }
 
@@ -928,15 +953,33 @@ tc_vis_kernel(const __grid_constant__ CUtensorMap rec_map, const __grid_constant
           const int s = (int)ring.s;
           const uint32_t par = ring.ph;
           const int rs = (int)(my_gs & (TC_NREC - 1));
+          // A launch of one simulation in cluster mode (split BF16) waits for
+          // the operand stage only once the first unit's values are in registers, so that the generators
+          // hold a stage for half of the time they take: of six stages, three
+          // teams generating leave the pushes, the MMAs and the releases of
+          // two CTAs more of the ring (350 antennas x 100k sources x 60 LSTs
+          // 4.95 -> 4.82 ms; without clusters, with 8 stages, in a batch or in
+          // the FP16 + FP8 form the registers held across the wait cost 1-4%).
+          // The others wait for the stage before the records.
+          //
           // A parity wait is exact only while the barrier's previous phase
           // has completed.  For the stage barrier that holds because this
           // team's previous stage passed it (teams <= stages).  For the
-          // record barrier it follows from this order: once stage gs is free
-          // the MMAs have consumed stage gs - NS, so the records of every
-          // stage up to gs - NS, gs - NREC among them (NREC >= NS), have
-          // landed -- even when a record copy is withheld (fault injection).
-          if (!wait_warp<kCluster>(smem_empty(s), par ^ 1, abort_flag, p.err, p.wait_ns)) { ok = false; break; }
+          // record barrier: this warp's previous stage gs - teams was free, so
+          // the MMAs had consumed stage gs - teams - NS, and the records of
+          // every stage up to that one, gs - NREC among them (NREC >= NS +
+          // teams), have landed -- even when a record copy is withheld (fault
+          // injection).  (With stage gs free first, NREC >= NS is enough.)
+          constexpr bool kLate = kCluster && !kTable && kForm == 0;
+          if (!kLate && !wait_warp<kCluster>(smem_empty(s), par ^ 1, abort_flag, p.err, p.wait_ns)) { ok = false; break; }
           if (!wait_warp(rec_full(rs), (my_gs / TC_NREC) & 1, abort_flag, p.err, p.wait_ns)) { ok = false; break; }
+          bool held = false;  // the operand stage is ours (kLate)
+          auto hold_stage = [&]() {
+            if (kLate && !held) {
+              held = true;
+              ok = wait_warp<kCluster>(smem_empty(s), par ^ 1, abort_flag, p.err, p.wait_ns);
+            }
+          };
           const SrcRec32* recs = reinterpret_cast<const SrcRec32*>(rec_smem + (size_t)rs * REC);
           const uint32_t stage_op = op_base + (uint32_t)s * stage_bytes;
           // unit u (sources 8 u .. 8 u + 7 of the stage) of slot index i
@@ -946,11 +989,13 @@ tc_vis_kernel(const __grid_constant__ CUtensorMap rec_map, const __grid_constant
               uint4 re_h = make_uint4(0, 0, 0, 0), im_h = re_h, re_l = re_h, im_l = re_h;
               if (u_ok[i]) {
                 float rv[8], iv[8];
-                gen_unit(recs + u * 8, i == 0 ? uc0 : Us[u_a[i]], beam + u_a[i], Np, dx, dy,
+                gen_unit<kForm == 0>(recs + u * 8, i == 0 ? uc0 : Us[u_a[i]], beam + u_a[i], Np, dx, dy,
                          dlim, 1.f, rv, iv);
                 split_pack(rv, re_h, re_l);
                 split_pack(iv, im_h, im_l);
               }
+              hold_stage();
+              if (kLate && !ok) return;
               sts128(tile + ((uint32_t)(u ^ r8) << 4), re_h);
               sts128(tile + ((uint32_t)((2 + u) ^ r8) << 4), im_h);
               sts128(tile + ((uint32_t)((4 + u) ^ r8) << 4), re_l);
@@ -960,11 +1005,13 @@ tc_vis_kernel(const __grid_constant__ CUtensorMap rec_map, const __grid_constant
               uint2 re_x = make_uint2(0, 0), im_x = re_x, re_l = re_x, im_l = re_x;
               if (u_ok[i]) {
                 float rv[8], iv[8];
-                gen_unit(recs + u * 8, i == 0 ? uc0 : Us[u_a[i]], beam + u_a[i], Np, dx, dy,
+                gen_unit<kForm == 0>(recs + u * 8, i == 0 ? uc0 : Us[u_a[i]], beam + u_a[i], Np, dx, dy,
                          dlim, csc, rv, iv);
                 split_f16_e4m3(rv, re_h, re_x, re_l);
                 split_f16_e4m3(iv, im_h, im_x, im_l);
               }
+              hold_stage();
+              if (kLate && !ok) return;
               sts128(tile + ((uint32_t)(u ^ r8) << 4), re_h);
               sts128(tile + ((uint32_t)((4 + u) ^ r8) << 4), im_h);
               const uint32_t t8 = tile + tile8_off + (uint32_t)(u & 1) * 8u;
@@ -978,7 +1025,7 @@ tc_vis_kernel(const __grid_constant__ CUtensorMap rec_map, const __grid_constant
           // one copy of the unit code (a second unrolled copy costs more in
           // instruction-cache misses than its static indices save)
 #pragma unroll 1
-          for (int k = 0; k < UPT; ++k) {
+          for (int k = 0; k < UPT && (!kLate || ok); ++k) {
             const int u = sg * UPT + k;
             if (kCluster) {
               // static unit indices keep the unit tables in registers (a CTA
@@ -992,6 +1039,7 @@ tc_vis_kernel(const __grid_constant__ CUtensorMap rec_map, const __grid_constant
                 if (i < nfill) unit(i, u);
             }
           }
+          if (kLate && !ok) break;
           // operands of this stage written: one arrival per warp (each lane
           // fences its own writes for the tensor core and the copy engine)
           fence_async_smem();
@@ -1506,9 +1554,9 @@ cudaError_t launch_form(const TcSimDesc* sims, int nsims, const void* rec, long 
   p.team_warps = team_warps;
   const int per_stage = TILES * p.max_slots * TC_SLOT;
   // records and the barrier block (barriers, item ring, TMEM holder: at most
-  // 8 (2 NREC + 3 NS + 3 + 2 RING + RING) + 8 = 472 bytes)
+  // 8 (2 NREC + 3 NS + 3 + 2 RING + RING) + 8 = 576 bytes)
   constexpr int TC_NREC = TcForm<kForm>::NREC;
-  const int fixed = TC_NREC * KS * 32 + 480;
+  const int fixed = TC_NREC * KS * 32 + 576;
   const int max_stages = std::min(TC_MAX_STAGES, (TC_SMEM_LIMIT - fixed) / per_stage);
   p.nstages = max_stages;
   if (sims[0].tune.stages > 0) p.nstages = std::min(p.nstages, sims[0].tune.stages);
@@ -1518,13 +1566,12 @@ cudaError_t launch_form(const TcSimDesc* sims, int nsims, const void* rec, long 
   // stages (each team's previous stage was released before it).  Small
   // teams of one-slot launches are widened, and a stage cap below the
   // number of teams raised, until that holds.
-  while ((TC_GEN_WARPS / p.team_warps > p.nstages || TC_GEN_WARPS / p.team_warps > TC_NREC) &&
+  while (TC_GEN_WARPS / p.team_warps > p.nstages &&
          p.team_warps < TC_TEAM_WARPS)
     p.team_warps *= 2;
   const int teams = std::max(TC_GEN_WARPS / p.team_warps, cluster ? TC_GEN_WARPS / TC_TEAM_WARPS : 1);
   p.nstages = std::min(max_stages, std::max(p.nstages, teams));
-  if (p.nstages < 2 || teams > p.nstages || TC_GEN_WARPS / p.team_warps > TC_NREC ||
-      p.nstages > TC_NREC)
+  if (p.nstages < 2 || teams > p.nstages || (kForm == 0 && teams + p.nstages > TC_NREC))
     return cudaErrorInvalidConfiguration;
   const int smem = fixed + p.nstages * per_stage;
   e = tc_configure();
