@@ -362,7 +362,7 @@ int run_device(hv_context* ctx, int method, const R* antpos, int nant, const dou
       // group table of the 128-antenna block pairs
       const size_t gbytes = tc_group_table_bytes(nant);
       std::string host(gbytes, '\0');
-      const int ngroups = tc_fill_group_table(nant, &host[0]);
+      const int ngroups = tc_fill_group_table(nant, form, &host[0]);
       HV_ENSURE(ctx->tcgroups, gbytes);
       HV_CK(cudaMemcpyAsync(ctx->tcgroups.p, host.data(), gbytes, cudaMemcpyHostToDevice, st));
       // batch of times per launch, bounded by the partial-sum and record caps
@@ -457,7 +457,8 @@ int run_device(hv_context* ctx, int method, const R* antpos, int nant, const dou
         if (nsrc > 0 && ctx->share.launched > 1) ctx->launches += ctx->share.launched - 1;
         HV_LAUNCH(1, launch_reduce<float>(static_cast<float*>(ctx->partial.p), slice_floats,
                                           counts + t0, nt, nfreq, t0, ntimes, chunk,
-                                          ceil_div(S1, chunk), Np, nant, true, out, st));
+                                          ceil_div(S1, chunk), Np, nant, tc_block_rows(nant, form),
+                                          out, st));
       }
     }
     return HV_OK;
@@ -487,7 +488,7 @@ int run_device(hv_context* ctx, int method, const R* antpos, int nant, const dou
                                            static_cast<R*>(ctx->partial.p), st),
                       st);
       HV_LAUNCH(1, launch_reduce<R>(static_cast<R*>(ctx->partial.p), 0, counts + t, 1, 1, 0, 1,
-                                    kPlainChunk, chunks, Np, nant, false, o, st));
+                                    kPlainChunk, chunks, Np, nant, 0, o, st));
     }
   }
   return HV_OK;

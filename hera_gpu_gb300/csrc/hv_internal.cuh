@@ -13,8 +13,8 @@
 //   partial [nchunk][2][Np][Np]   split-K partial sums over source chunks,
 //                                 plane 0 = Re V, plane 1 = Im V, stored
 //                                 [b][a] (a = row antenna, b = column antenna);
-//                                 the fused kernel's diagonal 128 x 128 blocks
-//                                 hold M in plane 1, with Im V = M - M^T
+//                                 the fused kernel's diagonal block pairs hold M
+//                                 in plane 1, with Im V = M - M^T
 // Np is nant rounded up to a multiple of 128; padded antennas have a zero
 // beam and so a zero phasor.
 #pragma once

@@ -33,6 +33,7 @@ struct PrepSim {
   float* partial;        // [T * F][nchunk][2][Np][Np]
   void* out;             // (F, T, nant, nant) complex64
   int nant, Np, T, F, S, P, rec_stride, chunk;
+  int block_rows;        // tc_block_rows(nant, 0)
 };
 // Prefix sums of the flattened index range of each batch launch (nsims + 1
 // entries each, device memory).
@@ -157,13 +158,13 @@ cudaError_t launch_herk_flagged(const F64Dims& d, int nz, const void* v, const i
 // chunks (ceil(count / chunk) of them) in order and write the full Hermitian
 // matrix (nant x nant complex R, row-major) to
 // out + ((f * ntimes_out) + t0 + tl) * nant * nant.  max_chunks: the most
-// chunks a slice can have (it picks the split of the work only).  antisym:
-// the partial sums of the fused kernel, whose diagonal 128 x 128 blocks hold M
-// in the imaginary plane, Im V = M - M^T.
+// chunks a slice can have (it picks the split of the work only).  block_rows:
+// 0, or the rows of the fused kernel's antenna blocks, whose diagonal pairs hold
+// M in the imaginary plane of its partial sums, Im V = M - M^T.
 template <typename R>
 cudaError_t launch_reduce(const R* partial, size_t slice_stride, const int* counts, int nt,
                           int nf, int t0, int ntimes_out, int chunk, int max_chunks, int Np,
-                          int nant, bool antisym, void* out, cudaStream_t st);
+                          int nant, int block_rows, void* out, cudaStream_t st);
 
 // --- hv_f64.cu -------------------------------------------------------------
 // FP64 product on the tensor cores.  Slices z = tl * nf + fl (nf of the
@@ -225,6 +226,9 @@ int tc_num_groups(int nant);
 // Generator warps per stage of the fused kernel for nant antennas (launches
 // whose simulations differ use the largest).
 int tc_team_warps(int nant);
+// Rows of the fused kernel's antenna blocks (32, 64, 96 or 128; one value a
+// launch) in a form (0 split BF16, 1 FP16 + FP8).
+int tc_block_rows(int nant, int form);
 // One-time launch attributes of the fused kernel (call outside stream capture).
 cudaError_t tc_configure();
 // All items of nsims simulations in one persistent launch; its CTAs claim
@@ -251,7 +255,7 @@ cudaError_t launch_tc_batch(const TcSimDesc* sims, int nsims, const void* rec, l
 size_t tc_partial_floats(int Np, int nsrc, int nslices, int chunk);
 int tc_chunk_sources(int nsrc, int nslices, int ngroups, int num_sms);
 size_t tc_group_table_bytes(int nant);
-int tc_fill_group_table(int nant, void* host_buf);
+int tc_fill_group_table(int nant, int form, void* host_buf);
 int tc_max_slots(int nant);
 
 }  // namespace hv

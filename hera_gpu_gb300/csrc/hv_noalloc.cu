@@ -152,7 +152,7 @@ extern "C" int hv_vis_gpu_noalloc(const void* d_antpos, int nant, double freq,
                                        Np, nant, beam_px, v, st));
     HV_NA_CK(launch_herk_plain<float>(v, counts + t, nsrc, Np, partial, st));
     HV_NA_CK(launch_reduce<float>(partial, 0, counts + t, 1, 1, 0, 1, kPlainChunk,
-                                  ceil_div(std::max(nsrc, 1), kPlainChunk), Np, nant, false,
+                                  ceil_div(std::max(nsrc, 1), kPlainChunk), Np, nant, 0,
                                   static_cast<float2*>(d_vis_out) + (size_t)t * NN, st));
   }
 #undef HV_NA_CK

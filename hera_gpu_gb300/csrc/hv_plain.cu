@@ -240,8 +240,8 @@ constexpr int kReduceAhead = 8;
 // slices x 2 chunks splitting it costs 10 us; from 34 chunks on it pays).
 constexpr int kReduceSplitChunks = 8;
 //
-// kAntisym (the fused kernel's partial sums): in the 128 x 128 blocks on the
-// diagonal the imaginary plane holds M with Im V = M - M^T, so their blocks sum
+// kAntisym (the fused kernel's partial sums): in the diagonal pairs of its
+// antenna blocks (block_rows antennas each) the imaginary plane holds M with Im V = M - M^T, so their blocks sum
 // M's transposed part as well (read along its rows, handed over through TM).
 template <typename R, int kCols, bool kAntisym>
 __device__ __forceinline__ void reduce_part(const R* __restrict__ partial_base,
@@ -249,7 +249,7 @@ __device__ __forceinline__ void reduce_part(const R* __restrict__ partial_base,
                                             int nf, int t0, int ntimes_out, int chunk, int Np,
                                             int nant,
                                             typename Traits<R>::C* __restrict__ out_base,
-                                            int tile, int part, int sl,
+                                            int block_rows, int tile, int part, int sl,
                                             typename Traits<R>::C (*T)[33], R (*TM)[33]) {
   using C = typename Traits<R>::C;
   const int nbt = ceil_div(nant, 32);
@@ -265,7 +265,7 @@ __device__ __forceinline__ void reduce_part(const R* __restrict__ partial_base,
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
   const size_t plane = (size_t)Np * Np;
   const int a = A * 32 + tx;
-  const bool antisym = kAntisym && A / (kAntPad / 32) == B / (kAntPad / 32);
+  const bool antisym = kAntisym && A / (block_rows / 32) == B / (block_rows / 32);
   if (antisym) {
 #pragma unroll 1
     for (int i = threadIdx.x; i < 32 * kCols; i += 256) {
@@ -334,13 +334,13 @@ template <typename R, int kCols, bool kAntisym>
 __global__ void __launch_bounds__(256)
 reduce_kernel(const R* __restrict__ partial_base, size_t slice_stride,
               const int* __restrict__ counts, int nf, int t0, int ntimes_out, int chunk, int Np,
-              int nant, typename Traits<R>::C* __restrict__ out_base) {
+              int nant, typename Traits<R>::C* __restrict__ out_base, int block_rows) {
   __shared__ typename Traits<R>::C T[kCols][33];
   __shared__ R TM[kAntisym ? kCols : 1][33];
   constexpr int kParts = 32 / kCols;
   reduce_part<R, kCols, kAntisym>(partial_base, slice_stride, counts, nf, t0, ntimes_out, chunk,
-                                  Np, nant, out_base, blockIdx.x / kParts, blockIdx.x % kParts,
-                                  blockIdx.y, T, TM);
+                                  Np, nant, out_base, block_rows, blockIdx.x / kParts,
+                                  blockIdx.x % kParts, blockIdx.y, T, TM);
 }
 
 // Every simulation of a batch: its split-K chunks reduced into its output.
@@ -356,7 +356,7 @@ reduce_batch_kernel(const PrepSim* __restrict__ sims, int nsims,
   const int local = (int)(blockIdx.x - __ldg(pre + si));
   const size_t slice = (size_t)ceil_div(sm.S > 0 ? sm.S : 1, sm.chunk) * 2 * sm.Np * sm.Np;
   reduce_part<float, 32, true>(sm.partial, slice, sm.counts, sm.F, 0, sm.T, sm.chunk, sm.Np,
-                               sm.nant, static_cast<float2*>(sm.out), local % tiles, 0,
+                               sm.nant, static_cast<float2*>(sm.out), sm.block_rows, local % tiles, 0,
                                local / tiles, T, TM);
 }
 
@@ -370,15 +370,15 @@ cudaError_t launch_reduce_batch(const PrepSim* sims, int nsims, const PrepPre& p
 template <typename R>
 cudaError_t launch_reduce(const R* partial, size_t slice_stride, const int* counts, int nt,
                           int nf, int t0, int ntimes_out, int chunk, int max_chunks, int Np,
-                          int nant, bool antisym, void* out, cudaStream_t st) {
+                          int nant, int block_rows, void* out, cudaStream_t st) {
   using C = typename Traits<R>::C;
   const int nbt = ceil_div(nant, 32);
   const bool split = max_chunks >= kReduceSplitChunks;
   const dim3 grid(nbt * (nbt + 1) / 2 * (split ? 4 : 1), nt * nf);
-  auto* kernel = split ? (antisym ? reduce_kernel<R, 8, true> : reduce_kernel<R, 8, false>)
-                       : (antisym ? reduce_kernel<R, 32, true> : reduce_kernel<R, 32, false>);
+  auto* kernel = split ? (block_rows ? reduce_kernel<R, 8, true> : reduce_kernel<R, 8, false>)
+                       : (block_rows ? reduce_kernel<R, 32, true> : reduce_kernel<R, 32, false>);
   kernel<<<grid, 256, 0, st>>>(partial, slice_stride, counts, nf, t0, ntimes_out, chunk, Np, nant,
-                               reinterpret_cast<C*>(out));
+                               reinterpret_cast<C*>(out), block_rows);
   return cudaGetLastError();
 }
 
@@ -386,7 +386,7 @@ template cudaError_t launch_gen_phasors<float>(const void*, const int*, int, con
 template cudaError_t launch_gen_phasors<double>(const void*, const int*, int, const void*, const double*, int, int, int, void*, cudaStream_t);
 template cudaError_t launch_herk_plain<float>(const void*, const int*, int, int, float*, cudaStream_t);
 template cudaError_t launch_herk_plain<double>(const void*, const int*, int, int, double*, cudaStream_t);
-template cudaError_t launch_reduce<float>(const float*, size_t, const int*, int, int, int, int, int, int, int, int, bool, void*, cudaStream_t);
-template cudaError_t launch_reduce<double>(const double*, size_t, const int*, int, int, int, int, int, int, int, int, bool, void*, cudaStream_t);
+template cudaError_t launch_reduce<float>(const float*, size_t, const int*, int, int, int, int, int, int, int, int, int, void*, cudaStream_t);
+template cudaError_t launch_reduce<double>(const double*, size_t, const int*, int, int, int, int, int, int, int, int, int, void*, cudaStream_t);
 
 }  // namespace hv

@@ -7,7 +7,8 @@
 // contracted on the tensor cores (tcgen05.mma, FP32 accumulators in TMEM).
 //
 // Work decomposition
-//   Antennas are cut into blocks of 128 (the MMA M).  The upper triangle of
+//   Antennas are cut into the fewest blocks of at most 128 (the MMA M), of 32,
+//   64, 96 or 128 rows each (tc_block_rows).  The upper triangle of
 //   block pairs (I <= J) is partitioned into groups of at most two pairs
 //   that share their row block: (I, J) and (I, J + 1), and the pairs that
 //   end a row on the last block, (I, nb - 1), taken transposed as
@@ -45,8 +46,10 @@
 //   last warp     cluster mode: pushes this CTA's tiles to peer CTAs.
 //
 // Operand layout of one stage (16 sources): one tile per slot, the slots'
-// tiles side by side (16 KB each: 128 rows x 128 bytes, K = 64 BF16 per
-// antenna row), within a row the K chunks of 16 bytes
+// tiles side by side (a block's rows x 128 bytes, K = 64 BF16 per antenna
+// row; the row block's operand is read as 128 rows whatever its block has, and
+// the accumulator lanes of the rows past it are never read), within a row the
+// K chunks of 16 bytes
 //   [Re hi s0-7, Re hi s8-15, Im hi s0-7, Im hi s8-15,
 //    Re lo s0-7, Re lo s8-15, Im lo s0-7, Im lo s8-15]
 //   so each MMA K-step (16 elements) holds the real or the imaginary parts
@@ -97,8 +100,8 @@
 
 namespace hv {
 
-constexpr int TC_ROWS = 128;          // antennas per block = MMA M
-constexpr int TC_SLOT = 16384;        // one operand tile: 128 rows x 128 B
+constexpr int TC_ROWS = 128;          // MMA M, the most antennas per block
+constexpr int TC_ROW_BYTES = 128;     // one antenna row of an operand tile
 // Sources per stage: 16 for split BF16 (one tile per slot: hi and lo of 16
 // sources), 32 for FP16 + FP8 (two tiles per slot, see above).
 // Record stages: at least the operand stages (and, for split BF16, whose
@@ -130,8 +133,9 @@ constexpr int TC_KS_MAX = 32;
 //    unit of 8 sources each).  Only three of its 64 KB stages fit beside the
 //    records, so a stage must be generated by every generator at once: with
 //    12 warps in three teams it ran 10% slower.
-// One-slot launches of up to 64 (32) antennas use teams of half (a
-// quarter) the full team, enough for their rows.
+// Fewer rows take smaller teams, and so more of them: split BF16 a warp for
+// each 32 rows of a block, FP16 + FP8 half (a quarter) of its warps for one-slot
+// launches of up to 64 (32) antennas.
 template <int kForm> struct TcLayout;
 template <> struct TcLayout<0> {
   static constexpr int GEN_WARPS = 12, TEAM = 4, NSG = 1;
@@ -142,7 +146,8 @@ template <> struct TcLayout<1> {
 template <int kForm> constexpr int tc_threads() { return TcLayout<kForm>::GEN_WARPS * 32 + 96; }
 static_assert(((tc_threads<0>() / 32 + 3) / 4) * 32 * 128 <= 16384,
               "split BF16: at most 4 warps a scheduler at 128 registers");
-constexpr int TC_MAX_STAGES = 8;
+// Operand stages: 8 unless more generator teams need one each.
+constexpr int TC_STAGES = 8, TC_MAX_STAGES = 12;
 // Sources accumulated in TMEM before the sum is added to the item's split-K
 // partial in global memory (FP32, round to nearest) and the accumulator
 // starts again.  The tensor core's accumulation into TMEM loses a fraction
@@ -155,8 +160,6 @@ constexpr int TC_MAX_STAGES = 8;
 #ifndef TC_FLUSH_SOURCES
 #define TC_FLUSH_SOURCES 2048
 #endif
-static_assert(2 * TC_MAX_STAGES <= TcForm<0>::NREC && TC_MAX_STAGES <= TcForm<1>::NREC,
-              "record stages >= operand stages (+ teams)");
 static_assert(TC_FLUSH_SOURCES % TC_KS_MAX == 0, "flush interval: whole stages of every form");
 constexpr int TC_TMEM_COLS = 512;
 constexpr int TC_SMEM_LIMIT = 227 * 1024;
@@ -172,13 +175,14 @@ struct TcGroup {
   int slot_block[3];
   int slot_rows[3];  // valid antenna rows of each slot's block
   int sa;            // slot of the row block (A operand); the column blocks (B) are slots 0, 1
-  int n_mma;         // MMA N: 128 + the columns of slot 1 for two pairs, else those of slot 0
+  int n_mma;         // MMA N: a block + the columns of slot 1 for two pairs, else those of slot 0
   // columns [neg_col, neg_col + neg_n) of the off-diagonal pairs (neg_n = 0:
   // none): the ones that take the -Re Im products (a diagonal pair's
   // imaginary part is M - M^T with M = Im Re^T, formed by the reduction)
   int neg_col, neg_n;
   int pI[2], pJ[2];  // row and column block of each pair; pI > pJ: computed below the diagonal
   int pN[2];         // valid columns of block pJ, rounded up to 16
+  int pM[2];         // valid rows of block pI
   // Cluster mode (one CTA per group, cluster rank = group index): every
   // block is generated by exactly one CTA of the cluster and written into
   // the shared memory of each CTA whose group uses it.
@@ -237,7 +241,8 @@ struct TcParams {
   unsigned long long* claim;
   int claim_mode;
   long long group_items;  // shared launch: cluster items x ngroups
-  int team_warps;  // generator warps per stage without clusters (a full team, or 1/2 or 1/4)
+  int team_warps;  // generator warps per stage
+  int rows;        // rows of an antenna block (tc_block_rows; one value a launch)
 };
 constexpr int kClaimCount = 0, kClaimFront = 1, kClaimBack = 2;
 // Items a CTA has claimed ahead of its slowest role (the ring of item
@@ -723,11 +728,13 @@ __device__ __forceinline__ bool decode_item(const TcParams& p, long long it, int
   return true;
 }
 
-// One CTA per SM; the launch bounds give each form's register budget (split
-// BF16: 15 warps, 128 registers a thread; FP16 + FP8: 19 warps, 96).
-template <bool kCluster, bool kTable, int kForm>
-__global__ void __launch_bounds__(tc_threads<kForm>(), 1)
-tc_vis_kernel(const __grid_constant__ CUtensorMap rec_map, const __grid_constant__ TcParams p) {
+// kFull: blocks of 128 rows and (split BF16) full teams, as compile-time
+// constants: with the sizes from the parameters these launches are 2-3% slower.
+template <bool kCluster, bool kTable, int kForm, bool kFull>
+__device__ __forceinline__ void tc_vis_body(const CUtensorMap& rec_map, const TcParams& p) {
+  const int block_rows = kFull ? TC_ROWS : p.rows;
+  const int team_warps =
+      kFull && (kForm == 0 || kCluster) ? TcLayout<kForm>::TEAM : p.team_warps;
   // warp roles: generators, then the TMA producer, the MMA issuer and the
   // cluster-mode pusher of tiles to peer CTAs
   constexpr int TC_GEN_WARPS = TcLayout<kForm>::GEN_WARPS;
@@ -740,9 +747,6 @@ tc_vis_kernel(const __grid_constant__ CUtensorMap rec_map, const __grid_constant
   constexpr int REC = KS * 32;                  // record bytes per stage
   constexpr int FLUSH = TC_FLUSH_SOURCES / KS;  // stages per accumulator flush
   constexpr int TC_NREC = TcForm<kForm>::NREC;  // record stages
-  // generator warps per stage in cluster mode (compile-time there; launches
-  // without clusters take theirs from the parameters)
-  constexpr int CL_TEAM = TcLayout<kForm>::TEAM;
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   // The operand tiles need a 1024-byte aligned base (the 128-byte swizzle
   // atoms); the launch reserves no slack for aligning it, which keeps the
@@ -758,7 +762,8 @@ tc_vis_kernel(const __grid_constant__ CUtensorMap rec_map, const __grid_constant
   const uint32_t op_base = smem_u32(smem);
   // a stage: the FP16 / split-BF16 tiles of every slot side by side, then
   // (FP16 + FP8 form) the FP8 tiles of every slot side by side
-  const uint32_t tile8_off = (uint32_t)p.max_slots * TC_SLOT;
+  const uint32_t slot_bytes = (uint32_t)block_rows * TC_ROW_BYTES;
+  const uint32_t tile8_off = (uint32_t)p.max_slots * slot_bytes;
   const uint32_t stage_bytes = (uint32_t)TILES * tile8_off;
   uint8_t* rec_smem = smem + (size_t)NS * stage_bytes;
   const uint32_t rec_base = smem_u32(rec_smem);
@@ -795,7 +800,7 @@ tc_vis_kernel(const __grid_constant__ CUtensorMap rec_map, const __grid_constant
   const TcGroup* mine = groups0 + rank;
   // cluster mode: operand bytes this CTA receives from peers per stage
   const uint32_t recv_bytes =
-      kCluster ? (uint32_t)__ldg(&mine->recv_slots) * (uint32_t)(TILES * TC_SLOT) : 0u;
+      kCluster ? (uint32_t)__ldg(&mine->recv_slots) * ((uint32_t)TILES * slot_bytes) : 0u;
   // cluster mode: does this CTA generate any block?
   const int nown = kCluster ? __ldg(&mine->nown) : 0;
   const bool generates = !kCluster || nown > 0;
@@ -803,7 +808,6 @@ tc_vis_kernel(const __grid_constant__ CUtensorMap rec_map, const __grid_constant
     // arrivals per stage on smem_full: one per generator warp of the team
     // (if this CTA generates) and, in cluster mode, the MMA thread's arming
     // of the bytes its peers push
-    const int team_warps = kCluster ? CL_TEAM : p.team_warps;
     const int full_count = (generates ? team_warps : 0) + (recv_bytes ? 1 : 0);
     const int empty_count = kCluster ? mine->empty_count : 1;
     for (int r = 0; r < TC_NREC; ++r) {
@@ -876,7 +880,6 @@ tc_vis_kernel(const __grid_constant__ CUtensorMap rec_map, const __grid_constant
   if (warp < TC_GEN_WARPS) {
     // ------------------------------------------------ phasor generators --
     const int tid = threadIdx.x;
-    const int team_warps = kCluster ? CL_TEAM : p.team_warps;
     const int nteams = TC_GEN_WARPS / team_warps;
     const int team = warp / team_warps;  // takes the stages with gs % nteams == team
     uint32_t gs = 0, ic = 0;
@@ -910,13 +913,13 @@ tc_vis_kernel(const __grid_constant__ CUtensorMap rec_map, const __grid_constant
       // this thread's units (fixed for the item): antenna row `row` and the
       // units of 8 sources [sg * upt, sg * upt + upt) of its team's stages,
       // in each slot it fills
-      // a team covers its rows (128, or fewer for the small teams of
-      // one-slot launches) with NSG thread groups along the stage
+      // a team covers its rows (the block's, or more where it had to be
+      // widened) with NSG thread groups along the stage
       constexpr int NSG = TcLayout<kForm>::NSG;
       constexpr int UPT = (KS / 8) / NSG;  // units per thread per stage
       static_assert(UPT >= 1 && UPT * NSG * 8 == KS, "a stage's units split evenly");
       const int tt = tid % (team_warps * 32);
-      const int nrows = kCluster ? TC_ROWS : team_warps * 32 / NSG;
+      const int nrows = team_warps * 32 / NSG;
       const int row = tt % nrows, sg = tt / nrows;
       int u_slot[3], u_a[3];
       bool u_ok[3];
@@ -927,7 +930,7 @@ tc_vis_kernel(const __grid_constant__ CUtensorMap rec_map, const __grid_constant
         const int srows = slot == 0 ? g_rows0 : (slot == 1 ? g_rows1 : g_rows2);
         const int sblk = slot == 0 ? g_blk0 : (slot == 1 ? g_blk1 : g_blk2);
         u_ok[i] = i < nfill && row < srows;
-        u_a[i] = sblk * TC_ROWS + row;
+        u_a[i] = sblk * block_rows + row;
       }
       // the phase coefficients of the first unit's antenna, fixed for the item
       Ucoef32 uc0 = {};
@@ -984,7 +987,7 @@ tc_vis_kernel(const __grid_constant__ CUtensorMap rec_map, const __grid_constant
           const uint32_t stage_op = op_base + (uint32_t)s * stage_bytes;
           // unit u (sources 8 u .. 8 u + 7 of the stage) of slot index i
           auto unit = [&](int i, int u) {
-            const uint32_t tile = stage_op + (uint32_t)u_slot[i] * TC_SLOT + rowoff;
+            const uint32_t tile = stage_op + (uint32_t)u_slot[i] * slot_bytes + rowoff;
             if constexpr (kForm == 0) {
               uint4 re_h = make_uint4(0, 0, 0, 0), im_h = re_h, re_l = re_h, im_l = re_h;
               if (u_ok[i]) {
@@ -996,6 +999,7 @@ tc_vis_kernel(const __grid_constant__ CUtensorMap rec_map, const __grid_constant
               }
               hold_stage();
               if (kLate && !ok) return;
+              if (!kFull && row >= block_rows) return;
               sts128(tile + ((uint32_t)(u ^ r8) << 4), re_h);
               sts128(tile + ((uint32_t)((2 + u) ^ r8) << 4), im_h);
               sts128(tile + ((uint32_t)((4 + u) ^ r8) << 4), re_l);
@@ -1010,8 +1014,7 @@ tc_vis_kernel(const __grid_constant__ CUtensorMap rec_map, const __grid_constant
                 split_f16_e4m3(rv, re_h, re_x, re_l);
                 split_f16_e4m3(iv, im_h, im_x, im_l);
               }
-              hold_stage();
-              if (kLate && !ok) return;
+              if (!kFull && row >= block_rows) return;
               sts128(tile + ((uint32_t)(u ^ r8) << 4), re_h);
               sts128(tile + ((uint32_t)((4 + u) ^ r8) << 4), im_h);
               const uint32_t t8 = tile + tile8_off + (uint32_t)(u & 1) * 8u;
@@ -1060,29 +1063,35 @@ tc_vis_kernel(const __grid_constant__ CUtensorMap rec_map, const __grid_constant
         const bool first = j0 == 0;
         if (!wait_warp(acc_full, ic & 1, abort_flag, p.err, p.wait_ns)) { ok = false; break; }
         tc_fence_after();
-        // a warp reads its lane quadrant q of TMEM; its 128-column blocks cb
-        // (pair cb & 1, plane cb >> 1: Re, Im) are every (generator warps /
-        // 4)-th from warp / 4
+        // a warp reads its lane quadrant q of TMEM (rows q * 32 .. of the row
+        // block); its column blocks cb (pair cb & 1, plane cb >> 1: Re, Im)
+        // are every (generator warps / 4)-th from warp / 4.  kTrim: quadrants
+        // and 32-column pieces past the block's valid rows and columns are
+        // skipped (in one-CTA FP16 + FP8 launches of 65-128 antennas the test
+        // costs 2-3% more than it saves).
+        constexpr bool kTrim = kForm == 0 || kCluster;
 #pragma unroll 1
         for (int cb = warp >> 2; cb < 4; cb += TC_GEN_WARPS / 4) {
           const int q = warp & 3;
           const int pr = cb & 1, plane = cb >> 1;
-          if (pr < g_npairs) {
+          if (pr < g_npairs && (!kTrim || q * 32 < __ldg(&gp->pM[pr]))) {
             const int I = __ldg(&gp->pI[pr]), J = __ldg(&gp->pJ[pr]);
             float* out = SIM_P(d, partial) +
                          (((size_t)d.sl * SIM_I(d, nchunk) + d.k) * 2 + plane) * (size_t)Np * Np;
-            const int a = I * TC_ROWS + q * 32 + lane;
+            const int a = I * block_rows + q * 32 + lane;
+            const uint32_t tcol = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(plane * 256 + pr * block_rows);
+            const int nc32 = kTrim ? (__ldg(&gp->pN[pr]) + 31) >> 5 : TC_ROWS / 32;
             if (I <= J) {
               // partial[b][a] = V[a][b], a contiguous across the warp
 #pragma unroll 1
-              for (int c32 = 0; c32 < 4; ++c32) {
+              for (int c32 = 0; c32 < nc32; ++c32) {
                 float v[32];
-                tmem_ld32(tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(cb * 128 + c32 * 32), v);
+                tmem_ld32(tcol + (uint32_t)(c32 * 32), v);
                 if (kForm == 1) {
 #pragma unroll
                   for (int c = 0; c < 32; ++c) v[c] *= inv_c2;
                 }
-                const int b0 = J * TC_ROWS + c32 * 32;
+                const int b0 = J * block_rows + c32 * 32;
                 if (first) {
 #pragma unroll
                   for (int c = 0; c < 32; ++c) out[(size_t)(b0 + c) * Np + a] = v[c];
@@ -1096,10 +1105,10 @@ tc_vis_kernel(const __grid_constant__ CUtensorMap rec_map, const __grid_constant
               // 32 consecutive b per lane
               const float sg_ = (plane ? -1.f : 1.f) * inv_c2;
 #pragma unroll 1
-              for (int c32 = 0; c32 < 4; ++c32) {
+              for (int c32 = 0; c32 < nc32; ++c32) {
                 float v[32];
-                tmem_ld32(tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(cb * 128 + c32 * 32), v);
-                float4* o4 = reinterpret_cast<float4*>(out + (size_t)a * Np + J * TC_ROWS + c32 * 32);
+                tmem_ld32(tcol + (uint32_t)(c32 * 32), v);
+                float4* o4 = reinterpret_cast<float4*>(out + (size_t)a * Np + J * block_rows + c32 * 32);
 #pragma unroll
                 for (int c = 0; c < 8; ++c) {
                   const float4 x = make_float4(sg_ * v[4 * c], sg_ * v[4 * c + 1],
@@ -1185,10 +1194,10 @@ tc_vis_kernel(const __grid_constant__ CUtensorMap rec_map, const __grid_constant
         const uint32_t abt = kForm == 0 ? 1u : 0u;  // BF16, or FP16 / E4M3
         const int neg_n = __ldg(&gp->neg_n);
         const uint32_t noff = (uint32_t)__ldg(&gp->neg_col);
-        const uint32_t b_neg = noff ? (uint32_t)(TC_SLOT >> 4) : 0u;  // slot 1's tile
+        const uint32_t b_neg = noff ? slot_bytes >> 4 : 0u;  // slot 1's tile
         const uint32_t idp = idesc_mma(nm, false, abt);
         const uint32_t idn = neg_n ? idesc_mma(neg_n, true, abt) : 0u;
-        const uint32_t a0 = desc_lo(op_base + (uint32_t)__ldg(&gp->sa) * TC_SLOT);
+        const uint32_t a0 = desc_lo(op_base + (uint32_t)__ldg(&gp->sa) * slot_bytes);
         const uint32_t b0 = desc_lo(op_base);
         for (int j0 = 0; j0 < d.nst && ok; j0 += FLUSH) {
           const int j1 = min(d.nst, j0 + FLUSH);
@@ -1242,14 +1251,14 @@ tc_vis_kernel(const __grid_constant__ CUtensorMap rec_map, const __grid_constant
         if (!wait1(gen_done(s), par, abort_flag, p.err, p.wait_ns)) { ok = false; break; }
         const uint32_t stage_op = op_base + (uint32_t)s * stage_bytes;
         for (int k = 0; k < nown; ++k) {
-          const uint32_t src = stage_op + (uint32_t)__ldg(&mine->own_slot[k]) * TC_SLOT;
+          const uint32_t src = stage_op + (uint32_t)__ldg(&mine->own_slot[k]) * slot_bytes;
           const int nd = __ldg(&mine->ndst[k]);
           for (int q = 0; q < nd; ++q) {
             const uint32_t rr = (uint32_t)__ldg(&mine->dst_rank[k][q]);
-            const uint32_t dst = stage_op + (uint32_t)__ldg(&mine->dst_slot[k][q]) * TC_SLOT;
+            const uint32_t dst = stage_op + (uint32_t)__ldg(&mine->dst_slot[k][q]) * slot_bytes;
 #pragma unroll
             for (int x = 0; x < TILES; ++x)
-              bulk_push(map_to_rank(dst + x * tile8_off, rr), src + x * tile8_off, TC_SLOT,
+              bulk_push(map_to_rank(dst + x * tile8_off, rr), src + x * tile8_off, slot_bytes,
                         map_to_rank(smem_full(s), rr));
           }
         }
@@ -1271,15 +1280,45 @@ tc_vis_kernel(const __grid_constant__ CUtensorMap rec_map, const __grid_constant
   }
 }
 
+// One CTA per SM; the launch bounds give each form's register budget (split
+// BF16: 15 warps, 128 registers a thread; FP16 + FP8: 19 warps, 96).
+template <bool kCluster, bool kTable, int kForm>
+__global__ void __launch_bounds__(tc_threads<kForm>(), 1)
+tc_vis_kernel(const __grid_constant__ CUtensorMap rec_map, const __grid_constant__ TcParams p) {
+  if constexpr (kForm == 1) {
+    tc_vis_body<kCluster, kTable, kForm, true>(rec_map, p);
+  } else {
+    if (p.rows == TC_ROWS && p.team_warps == TcLayout<kForm>::TEAM)
+      tc_vis_body<kCluster, kTable, kForm, true>(rec_map, p);
+    else
+      tc_vis_body<kCluster, kTable, kForm, false>(rec_map, p);
+  }
+}
+
 #undef SIM_I
 #undef SIM_P
 
 // ------------------------------------------------------------------- host --
+// Rows of an antenna block: as few blocks of at most 128 as there can be, evenly
+// filled, in multiples of 32 (a generator warp, a TMEM lane quadrant).  A
+// block's generators take a time of their own however few rows it has, so 158
+// antennas as 96 + 62 keep two CTAs of a cluster evenly busy, where 128 + 30
+// leave one nearly idle; and blocks of 32, 64 and 96 rows have smaller teams,
+// tiles and accumulators.  Split BF16, 4 channels x 20 LSTs x 50k sources: 80
+// antennas 963 -> 886 us, 140 antennas 1931 -> 1802; 270 antennas, 2 channels,
+// 2012 -> 1900.  The FP16 + FP8 form keeps 128 rows: its single team gains on
+// some sizes and loses as much on others.
+int tc_block_rows(int nant, int form) {
+  if (form != 0) return TC_ROWS;
+  const int nb = ceil_div(nant, TC_ROWS);
+  return ceil_div(ceil_div(nant, nb), 32) * 32;
+}
+
 namespace {
 
-std::vector<TcGroup> make_groups(int nant) {
-  const int nb = ceil_div(nant, TC_ROWS);
-  auto rows_of = [&](int blk) { return std::min(TC_ROWS, nant - blk * TC_ROWS); };
+std::vector<TcGroup> make_groups(int nant, int form = 0) {
+  const int BR = tc_block_rows(nant, form), nb = ceil_div(nant, BR);
+  auto rows_of = [&](int blk) { return std::min(BR, nant - blk * BR); };
   auto ncols = [&](int blk) { return ((rows_of(blk) + 15) / 16) * 16; };
   // (row block, column block) pairs of each group; the column blocks of a
   // group are different and only the last may be partly valid
@@ -1315,17 +1354,18 @@ std::vector<TcGroup> make_groups(int nant) {
       g.pI[q] = prs[q].first;
       g.pJ[q] = prs[q].second;
       g.pN[q] = ncols(prs[q].second);
+      g.pM[q] = rows_of(prs[q].first);
       slot_of(prs[q].second);
     }
     g.sa = slot_of(prs[0].first);
-    g.n_mma = g.npairs == 2 ? TC_ROWS + g.pN[1] : g.pN[0];
+    g.n_mma = g.npairs == 2 ? BR + g.pN[1] : g.pN[0];
     g.neg_col = 0;
     g.neg_n = g.n_mma;
     if (g.pI[0] == g.pJ[0]) {  // the first pair is diagonal
-      g.neg_col = TC_ROWS;
+      g.neg_col = BR;
       g.neg_n = g.npairs == 2 ? g.pN[1] : 0;
     } else if (g.npairs == 2 && g.pI[1] == g.pJ[1]) {
-      g.neg_n = TC_ROWS;
+      g.neg_n = BR;
     }
     out.push_back(g);
   }
@@ -1335,9 +1375,9 @@ std::vector<TcGroup> make_groups(int nant) {
 // Cluster mode: each block is generated by one CTA of the cluster (among
 // the groups that use it, the one with the fewest generated rows so far) and
 // sent to the others; fills the sharing fields of every group.
-void plan_cluster(std::vector<TcGroup>& gs, int nant) {
+void plan_cluster(std::vector<TcGroup>& gs, int nant, int form) {
   const int C = (int)gs.size();
-  const int nb = ceil_div(nant, TC_ROWS);
+  const int BR = tc_block_rows(nant, form), nb = ceil_div(nant, BR);
   std::vector<int> load(C, 0);
   auto slot_in = [&](int g, int blk) {
     for (int s = 0; s < gs[g].nslots; ++s)
@@ -1353,7 +1393,7 @@ void plan_cluster(std::vector<TcGroup>& gs, int nant) {
     for (int g = 0; g < C; ++g)
       if (slot_in(g, b) >= 0 && (owner < 0 || load[g] < load[owner])) owner = g;
     if (owner < 0) continue;
-    load[owner] += std::min(TC_ROWS, nant - b * TC_ROWS);
+    load[owner] += std::min(BR, nant - b * BR);
     TcGroup& o = gs[owner];
     const int k = o.nown++;
     o.own_slot[k] = slot_in(owner, b);
@@ -1414,6 +1454,7 @@ namespace {
 template <int kForm>
 int team_warps_for(int nant) {
   constexpr int T = TcLayout<kForm>::TEAM;
+  if (kForm == 0) return tc_block_rows(nant, 0) / 32;
   return nant <= 32 ? T / 4 : nant <= 64 ? T / 2 : T;
 }
 }  // namespace
@@ -1422,9 +1463,9 @@ int tc_team_warps(int nant) { return team_warps_for<0>(nant); }
 
 size_t tc_group_table_bytes(int nant) { return sizeof(TcGroup) * make_groups(nant).size(); }
 
-int tc_fill_group_table(int nant, void* host_buf) {
-  auto g = make_groups(nant);
-  if (use_cluster((int)g.size())) plan_cluster(g, nant);
+int tc_fill_group_table(int nant, int form, void* host_buf) {
+  auto g = make_groups(nant, form);
+  if (use_cluster((int)g.size())) plan_cluster(g, nant, form);
   std::copy(g.begin(), g.end(), static_cast<TcGroup*>(host_buf));
   return (int)g.size();
 }
@@ -1499,6 +1540,8 @@ cudaError_t launch_form(const TcSimDesc* sims, int nsims, const void* rec, long 
   int max_slots = 1, team_warps = 1;
   for (int i = 0; i < nsims; ++i) {
     if (sims[i].ngroups != sims[0].ngroups) cluster = false;
+    if (tc_block_rows(sims[i].nant, kForm) != tc_block_rows(sims[0].nant, kForm))
+      return cudaErrorInvalidValue;
     max_slots = std::max(max_slots, sims[i].max_slots);
     team_warps = std::max(team_warps, team_warps_for<kForm>(sims[i].nant));
   }
@@ -1552,26 +1595,35 @@ cudaError_t launch_form(const TcSimDesc* sims, int nsims, const void* rec, long 
   p.wait_ns = wait_ns ? wait_ns : TC_WAIT_NS;
   p.stall = stall;
   p.team_warps = team_warps;
-  const int per_stage = TILES * p.max_slots * TC_SLOT;
-  // records and the barrier block (barriers, item ring, TMEM holder: at most
-  // 8 (2 NREC + 3 NS + 3 + 2 RING + RING) + 8 = 576 bytes)
+  p.rows = tc_block_rows(sims[0].nant, kForm);
+  const int slot = p.rows * TC_ROW_BYTES;
+  const int per_stage = TILES * p.max_slots * slot;
+  // records and the barrier block (barriers, item ring, TMEM holder);
   constexpr int TC_NREC = TcForm<kForm>::NREC;
-  const int fixed = TC_NREC * KS * 32 + 576;
-  const int max_stages = std::min(TC_MAX_STAGES, (TC_SMEM_LIMIT - fixed) / per_stage);
-  p.nstages = max_stages;
+  // and, behind the last tile, the rows past its block that the row operand
+  // is read with
+  const int fixed = std::max(TC_NREC * KS * 32 + 8 * (2 * TC_NREC + 3 * TC_MAX_STAGES + 3 + 3 * TC_ITEM_RING) + 8,
+                             TC_ROWS * TC_ROW_BYTES - slot);
+  const int max_stages = std::min(kForm == 0 ? TC_MAX_STAGES : TC_STAGES,
+                                  (TC_SMEM_LIMIT - fixed) / per_stage);
+  p.nstages = std::min(max_stages, TC_STAGES);
   if (sims[0].tune.stages > 0) p.nstages = std::min(p.nstages, sims[0].tune.stages);
   // A team waits on a stage's barriers by phase parity, which tells apart
   // only consecutive phases: a team may run at most one round of a stage
   // ahead of the MMAs, which holds while the teams are no more than the
-  // stages (each team's previous stage was released before it).  Small
-  // teams of one-slot launches are widened, and a stage cap below the
-  // number of teams raised, until that holds.
-  while (TC_GEN_WARPS / p.team_warps > p.nstages &&
-         p.team_warps < TC_TEAM_WARPS)
+  // stages (each team's previous stage was released before it).  Small teams
+  // are widened where the shared memory (or a stage cap) does not hold a stage
+  // for each, and the stages raised to the teams otherwise.
+  while (TC_GEN_WARPS / p.team_warps >
+             (sims[0].tune.stages > 0 ? std::min(max_stages, sims[0].tune.stages) : max_stages) &&
+         2 * p.team_warps <= TC_TEAM_WARPS)
     p.team_warps *= 2;
-  const int teams = std::max(TC_GEN_WARPS / p.team_warps, cluster ? TC_GEN_WARPS / TC_TEAM_WARPS : 1);
+  const int teams = TC_GEN_WARPS / p.team_warps;
   p.nstages = std::min(max_stages, std::max(p.nstages, teams));
-  if (p.nstages < 2 || teams > p.nstages || (kForm == 0 && teams + p.nstages > TC_NREC))
+  // records: at least a stage each, and in cluster mode (split BF16) a team
+  // more (see the generators)
+  if (p.nstages < 2 || teams > p.nstages || p.nstages > TC_NREC ||
+      (kForm == 0 && cluster && teams + p.nstages > TC_NREC))
     return cudaErrorInvalidConfiguration;
   const int smem = fixed + p.nstages * per_stage;
   e = tc_configure();
@@ -1618,8 +1670,8 @@ cudaError_t launch_form(const TcSimDesc* sims, int nsims, const void* rec, long 
   cfg.gridDim = dim3((unsigned)(C * (num_sms / C)));
   // co-resident clusters for this cluster size and shared memory (cached:
   // the query is host-side and stays valid)
-  static int cached_n[2][TC_MAX_CLUSTER + 1][TC_MAX_STAGES + 1] = {};
-  int& nclusters = cached_n[table][C][p.nstages];
+  static int cached_n[2][TC_MAX_CLUSTER + 1][TC_MAX_STAGES + 1][TC_ROWS / 32 + 1] = {};
+  int& nclusters = cached_n[table][C][p.nstages][p.rows / 32];
   if (nclusters == 0) {
     e = table ? cudaOccupancyMaxActiveClusters(&nclusters, tc_vis_kernel<true, true, kForm>,
                                                &cfg)

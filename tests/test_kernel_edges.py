@@ -210,3 +210,23 @@ def test_omnical_layouts(nants, kind):
     np.testing.assert_array_equal(got["iters"], ref["iters"])
     again = omnical(ggu, *[x[1:] for x in a], 1e-10, 12, precision=1)
     np.testing.assert_array_equal(again["gains"], got["gains"][1:])
+
+
+# antenna blocks of the fused forms (32, 64, 96 and 128 rows; one to five
+# blocks), at their edges
+@gpu
+@pytest.mark.parametrize("method", ["tc", "tc_fp16"])
+@pytest.mark.parametrize("nant", [31, 32, 33, 64, 65, 96, 97, 128, 129, 161, 192, 193, 257, 288,
+                                  289, 385, 520, 641])
+def test_antenna_blocks(nant, method):
+    args = sim(nant, 700, ntimes=2, seed=nant)
+    v = vis_gpu(*args, precision=1, method=method)
+    check_hermitian(v)
+    ref = vis_oracle(*[a.astype(np.float64) if isinstance(a, np.ndarray) else a for a in args])
+    assert rel_frobenius(v, ref).max() <= 1e-4
+    if method == "tc":
+        # every entry on the scale of its antennas' powers (split BF16 operands
+        # carry 16 bits): a misplaced block or a sign of one pair would be of
+        # order 1
+        p = np.sqrt(np.einsum("taa->ta", ref.real))
+        assert np.abs(v - ref).max() <= 1e-4 * (p[:, :, None] * p[:, None, :]).max()
