@@ -134,14 +134,18 @@ __device__ __forceinline__ int med3(int a, int b, int c) {
 }
 
 constexpr int kStripWarps = 4;  // warps a block, each with its own strip or rows
-constexpr int kStripRows = 16;  // output rows a warp takes (8 and 32 were slower for one window or another)
+// Output rows a warp takes, at most (8 and 32 were slower for one window or
+// another at full size); fewer, down to 2, while that leaves fewer warps than
+// kStripFill: an image of 100 x 100 is bound by its warps' serial rows.
+constexpr int kStripRows = 16, kStripFill = 152 * 8;
 
 // The strip of a warp: warps of consecutive index take consecutive strips of
 // the same rows.
-__device__ __forceinline__ bool strip_of_warp(int nstrips, int rows, int& strip, int& row0) {
+__device__ __forceinline__ bool strip_of_warp(int nstrips, int rows, int take, int& strip,
+                                              int& row0) {
   const long long w = (long long)blockIdx.x * kStripWarps + (threadIdx.x >> 5);
   strip = (int)(w % nstrips);
-  const long long r = w / nstrips * kStripRows;
+  const long long r = w / nstrips * take;
   row0 = (int)r;
   return r < rows;
 }
@@ -195,14 +199,14 @@ __device__ __forceinline__ void expand_row4(const Row4& x, int lane, int (&k)[6]
 template <bool kVec>
 __global__ void __launch_bounds__(kStripWarps * 32)
 median3x3_kernel(const float* __restrict__ in, float* __restrict__ out, int rows, int cols,
-                 int nstrips) {
+                 int nstrips, int take) {
   int strip, row0;
-  if (!strip_of_warp(nstrips, rows, strip, row0)) return;
+  if (!strip_of_warp(nstrips, rows, take, strip, row0)) return;
   const int lane = threadIdx.x & 31, c = strip * 128 + 4 * lane;
   const size_t plane = (size_t)rows * cols;
   const float* img = in + (size_t)blockIdx.y * plane;
   float* dst = out + (size_t)blockIdx.y * plane;
-  const int row1 = min(rows, row0 + kStripRows);
+  const int row1 = min(rows, row0 + take);
   int ka[6], kb[6];
   expand_row4(load_row4<kVec>(img, row0 - 1, rows, cols, c, lane), lane, ka);
   expand_row4(load_row4<kVec>(img, row0, rows, cols, c, lane), lane, kb);
@@ -351,13 +355,13 @@ __device__ __forceinline__ List<N> middle(const List<NA>& a) {
 template <int H, int W>
 __global__ void __launch_bounds__(kStripWarps * 32, 4)
 median_merge_kernel(const float* __restrict__ in, float* __restrict__ out, int rows, int cols,
-                    int nstrips) {
+                    int nstrips, int take) {
   static_assert(H % 2 == 1 && W % 2 == 1 && W <= 11, "odd windows");
   constexpr int kHalf = (W - 1) / 2;
   constexpr int kPairs = 31 - kHalf;
   constexpr int kLow = H * W / 2 - H;  // of the shared elements, ranks kLow .. kLow + H
   int strip, row0;
-  if (!strip_of_warp(nstrips, rows, strip, row0)) return;
+  if (!strip_of_warp(nstrips, rows, take, strip, row0)) return;
   const int lane = threadIdx.x & 31;
   const size_t plane = (size_t)rows * cols;
   const float* img = in + (size_t)blockIdx.y * plane;
@@ -368,7 +372,7 @@ median_merge_kernel(const float* __restrict__ in, float* __restrict__ out, int r
   const int x0 = c - W / 2 + 1;
   const bool in0 = x0 >= 0 && x0 < cols, in1 = x0 + 1 >= 0 && x0 + 1 < cols;
   const bool mine = lane >= 1 && lane <= kPairs;
-  const int row1 = min(rows, row0 + kStripRows);
+  const int row1 = min(rows, row0 + take);
   int a[H], b[H];
   auto load = [&](int r, float& u, float& v) {
     u = v = 0.f;
@@ -428,13 +432,22 @@ median_merge_kernel(const float* __restrict__ in, float* __restrict__ out, int r
   }
 }
 
+// Rows a warp takes and the grid of a strip launch.
+int strip_grid(int nstrips, int rows, int nimg, dim3* grid) {
+  auto warps = [&](int take) { return (long long)nstrips * ((rows + take - 1) / take); };
+  int take = kStripRows;
+  while (take > 2 && warps(take) * nimg < kStripFill) take /= 2;
+  *grid = dim3((unsigned)((warps(take) + kStripWarps - 1) / kStripWarps), nimg);
+  return take;
+}
 template <int H, int W>
 bool launch_merge(const float* d_in, float* d_out, int nimg, int rows, int cols, cudaStream_t st) {
   constexpr int kOut = 2 * (31 - (W - 1) / 2);
   const int nstrips = (cols + kOut - 1) / kOut;
-  const long long warps = (long long)nstrips * ((rows + kStripRows - 1) / kStripRows);
-  median_merge_kernel<H, W><<<dim3((unsigned)((warps + kStripWarps - 1) / kStripWarps), nimg),
-                              kStripWarps * 32, 0, st>>>(d_in, d_out, rows, cols, nstrips);
+  dim3 grid;
+  const int take = strip_grid(nstrips, rows, nimg, &grid);
+  median_merge_kernel<H, W><<<grid, kStripWarps * 32, 0, st>>>(d_in, d_out, rows, cols, nstrips,
+                                                               take);
   return true;
 }
 template <int H>
@@ -454,13 +467,15 @@ bool launch_strips(const float* d_in, float* d_out, int nimg, int rows, int cols
                    cudaStream_t st) {
   if (k0 == 3 && k1 == 3) {
     const int nstrips = (cols + 127) / 128;
-    const long long warps = (long long)nstrips * ((rows + kStripRows - 1) / kStripRows);
-    const dim3 grid((unsigned)((warps + kStripWarps - 1) / kStripWarps), nimg);
+    dim3 grid;
+    const int take = strip_grid(nstrips, rows, nimg, &grid);
     if ((cols & 3) == 0 &&
         ((reinterpret_cast<uintptr_t>(d_in) | reinterpret_cast<uintptr_t>(d_out)) & 15) == 0)
-      median3x3_kernel<true><<<grid, kStripWarps * 32, 0, st>>>(d_in, d_out, rows, cols, nstrips);
+      median3x3_kernel<true><<<grid, kStripWarps * 32, 0, st>>>(d_in, d_out, rows, cols, nstrips,
+                                                                take);
     else
-      median3x3_kernel<false><<<grid, kStripWarps * 32, 0, st>>>(d_in, d_out, rows, cols, nstrips);
+      median3x3_kernel<false><<<grid, kStripWarps * 32, 0, st>>>(d_in, d_out, rows, cols, nstrips,
+                                                                take);
     return true;
   }
   switch (k0) {
