@@ -170,6 +170,16 @@ int ensure(hv_context* ctx, DevBuf& b, size_t bytes) {
   return HV_OK;
 }
 
+// Whether buffers can grow to the wanted sizes, ensure()'s slack included,
+// within the budget: asked before any of them grows, since one grown for more
+// work than fits would leave less room for the others.
+bool fits(const hv_context* ctx, const std::pair<DevBuf*, size_t>* want, size_t n) {
+  size_t grow = 0;
+  for (size_t i = 0; i < n; ++i)
+    grow += want[i].second > want[i].first->cap ? want[i].second - want[i].first->cap : 0;
+  return !ctx->budget || ctx->held + grow + grow / 8 + 256 * n <= ctx->budget;
+}
+
 // Page-locked host buffer that stays valid for the copies queued from it.
 int ensure_host(hv_context* ctx, HostBuf& b, size_t bytes) {
   if (b.cap >= bytes) return HV_OK;
@@ -221,6 +231,9 @@ int check_shapes(hv_context* ctx, int precision, int method, int nant, int nfreq
 // records of one batch of times.
 constexpr size_t kTcPartialCap = size_t(6) << 30;
 constexpr size_t kTcRecCap = size_t(4) << 30;
+// Phasors and partial sums of the slices that one launch of the plain form
+// takes (a slice of 350 antennas x 100k sources has 350 MB).
+constexpr size_t kPlainCap = size_t(2) << 30;
 
 // FP64 product on the tensor cores (hv_f64.cu) for every slice; HV_OK, an
 // error, or -1: the SIMT product is to be used (arrays whose class sums would
@@ -269,12 +282,7 @@ int run_f64(hv_context* ctx, const double* eq2tops, const double* crd_eq, const 
         {&ctx->f64_small, f64_table_bytes() + b_small * n},
         {&ctx->rec, b_rec * ntb},
         {&ctx->blkcounts, sizeof(int) * (size_t)prep_blocks(nsrc) * ntb}};
-    // before any buffer grows: a buffer grown for more slices than fit would
-    // leave less room for the others
-    size_t grow = 0;
-    for (auto& w : want) grow += w.second > w.first->cap ? w.second - w.first->cap : 0;
-    grow += grow / 8 + 256 * std::size(want);  // ensure()'s slack
-    if (ctx->budget && ctx->held + grow > ctx->budget) continue;
+    if (!fits(ctx, want, std::size(want))) continue;
     int r = HV_OK;
     for (auto& w : want)
       if (r == HV_OK) r = ensure(ctx, *w.first, w.second);
@@ -470,25 +478,57 @@ int run_device(hv_context* ctx, int method, const R* antpos, int nant, const dou
     if (r >= 0) return r;
   }
 
-  // plain form: one time at a time, one frequency at a time
+  // plain form: as many slices a launch (whole times, or some frequencies of
+  // one time) as kPlainCap and the budget hold; a slice's result does not
+  // depend on them
   const int chunks = ceil_div(S1, kPlainChunk);
-  HV_ENSURE(ctx->partial, sizeof(R) * (size_t)chunks * 2 * Np * Np);
-  HV_ENSURE(ctx->v, sizeof(C) * (size_t)S1 * Np);
-  HV_ENSURE(ctx->rec, sizeof(Rec) * (size_t)S1);
-  HV_ENSURE(ctx->blkcounts, sizeof(int) * (size_t)prep_blocks(nsrc));
-  for (int t = 0; t < ntimes; ++t) {
-    HV_LAUNCH(2, launch_prep<R>(crd_eq, I_sky, nsrc, eq2tops, t, 1, P,
-                                static_cast<int*>(ctx->blkcounts.p), ctx->rec.p, counts + t, st));
-    const U* Ut = static_cast<const U*>(ctx->ucoef.p) + (size_t)t * nfreq * Np;
-    for (int f = 0; f < nfreq; ++f) {
-      C* o = static_cast<C*>(out) + ((size_t)f * ntimes + t) * NN;
-      HV_LAUNCH(1, launch_gen_phasors<R>(ctx->rec.p, counts + t, nsrc, Ut + (size_t)f * Np,
-                                         beamT + (size_t)f * PP * Np, Np, nant, P, ctx->v.p, st));
-      HV_LAUNCH_TIMED(launch_herk_plain<R>(ctx->v.p, counts + t, nsrc, Np,
-                                           static_cast<R*>(ctx->partial.p), st),
+  const size_t b_part = sizeof(R) * (size_t)chunks * 2 * Np * Np, b_v = sizeof(C) * (size_t)S1 * Np;
+  long long nz = std::max<long long>(1, std::min<long long>(
+      std::min<long long>(32768, (long long)ntimes * nfreq), (long long)(kPlainCap / (b_part + b_v))));
+  int ntb = 1, nfb = 1;
+  for (;; nz /= 2) {
+    nfb = (int)std::min<long long>(nfreq, nz);
+    ntb = nfb == nfreq ? (int)std::max<long long>(1, std::min<long long>(ntimes, nz / nfreq)) : 1;
+    const size_t n = (size_t)ntb * nfb;
+    const std::pair<DevBuf*, size_t> want[] = {
+        {&ctx->partial, b_part * n},
+        {&ctx->v, b_v * n},
+        {&ctx->rec, sizeof(Rec) * (size_t)S1 * ntb},
+        {&ctx->blkcounts, sizeof(int) * (size_t)prep_blocks(nsrc) * ntb}};
+    if (n > 1 && !fits(ctx, want, std::size(want))) continue;
+    int r = HV_OK;
+    for (auto& w : want)
+      if (r == HV_OK) r = ensure(ctx, *w.first, w.second);
+    if (r == HV_OK) break;
+    if (r != HV_ERR_OOM || n == 1) return r;
+    ctx->err.clear();
+  }
+  PlainDims d{};
+  d.u_nf = nfreq;
+  d.nant = nant;
+  d.Np = Np;
+  d.rec_stride = (size_t)S1;
+  d.v_stride = (size_t)S1 * Np;
+  d.p_stride = (size_t)chunks * 2 * Np * Np;
+  for (int t0 = 0; t0 < ntimes; t0 += ntb) {
+    const int nt = std::min(ntb, ntimes - t0);
+    HV_LAUNCH(2, launch_prep_strided<R>(crd_eq, I_sky, nsrc, eq2tops, t0, nt, P,
+                                        static_cast<int*>(ctx->blkcounts.p), ctx->rec.p,
+                                        (size_t)S1, counts + t0, st));
+    d.counts = counts + t0;
+    for (int f0 = 0; f0 < nfreq; f0 += nfb) {
+      d.nf = std::min(nfb, nfreq - f0);
+      const int n = nt * d.nf;
+      HV_LAUNCH(1, launch_gen_phasors<R>(
+                       d, n, ctx->rec.p, nsrc,
+                       static_cast<const U*>(ctx->ucoef.p) + ((size_t)t0 * nfreq + f0) * Np,
+                       beamT + (size_t)f0 * PP * Np, P, ctx->v.p, st));
+      HV_LAUNCH_TIMED(launch_herk_plain<R>(d, n, ctx->v.p, nsrc, static_cast<R*>(ctx->partial.p),
+                                           st),
                       st);
-      HV_LAUNCH(1, launch_reduce<R>(static_cast<R*>(ctx->partial.p), 0, counts + t, 1, 1, 0, 1,
-                                    kPlainChunk, chunks, Np, nant, 0, o, st));
+      HV_LAUNCH(1, launch_reduce<R>(static_cast<R*>(ctx->partial.p), d.p_stride, counts + t0, nt,
+                                    d.nf, t0, ntimes, kPlainChunk, chunks, Np, nant, 0,
+                                    static_cast<C*>(out) + (size_t)f0 * ntimes * NN, st));
     }
   }
   return HV_OK;

@@ -134,17 +134,28 @@ cudaError_t launch_slice_bound(const void* rec, size_t rec_stride, const int* co
 // Source chunk of the split-K sum over sources (plain path).
 constexpr int kPlainChunk = 4096;
 
-// v[s][a] (complex, Np per source) for the count[0] records of one slice.
-template <typename R>
-cudaError_t launch_gen_phasors(const void* rec, const int* count, int nsrc_max,
-                               const void* U, const R* beamT, int Np, int nant, int P,
-                               void* v, cudaStream_t st);
+// Slices of one launch: z = tl * nf + fl (nf of the call's u_nf frequencies),
+// buffers with a stride a slice.
+struct PlainDims {
+  const int* counts;  // sources above the horizon per time
+  int nf, u_nf;       // frequencies of the launch, and of U
+  int nant, Np;
+  size_t rec_stride;  // records a time
+  size_t v_stride;    // phasors a slice
+  size_t p_stride;    // partial sums a slice
+};
 
-// Upper-triangle SIMT Hermitian product of v into partial sums, one chunk of
+// v[z][s][a] (complex, Np per source) for every record of every slice.  U,
+// beamT: of the launch's first slice.
+template <typename R>
+cudaError_t launch_gen_phasors(const PlainDims& d, int nz, const void* rec, int nsrc_max,
+                               const void* U, const R* beamT, int P, void* v, cudaStream_t st);
+
+// Upper-triangle SIMT Hermitian products of v into partial sums, one chunk of
 // kPlainChunk sources per grid row.
 template <typename R>
-cudaError_t launch_herk_plain(const void* v, const int* count, int nsrc_max, int Np,
-                              R* partial, cudaStream_t st);
+cudaError_t launch_herk_plain(const PlainDims& d, int nz, const void* v, int nsrc_max, R* partial,
+                              cudaStream_t st);
 
 // The same for nz slices in FP64, only those with flags[z] set (hv_f64.cu):
 // the sources of window d, their chunks' sums at partial + z *

@@ -146,11 +146,12 @@ extern "C" int hv_vis_gpu_noalloc(const void* d_antpos, int nant, double freq,
                                         Np, beamT, st));
   HV_NA_CK(launch_ucoef<float>(antpos, nant, Np, e2t, 0, ntimes, d_freq, 1, U, st));
   for (int t = 0; t < ntimes; ++t) {
+    const PlainDims d{counts + t, 1, 1, nant, Np, 0, 0, 0};
     HV_NA_CK(launch_prep<float>(crd, I, nsrc, e2t, t, 1, beam_px, blk, rec, counts + t, st));
-    HV_NA_CK(launch_gen_phasors<float>(rec, counts + t, nsrc,
+    HV_NA_CK(launch_gen_phasors<float>(d, 1, rec, nsrc,
                                        static_cast<const Ucoef32*>(U) + (size_t)t * Np, beamT,
-                                       Np, nant, beam_px, v, st));
-    HV_NA_CK(launch_herk_plain<float>(v, counts + t, nsrc, Np, partial, st));
+                                       beam_px, v, st));
+    HV_NA_CK(launch_herk_plain<float>(d, 1, v, nsrc, partial, st));
     HV_NA_CK(launch_reduce<float>(partial, 0, counts + t, 1, 1, 0, 1, kPlainChunk,
                                   ceil_div(std::max(nsrc, 1), kPlainChunk), Np, nant, 0,
                                   static_cast<float2*>(d_vis_out) + (size_t)t * NN, st));

@@ -12,6 +12,8 @@
 //   reduce      : sums the chunk partials in a fixed order (compensated in
 //                 FP32) and writes the full Hermitian matrix, replacing the
 //                 host-side sum over chunks of vis.py:258.
+#include <algorithm>
+
 #include "hv_internal.cuh"
 #include "hv_kernels.h"
 
@@ -25,39 +27,47 @@ __device__ __forceinline__ double2 make_phasor(const SrcRec64& r, const Ucoef64&
   return phasor64(r, u, A);
 }
 
+// A warp generates kGenSpan sources for 32 antennas, whose coefficients stay in
+// its registers.  Slice z of the launch: time z / nf, frequency z % nf.
+constexpr int kGenSpan = 64;
 template <typename R>
 __global__ void __launch_bounds__(256)
-gen_phasors_kernel(const typename Traits<R>::Rec* __restrict__ rec, const int* __restrict__ count,
+gen_phasors_kernel(const PlainDims d, const typename Traits<R>::Rec* __restrict__ rec,
                    const typename Traits<R>::U* __restrict__ U, const R* __restrict__ beamT,
-                   int Np, int nant, int dx, int dy, typename Traits<R>::C* __restrict__ v) {
+                   int PP, int dx, int dy, typename Traits<R>::C* __restrict__ v) {
   using C = typename Traits<R>::C;
-  const int n = *count;
-  const int lane = threadIdx.x & 31;
-  const int wpb = blockDim.x >> 5;
-  for (int s = blockIdx.x * wpb + (threadIdx.x >> 5); s < n; s += gridDim.x * wpb) {
-    const typename Traits<R>::Rec r = rec[s];
-    for (int a = lane; a < Np; a += 32) {
-      C val;
-      val.x = R(0); val.y = R(0);
-      if (a < nant) {
-        const R A = beam_bilinear<R>(beamT, Np, a, r, dx, dy);
-        val = make_phasor(r, U[a], A);
-      }
-      v[(size_t)s * Np + a] = val;
+  const int z = blockIdx.y, tl = z / d.nf, f = z % d.nf;
+  const int n = d.counts[tl];
+  const int groups = d.Np / 32;
+  const long long job = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
+  const long long s0 = job / groups * kGenSpan;
+  if (s0 >= n) return;
+  const int a = (int)(job % groups) * 32 + (threadIdx.x & 31);
+  const typename Traits<R>::U u = U[((size_t)tl * d.u_nf + f) * d.Np + a];
+  const R* beam = beamT + (size_t)f * PP * d.Np;
+  rec += (size_t)tl * d.rec_stride;
+  v += (size_t)z * d.v_stride + a;
+  const int s1 = (int)min((long long)n, s0 + kGenSpan);
+#pragma unroll 2
+  for (int s = (int)s0; s < s1; ++s) {
+    C val;
+    val.x = R(0); val.y = R(0);
+    if (a < d.nant) {
+      const typename Traits<R>::Rec r = rec[s];
+      val = make_phasor(r, u, beam_bilinear<R>(beam, d.Np, a, r, dx, dy));
     }
+    v[(size_t)s * d.Np] = val;
   }
 }
 
 template <typename R>
-cudaError_t launch_gen_phasors(const void* rec, const int* count, int nsrc_max,
-                               const void* U, const R* beamT, int Np, int nant, int P,
-                               void* v, cudaStream_t st) {
+cudaError_t launch_gen_phasors(const PlainDims& d, int nz, const void* rec, int nsrc_max,
+                               const void* U, const R* beamT, int P, void* v, cudaStream_t st) {
   const int dx = P > 1 ? 1 : 0, dy = P > 1 ? P : 0;
-  int blocks = ceil_div(nsrc_max > 0 ? nsrc_max : 1, 8);
-  if (blocks > 152 * 64) blocks = 152 * 64;
-  gen_phasors_kernel<R><<<blocks, 256, 0, st>>>(
-      reinterpret_cast<const typename Traits<R>::Rec*>(rec), count,
-      reinterpret_cast<const typename Traits<R>::U*>(U), beamT, Np, nant, dx, dy,
+  const long long jobs = (long long)ceil_div(std::max(nsrc_max, 1), kGenSpan) * (d.Np / 32);
+  gen_phasors_kernel<R><<<dim3((unsigned)((jobs + 7) / 8), nz), 256, 0, st>>>(
+      d, reinterpret_cast<const typename Traits<R>::Rec*>(rec),
+      reinterpret_cast<const typename Traits<R>::U*>(U), beamT, P * P, dx, dy,
       reinterpret_cast<typename Traits<R>::C*>(v));
   return cudaGetLastError();
 }
@@ -72,10 +82,12 @@ __device__ __forceinline__ void decode_upper(int t, int nb, int& I, int& J) {
   J = I + t;
 }
 
-template <typename R>
-__device__ __forceinline__ void herk_tile(const typename Traits<R>::C* __restrict__ v, int n,
-                                          int Np, R* __restrict__ partial) {
-  using C = typename Traits<R>::C;
+// FP64: one tile of a chunk, 4 x 4 outputs a thread; bound by the FP64 pipe
+// (2 FMA a clock and SM).
+__device__ __forceinline__ void herk_tile(const double2* __restrict__ v, int n, int Np,
+                                          double* __restrict__ partial) {
+  using R = double;
+  using C = double2;
   const int s0 = blockIdx.y * kPlainChunk;
   if (s0 >= n) return;
   const int s1 = min(s0 + kPlainChunk, n);
@@ -115,19 +127,6 @@ __device__ __forceinline__ void herk_tile(const typename Traits<R>::C* __restric
     }
     __syncthreads();
     if (s + kHK < s1) gload(s + kHK);
-    // FP32: each stage's 16 sources are summed from zero and the stage sum
-    // is added to the running total, so the total's rounding walks over
-    // kPlainChunk / 16 additions instead of kPlainChunk (about 4x less
-    // error at the same chunk); FP64 sums straight into the total
-    constexpr bool kTwoLevel = sizeof(R) == 4;
-    R st_re[4][4], st_im[4][4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        st_re[i][j] = kTwoLevel ? R(0) : acc_re[i][j];
-        st_im[i][j] = kTwoLevel ? R(0) : acc_im[i][j];
-      }
 #pragma unroll
     for (int k = 0; k < kHK; ++k) {
       C a[4], b[4];
@@ -140,17 +139,10 @@ __device__ __forceinline__ void herk_tile(const typename Traits<R>::C* __restric
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
           // v_a conj(v_b) = (ar br + ai bi) + i (ai br - ar bi)
-          st_re[i][j] = fma(a[i].x, b[j].x, fma(a[i].y, b[j].y, st_re[i][j]));
-          st_im[i][j] = fma(a[i].y, b[j].x, fma(-a[i].x, b[j].y, st_im[i][j]));
+          acc_re[i][j] = fma(a[i].x, b[j].x, fma(a[i].y, b[j].y, acc_re[i][j]));
+          acc_im[i][j] = fma(a[i].y, b[j].x, fma(-a[i].x, b[j].y, acc_im[i][j]));
         }
     }
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        acc_re[i][j] = kTwoLevel ? acc_re[i][j] + st_re[i][j] : st_re[i][j];
-        acc_im[i][j] = kTwoLevel ? acc_im[i][j] + st_im[i][j] : st_im[i][j];
-      }
     __syncthreads();
   }
   R* pre = partial + (size_t)blockIdx.y * 2 * Np * Np;
@@ -167,11 +159,127 @@ __device__ __forceinline__ void herk_tile(const typename Traits<R>::C* __restric
   }
 }
 
-template <typename R>
+// Pairs of FP32 values in one 64-bit register, combined by the packed FMA
+// (two of them a lane and instruction, each rounded as a scalar one).
+using F2 = unsigned long long;
+__device__ __forceinline__ F2 fma2(F2 a, F2 b, F2 c) {
+  F2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ F2 add2(F2 a, F2 b) {
+  F2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ F2 pack2(float lo, float hi) {
+  F2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ float half2(F2 v, int h) {
+  float lo, hi;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+  return h ? hi : lo;
+}
+
+// FP32: a 64 x 64 tile of a chunk, 4 (rows a) x 4 (columns b) outputs a thread.
+// Bound by the FMA pipe and by the shared-memory reads that feed it.  The
+// columns' values are kept as separate real and imaginary arrays, read as
+// pairs without bank conflicts; the rows' values doubled (ar ar ai ai), so that
+// a packed FMA takes them as they come (a warp reads only two distinct ones at
+// a time, a broadcast).  Two buffers, one barrier a stage of 16 sources.  Each
+// stage is summed from zero and added to the running total, so the total's
+// rounding walks over kPlainChunk / 16 additions instead of kPlainChunk (about
+// 4x less error at the same chunk).  Measured on GB300, 350 antennas x 50k
+// sources (ncu): scalar FMAs on interleaved complex values, whose column reads
+// had two-way bank conflicts, 872 us; @HK@.
+__global__ void __launch_bounds__(256, 2)
+herk_plain_kernel(const PlainDims d, const float2* __restrict__ v_base,
+                  float* __restrict__ partial) {
+  const int z = blockIdx.z;
+  const int n = d.counts[z / d.nf], Np = d.Np;
+  const int s0 = blockIdx.y * kPlainChunk;
+  if (s0 >= n) return;
+  const int s1 = min(s0 + kPlainChunk, n);
+  int I, J;
+  decode_upper(blockIdx.x, Np / kHT, I, J);
+  const float2* v = v_base + (size_t)z * d.v_stride;
+  __shared__ __align__(16) float4 As[2][kHK][kHT];
+  __shared__ __align__(16) float Br[2][kHK][kHT], Bi[2][kHK][kHT];
+  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+  F2 acc_re[4][2] = {}, acc_im[4][2] = {};
+  const float2* vA = v + (size_t)I * kHT;
+  const float2* vB = v + (size_t)J * kHT;
+  const int c = threadIdx.x & 63, k0 = threadIdx.x >> 6;  // this thread loads sources k0 + 4 q
+  float2 ra[4], rb[4];
+  auto gload = [&](int s) {
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int k = s + k0 + 4 * q;
+      const bool ok = k < s1;
+      ra[q] = ok ? vA[(size_t)k * Np + c] : make_float2(0.f, 0.f);
+      rb[q] = ok ? vB[(size_t)k * Np + c] : make_float2(0.f, 0.f);
+    }
+  };
+  gload(s0);
+  int buf = 0;
+  const F2 minus = pack2(-1.f, -1.f);
+  for (int s = s0; s < s1; s += kHK, buf ^= 1) {
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      As[buf][k0 + 4 * q][c] = make_float4(ra[q].x, ra[q].x, ra[q].y, ra[q].y);
+      Br[buf][k0 + 4 * q][c] = rb[q].x;
+      Bi[buf][k0 + 4 * q][c] = rb[q].y;
+    }
+    __syncthreads();  // (the other buffer's readers are past it before the next)
+    if (s + kHK < s1) gload(s + kHK);
+    F2 st_re[4][2] = {}, st_im[4][2] = {};
+#pragma unroll
+    for (int k = 0; k < kHK; ++k) {
+      const ulonglong2 br = *reinterpret_cast<const ulonglong2*>(&Br[buf][k][tx * 4]);
+      const ulonglong2 bi = *reinterpret_cast<const ulonglong2*>(&Bi[buf][k][tx * 4]);
+      const F2 b_re[2] = {br.x, br.y}, b_im[2] = {bi.x, bi.y};
+      const F2 b_ni[2] = {fma2(bi.x, minus, 0ull), fma2(bi.y, minus, 0ull)};
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const ulonglong2 a = *reinterpret_cast<const ulonglong2*>(&As[buf][k][ty * 4 + i]);
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          // v_a conj(v_b) = (ar br + ai bi) + i (ai br - ar bi)
+          st_re[i][j] = fma2(a.x, b_re[j], fma2(a.y, b_im[j], st_re[i][j]));
+          st_im[i][j] = fma2(a.y, b_re[j], fma2(a.x, b_ni[j], st_im[i][j]));
+        }
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        acc_re[i][j] = add2(acc_re[i][j], st_re[i][j]);
+        acc_im[i][j] = add2(acc_im[i][j], st_im[i][j]);
+      }
+  }
+  float* pre = partial + (size_t)z * d.p_stride + (size_t)blockIdx.y * 2 * Np * Np +
+               (size_t)(J * kHT + tx * 4) * Np + I * kHT + ty * 4;
+  float* pim = pre + (size_t)Np * Np;
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    *reinterpret_cast<float4*>(pre + (size_t)j * Np) =
+        make_float4(half2(acc_re[0][j >> 1], j & 1), half2(acc_re[1][j >> 1], j & 1),
+                    half2(acc_re[2][j >> 1], j & 1), half2(acc_re[3][j >> 1], j & 1));
+    *reinterpret_cast<float4*>(pim + (size_t)j * Np) =
+        make_float4(half2(acc_im[0][j >> 1], j & 1), half2(acc_im[1][j >> 1], j & 1),
+                    half2(acc_im[2][j >> 1], j & 1), half2(acc_im[3][j >> 1], j & 1));
+  }
+}
+
 __global__ void __launch_bounds__(256)
-herk_plain_kernel(const typename Traits<R>::C* __restrict__ v, const int* __restrict__ count,
-                  int Np, R* __restrict__ partial) {
-  herk_tile<R>(v, *count, Np, partial);
+herk_plain_f64_kernel(const PlainDims d, const double2* __restrict__ v,
+                      double* __restrict__ partial) {
+  const int z = blockIdx.z;
+  herk_tile(v + (size_t)z * d.v_stride, d.counts[z / d.nf], d.Np,
+            partial + (size_t)z * d.p_stride);
 }
 
 __global__ void __launch_bounds__(256)
@@ -181,7 +289,7 @@ herk_flagged_kernel(const F64Dims d, const double2* __restrict__ v,
   const int z = blockIdx.z;
   if (!flags[z]) return;
   const int n = max(0, min(d.counts[z / d.nf] - d.s0, d.S));
-  herk_tile<double>(v + (size_t)z * d.v_stride, n, d.Np, partial + (size_t)z * partial_stride);
+  herk_tile(v + (size_t)z * d.v_stride, n, d.Np, partial + (size_t)z * partial_stride);
 }
 
 cudaError_t launch_herk_flagged(const F64Dims& d, int nz, const void* v, const int* flags,
@@ -194,14 +302,14 @@ cudaError_t launch_herk_flagged(const F64Dims& d, int nz, const void* v, const i
 }
 
 template <typename R>
-cudaError_t launch_herk_plain(const void* v, const int* count, int nsrc_max, int Np,
-                              R* partial, cudaStream_t st) {
-  const int nb = Np / kHT;
-  const int tiles = nb * (nb + 1) / 2;
-  const int chunks = nsrc_max > 0 ? ceil_div(nsrc_max, kPlainChunk) : 1;
-  dim3 grid(tiles, chunks);
-  herk_plain_kernel<R><<<grid, 256, 0, st>>>(
-      reinterpret_cast<const typename Traits<R>::C*>(v), count, Np, partial);
+cudaError_t launch_herk_plain(const PlainDims& d, int nz, const void* v, int nsrc_max, R* partial,
+                              cudaStream_t st) {
+  const int nb = d.Np / kHT;
+  const dim3 grid(nb * (nb + 1) / 2, ceil_div(std::max(nsrc_max, 1), kPlainChunk), nz);
+  if constexpr (sizeof(R) == 4)
+    herk_plain_kernel<<<grid, 256, 0, st>>>(d, static_cast<const float2*>(v), partial);
+  else
+    herk_plain_f64_kernel<<<grid, 256, 0, st>>>(d, static_cast<const double2*>(v), partial);
   return cudaGetLastError();
 }
 
@@ -382,10 +490,10 @@ cudaError_t launch_reduce(const R* partial, size_t slice_stride, const int* coun
   return cudaGetLastError();
 }
 
-template cudaError_t launch_gen_phasors<float>(const void*, const int*, int, const void*, const float*, int, int, int, void*, cudaStream_t);
-template cudaError_t launch_gen_phasors<double>(const void*, const int*, int, const void*, const double*, int, int, int, void*, cudaStream_t);
-template cudaError_t launch_herk_plain<float>(const void*, const int*, int, int, float*, cudaStream_t);
-template cudaError_t launch_herk_plain<double>(const void*, const int*, int, int, double*, cudaStream_t);
+template cudaError_t launch_gen_phasors<float>(const PlainDims&, int, const void*, int, const void*, const float*, int, void*, cudaStream_t);
+template cudaError_t launch_gen_phasors<double>(const PlainDims&, int, const void*, int, const void*, const double*, int, void*, cudaStream_t);
+template cudaError_t launch_herk_plain<float>(const PlainDims&, int, const void*, int, float*, cudaStream_t);
+template cudaError_t launch_herk_plain<double>(const PlainDims&, int, const void*, int, double*, cudaStream_t);
 template cudaError_t launch_reduce<float>(const float*, size_t, const int*, int, int, int, int, int, int, int, int, int, void*, cudaStream_t);
 template cudaError_t launch_reduce<double>(const double*, size_t, const int*, int, int, int, int, int, int, int, int, int, void*, cudaStream_t);
 
