@@ -124,7 +124,8 @@ def sources_up(w, t):
 
 
 def tc_chunk(nsrc, nslices, ngroups, num_sms):
-    """Split-K chunk the library picks (hv_tc.cu tc_chunk_sources)."""
+    """Split-K chunk the library picks (hv_tc.cu tc_chunk_sources) where the
+    items fill the GPU."""
     nchunk = max(1, -(-40 * num_sms // (nslices * ngroups)))
     c = -(-max(nsrc // 2, 1) // nchunk)
     c = min(32768, max(1024, c))

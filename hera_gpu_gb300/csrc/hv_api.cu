@@ -377,7 +377,7 @@ int run_device(hv_context* ctx, int method, const R* antpos, int nant, const dou
       int ntb = ntimes, chunk = 0;
       size_t slice_floats = 0;
       for (;;) {
-        chunk = tc_chunk_sources(S1, ntb * nfreq, ngroups, ctx->num_sms);
+        chunk = tc_chunk_sources(S1, ntb, nfreq, ngroups, tc_block_rows(nant, form), ctx->num_sms);
         slice_floats = tc_partial_floats(Np, S1, 1, chunk);
         const size_t pbytes = sizeof(float) * slice_floats * (size_t)ntb * nfreq;
         const size_t rbytes = sizeof(Rec) * (size_t)ntb * (((size_t)S1 + 31) / 32 * 32);

@@ -264,7 +264,7 @@ cudaError_t launch_tc_batch(const TcSimDesc* sims, int nsims, const void* rec, l
                             int num_sms, cudaStream_t st, unsigned long long wait_ns = 0,
                             int stall = 0, TcShare* share = nullptr);
 size_t tc_partial_floats(int Np, int nsrc, int nslices, int chunk);
-int tc_chunk_sources(int nsrc, int nslices, int ngroups, int num_sms);
+int tc_chunk_sources(int nsrc, int ntimes, int nfreq, int ngroups, int block_rows, int num_sms);
 size_t tc_group_table_bytes(int nant);
 int tc_fill_group_table(int nant, int form, void* host_buf);
 int tc_max_slots(int nant);

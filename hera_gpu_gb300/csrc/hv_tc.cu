@@ -1470,13 +1470,13 @@ int tc_fill_group_table(int nant, int form, void* host_buf) {
   return (int)g.size();
 }
 
-int tc_chunk_sources(int nsrc, int nslices, int ngroups, int num_sms) {
+int tc_chunk_sources(int nsrc, int ntimes, int nfreq, int ngroups, int block_rows, int num_sms) {
   // about 40 items per cluster (or per CTA without clusters), so that the
   // run-time claiming leaves a short tail, in chunks of 1k-32k sources
   // (about half the catalogue is above the horizon)
+  const long long nslices = (long long)ntimes * nfreq;
   const long long nchunk =
-      std::max<long long>(1, (40LL * num_sms + (long long)nslices * ngroups - 1) /
-                                 ((long long)nslices * ngroups));
+      std::max<long long>(1, (40LL * num_sms + nslices * ngroups - 1) / (nslices * ngroups));
   const long long up = std::max(nsrc / 2, 1);
   long long c = (up + nchunk - 1) / nchunk;
   c = std::min<long long>(32768, std::max<long long>(1024, c));
@@ -1485,6 +1485,33 @@ int tc_chunk_sources(int nsrc, int nslices, int ngroups, int num_sms) {
   // 1M sources x 16 slices: 4128 sources took three flushes, 4096 take two)
   const long long unit = c > TC_FLUSH_SOURCES ? TC_FLUSH_SOURCES : 32;
   c = (c + unit / 2) / unit * unit;
+  // Small calls, which leave clusters (or CTAs) without an item at the shortest
+  // of those chunks: the chunk with the shortest span, an item costing its
+  // sources and a part for its partial sums (as many sources as their write and
+  // reduction take; they grow with the block).  Clusters: 11/12 of the SMs (46
+  // of 3 CTAs and 29 of 5 are resident together).  16 antennas x 1000 sources x
+  // 10 slices 82 -> 68 us a call, 64 x 3000 x 4 121 -> 82, 140 x 2000 x 8
+  // 174 -> 104, 200 x 20000 x 1 250 -> 152, 350 x 3000 x 5 220 -> 164; a few
+  // items more than the workers (350 x 100000 x 1) gained nothing from it.
+  //
+  // It is chosen for the slices of one frequency, so that a call of a few
+  // frequencies sums as their single calls do, and taken for them where it
+  // shortens the whole call by a third (350 x 20000 x 2 frequencies, just short
+  // of that: 254 -> 262 us with it, for the partial sums of 90 items).
+  const long long workers =
+      std::max(1, use_cluster(ngroups) ? num_sms * 11 / (12 * ngroups) : num_sms);
+  const long long fixed = use_cluster(ngroups) ? 192 : 32 + block_rows;
+  const long long units = use_cluster(ngroups) ? 1 : ngroups;
+  auto span = [&](long long x, long long slices) {
+    const long long items = slices * units * ((up + x - 1) / x);
+    return (items + workers - 1) / workers * (std::min(x, up) + fixed);
+  };
+  if (c == 1024 && nslices * units * ((up + c - 1) / c) < workers) {
+    long long best = c;
+    for (long long x = c - 32; x >= 64; x -= 32)
+      if (span(x, ntimes) < span(best, ntimes)) best = x;
+    if (nfreq == 1 || 3 * span(best, nslices) < 2 * span(c, nslices)) c = best;
+  }
   return (int)c;
 }
 

@@ -230,3 +230,19 @@ def test_antenna_blocks(nant, method):
         # order 1
         p = np.sqrt(np.einsum("taa->ta", ref.real))
         assert np.abs(v - ref).max() <= 1e-4 * (p[:, :, None] * p[:, None, :]).max()
+
+
+# calls that leave CTAs or clusters idle at the shortest regular chunk take
+# shorter ones: one source, one chunk, a last chunk of a few sources
+@gpu
+@pytest.mark.parametrize("method", ["tc", "tc_fp16"])
+@pytest.mark.parametrize("nant,nsrc,ntimes", [(16, 1, 1), (16, 130, 1), (40, 2047, 7), (200, 257, 1),
+                                              (200, 20000, 1), (350, 3001, 5), (641, 4099, 2)])
+def test_small_call_chunks(nant, nsrc, ntimes, method):
+    args = sim(nant, nsrc, ntimes=ntimes, seed=nsrc)
+    v = vis_gpu(*args, precision=1, method=method)
+    check_hermitian(v)
+    ref = vis_oracle(*[a.astype(np.float64) if isinstance(a, np.ndarray) else a for a in args])
+    up = np.abs(ref).max(axis=(1, 2)) > 0
+    assert rel_frobenius(v[up], ref[up]).max(initial=0) <= 1e-4
+    assert not v[~up].any()
