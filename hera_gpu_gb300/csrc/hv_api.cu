@@ -358,9 +358,12 @@ int run_device(hv_context* ctx, int method, const R* antpos, int nant, const dou
   HV_ENSURE(ctx->ucoef, sizeof(U) * (size_t)ntimes * nfreq * Np);
   HV_ENSURE(ctx->counts, sizeof(int) * (size_t)ntimes);
   R* beamT = static_cast<R*>(ctx->beamT.p);
-  HV_LAUNCH(1, launch_beam_transpose<R>(bm, nfreq, nant, P, Np, beamT, st));
-  HV_LAUNCH(1, launch_ucoef<R>(antpos, nant, Np, eq2tops, 0, ntimes,
-                               static_cast<const double*>(ctx->freqs.p), nfreq, ctx->ucoef.p, st));
+  if (!tc) {  // the fused forms do both, and more, in launch_setup
+    HV_LAUNCH(1, launch_beam_transpose<R>(bm, nfreq, nant, P, Np, beamT, st));
+    HV_LAUNCH(1, launch_ucoef<R>(antpos, nant, Np, eq2tops, 0, ntimes,
+                                 static_cast<const double*>(ctx->freqs.p), nfreq, ctx->ucoef.p,
+                                 st));
+  }
   int* counts = static_cast<int*>(ctx->counts.p);
   const size_t NN = (size_t)nant * nant;
   const int S1 = nsrc > 0 ? nsrc : 1;
@@ -390,8 +393,25 @@ int run_device(hv_context* ctx, int method, const R* antpos, int nant, const dou
       HV_ENSURE(ctx->blkcounts, sizeof(int) * (size_t)prep_blocks(nsrc) * ntb);
       // per-slice bound of |U|_1, and the catalogue in spatial order
       HV_ENSURE(ctx->umax, sizeof(float) * (size_t)ntimes * nfreq);
-      HV_LAUNCH(1, launch_ubound(ctx->ucoef.p, ntimes * nfreq, Np,
-                                 static_cast<float*>(ctx->umax.p), st));
+      const R* crd_use = crd_eq;
+      const R* I_use = I_sky;
+      if (nsrc > 0) {
+        HV_ENSURE(ctx->sortkv, sizeof(unsigned long long) * (size_t)nsrc);
+        HV_ENSURE(ctx->crd_sorted, sizeof(float) * 3 * (size_t)nsrc);
+        HV_ENSURE(ctx->I_sorted, sizeof(float) * (size_t)nsrc);
+        crd_use = static_cast<const R*>(ctx->crd_sorted.p);
+        I_use = static_cast<const R*>(ctx->I_sorted.p);
+      }
+      float* crd_s = static_cast<float*>(ctx->crd_sorted.p);
+      float* I_s = static_cast<float*>(ctx->I_sorted.p);
+      HV_LAUNCH(1, launch_setup(reinterpret_cast<const float*>(bm), nfreq, nant, P, Np,
+                                reinterpret_cast<float*>(beamT),
+                                reinterpret_cast<const float*>(antpos),
+                                reinterpret_cast<const float*>(eq2tops), ntimes,
+                                static_cast<const double*>(ctx->freqs.p), ctx->ucoef.p,
+                                static_cast<float*>(ctx->umax.p),
+                                reinterpret_cast<const float*>(crd_eq),
+                                reinterpret_cast<const float*>(I_sky), nsrc, crd_s, I_s, st));
       // FP16 + FP8 form: the beam's largest value per pixel, for the slices'
       // scales
       if (form == 1) {
@@ -400,12 +420,7 @@ int run_device(hv_context* ctx, int method, const R* antpos, int nant, const dou
         HV_LAUNCH(1, launch_beam_pixmax(reinterpret_cast<const float*>(beamT), nfreq, P, Np,
                                         static_cast<float*>(ctx->pixmax.p), st));
       }
-      const R* crd_use = crd_eq;
-      const R* I_use = I_sky;
-      if (nsrc > 0) {
-        HV_ENSURE(ctx->sortkv, sizeof(unsigned long long) * (size_t)nsrc);
-        HV_ENSURE(ctx->crd_sorted, sizeof(float) * 3 * (size_t)nsrc);
-        HV_ENSURE(ctx->I_sorted, sizeof(float) * (size_t)nsrc);
+      if (sort_table_bytes(nsrc) > 0) {
         // the sort's digit tables (half a byte a source) use the partial sums'
         // buffer (at least 4 bytes a source and 128 KB), not yet in use
         if (sort_table_bytes(nsrc) > ctx->partial.cap)
@@ -413,12 +428,8 @@ int run_device(hv_context* ctx, int method, const R* antpos, int nant, const dou
         int nl = 0;
         HV_CK(launch_sort_sources(reinterpret_cast<const float*>(crd_eq),
                                   reinterpret_cast<const float*>(I_sky), nsrc, ctx->sortkv.p,
-                                  ctx->partial.p,
-                                  static_cast<float*>(ctx->crd_sorted.p),
-                                  static_cast<float*>(ctx->I_sorted.p), &nl, st));
+                                  ctx->partial.p, crd_s, I_s, &nl, st));
         ctx->launches += nl;
-        crd_use = static_cast<const R*>(ctx->crd_sorted.p);
-        I_use = static_cast<const R*>(ctx->I_sorted.p);
       }
       for (int t0 = 0; t0 < ntimes; t0 += ntb) {
         const int nt = std::min(ntb, ntimes - t0);

@@ -59,8 +59,7 @@ struct PrepTotals {
 cudaError_t launch_prepare_batch(const PrepSim* sims, int nsims, const PrepPre& pre,
                                  const PrepTotals& tot, int* launches, cudaStream_t st);
 // The spatial sort of every simulation of a batch (hv_sort.cu): each one's
-// keys are sorted within its own segment, exactly as launch_sort_sources
-// sorts them alone.
+// keys are sorted within its own segment, exactly as they are sorted alone.
 cudaError_t launch_sort_batch(const PrepSim* sims, int nsims, const PrepPre& pre,
                               const PrepTotals& tot, int* launches, cudaStream_t st);
 // The split-K reduction of every simulation of a batch into its output.
@@ -91,15 +90,22 @@ cudaError_t launch_prep(const R* crd_eq, const R* I_sky, int nsrc, const R* eq2t
                         int t0, int nt, int P, int* block_counts, void* rec,
                         int* count, cudaStream_t st);
 
-// Bound max_a (|U_x| + |U_y| + |U_z|) of every (time, frequency) slice of U
-// (nslices x Np Ucoef32) into umax[nslices] (used by the fused kernel to
-// decide when a phase may be taken relative to a nearby source).
-cudaError_t launch_ubound(const void* U, int nslices, int Np, float* umax, cudaStream_t st);
+// The setup of a fused-form call, in one launch: beamT as
+// launch_beam_transpose, U as launch_ucoef (times [0, ntimes)), the bound
+// max_a (|U_x| + |U_y| + |U_z|) of every (time, frequency) slice into umax (the
+// fused kernel decides by it when a phase may be taken relative to a nearby
+// source), and, for a catalogue without sort tables (sort_table_bytes is 0),
+// its spatial order into crd_s and I_s.
+cudaError_t launch_setup(const float* bm, int nfreq, int nant, int P, int Np, float* beamT,
+                         const float* antpos, const float* eq2tops, int ntimes,
+                         const double* d_freqs, void* U, float* umax, const float* crd_eq,
+                         const float* I, int nsrc, float* crd_s, float* I_s, cudaStream_t st);
 
 // --- hv_sort.cu ------------------------------------------------------------
 // Spatial (Morton) order of the sources: kv_buf needs nsrc 64-bit words and
 // table_buf sort_table_bytes(nsrc); writes the permuted crd_eq (3 x nsrc, at
 // an 8-byte aligned address: it holds sort words in between) and I_sky.
+// Catalogues without tables (sort_table_bytes 0) are ordered by launch_setup.
 // *launches is set to the number of kernels launched.
 size_t sort_table_bytes(int nsrc);
 cudaError_t launch_sort_sources(const float* crd_eq, const float* I_sky, int nsrc, void* kv_buf,
@@ -220,7 +226,7 @@ struct TcSimDesc {
   const int* counts;    // [nt] sources above the horizon per time
   const void* U;        // Ucoef32 [nt][nf][Np]
   const float* beamT;   // [nf][P*P][Np]
-  const float* umax;    // [nt * nf] bound of |U|_1 per slice (launch_ubound)
+  const float* umax;    // [nt * nf] bound of |U|_1 per slice (launch_setup)
   const float* sbound;  // [nt * nf] bound of |A| sqrt(I) per slice (form 1; launch_slice_bound)
   float* partial;       // [nt * nf][ceil(nsrc / chunk)][2][Np][Np]
   const void* groups;   // device group table (tc_fill_group_table for this nant)

@@ -19,25 +19,28 @@
 
 #include "hv_internal.cuh"
 #include "hv_kernels.h"
+#include "hv_spatial.cuh"
 
 namespace hv {
 
 // ---------------------------------------------------------------- beam ----
-// One 32 x 32 (pixel, antenna) tile of frequency f (block 32 x 8 threads).
+// One 32 x 32 (pixel, antenna) tile of frequency f, by rows of 32 threads
+// (thread tx of row ty of ny).
 template <typename R>
 __device__ __forceinline__ void beam_transpose_tile(const R* __restrict__ bm, int nant, int PP,
                                                     int Np, R* __restrict__ beamT, int f,
-                                                    int pix0, int a0, R (*tile)[33]) {
+                                                    int pix0, int a0, R (*tile)[33], int tx,
+                                                    int ty, int ny) {
   const R* src = bm + (size_t)f * nant * PP;
   R* dst = beamT + (size_t)f * PP * Np;
-  for (int j = threadIdx.y; j < 32; j += blockDim.y) {
-    const int a = a0 + j, pix = pix0 + threadIdx.x;
-    tile[j][threadIdx.x] = (a < nant && pix < PP) ? src[(size_t)a * PP + pix] : R(0);
+  for (int j = ty; j < 32; j += ny) {
+    const int a = a0 + j, pix = pix0 + tx;
+    tile[j][tx] = (a < nant && pix < PP) ? src[(size_t)a * PP + pix] : R(0);
   }
   __syncthreads();
-  for (int j = threadIdx.y; j < 32; j += blockDim.y) {
-    const int pix = pix0 + j, a = a0 + threadIdx.x;
-    if (pix < PP && a < Np) dst[(size_t)pix * Np + a] = tile[threadIdx.x][j];
+  for (int j = ty; j < 32; j += ny) {
+    const int pix = pix0 + j, a = a0 + tx;
+    if (pix < PP && a < Np) dst[(size_t)pix * Np + a] = tile[tx][j];
   }
 }
 
@@ -46,7 +49,7 @@ __global__ void beam_transpose_kernel(const R* __restrict__ bm, int nant, int PP
                                       R* __restrict__ beamT) {
   __shared__ R tile[32][33];
   beam_transpose_tile<R>(bm, nant, PP, Np, beamT, blockIdx.z, blockIdx.x * 32, blockIdx.y * 32,
-                         tile);
+                         tile, threadIdx.x, threadIdx.y, blockDim.y);
 }
 
 template <typename R>
@@ -140,14 +143,77 @@ __device__ __forceinline__ void ubound_slice(const Ucoef32* __restrict__ u, int 
   }
 }
 
+// --------------------------------------------------------------- setup ----
+// What a call of the fused forms does before its first time, in one launch of
+// blocks with different parts.  The parts are independent, and each alone is
+// mostly its launch: for 16 antennas x 1000 sources x 10 times (ncu) 6.4 us
+// together, against 3.2 (beam), 4.9 + 3.3 (coefficients and bound) and 12.7
+// (order, a radix sort by one block); 32 antennas x 5000 sources x 6 slices
+// took 138 us a call, now 71, and 512 x 3072 x 10 from the host 474, now 444.
+//   blocks [0, nsort)     the spatial order of a small catalogue (kSort)
+//   the next nslices      a slice's phase coefficients and their bound
+//   the rest              tiles of the beam transpose
+struct SetupDims {
+  int nant, Np, nfreq, nslices, PP;
+  int nsort, nsrc;
+  int tiles_x, tiles_y;  // tiles along the pixels and the antennas
+};
+
+template <bool kSort>
 __global__ void __launch_bounds__(256)
-ubound_kernel(const Ucoef32* __restrict__ U, int Np, float* __restrict__ umax) {
-  __shared__ float red[8];
-  ubound_slice(U + (size_t)blockIdx.x * Np, Np, umax + blockIdx.x, red);
+setup_kernel(const SetupDims d, const float* __restrict__ bm, float* __restrict__ beamT,
+             const float* __restrict__ antpos, const float* __restrict__ eq2tops,
+             const double* __restrict__ freqs, Ucoef32* __restrict__ U, float* __restrict__ umax,
+             const float* __restrict__ crd_eq, const float* __restrict__ I,
+             float* __restrict__ crd_s, float* __restrict__ I_s) {
+  static_assert(kRankThreads == 256, "one block size for every part");
+  constexpr int kBytes = kSort ? 4 * kRankSort : 32 * 33 * 4;
+  __shared__ __align__(16) uint8_t smem[kBytes];
+  int b = blockIdx.x;
+  if (b < d.nsort) {
+    if constexpr (kSort)
+      rank_sort_block(crd_eq, I, d.nsrc, crd_s, I_s, b, reinterpret_cast<uint32_t*>(smem));
+    return;
+  }
+  b -= d.nsort;
+  if (b < d.nslices) {
+    const size_t i0 = (size_t)b * d.Np;
+    for (int a = threadIdx.x; a < d.Np; a += 256)
+      ucoef_element<float>(antpos, d.nant, d.Np, eq2tops, 0, freqs, d.nfreq, U, i0 + a);
+    // (a thread reads what it wrote)
+    ubound_slice(U + i0, d.Np, umax + b, reinterpret_cast<float*>(smem));
+    return;
+  }
+  b -= d.nslices;
+  const int x = b % d.tiles_x, y = b / d.tiles_x % d.tiles_y, f = b / d.tiles_x / d.tiles_y;
+  beam_transpose_tile<float>(bm, d.nant, d.PP, d.Np, beamT, f, x * 32, y * 32,
+                             reinterpret_cast<float(*)[33]>(smem), threadIdx.x & 31,
+                             threadIdx.x >> 5, 8);
 }
 
-cudaError_t launch_ubound(const void* U, int nslices, int Np, float* umax, cudaStream_t st) {
-  ubound_kernel<<<nslices, 256, 0, st>>>(static_cast<const Ucoef32*>(U), Np, umax);
+cudaError_t launch_setup(const float* bm, int nfreq, int nant, int P, int Np, float* beamT,
+                         const float* antpos, const float* eq2tops, int ntimes,
+                         const double* d_freqs, void* U, float* umax, const float* crd_eq,
+                         const float* I, int nsrc, float* crd_s, float* I_s, cudaStream_t st) {
+  SetupDims d{};
+  d.nant = nant;
+  d.Np = Np;
+  d.nfreq = nfreq;
+  d.nslices = ntimes * nfreq;
+  d.PP = P * P;
+  d.nsort = nsrc <= kRankSort ? ceil_div(nsrc, kRankSources) : 0;
+  d.nsrc = nsrc;
+  d.tiles_x = ceil_div(d.PP, 32);
+  d.tiles_y = Np / 32;
+  const long long blocks = (long long)d.nsort + d.nslices + (long long)d.tiles_x * d.tiles_y * nfreq;
+  if (blocks > 0x7fffffffLL) return cudaErrorInvalidValue;
+  Ucoef32* u = static_cast<Ucoef32*>(U);
+  if (d.nsort)
+    setup_kernel<true><<<(int)blocks, 256, 0, st>>>(d, bm, beamT, antpos, eq2tops, d_freqs, u,
+                                                    umax, crd_eq, I, crd_s, I_s);
+  else
+    setup_kernel<false><<<(int)blocks, 256, 0, st>>>(d, bm, beamT, antpos, eq2tops, d_freqs, u,
+                                                     umax, crd_eq, I, crd_s, I_s);
   return cudaGetLastError();
 }
 
@@ -650,7 +716,7 @@ beam_transpose_batch_kernel(const PrepSim* __restrict__ sims, int nsims,
   const int f = (int)(local / ((long long)tx * ty));
   const int rem = (int)(local % ((long long)tx * ty));
   beam_transpose_tile<float>(sm.bm, sm.nant, PP, sm.Np, sm.beamT, f, (rem % tx) * 32,
-                             (rem / tx) * 32, tile);
+                             (rem / tx) * 32, tile, threadIdx.x, threadIdx.y, blockDim.y);
 }
 
 __global__ void __launch_bounds__(256)

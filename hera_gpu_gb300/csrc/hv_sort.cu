@@ -7,63 +7,29 @@
 // reference source.  Rotation to topocentric is an isometry, so an order
 // that is local on the equatorial sphere stays local at every time.
 //
-// Key: Morton code (16 bits per axis) of the octahedral projection of the
-// unit vector.  Sort: by the words (key << 32 | index) -- a total order, so
+// Sort: by the words (key << 32 | index) of hv_spatial.cuh -- a total order, so
 // the permutation (and every result downstream) is deterministic -- with a
-// radix sort for one catalogue and a segmented bitonic network for a batch.
+// radix sort for one catalogue (one of at most kRankSort sources is ordered by
+// counting, among the call's setup) and a segmented bitonic network for a
+// batch.
 #include <algorithm>
 #include <utility>
 
 #include "hv_internal.cuh"
 #include "hv_kernels.h"
+#include "hv_spatial.cuh"
 
 namespace hv {
-
-__device__ __forceinline__ uint32_t spread16(uint32_t a) {
-  a = (a | (a << 8)) & 0x00FF00FFu;
-  a = (a | (a << 4)) & 0x0F0F0F0Fu;
-  a = (a | (a << 2)) & 0x33333333u;
-  a = (a | (a << 1)) & 0x55555555u;
-  return a;
-}
-
-// Sort word of source i: (Morton key << 32) | i, or all ones for padding.
-__device__ __forceinline__ unsigned long long sort_word(const float* __restrict__ crd_eq,
-                                                        int nsrc, int i) {
-  unsigned long long v = ~0ull;
-  {
-    if (i < nsrc) {
-      const float x = crd_eq[i], y = crd_eq[(size_t)nsrc + i], z = crd_eq[2 * (size_t)nsrc + i];
-      const float n = fabsf(x) + fabsf(y) + fabsf(z);
-      float u = n > 0.f ? x / n : 0.f, w = n > 0.f ? y / n : 0.f;
-      if (z < 0.f) {
-        const float uu = (1.f - fabsf(w)) * (u < 0.f ? -1.f : 1.f);
-        const float ww = (1.f - fabsf(u)) * (w < 0.f ? -1.f : 1.f);
-        u = uu;
-        w = ww;
-      }
-      // NaN-safe quantisation to [0, 65535]
-      const float qu = fminf(fmaxf((u + 1.f) * 32767.5f, 0.f), 65535.f);
-      const float qw = fminf(fmaxf((w + 1.f) * 32767.5f, 0.f), 65535.f);
-      const uint32_t key = spread16((uint32_t)qu) | (spread16((uint32_t)qw) << 1);
-      v = ((unsigned long long)key << 32) | (uint32_t)i;
-    }
-  }
-  return v;
-}
 
 // -------------------------------------------------------- single call ----
 // Least-significant-digit radix sort of the words by key, four stable passes
 // of 8 bits, so that equal keys keep their index order: the order of the
 // (key, index) words.  It is bound by launches and latency (a 1M-source
 // catalogue is 8 MB).  Measured on GB300 under ncu, gather included: 139 us
-// at 1M sources (12 launches), 71 us at 100k; 12.7 us at 1000 by one block.
-// A bitonic network of the words took 444 us (57 launches), 138 us and 28 us.
+// at 1M sources (12 launches), 71 us at 100k.  A bitonic network of the words
+// took 444 us (57 launches) and 138 us.
 constexpr int kRadixTile = 2048;   // words a block, 8 a thread
 constexpr int kRadixThreads = 256;
-// Up to this many sources one block sorts in shared memory, in one launch.
-constexpr int kSmallSort = 4096;
-constexpr int kSmallThreads = 512;
 
 // Stable ranks within a warp's row of 32 digits: the lanes of the same digit
 // (match) take consecutive ranks from the warp's counter of that digit.
@@ -199,89 +165,14 @@ radix_scatter_kernel(const unsigned long long* __restrict__ src, int n, int shif
   }
 }
 
-// Catalogues of up to kSmallSort sources: the same passes by one block, the
-// words in registers between exchanges through shared memory.
-__global__ void __launch_bounds__(kSmallThreads)
-small_sort_kernel(const float* __restrict__ crd_eq, const float* __restrict__ I, int n,
-                  float* __restrict__ crd_s, float* __restrict__ I_s) {
-  constexpr int W = kSmallThreads / 32, R = kSmallSort / kSmallThreads;
-  __shared__ unsigned long long buf[kSmallSort];
-  __shared__ unsigned short cnt[W][256];
-  __shared__ int ws[8];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int rows = ceil_div(n, kSmallThreads);  // rows of 32 words a warp
-  const int base = warp * 32 * rows + lane;
-  unsigned long long w[R];
-  int rank[R];
-#pragma unroll
-  for (int r = 0; r < R; ++r) w[r] = r < rows ? sort_word(crd_eq, n, base + r * 32) : ~0ull;
-#pragma unroll 1
-  for (int shift = 32; shift < 64; shift += 8) {
-    for (int i = threadIdx.x; i < W * 128; i += kSmallThreads)
-      reinterpret_cast<uint32_t*>(&cnt[0][0])[i] = 0;
-    __syncthreads();
-    // padding words (all ones) come after every source: they rank as digit
-    // 255, and passes are stable
-#pragma unroll
-    for (int r = 0; r < R; ++r)
-      if (r < rows) {
-        const int d = (int)(w[r] >> shift) & 255;
-        const unsigned peers = __match_any_sync(0xffffffffu, d);
-        const int leader = __ffs(peers) - 1;
-        int b = 0;
-        if (lane == leader) {
-          b = cnt[warp][d];
-          cnt[warp][d] = (unsigned short)(b + __popc(peers));
-        }
-        __syncwarp();
-        rank[r] = __shfl_sync(0xffffffffu, b, leader) + __popc(peers & ((1u << lane) - 1u));
-      }
-    __syncthreads();
-    int tot = 0;
-    if (threadIdx.x < 256)
-      for (int k = 0; k < W; ++k) tot += cnt[k][threadIdx.x];
-    int run = prefix256(tot, ws);
-    if (threadIdx.x < 256)
-      for (int k = 0; k < W; ++k) {
-        const int c = cnt[k][threadIdx.x];
-        cnt[k][threadIdx.x] = (unsigned short)run;
-        run += c;
-      }
-    __syncthreads();
-#pragma unroll
-    for (int r = 0; r < R; ++r)
-      if (r < rows) buf[cnt[warp][(int)(w[r] >> shift) & 255] + rank[r]] = w[r];
-    __syncthreads();
-#pragma unroll
-    for (int r = 0; r < R; ++r)
-      if (r < rows) w[r] = buf[base + r * 32];
-    __syncthreads();
-  }
-#pragma unroll
-  for (int r = 0; r < R; ++r) {
-    const int pos = base + r * 32;
-    if (r >= rows || pos >= n) continue;
-    const uint32_t i = (uint32_t)w[r];
-    crd_s[pos] = crd_eq[i];
-    crd_s[(size_t)n + pos] = crd_eq[(size_t)n + i];
-    crd_s[2 * (size_t)n + pos] = crd_eq[2 * (size_t)n + i];
-    I_s[pos] = I[i];
-  }
-}
-
 size_t sort_table_bytes(int nsrc) {
-  return nsrc <= kSmallSort ? 0
+  return nsrc <= kRankSort ? 0
                             : sizeof(int) * 256 * ((size_t)ceil_div(nsrc, kRadixTile) + 1);
 }
 
 cudaError_t launch_sort_sources(const float* crd_eq, const float* I_sky, int nsrc, void* kv_buf,
                                 void* table_buf, float* crd_sorted, float* I_sorted,
                                 int* launches, cudaStream_t st) {
-  if (nsrc <= kSmallSort) {
-    small_sort_kernel<<<1, kSmallThreads, 0, st>>>(crd_eq, I_sky, nsrc, crd_sorted, I_sorted);
-    if (launches) *launches = 1;
-    return cudaGetLastError();
-  }
   // the words go back and forth between crd_sorted (12 bytes a source, not
   // written as such before the last pass, which reads kv) and kv
   auto* a = reinterpret_cast<unsigned long long*>(crd_sorted);
@@ -314,7 +205,7 @@ constexpr int kSortTile = 2048;  // elements sorted in shared memory per block
 // Every simulation of a batch sorted in one set of launches: simulation s
 // owns a segment of sort_pad(S_s) words (its own kv buffer), and each pass
 // of a bitonic network runs within every segment long enough for it, so a
-// simulation's order is exactly the one launch_sort_sources gives it alone.
+// simulation's order is exactly the one it gets alone.
 __global__ void sort_keys_batch_kernel(const PrepSim* __restrict__ sims, int nsims,
                                        const long long* __restrict__ pre, long long total) {
   for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < total;
