@@ -307,7 +307,7 @@ int run_f64(hv_context* ctx, const double* eq2tops, const double* crd_eq, const 
   d.w_stride = b_w / sizeof(long long);
   for (int t0 = 0; t0 < ntimes; t0 += ntb) {
     const int nt = std::min(ntb, ntimes - t0);
-    HV_LAUNCH(2, launch_prep_strided<double>(crd_eq, I_sky, nsrc, eq2tops, t0, nt, P,
+    HV_LAUNCH(prep_launches(nsrc), launch_prep_strided<double>(crd_eq, I_sky, nsrc, eq2tops, t0, nt, P,
                                              static_cast<int*>(ctx->blkcounts.p), ctx->rec.p,
                                              (size_t)S1, counts + t0, st));
     d.counts = counts + t0;
@@ -433,10 +433,11 @@ int run_device(hv_context* ctx, int method, const R* antpos, int nant, const dou
       }
       for (int t0 = 0; t0 < ntimes; t0 += ntb) {
         const int nt = std::min(ntb, ntimes - t0);
-        HV_LAUNCH(2, launch_prep_strided<R>(crd_use, I_use, nsrc, eq2tops, t0, nt, P,
+        HV_LAUNCH(prep_launches(nsrc), launch_prep_strided<R>(crd_use, I_use, nsrc, eq2tops, t0, nt, P,
                                             static_cast<int*>(ctx->blkcounts.p), ctx->rec.p,
                                             rec_stride, counts + t0, st));
-        HV_LAUNCH(1, launch_tc_relative(ctx->rec.p, rec_stride, counts + t0, nt, nsrc, st));
+        HV_LAUNCH(1, launch_tc_relative(ctx->rec.p, rec_stride, counts + t0, nt, nsrc, ctx->d_claim,
+                                        st));
         float* sbound = nullptr;
         if (form == 1) {
           sbound = static_cast<float*>(ctx->sbound.p) + (size_t)t0 * nfreq;
@@ -446,6 +447,7 @@ int run_device(hv_context* ctx, int method, const R* antpos, int nant, const dou
         }
         TcSimDesc L{};
         L.sbound = sbound;
+        L.claim_zeroed = true;
         L.form = form;
         L.tune = ctx->tune;
         L.counts = counts + t0;
@@ -523,7 +525,7 @@ int run_device(hv_context* ctx, int method, const R* antpos, int nant, const dou
   d.p_stride = (size_t)chunks * 2 * Np * Np;
   for (int t0 = 0; t0 < ntimes; t0 += ntb) {
     const int nt = std::min(ntb, ntimes - t0);
-    HV_LAUNCH(2, launch_prep_strided<R>(crd_eq, I_sky, nsrc, eq2tops, t0, nt, P,
+    HV_LAUNCH(prep_launches(nsrc), launch_prep_strided<R>(crd_eq, I_sky, nsrc, eq2tops, t0, nt, P,
                                         static_cast<int*>(ctx->blkcounts.p), ctx->rec.p,
                                         (size_t)S1, counts + t0, st));
     d.counts = counts + t0;

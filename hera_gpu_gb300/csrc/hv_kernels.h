@@ -79,8 +79,9 @@ cudaError_t launch_ucoef(const R* antpos, int nant, int Np, const R* eq2tops, in
                          int nt, const double* d_freqs, int nfreq, void* U,
                          cudaStream_t st);
 
-// Number of prep blocks for nsrc sources.
+// Number of prep blocks for nsrc sources, and launches of launch_prep.
 int prep_blocks(int nsrc);
+int prep_launches(int nsrc);
 
 // Horizon cut + beam corner for times [t0, t0 + nt): records of the sources
 // with z > 0, in input order, into rec + tt * nsrc; counts into count[tt].
@@ -122,9 +123,10 @@ cudaError_t launch_prep_strided(const R* crd_eq, const R* I_sky, int nsrc, const
 
 // Fused-path record preparation (hv_prep.cu): per-unit spread of directions
 // in the pad word of each unit's first record, zero padding to a multiple of
-// 32 (rec_stride >= round_up(nsrc, 32)).
+// 32 (rec_stride >= round_up(nsrc, 32)); the item counter of the fused launch
+// that follows is set to zero along with it.
 cudaError_t launch_tc_relative(void* rec, size_t rec_stride, const int* counts, int nt, int nsrc,
-                               cudaStream_t st);
+                               unsigned long long* claim, cudaStream_t st);
 
 // FP16 + FP8 form: pixmax[f][pix] = max over antennas of |beamT[f][pix][a]|
 // (nfreq * P * P floats).
@@ -237,6 +239,7 @@ struct TcSimDesc {
   int chunk;            // sources per split-K chunk (multiple of 32)
   int form;             // 0: split BF16; 1: FP16 + FP8 (needs sbound)
   TcTune tune;          // launch shape (the first simulation's applies to a launch)
+  bool claim_zeroed;    // launch_tc_relative, ahead in the stream, zeroed the claim counter
 };
 size_t tc_sim_table_bytes(int nsims);
 int tc_num_groups(int nant);

@@ -1608,8 +1608,10 @@ cudaError_t launch_form(const TcSimDesc* sims, int nsims, const void* rec, long 
   }
 
   // the claim counter starts at zero (in stream order, before the launches)
-  e = cudaMemsetAsync(claim, 0, sizeof(unsigned long long), st);
-  if (e != cudaSuccess) return e;
+  if (!sims[0].claim_zeroed) {
+    e = cudaMemsetAsync(claim, 0, sizeof(unsigned long long), st);
+    if (e != cudaSuccess) return e;
+  }
   TcParams p{};
   p.claim = claim;
   p.claim_mode = kClaimCount;

@@ -246,3 +246,18 @@ def test_small_call_chunks(nant, nsrc, ntimes, method):
     up = np.abs(ref).max(axis=(1, 2)) > 0
     assert rel_frobenius(v[up], ref[up]).max(initial=0) <= 1e-4
     assert not v[~up].any()
+
+
+# order of the records: by counting (one pixel, a few, a box of hundreds) and
+# by sorting (a box beyond 512 pixels); blocks of 1024 sources that form the
+# counts before them (up to 4096 sources) and that read them.  A lost or
+# doubled source is of order 1 / sqrt(nsrc) >= 1e-2, far above the tolerance
+@gpu
+@pytest.mark.parametrize("P", [2, 15, 63, 301])
+@pytest.mark.parametrize("nsrc", [31, 1023, 1025, 4096, 4097, 8193])
+def test_record_order(nsrc, P):
+    args = sim(4, nsrc, ntimes=2, P=P, seed=nsrc + P)
+    v = vis_gpu(*args, precision=1, method="tc")
+    check_hermitian(v)
+    ref = vis_oracle(*[a.astype(np.float64) if isinstance(a, np.ndarray) else a for a in args])
+    assert rel_frobenius(v, ref).max() <= 1e-4
