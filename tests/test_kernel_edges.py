@@ -261,3 +261,18 @@ def test_record_order(nsrc, P):
     check_hermitian(v)
     ref = vis_oracle(*[a.astype(np.float64) if isinstance(a, np.ndarray) else a for a in args])
     assert rel_frobenius(v, ref).max() <= 1e-4
+
+
+# host calls around the limits of page-locked staging (512 KB of inputs, 64 KB
+# of output: 90 antennas), small and large ones in turn through one context
+@gpu
+def test_host_calls_staged_and_not():
+    cases = [sim(nant, nsrc, seed=nsrc) for nant, nsrc in
+             [(90, 1000), (91, 27000), (90, 26000), (91, 1000), (8, 40000), (8, 1)]]
+    first = [vis_gpu(*a, precision=1, method="tc") for a in cases]
+    for a, v in zip(cases, first):
+        ref = vis_oracle(*[x.astype(np.float64) if isinstance(x, np.ndarray) else x for x in a])
+        if ref.any():
+            assert rel_frobenius(v, ref).max() <= 1e-4
+    for a, v in zip(cases[::-1], first[::-1]):
+        np.testing.assert_array_equal(vis_gpu(*a, precision=1, method="tc"), v)
