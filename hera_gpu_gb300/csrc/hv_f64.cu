@@ -21,14 +21,15 @@
 //     classes a word, added with integer reductions: exact and independent of
 //     order), and are converted once, smallest class first, in FP64.
 // The result is deterministic, and its distance from an exact evaluation is
-// set by the rounding of the FP64 phases: relative Frobenius errors against
-// 113-bit arithmetic of 3.9e-15 at 16 antennas x 1000 sources (SIMT product
-// 4.0e-15), 6.8e-15 at 40 x 2000 (6.9e-15), and 2.4e-16 on a 2.5 m array, where
-// the phases are exact enough to show the product (1.1e-15).
+// set by the rounding of U (the phases themselves are formed in integers):
+// relative Frobenius errors against 113-bit arithmetic of 3.6e-15 at 16
+// antennas x 1000 sources (SIMT product 4.0e-15), 5.5e-15 at 40 x 2000
+// (6.9e-15), and 2.2e-16 on a 2.5 m array, where the phases are exact enough to
+// show the product (1.1e-15).
 //
 // Measured on GB300, one slice of 350 antennas x 50k sources above the horizon
-// (ncu): phasors 0.80 ms, digits 0.24 ms, class sums 0.93 ms, conversion 0.02
-// ms; with SIMT 1.30 ms and 32.8 ms.  A call of 3 such slices 102.6 -> 5.44 ms.
+// (ncu): phasors 0.33 ms, digits 0.25 ms, class sums 0.92 ms, conversion 0.02
+// ms; with SIMT 1.30 ms and 32.8 ms.  A call of 3 such slices 102.6 -> 4.12 ms.
 //
 // Slices whose phasors are not finite, or whose antenna scales leave
 // [2^-400, 2^400], are flagged on the device and take the SIMT product of
@@ -63,38 +64,104 @@ __device__ __forceinline__ int window_count(const F64Dims& d, int z) {
 }
 
 // --------------------------------------------------------------- gen64 ----
-__global__ void sincos_table_kernel(double2* __restrict__ tab) {
+constexpr long long kTwoPi = 7244019458077122842ll;  // 2 pi 2^60
+
+// cos and sin of the multiples of 1/1024 cycle, in units of 2^-62 and within a
+// few of them: Taylor series up to pi / 4 in integers, and symmetry.
+__global__ void sincos_table_kernel(longlong2* __restrict__ tab) {
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k < kTable) {
-    double s, c;
-    sincospi(k * (2.0 / kTable), &s, &c);
-    tab[k] = make_double2(c, s);
+  if (k >= kTable) return;
+  static_assert(kTable == 1024, "quadrants of 256");
+  const int m = k & 255, j = m > 128 ? 256 - m : m;
+  auto mul = [](long long a, long long b) { return (long long)((__int128)a * b >> 62); };
+  const long long th = (long long)((__int128)kTwoPi * j >> 8);  // 2 pi j / 1024
+  const long long t2 = mul(th, th);
+  long long c = 1ll << 62, s = th, tc = c, ts = th;
+  for (int i = 1; i <= 10; ++i) {
+    tc = -mul(tc, t2) / ((2 * i - 1) * (2 * i));
+    ts = -mul(ts, t2) / (2 * i * (2 * i + 1));
+    c += tc;
+    s += ts;
   }
+  const long long x = m > 128 ? s : c, y = m > 128 ? c : s;  // first quadrant
+  const int q = k >> 8;
+  tab[k] = q == 0   ? make_longlong2(x, y)
+           : q == 1 ? make_longlong2(-y, x)
+           : q == 2 ? make_longlong2(-x, -y)
+                    : make_longlong2(y, -x);
+}
+
+// Smallest E >= 0 with every |component| < 2^E (above 1000 if one is not
+// finite), and a component in units of 2^(E - 62).
+__device__ __forceinline__ int fixed_exponent(double x, double y, double z) {
+  const int m = max(__double2hiint(x) & 0x7fffffff,
+                    max(__double2hiint(y) & 0x7fffffff, __double2hiint(z) & 0x7fffffff));
+  return max(0, (m >> 20) - 1022);
+}
+__device__ __forceinline__ long long to_fixed(double x, int E) {
+  return __double2ll_rn(x * __hiloint2double((1023 + 62 - E) << 20, 0));
+}
+
+// cos and sin, in units of 2^-62, of a phase in units of 2^-64 cycle: its
+// nearest multiple of 1/1024 cycle from the table, the rest r (|r| <= 2^-11
+// cycles) by the Taylor series in theta = 2 pi r up to theta^5, whose first
+// dropped terms are below 2e-18, and the addition theorem.  Every product
+// keeps an error below 2^-58.
+__device__ __forceinline__ void sincos_fixed(unsigned long long ph,
+                                             const longlong2* __restrict__ tab, long long& cs,
+                                             long long& sn) {
+  const uint32_t k = (uint32_t)((ph + (1ull << 53)) >> 54);  // mod 1024
+  const long long r = (long long)(ph - ((unsigned long long)k << 54));
+  const longlong2 t = tab[k];
+  const long long th = __mul64hi(r << 9, kTwoPi);               // theta 2^69
+  const unsigned long long h = (unsigned long long)__mul64hi(th, th);  // theta^2 2^74
+  const uint32_t hq = (uint32_t)(h >> 26);                      // theta^2 2^48
+  const uint32_t q4 = __umulhi(hq, hq);                         // theta^4 2^64
+  // theta^2 / 6 - theta^4 / 120, 2^50
+  const int w = (int)(__umulhi(hq, 2863311531u) - __umulhi(q4, 2185u));
+  // sin theta 2^64 and (1 - cos theta) 2^64 (in this sign: nvcc 13.0 makes
+  // -2^32 of the difference 0 - 0 the other way round)
+  const long long sr = (th >> 5) - (((long long)(int)(th >> 30) * w) >> 25);
+  const long long cr = (long long)((h >> 11) - __umulhi(q4, 178956971u));
+  const long long s7 = sr << 7, c16 = cr << 16;
+  cs = t.x - (__mul64hi(t.x, c16) >> 16) - (__mul64hi(t.y, s7) >> 7);
+  sn = t.y - (__mul64hi(t.y, c16) >> 16) + (__mul64hi(t.x, s7) >> 7);
+}
+// x 2^-62, rounded once.
+__device__ __forceinline__ double from_fixed62(long long x) {
+  const double d = (double)x;
+  const int hi = __double2hiint(d);
+  return __hiloint2double(x == 0 ? 0 : hi - (62 << 20), __double2loint(d));
 }
 
 // One source of a warp's batch, as its 32 antennas read it.
 struct GenSrc {
-  double sx, sy, sz;
+  long long sx, sy, sz;       // direction, units of 2^(e - 62)
   double w00, w01, w10, w11;  // bilinear weights times sqrt(I)
   long long pix;
+  int e;
 };
 
 // A warp generates kGenSrc sources for 32 antennas: U stays in registers, a
-// source's weights are formed once per warp.  Bound by the FP64 pipe: 22
-// instructions a phasor (3 phase, 3 reduction, 12 sine and cosine, 4 beam and
-// amplitude; 2 products), against 46 of the form with sincospi and lerps,
-// which took 1.30 ms for 350 antennas x 50k sources.
+// source's weights are formed once per warp.
 //
-// Sine and cosine: the phase's nearest multiple of 1/1024 cycle, k, comes
-// from a table; the rest r (exact, |r| <= 2^-11 cycles) from the Taylor series
-// in 2 pi r, whose first dropped terms are below 2e-18; then the addition
-// theorem.  The integer cycles drop out with k modulo 1024.
+// The phase and its sine and cosine are formed in 64-bit integers: the FP64
+// pipe takes 16 clocks for an instruction of a warp, as long as some 40
+// integer ones.  U and the direction are rounded to 62 bits below a power of
+// two each, their products summed exactly in 128 bits, of which the 64 below
+// one cycle are kept: the phase is off by at most 2^-60 of the largest |U| times
+// |s|, where an FP64 sum is by about 2^-53 of it.  8 FP64 instructions
+// remain a phasor (4 beam and amplitude, 2 conversions, 2 products).  350
+// antennas x 50k sources: 0.33 ms, against 0.80 with 22 FP64 instructions (the
+// phase, its reduction and the series in FP64) and 1.30 with sincospi.
+// Phases of 2^56 cycles and more, and those that are not finite, take the FP64
+// sum and the library functions.
 __global__ void __launch_bounds__(kGenWarps * 32)
 gen64_kernel(const F64Dims d, const SrcRec64* __restrict__ rec, size_t rec_stride,
              const Ucoef64* __restrict__ U, const double* __restrict__ beamT, int PP, int dx,
-             int dy, const double2* __restrict__ table, double2* __restrict__ v,
+             int dy, const longlong2* __restrict__ table, double2* __restrict__ v,
              uint32_t* __restrict__ rowmax) {
-  __shared__ double2 tab[kTable];
+  __shared__ longlong2 tab[kTable];
   __shared__ GenSrc src[kGenWarps][32];
   const int z = blockIdx.z, n = window_count(d, z);
   const int ng = ceil_div(d.nant, 32);
@@ -110,7 +177,16 @@ gen64_kernel(const F64Dims d, const SrcRec64* __restrict__ rec, size_t rec_strid
   const int tl = z / d.nf, f = z % d.nf;
   rec += (size_t)tl * rec_stride + d.s0;
   // padded antennas (a < Np) have U = 0 and a zero beam; they are not stored
-  const Ucoef64 u = U[((size_t)tl * d.u_nf + f) * d.Np + a];
+  U += ((size_t)tl * d.u_nf + f) * d.Np + a;
+  long long ux, uy, uz;
+  int ue;
+  {
+    const Ucoef64 u = *U;
+    ue = fixed_exponent(u.x, u.y, u.z);
+    ux = to_fixed(u.x, ue);
+    uy = to_fixed(u.y, ue);
+    uz = to_fixed(u.z, ue);
+  }
   const double* beam = beamT + (size_t)f * PP * d.Np + a;
   double2* out = v + (size_t)z * d.v_stride + a;
   uint32_t top = 0, low = 0;
@@ -121,7 +197,10 @@ gen64_kernel(const F64Dims d, const SrcRec64* __restrict__ rec, size_t rec_strid
     if (lane < m) {
       const SrcRec64 r = rec[s0 + lane];
       GenSrc g;
-      g.sx = r.sx; g.sy = r.sy; g.sz = r.sz;
+      g.e = fixed_exponent(r.sx, r.sy, r.sz);
+      g.sx = to_fixed(r.sx, g.e);
+      g.sy = to_fixed(r.sy, g.e);
+      g.sz = to_fixed(r.sz, g.e);
       const double y1 = r.amp * r.fy, y0 = fma(-r.amp, r.fy, r.amp);
       g.w01 = y0 * r.fx;
       g.w00 = fma(-y0, r.fx, y0);
@@ -138,24 +217,19 @@ gen64_kernel(const F64Dims d, const SrcRec64* __restrict__ rec, size_t rec_strid
       const double b00 = __ldg(bp), b01 = __ldg(bp + (size_t)dx * d.Np),
                    b10 = __ldg(bp + (size_t)dy * d.Np), b11 = __ldg(bp + (size_t)(dx + dy) * d.Np);
       const double A = fma(g.w11, b11, fma(g.w10, b10, fma(g.w01, b01, g.w00 * b00)));
-      const double ph = fma(u.x, g.sx, fma(u.y, g.sy, u.z * g.sz));
       double sn, cs;
-      // |ph| < 2^40 cycles (the magic sum below is exact there); else, and
-      // for a phase that is not finite, the library functions
-      if ((uint32_t)(__double2hiint(ph) & 0x7fffffff) < 0x42700000u) {
-        constexpr double kMagic = 6755399441055744.0;  // 1.5 * 2^52
-        const double t = fma(ph, (double)kTable, kMagic);
-        const double r = fma(t - kMagic, -1.0 / kTable, ph);
-        const double2 cs0 = tab[__double2loint(t) & (kTable - 1)];
-        constexpr double k1 = 6.283185307179586477, k2 = -19.739208802178717238,
-                         k3 = -41.341702240399760234, k4 = 64.939394022668291491,
-                         k5 = 81.605249276075054203;  // +-(2 pi)^i / i!
-        const double r2 = r * r;
-        const double sr = r * fma(r2, fma(r2, k5, k3), k1);  // sin 2 pi r
-        const double cr = r2 * fma(r2, k4, k2);              // cos 2 pi r - 1
-        sn = fma(cs0.x, sr, fma(cs0.y, cr, cs0.y));
-        cs = fma(-cs0.y, sr, fma(cs0.x, cr, cs0.x));
+      // the sum is in units of 2^(ue + e - 124) cycles, below 3 x 2^124
+      const int sh = 60 - ue - g.e;
+      if (sh >= 4) {
+        const __int128 p = (__int128)ux * g.sx + (__int128)uy * g.sy + (__int128)uz * g.sz;
+        long long ci, si;
+        sincos_fixed((unsigned long long)(p >> sh), tab, ci, si);
+        cs = from_fixed62(ci);
+        sn = from_fixed62(si);
       } else {
+        const Ucoef64 u = *U;
+        const SrcRec64 r = rec[s0 + s];
+        const double ph = fma(u.x, r.sx, fma(u.y, r.sy, u.z * r.sz));
         sincospi(2.0 * (ph - rint(ph)), &sn, &cs);
       }
       const double re = A * cs, im = A * sn;
@@ -524,10 +598,10 @@ size_t f64_digit_bytes(int Np, int S) {
   return std::max(dig, part);
 }
 size_t f64_word_bytes(int Np) { return sizeof(long long) * 2 * kGroups * (size_t)Np * Np; }
-size_t f64_table_bytes() { return sizeof(double2) * kTable; }
+size_t f64_table_bytes() { return sizeof(longlong2) * kTable; }
 
 cudaError_t launch_f64_table(void* table, cudaStream_t st) {
-  sincos_table_kernel<<<kTable / 256, 256, 0, st>>>(static_cast<double2*>(table));
+  sincos_table_kernel<<<kTable / 256, 256, 0, st>>>(static_cast<longlong2*>(table));
   return cudaGetLastError();
 }
 
@@ -538,7 +612,7 @@ cudaError_t launch_f64_phasors(const F64Dims& d, int nz, const void* rec, size_t
   const dim3 grid((unsigned)((jobs + kGenWarps - 1) / kGenWarps), 1, nz);
   gen64_kernel<<<grid, kGenWarps * 32, 0, st>>>(
       d, static_cast<const SrcRec64*>(rec), rec_stride, static_cast<const Ucoef64*>(U), beamT,
-      P * P, P > 1 ? 1 : 0, P > 1 ? P : 0, static_cast<const double2*>(table),
+      P * P, P > 1 ? 1 : 0, P > 1 ? P : 0, static_cast<const longlong2*>(table),
       static_cast<double2*>(v), rowmax);
   return cudaGetLastError();
 }

@@ -105,6 +105,33 @@ def test_fp64_product_under_a_budget():
             assert np.abs(v - full).max() <= F64_TOL * np.abs(full).max()
 
 
+# phases in fixed point: arrays from a micrometre to a light second.  Both
+# sides round U and the oracle its phase sums in FP64: 8 roundings of the
+# largest |U| in cycles, and 1e-14 for the amplitudes
+@gpu
+@pytest.mark.parametrize("scale", [1e-8, 1e-3, 1.0, 1e3, 1e6])
+def test_fp64_phases(scale):
+    args = list(sim(24, 700, ntimes=2, seed=7, dtype=np.float64))
+    args[0] = args[0] * scale
+    v = vis_gpu(*args, precision=2)
+    check_hermitian(v)
+    cycles = np.sqrt((args[0] ** 2).sum(axis=1)).max() * args[1] / 299792458.0
+    tol = 1e-14 + 2 * np.pi * 8 * 2.0 ** -53 * cycles
+    assert rel_frobenius(v, vis_oracle(*args)).max() <= tol
+
+
+# phases of 2^56 cycles and more carry no information, but stay phases: the
+# autocorrelations do not know them
+@gpu
+def test_fp64_phases_beyond_fixed_point():
+    args = list(sim(24, 700, ntimes=2, seed=7, dtype=np.float64))
+    near = vis_gpu(*args, precision=2)
+    args[0] = args[0] * 2.0 ** 60
+    v = vis_gpu(*args, precision=2)
+    check_hermitian(v)
+    np.testing.assert_allclose(np.einsum("taa->ta", v), np.einsum("taa->ta", near), rtol=1e-13)
+
+
 # antennas of very different scale, a dark antenna, and scales outside the
 # digit form's range (2^-400): the slice takes the SIMT product
 @gpu
