@@ -28,8 +28,9 @@
 // show the product (1.1e-15).
 //
 // Measured on GB300, one slice of 350 antennas x 50k sources above the horizon
-// (ncu): phasors 0.33 ms, digits 0.25 ms, class sums 0.92 ms, conversion 0.02
-// ms; with SIMT 1.30 ms and 32.8 ms.  A call of 3 such slices 102.6 -> 4.12 ms.
+// (ncu): phasors 0.33 ms, digits 0.25 ms, class sums 0.72 ms (0.63 of a call of
+// more slices), conversion 0.02 ms; with SIMT 1.30 ms and 32.8 ms.  A call of 3
+// such slices 102.6 -> 3.74 ms.
 //
 // Slices whose phasors are not finite, or whose antenna scales leave
 // [2^-400, 2^400], are flagged on the device and take the SIMT product of
@@ -336,13 +337,25 @@ digits64_kernel(const F64Dims d, const double2* __restrict__ v,
 
 // --------------------------------------------------------------- mma64 ----
 // A work item: a pair of antenna blocks, a chunk of source steps and a unit,
-// two neighbouring classes over a range of A digits i0 .. i1 (at most 6, so
-// that two stages of the planes they need fit in shared memory).  Real and
-// imaginary sums of both classes fill the 512 TMEM columns.  Units in order of
-// falling cost (digit pairs).
+// which fills the 512 TMEM columns with the real and imaginary sums of two
+// accumulators.  Units in order of falling cost (digit pairs).
+//
+// Two different blocks: two neighbouring classes, 2 g and 2 g + 1, over a range
+// of A digits i0 .. i1 (at most 6, so that two stages of the planes they need
+// fit in shared memory), added to word g as 32 x the one + the other.
+//
+// A block with itself: the sum S over the digit pairs (i, j) of a class is
+// Hermitian, the pairs (i, j) and (j, i) each other's adjoint.  So the units 0-5
+// take the pairs i < j only, with twice the weight, others the pairs (i, i) of
+// two digits 2 k and 2 k + 1 (the even classes 4 k and 4 k + 2, words 2 k and
+// 2 k + 1), and the conversion takes (S + S^H) / 2: 42 digit pairs instead
+// of 78, and the digits are read once.  Three blocks: 0.93 -> 0.86 ms a slice.
 constexpr int kUnits = 9;
 __constant__ int8_t kUnit[kUnits][3] = {{5, 0, 5}, {5, 6, 11}, {2, 0, 5}, {4, 0, 4}, {4, 5, 9},
                                         {3, 0, 3}, {3, 4, 7},  {1, 0, 3}, {0, 0, 1}};
+// {g, 0} or {k, 1} of a block with itself
+__constant__ int8_t kOwnUnit[kUnits][2] = {{5, 0}, {4, 0}, {3, 0}, {2, 0}, {1, 0},
+                                           {0, 1}, {1, 1}, {2, 1}, {0, 0}};
 constexpr int kMaxA = 6, kMaxB = 7;        // digits a unit needs of A and of B
 constexpr int kStageBytes = (kMaxA + kMaxB) * 2 * kTile;
 constexpr int kStages = 2;
@@ -377,22 +390,33 @@ __device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_
       : "memory");
 }
 
+__device__ __forceinline__ void add_word(unsigned long long* w, long long x) {
+  asm volatile("red.global.add.u64 [%0], %1;" ::"l"(w), "l"((unsigned long long)x) : "memory");
+}
+
 __global__ void __launch_bounds__(kMmaThreads, 1)
 mma64_kernel(const F64Dims d, const uint8_t* __restrict__ dig, const int* __restrict__ flags,
              long long* __restrict__ W, int npairs, int nchunks, int chunk_steps, int* err,
              unsigned long long wait_ns) {
   extern __shared__ __align__(1024) uint8_t smem[];
-  const int item = blockIdx.x;
-  const int chunk = item % nchunks, pair = (item / nchunks) % npairs,
-            z = item / (nchunks * npairs);
+  // all pairs and units of a chunk together: they read the same digits, 14 MB
+  // a chunk of 46 steps and 3 blocks, from L2 (a sweep of all chunks a unit
+  // read 5 GB from HBM a slice, 0.86 -> 0.79 ms at one)
+  const int pair = blockIdx.x % npairs, unit = blockIdx.x / npairs % kUnits;
+  const int cz = blockIdx.x / (npairs * kUnits), chunk = cz % nchunks, z = cz / nchunks;
   const int steps = ceil_div(window_count(d, z), 32);
   const int k0 = chunk * chunk_steps, k1 = min(steps, k0 + chunk_steps);
   if (k0 >= k1 || flags[z]) return;
-  const int g = kUnit[blockIdx.y][0], i0 = kUnit[blockIdx.y][1], i1 = kUnit[blockIdx.y][2];
-  const int j0 = max(0, 2 * g - i1), j1 = 2 * g + 1 - i0;
   int I = 0, J = pair;
   for (const int nb = d.Np / 128; J >= nb - I; ++I) J -= nb - I;
   J += I;
+  // digits of A and of B
+  const bool own = I == J, same = own && kOwnUnit[unit][1];
+  const int g = own ? kOwnUnit[unit][0] : kUnit[unit][0];
+  const int i0 = same ? 2 * g : own ? 0 : kUnit[unit][1];
+  const int i1 = same ? 2 * g + 1 : own ? g : kUnit[unit][2];
+  const int j0 = same ? i0 : own ? g + 1 : max(0, 2 * g - i1);
+  const int j1 = same ? i1 : 2 * g + 1 - i0;
   const uint32_t base = smem_u32(smem);
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + kStages * kStageBytes);
   const uint32_t bar0 = smem_u32(bars);
@@ -435,9 +459,9 @@ mma64_kernel(const F64Dims d, const uint8_t* __restrict__ dig, const int* __rest
       const int s = k % kStages;
       if (!wait1(empty(s), ((k / kStages) & 1) ^ 1, abort_flag, err, wait_ns)) break;
       const uint32_t st = base + (uint32_t)s * kStageBytes;
-      mbar_expect_tx(full(s), na + nb);
+      mbar_expect_tx(full(s), same ? na : na + nb);
       bulk_load(st, pa, na, full(s));
-      bulk_load(st + kMaxA * 2 * kTile, pb, nb, full(s));
+      if (!same) bulk_load(st + kMaxA * 2 * kTile, pb, nb, full(s));
     }
     // copies still in flight land before the CTA can exit
     for (int q = max(0, k - kStages); q < k; ++q)
@@ -449,15 +473,16 @@ mma64_kernel(const F64Dims d, const uint8_t* __restrict__ dig, const int* __rest
       if (!wait1(full(s), (k / kStages) & 1, abort_flag, err, wait_ns)) break;
       tc_fence_after();
       const uint32_t st = base + (uint32_t)s * kStageBytes;
-      const uint32_t a0 = plain_desc_lo(st), b0 = plain_desc_lo(st + kMaxA * 2 * kTile);
+      const uint32_t a0 = plain_desc_lo(st);
+      const uint32_t b0 = same ? a0 : plain_desc_lo(st + kMaxA * 2 * kTile);
       constexpr uint32_t kP = kTile >> 4;  // descriptor units of a plane
 #pragma unroll 1
       for (int q = 0; q < 2; ++q) {
         const uint32_t dre = tmem + 256u * q, dim = dre + 128u;
         uint32_t acc = k > 0;
         for (int i = i0; i <= i1; ++i) {
-          const int j = 2 * g + q - i;
-          if (j < 0 || j > j1) continue;
+          const int j = same ? i : 2 * g + q - i;
+          if (j < j0 || j > j1 || (same && i != i0 + q)) continue;
           const uint32_t a = a0 + (uint32_t)(i - i0) * 2 * kP, b = b0 + (uint32_t)(j - j0) * 2 * kP;
           mma64(dre, a, b, idp, acc);           // Re Re
           mma64(dim, a + kP, b, idp, acc);      // Im Re
@@ -473,16 +498,20 @@ mma64_kernel(const F64Dims d, const uint8_t* __restrict__ dig, const int* __rest
     wait_drain(done, 0, err, wait_ns);
   }
   __syncwarp();
-  // the class sums, exact integers: two classes a word, added to the slice's
-  // words (W[g][re / im][b][a], a contiguous across a warp)
+  // the sums, exact integers, added to the slice's words (W[g][re / im][b][a],
+  // a contiguous across a warp)
   const bool ok = wait_warp(done, 0, abort_flag, err, wait_ns) && !*abort_flag;
   tc_fence_after();
   if (ok) {
     const int q = warp & 3, ri = warp >> 2;
     const int a = I * 128 + q * 32 + lane;
+    const size_t plane = (size_t)d.Np * d.Np;
     unsigned long long* w = reinterpret_cast<unsigned long long*>(W) + (size_t)z * d.w_stride +
-                            (size_t)(2 * g + ri) * d.Np * d.Np + (size_t)J * 128 * d.Np + a;
+                            (size_t)(2 * (same ? 2 * g : g) + ri) * plane +
+                            (size_t)J * 128 * d.Np + a;
     const uint32_t tq = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)ri * 128u;
+    const long long weight = own ? 2 : 1;
+    const bool no_hi = own && !same && g == 0;  // (no pair i < j in class 0)
 #pragma unroll 1
     for (int c = 0; c < 128; c += 32) {
       float hi[32], lo[32];
@@ -490,10 +519,14 @@ mma64_kernel(const F64Dims d, const uint8_t* __restrict__ dig, const int* __rest
       tmem_ld32(tq + 256u + c, lo);
 #pragma unroll
       for (int x = 0; x < 32; ++x) {
-        const long long sum = 32ll * __float2int_rn(hi[x]) + __float2int_rn(lo[x]);
-        asm volatile("red.global.add.u64 [%0], %1;" ::"l"(w + (size_t)(c + x) * d.Np),
-                     "l"((unsigned long long)sum)
-                     : "memory");
+        if (no_hi) hi[x] = 0.f;
+        unsigned long long* wx = w + (size_t)(c + x) * d.Np;
+        if (same) {
+          add_word(wx, 32ll * __float2int_rn(hi[x]));
+          add_word(wx + 2 * plane, 32ll * __float2int_rn(lo[x]));
+        } else {
+          add_word(wx, weight * (32ll * __float2int_rn(hi[x]) + __float2int_rn(lo[x])));
+        }
       }
     }
   }
@@ -529,6 +562,7 @@ final64_kernel(const F64Dims d, const long long* __restrict__ W,
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
   const size_t plane = (size_t)d.Np * d.Np;
   const bool simt = flags[z] != 0;
+  const bool own = A / 4 == B / 4;  // a block of 128 with itself
   const int a = A * 32 + tx;
   int fa = 0;
   if (a < d.nant) row_field(rowmax[(size_t)z * d.Np + a], fa);
@@ -552,6 +586,14 @@ final64_kernel(const F64Dims d, const long long* __restrict__ W,
           x[g] = w[(size_t)(2 * g) * plane];
           y[g] = w[(size_t)(2 * g + 1) * plane];
         }
+        if (own) {  // S + S^H, exact
+          const long long* wt = W + (size_t)z * d.w_stride + (size_t)a * d.Np + b;
+#pragma unroll
+          for (int g = 0; g < kGroups; ++g) {
+            x[g] += wt[(size_t)(2 * g) * plane];
+            y[g] -= wt[(size_t)(2 * g + 1) * plane];
+          }
+        }
 #pragma unroll
         for (int g = kGroups - 1; g >= 0; --g) {
           val.x = fma(val.x, 0x1p-10, (double)x[g]);
@@ -559,7 +601,7 @@ final64_kernel(const F64Dims d, const long long* __restrict__ W,
         }
         int fb;
         row_field(rowmax[(size_t)z * d.Np + b], fb);
-        const int e = fa + fb - 2 * 1022 - 13;
+        const int e = fa + fb - 2 * 1022 - 13 - (own ? 1 : 0);
         val.x = scalbn(val.x, e);
         val.y = scalbn(val.y, e);
       }
@@ -627,15 +669,16 @@ cudaError_t launch_f64_product(const F64Dims& d, int nz, const void* v, const ui
   if (e != cudaSuccess) return e;
   e = cudaFuncSetAttribute(mma64_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMmaSmem);
   if (e != cudaSuccess) return e;
-  // about 12 items an SM over the window (half of it above the horizon), so
-  // that the last wave is short; at least 8 steps, so that an item's start and
-  // reductions stay small beside its MMAs (64 clocks each, 12 to 48 a step)
+  // about 4 items an SM over the window (half of it above the horizon): an
+  // item's start and its reductions take as long as some 20 steps (200
+  // antennas x 50k sources 550 us a call at 12 items an SM, 499 at 4, 500 at
+  // 3); at least 8 steps
   const long long units = (long long)kUnits * npairs * nz;
   const long long per_sm = (units * std::max(1, d.nks / 2) + num_sms - 1) / num_sms;
-  const int steps = (int)std::min<long long>(kMaxChunkSteps, std::max<long long>(8, per_sm / 12));
+  const int steps = (int)std::min<long long>(kMaxChunkSteps, std::max<long long>(8, per_sm / 4));
   const int nchunks = ceil_div(d.nks, steps);
-  const dim3 grid((unsigned)((long long)nchunks * npairs * nz), kUnits);
-  mma64_kernel<<<grid, kMmaThreads, kMmaSmem, st>>>(
+  const unsigned items = (unsigned)((long long)nchunks * npairs * nz * kUnits);
+  mma64_kernel<<<items, kMmaThreads, kMmaSmem, st>>>(
       d, static_cast<const uint8_t*>(dig), flags, W, npairs, nchunks, steps, err,
       wait_ns ? wait_ns : 10000000000ull);
   return cudaGetLastError();
