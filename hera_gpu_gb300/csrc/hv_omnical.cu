@@ -33,6 +33,7 @@
 #include <algorithm>
 #include <cstdint>
 #include <cstdio>
+#include <numeric>
 #include <vector>
 
 #include "heravis.h"
@@ -77,6 +78,7 @@ struct OmParams {
   const uint2* bl;        // [nbls] (i | j << 16, k)
   const int* seg_off;     // [npanels][nants + nubls + 1] into seg_ent
   const uint32_t* seg_ent;// baseline within its panel | (conjugate << 31)
+  const int* seg_ord;     // [npanels][nants + nubls] segments, longest first
   const typename Cx<R>::T* data;  // [ndata][nbls]
   const R* wgts;                  // [ndata][nbls]
   typename Cx<R>::T* gains;       // [ndata][nants], in/out
@@ -145,19 +147,23 @@ __device__ void block_sum3(R& a, R& b, R& c, R* red) {
 // For every segment s of the incidence list: a group of G lanes sums
 // val(entry) over the segment's entries (lane l takes entries l, l + G, ...,
 // kGU at a time, added in that order; then a butterfly over the group) and
-// lane 0 of the group calls out(s, sum).  The loop over segments is uniform
-// across the block, so every lane takes part in every shuffle.
+// lane 0 of the group calls out(s, sum).  The groups take the segments in the
+// order ord, by falling length, so that those of a warp are about as long.  The
+// loop over segments is uniform across the block, so every lane takes part in
+// every shuffle.
 template <int kGU, typename V, typename Val, typename Out>
 __device__ __forceinline__ void seg_gather(const int* __restrict__ off,
-                                           const uint32_t* __restrict__ ent, int nseg, int G,
-                                           Val val, Out out) {
+                                           const uint32_t* __restrict__ ent,
+                                           const int* __restrict__ ord, int nseg, int G, Val val,
+                                           Out out) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int per_warp = 32 / G, ngroups = (blockDim.x >> 5) * per_warp;
   const int gid = warp * per_warp + lane / G, gl = lane & (G - 1);
   for (int base = 0; base < nseg; base += ngroups) {
-    const int s = base + gid;
+    const bool has = base + gid < nseg;
+    const int s = has ? __ldg(ord + base + gid) : 0;
     V acc = V{};
-    if (s < nseg) {
+    if (has) {
       const int e1 = __ldg(off + s + 1);
       int e = __ldg(off + s) + gl;
       for (; e + (kGU - 1) * G < e1; e += kGU * G) {
@@ -170,7 +176,7 @@ __device__ __forceinline__ void seg_gather(const int* __restrict__ off,
       for (; e < e1; e += G) acc = acc + val(__ldg(ent + e));
     }
     for (int o = G >> 1; o > 0; o >>= 1) acc = acc + V::shfl_xor(acc, o);
-    if (gl == 0 && s < nseg) out(s, acc);
+    if (gl == 0 && has) out(s, acc);
   }
 }
 
@@ -252,11 +258,14 @@ __device__ __forceinline__ R chisq_part(const C* sol, int nants, const uint2* __
 //
 // kFactored (float64, which is bound by the FP64 pipe): the ratios are kept
 // multiplied into the factors, p_a = conj(g_a) ra_a and c_k = conj(u_k) ru_k,
-// so that d_b = data_b w_b p_i conj(p_j) c_k takes 14 operations instead of 17;
-// the weights come from the factors' magnitudes (3 instead of 11), and a step
-// divides once a segment instead of twice: 12 iterations of 1000 problems of 54
-// antennas 1.72 and 1.52 ms, of 200 of 180 antennas 5.05 and 4.41 ms.  It takes 8 bytes more of shared
-// memory a segment; problems that only fit without it go without.
+// so that d_b = data_b w_b p_i conj(p_j) c_k takes 14 operations instead of 17,
+// and 12 where data w is kept in shared memory (chi^2 reads the data again);
+// the weights come from the factors' magnitudes (3 instead of 11), and gain /
+// weight is divided when the weights are formed.  12 iterations of 1000 problems
+// of 54 antennas: 1.72 ms without, 1.52 with data and w kept apart and the
+// segments gathered in their own order, 1.43 now; 200 of 180 antennas 5.05, 4.42
+// and 4.37 ms.  It takes 8 bytes more of shared memory a segment; problems that
+// only fit without it go without.
 template <typename R, bool kDataShared, bool kFactored>
 __global__ void __launch_bounds__(kOmMaxThreads, OM_MINB) omnical_kernel(const OmParams<R> p) {
   using C = typename Cx<R>::T;
@@ -296,17 +305,24 @@ __global__ void __launch_bounds__(kOmMaxThreads, OM_MINB) omnical_kernel(const O
     for (int k = tid; k < nubls; k += nt) solA[nants + k] = p.ubls[(size_t)prob * nubls + k];
     if (kDataShared) {
       for (int b = tid; b < nbls; b += nt) {
-        sdata[b] = __ldg(gdata + b);
-        sw[b] = __ldg(gwgt + b);
+        C x = __ldg(gdata + b);
+        const R w = __ldg(gwgt + b);
+        if (kFactored) {  // data w: what an iteration needs
+          x.x *= w;
+          x.y *= w;
+        }
+        sdata[b] = x;
+        sw[b] = w;
       }
     }
     const C* const data = kDataShared ? sdata : gdata;
+    const C* const cdata = kDataShared && !kFactored ? sdata : gdata;  // for chi^2
     const R* const wgt = kDataShared ? sw : gwgt;
     __syncthreads();
     C *sol = solA, *nsol = solB;
 
     // chi^2 of the starting solution (redcal.py:566-577)
-    R chisq = chisq_part(sol, nants, bl, data, wgt, nbls), z1 = 0, z2 = 0;
+    R chisq = chisq_part(sol, nants, bl, cdata, wgt, nbls), z1 = 0, z2 = 0;
     block_sum3(chisq, z1, z2, red);
     R conv = 0;
     uint32_t iters = 0;
@@ -331,9 +347,13 @@ __global__ void __launch_bounds__(kOmMaxThreads, OM_MINB) omnical_kernel(const O
           }
           __syncthreads();
           seg_gather<Unroll<R>::gather, RealV<R>>(
-              p.seg_off + (size_t)pn * (nseg + 1), p.seg_ent, nseg, p.group,
+              p.seg_off + (size_t)pn * (nseg + 1), p.seg_ent,
+              p.seg_ord + (size_t)pn * nseg, nseg, p.group,
               [&](uint32_t e) { return RealV<R>{dw[e & 0x7fffffffu]}; },
-              [&](int s, RealV<R> v) { gw[s] = pn ? gw[s] + v.v : v.v; });
+              [&](int s, RealV<R> v) {
+                const R x = pn ? gw[s] + v.v : v.v;
+                gw[s] = kFactored && pn == np - 1 ? gs / x : x;
+              });
           __syncthreads();  // dw is overwritten below
         }
       } else {
@@ -363,7 +383,7 @@ __global__ void __launch_bounds__(kOmMaxThreads, OM_MINB) omnical_kernel(const O
             if (c0 + q * nt < nb) {
               e[q] = bl[b0 + c0 + q * nt];
               x[q] = data[b0 + c0 + q * nt];
-              w[q] = wgt[b0 + c0 + q * nt];
+              if (!(kFactored && kDataShared)) w[q] = wgt[b0 + c0 + q * nt];
             }
 #pragma unroll
           for (int q = 0; q < U; ++q)
@@ -371,8 +391,10 @@ __global__ void __launch_bounds__(kOmMaxThreads, OM_MINB) omnical_kernel(const O
               const int i = e[q].x & 0xffffu, j = e[q].x >> 16;
               C z;
               if constexpr (kFactored) {
-                x[q].x *= w[q];
-                x[q].y *= w[q];
+                if constexpr (!kDataShared) {
+                  x[q].x *= w[q];
+                  x[q].y *= w[q];
+                }
                 z = cmul(cmul(x[q], cmul(pc[i], conjc(pc[j]))), pc[nants + e[q].y]);
               } else {
                 const C m = model(sol, nants, e[q]);
@@ -387,7 +409,8 @@ __global__ void __launch_bounds__(kOmMaxThreads, OM_MINB) omnical_kernel(const O
         __syncthreads();
         const bool last = pn == np - 1;
         seg_gather<Unroll<R>::gather, CplxV<R>>(
-            p.seg_off + (size_t)pn * (nseg + 1), p.seg_ent, nseg, p.group,
+            p.seg_off + (size_t)pn * (nseg + 1), p.seg_ent,
+            p.seg_ord + (size_t)pn * nseg, nseg, p.group,
             [&](uint32_t e) {
               const C z = d[e & 0x7fffffffu];
               return CplxV<R>{z.x, (e >> 31) ? -z.y : z.y};
@@ -405,7 +428,7 @@ __global__ void __launch_bounds__(kOmMaxThreads, OM_MINB) omnical_kernel(const O
                 return;
               }
               if constexpr (kFactored) {
-                const R q = gs / gw[s];
+                const R q = gw[s];  // gain / weight
                 f.x = one_m + q * v.x;
                 f.y = q * v.y;
               } else {
@@ -423,7 +446,7 @@ __global__ void __launch_bounds__(kOmMaxThreads, OM_MINB) omnical_kernel(const O
       }
       // convergence and chi^2 of the stepped solution (calc_conv,
       // calc_chisq, update_active)
-      R nchisq = chisq_part(nsol, nants, bl, data, wgt, nbls), csum = 0, cwgt = 0;
+      R nchisq = chisq_part(nsol, nants, bl, cdata, wgt, nbls), csum = 0, cwgt = 0;
       for (int s = tid; s < nseg; s += nt) {
         const C x = nsol[s], y = sol[s];
         const R dx = x.x - y.x, dy = x.y - y.y;
@@ -928,7 +951,8 @@ void build_csr(const uint32_t* ggu, int nbls, int nants, int nubls, int panel, i
                std::vector<uint2>& bl, std::vector<int>& off, std::vector<uint32_t>& ent) {
   const int nseg = nants + nubls;
   bl.resize(nbls);
-  off.assign((size_t)npanels * (nseg + 1), 0);
+  // the panels' offsets, then each panel's segments by falling length
+  off.assign((size_t)npanels * (2 * nseg + 1), 0);
   ent.resize((size_t)3 * nbls);
   size_t base = 0;
   for (int pn = 0; pn < npanels; ++pn) {
@@ -942,6 +966,9 @@ void build_csr(const uint32_t* ggu, int nbls, int nants, int nubls, int panel, i
     }
     o[0] = (int)base;
     for (int s = 0; s < nseg; ++s) o[s + 1] = o[s] + cnt[s + 1];
+    int* ord = off.data() + (size_t)npanels * (nseg + 1) + (size_t)pn * nseg;
+    std::iota(ord, ord + nseg, 0);
+    std::stable_sort(ord, ord + nseg, [&](int x, int y) { return cnt[x + 1] > cnt[y + 1]; });
     std::vector<int> pos(o, o + nseg);
     for (int b = b0; b < b1; ++b) {
       const uint32_t i = ggu[3 * b], j = ggu[3 * b + 1], k = ggu[3 * b + 2];
@@ -1096,6 +1123,7 @@ int run_typed(hv_context* ctx, const uint32_t* ggu, int nbls, void* d_gains, int
     p.npanels = pl.npanels;
     p.bl = reinterpret_cast<const uint2*>(b8);
     p.seg_off = reinterpret_cast<const int*>(b8 + o_off);
+    p.seg_ord = p.seg_off + (size_t)pl.npanels * (nants + nubls + 1);
     p.seg_ent = reinterpret_cast<const uint32_t*>(b8 + o_ent);
     p.data = static_cast<const C*>(d_data);
     p.wgts = static_cast<const R*>(d_wgts);

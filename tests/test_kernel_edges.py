@@ -239,6 +239,29 @@ def test_omnical_layouts(nants, kind):
     np.testing.assert_array_equal(again["gains"], got["gains"][1:])
 
 
+# omnical in float64: everything in shared memory (data times weights kept), and
+# panels of baselines, with flagged samples.  A dozen iterations of 1e-16 a step
+# and term stay far below 1e-11 of the largest gain
+@gpu
+@pytest.mark.parametrize("nants", [3, 19, 54, 91, 150, 200])
+def test_omnical_float64_layouts(nants):
+    from hera_gpu_gb300 import omnical
+    from oracle import omnical_oracle
+    ggu, nubls = synth.hex_redundant_layout(nants)
+    g0, u0, d, w = synth.redundant_data(ggu, nubls, 3, seed=nants, noise=0.05)
+    w = np.where(np.random.default_rng(nants).random(w.shape) < 0.05, 0.0, w)
+    a = [x.astype(t) for x, t in ((g0, np.complex128), (u0, np.complex128), (d, np.complex128),
+                                  (w, np.float64))]
+    got = omnical(ggu, *a, 1e-10, 12, precision=2)
+    ref = omnical_oracle(ggu, *a, 1e-10, 12, precision=2)
+    for x in ("gains", "ubls"):  # (a unique baseline may be flagged altogether)
+        finite = np.isfinite(ref[x])
+        np.testing.assert_array_equal(np.isfinite(got[x]), finite)
+        assert (np.abs(got[x] - ref[x])[finite].max(initial=0)
+                <= 1e-11 * np.abs(ref[x][finite]).max(initial=1))
+    np.testing.assert_array_equal(got["iters"], ref["iters"])
+
+
 # antenna blocks of the fused forms (32, 64, 96 and 128 rows; one to five
 # blocks), at their edges
 @gpu
