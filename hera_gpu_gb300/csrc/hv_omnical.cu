@@ -49,7 +49,6 @@ template <> struct Cx<double> { using T = double2; };
 //   OM_UNROLL_*  baselines a thread takes per pass of the per-baseline loops
 //   OM_GATHER_*  incidence entries a lane loads ahead in the segment gathers
 //   OM_MINB      CTAs of 512 threads an SM (2: 64 registers a thread)
-//   OM_GK_D      float64 gathers: at least this many entries a lane
 //   OM_WANT_*    CTAs of 512 threads an SM the panels of baselines are sized for
 #ifndef OM_UNROLL_F
 #define OM_UNROLL_F 1
@@ -59,9 +58,6 @@ template <> struct Cx<double> { using T = double2; };
 #endif
 #ifndef OM_MINB
 #define OM_MINB 2
-#endif
-#ifndef OM_GK_D
-#define OM_GK_D 16
 #endif
 #ifndef OM_WANT_F
 #define OM_WANT_F 2
@@ -877,15 +873,15 @@ struct Plan {
   size_t smem = 0;
 };
 
-// Launch shape: threads = about half the baselines (64 .. 512); everything
+// Launch shape: threads = about half the baselines (64 .. max_threads); everything
 // in shared memory when that leaves 16 warps an SM, else panels of
 // baselines sized for two CTAs (or the thread limit) an SM.
 template <typename R>
-int make_plan(int nants, int nubls, int nbls, bool factored, Plan* out) {
+int make_plan(int nants, int nubls, int nbls, bool factored, int max_threads, Plan* out) {
   using C = typename Cx<R>::T;
   Plan pl;
   const int t = ((nbls / 2 + 31) / 32) * 32;
-  pl.threads = std::max(64, std::min(kOmMaxThreads, t));
+  pl.threads = std::max(64, std::min(max_threads, t));
   const size_t nseg = (size_t)nants + nubls;
   pl.factored = factored;
   const size_t fixed =
@@ -913,16 +909,33 @@ int make_plan(int nants, int nubls, int nbls, bool factored, Plan* out) {
   // lanes per segment, a power of two <= 32, from the mean segment length
   // of a panel: float32 (latency-bound) about its square root; float64
   // (bound by the FP64 pipe, where each level of the butterfly over the
-  // lanes costs adds) at least OM_GK_D entries a lane
+  // lanes costs adds) 2 from a length of 22 on (a CTA of at most 256 threads,
+  // whose lanes are soon all taken: 26), 4 from four times that.  Measured, one
+  // and two lanes: 54 antennas (28.2, 256 threads) 1.38 and 1.27 ms, 45 (23.0)
+  // 1.29 and 1.36, 180 (22.8, 512 threads) 4.36 and 4.08; two and four lanes:
+  // 61 (32.5, 256) 1.32 and 1.44, 135 (34.2, 512) 2.22 and 2.39.
   const double mean = nseg ? 3.0 * pl.panel / nseg : 1.0;
   int g = 1;
   if (sizeof(R) == 4)
     while (g < 32 && 4.0 * g * g <= mean) g *= 2;
   else
-    while (g < 32 && 2.0 * g * OM_GK_D <= mean) g *= 2;
+    while (g < 32 && (pl.threads > 256 ? 22.0 : 26.0) * g * g <= mean) g *= 2;
   pl.group = g;
   *out = pl;
   return HV_OK;
+}
+
+// The plan of a call.  Float64 takes CTAs of 256 threads where all baselines or
+// half of them fit in shared memory: more problems an SM, whose barriers and
+// serial sums overlap.  Measured, 512 and 256 threads: 37 antennas 1.09 and 0.96
+// ms, 70 (two CTAs of either) 1.26 and 1.16, 90 (one panel and two) 1.95 and
+// 1.93; 100 (one panel and three) 1.80 and 2.02, 180 4.36 and 7.16.
+template <typename R>
+int choose_plan(int nants, int nubls, int nbls, bool factored, Plan* out) {
+  if (sizeof(R) == 8 && make_plan<R>(nants, nubls, nbls, factored, 256, out) == HV_OK &&
+      out->npanels <= 2)
+    return HV_OK;
+  return make_plan<R>(nants, nubls, nbls, factored, kOmMaxThreads, out);
 }
 
 int fail(hv_context* ctx, int code, const char* msg) {
@@ -1070,8 +1083,8 @@ int run_typed(hv_context* ctx, const uint32_t* ggu, int nbls, void* d_gains, int
                        d_conv, st);
   }
   Plan pl;
-  if ((sizeof(R) == 4 || make_plan<R>(nants, nubls, nbls, true, &pl) != HV_OK) &&
-      make_plan<R>(nants, nubls, nbls, false, &pl) != HV_OK)
+  if ((sizeof(R) == 4 || choose_plan<R>(nants, nubls, nbls, true, &pl) != HV_OK) &&
+      choose_plan<R>(nants, nubls, nbls, false, &pl) != HV_OK)
     return fail(ctx, HV_ERR_ARG, "omnical: too many antennas and unique baselines for one CTA");
   std::vector<uint2> bl;
   std::vector<int> off;
