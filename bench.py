@@ -126,11 +126,12 @@ def sources_up(w, t):
 def tc_chunk(nsrc, nslices, ngroups, num_sms):
     """Split-K chunk the library picks (hv_tc.cu tc_chunk_sources) where the
     items fill the GPU."""
-    nchunk = max(1, -(-40 * num_sms // (nslices * ngroups)))
-    c = -(-max(nsrc // 2, 1) // nchunk)
-    c = min(32768, max(1024, c))
-    unit = 2048 if c > 2048 else 32
-    return (c + unit // 2) // unit * unit
+    up = max(nsrc // 2, 1)
+    nrun = max(1, -(-40 * num_sms // (nslices * ngroups)))
+    run = min((max(1024, -(-up // nrun)) + 16) // 32 * 32, 2048)
+    return min(range(run, 32769, run),
+               key=lambda c: min(nslices, 1 << 20) * ngroups * (up + 320 * -(-up // c))
+               + num_sms * (min(c, up) + 320))
 
 
 def tc_groups(nant):

@@ -380,10 +380,11 @@ int run_device(hv_context* ctx, int method, const R* antpos, int nant, const dou
       HV_ENSURE(ctx->tcgroups, gbytes);
       HV_CK(cudaMemcpyAsync(ctx->tcgroups.p, host.data(), gbytes, cudaMemcpyHostToDevice, st));
       // batch of times per launch, bounded by the partial-sum and record caps
-      int ntb = ntimes, chunk = 0;
+      int ntb = ntimes, chunk = 0, flush = 0;
       size_t slice_floats = 0;
       for (;;) {
-        chunk = tc_chunk_sources(S1, ntb, nfreq, ngroups, tc_block_rows(nant, form), ctx->num_sms);
+        chunk = tc_chunk_sources(S1, ntb, nfreq, ngroups, tc_block_rows(nant, form), ctx->num_sms,
+                                 &flush);
         slice_floats = tc_partial_floats(Np, S1, 1, chunk);
         const size_t pbytes = sizeof(float) * slice_floats * (size_t)ntb * nfreq;
         const size_t rbytes = sizeof(Rec) * (size_t)ntb * (((size_t)S1 + 31) / 32 * 32);
@@ -470,6 +471,7 @@ int run_device(hv_context* ctx, int method, const R* antpos, int nant, const dou
         L.P = P;
         L.nsrc = nsrc;
         L.chunk = chunk;
+        L.flush = flush;
         HV_ENSURE(ctx->tctable, tc_sim_table_bytes(1));
         HV_HOST_ENSURE(ctx->tctable_h, tc_sim_table_bytes(1));
         if (nsrc > 0)

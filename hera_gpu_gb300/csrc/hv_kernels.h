@@ -237,6 +237,8 @@ struct TcSimDesc {
   int rec_stride;       // records per time, a multiple of 32 >= nsrc
   int nt, nf, Np, nant, P, nsrc;
   int chunk;            // sources per split-K chunk (multiple of 32)
+  int flush;            // sources per accumulator flush (multiple of 32; 0: the most there may
+                        // be); the first simulation's applies to a launch
   int form;             // 0: split BF16; 1: FP16 + FP8 (needs sbound)
   TcTune tune;          // launch shape (the first simulation's applies to a launch)
   bool claim_zeroed;    // launch_tc_relative, ahead in the stream, zeroed the claim counter
@@ -273,7 +275,8 @@ cudaError_t launch_tc_batch(const TcSimDesc* sims, int nsims, const void* rec, l
                             int num_sms, cudaStream_t st, unsigned long long wait_ns = 0,
                             int stall = 0, TcShare* share = nullptr);
 size_t tc_partial_floats(int Np, int nsrc, int nslices, int chunk);
-int tc_chunk_sources(int nsrc, int ntimes, int nfreq, int ngroups, int block_rows, int num_sms);
+int tc_chunk_sources(int nsrc, int ntimes, int nfreq, int ngroups, int block_rows, int num_sms,
+                     int* flush);
 size_t tc_group_table_bytes(int nant);
 int tc_fill_group_table(int nant, int form, void* host_buf);
 int tc_max_slots(int nant);

@@ -34,8 +34,8 @@
 //                 the phase in cycles reduced exactly in FP32
 //                 (phase_cycles32), sincos, v = A sqrt(I) e^{2 pi i phi},
 //                 the split of v, stored to the canonical K-major
-//                 128-byte-swizzled UMMA layout.  Every TC_FLUSH_SOURCES
-//                 sources of an item, and after its last stage, they drain
+//                 128-byte-swizzled UMMA layout.  Every TcParams::flush
+//                 stages of an item, and after its last stage, they drain
 //                 TMEM into the item's partial buffer (epilogue).
 //   next warp     TMA producer: each stage's source records, one 2-D
 //                 cp.async.bulk.tensor into shared memory.  Its first thread
@@ -155,8 +155,8 @@ constexpr int TC_STAGES = 8, TC_MAX_STAGES = 12;
 // its error grows with the number of additions into one value: measured
 // against the FP64 oracle at 350 antennas x 1M sources, the relative error
 // of an autocorrelation summed over 16384 sources is -1e-4, over 1024
-// sources -1.3e-5.  TC_FLUSH_SOURCES (a multiple of every stage size) per
-// flush bound it.
+// sources -1.3e-5.  At most TC_FLUSH_SOURCES (a multiple of every stage size)
+// per flush bound it (see tc_chunk_sources).
 #ifndef TC_FLUSH_SOURCES
 #define TC_FLUSH_SOURCES 2048
 #endif
@@ -243,6 +243,7 @@ struct TcParams {
   long long group_items;  // shared launch: cluster items x ngroups
   int team_warps;  // generator warps per stage
   int rows;        // rows of an antenna block (tc_block_rows; one value a launch)
+  int flush;       // stages per accumulator flush
 };
 constexpr int kClaimCount = 0, kClaimFront = 1, kClaimBack = 2;
 // Items a CTA has claimed ahead of its slowest role (the ring of item
@@ -745,7 +746,7 @@ __device__ __forceinline__ void tc_vis_body(const CUtensorMap& rec_map, const Tc
   constexpr int KS = TcForm<kForm>::KS;         // sources per stage
   constexpr int TILES = TcForm<kForm>::TILES;   // tiles per slot per stage
   constexpr int REC = KS * 32;                  // record bytes per stage
-  constexpr int FLUSH = TC_FLUSH_SOURCES / KS;  // stages per accumulator flush
+  const int FLUSH = p.flush;  // stages per accumulator flush
   constexpr int TC_NREC = TcForm<kForm>::NREC;  // record stages
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   // The operand tiles need a 1024-byte aligned base (the 128-byte swizzle
@@ -1470,21 +1471,37 @@ int tc_fill_group_table(int nant, int form, void* host_buf) {
   return (int)g.size();
 }
 
-int tc_chunk_sources(int nsrc, int ntimes, int nfreq, int ngroups, int block_rows, int num_sms) {
-  // about 40 items per cluster (or per CTA without clusters), so that the
-  // run-time claiming leaves a short tail, in chunks of 1k-32k sources
-  // (about half the catalogue is above the horizon)
+int tc_chunk_sources(int nsrc, int ntimes, int nfreq, int ngroups, int block_rows, int num_sms,
+                     int* flush) {
+  // Sources an accumulator sums before it is flushed: as many as give about 40
+  // runs a cluster (or CTA), 1024 to TC_FLUSH_SOURCES, in whole stages (the
+  // error grows with the run; about half the catalogue is above the horizon).
   const long long nslices = (long long)ntimes * nfreq;
-  const long long nchunk =
-      std::max<long long>(1, (40LL * num_sms + nslices * ngroups - 1) / (nslices * ngroups));
   const long long up = std::max(nsrc / 2, 1);
-  long long c = (up + nchunk - 1) / nchunk;
-  c = std::min<long long>(32768, std::max<long long>(1024, c));
-  // whole stages; above one accumulator flush, whole flushes: a chunk a few
-  // stages longer than that pays another epilogue for them (350 antennas x
-  // 1M sources x 16 slices: 4128 sources took three flushes, 4096 take two)
-  const long long unit = c > TC_FLUSH_SOURCES ? TC_FLUSH_SOURCES : 32;
-  c = (c + unit / 2) / unit * unit;
+  const long long nrun =
+      std::max<long long>(1, (40LL * num_sms + nslices * ngroups - 1) / (nslices * ngroups));
+  long long run = std::max<long long>(1024, (up + nrun - 1) / nrun);
+  run = std::min<long long>((run + 16) / 32 * 32, TC_FLUSH_SOURCES);
+  // The chunk: the number of runs with the least cost, which is the sources of
+  // the slices' items and `start` more an item (its start, and its partial sums
+  // through HBM to the reduction) spread over the SMs, and one item for the tail
+  // of the run-time claiming.  Measured, against chunks of one run: 350 antennas
+  // x 50k sources above the horizon x 60 slices (runs of 1472) 4.67 -> 4.41 ms,
+  // 100k x 16 (1024) 3.04 -> 2.47, 524k x 16 (2048; two runs before) 10.75 ->
+  // 10.41, 203 antennas x 50k x 80 (1312) 3.51 -> 3.24; half of `start` took
+  // 2.61 ms for the second, twice of it 1.52 instead of 1.38 for 200 antennas x
+  // 100k x 16.
+  const int start = 64 + 2 * block_rows;
+  long long c = 0, least = 0;
+  for (long long x = run; x <= 32768; x += run) {
+    const long long cost = std::min<long long>(nslices, 1 << 20) * ngroups *
+                               (up + start * ((up + x - 1) / x)) +
+                           num_sms * (std::min(x, up) + start);
+    if (c == 0 || cost < least) {
+      c = x;
+      least = cost;
+    }
+  }
   // Small calls, which leave clusters (or CTAs) without an item at the shortest
   // of those chunks: the chunk with the shortest span, an item costing its
   // sources and a part for its partial sums (as many sources as their write and
@@ -1510,8 +1527,9 @@ int tc_chunk_sources(int nsrc, int ntimes, int nfreq, int ngroups, int block_row
     long long best = c;
     for (long long x = c - 32; x >= 64; x -= 32)
       if (span(x, ntimes) < span(best, ntimes)) best = x;
-    if (nfreq == 1 || 3 * span(best, nslices) < 2 * span(c, nslices)) c = best;
+    if (nfreq == 1 || 3 * span(best, nslices) < 2 * span(c, nslices)) run = c = best;
   }
+  *flush = (int)run;
   return (int)c;
 }
 
@@ -1623,6 +1641,7 @@ cudaError_t launch_form(const TcSimDesc* sims, int nsims, const void* rec, long 
   p.err = err;
   p.wait_ns = wait_ns ? wait_ns : TC_WAIT_NS;
   p.stall = stall;
+  p.flush = (sims[0].flush > 0 ? sims[0].flush : TC_FLUSH_SOURCES) / KS;
   p.team_warps = team_warps;
   p.rows = tc_block_rows(sims[0].nant, kForm);
   const int slot = p.rows * TC_ROW_BYTES;

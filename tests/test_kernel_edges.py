@@ -326,3 +326,18 @@ def test_host_calls_staged_and_not():
             assert rel_frobenius(v, ref).max() <= 1e-4
     for a, v in zip(cases[::-1], first[::-1]):
         np.testing.assert_array_equal(vis_gpu(*a, precision=1, method="tc"), v)
+
+
+# chunks of several accumulator runs: a last chunk of one run and less, chunks
+# beyond the sources above the horizon
+@gpu
+@pytest.mark.parametrize("method", ["tc", "tc_fp16"])
+@pytest.mark.parametrize("nant,nsrc,ntimes", [(33, 20000, 60), (70, 6100, 200), (260, 9000, 40)])
+def test_chunks_of_several_runs(nant, nsrc, ntimes, method):
+    args = sim(nant, nsrc, ntimes=ntimes, seed=nant)
+    v = vis_gpu(*args, precision=1, method=method)
+    check_hermitian(v)
+    t = [0, ntimes // 2, ntimes - 1]
+    part = (args[0], args[1], args[2][t], *args[3:])
+    ref = vis_oracle(*[a.astype(np.float64) if isinstance(a, np.ndarray) else a for a in part])
+    assert rel_frobenius(v[t], ref).max() <= 1e-4
