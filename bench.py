@@ -136,22 +136,23 @@ def tc_chunk(nsrc, nslices, ngroups, num_sms):
 
 def tc_groups(nant):
     """The fused kernel's block-pair groups (hv_tc.cu make_groups): per group
-    its MMA N.  Pairs (I, J), (I, J + 1) share row block I; the pairs left
-    over at the end of a row, (I, nb - 1), are taken as (nb - 1, I) and
-    paired in ascending I."""
+    the columns of its four MMAs a product, as multiples of one.  Pairs (I, J),
+    (I, J + 1) share row block I; the pairs left over at the end of a row,
+    (I, nb - 1), are taken as (nb - 1, I) and paired in ascending I.  A block
+    with itself takes three of the four MMAs."""
     nb = (nant + 127) // 128
     ncols = [(min(128, nant - 128 * b) + 15) // 16 * 16 for b in range(nb)]
     groups, singles = [], []
     for I in range(nb):
         J = I
         while J + 1 < nb:
-            groups.append(128 + ncols[J + 1])
+            groups.append([(128, I == J), (ncols[J + 1], False)])
             J += 2
         if J < nb:
-            singles.append(I)
+            singles.append((ncols[I], I == nb - 1))
     for k in range(0, len(singles), 2):
-        groups.append(128 + ncols[singles[k + 1]] if k + 1 < len(singles) else ncols[singles[k]])
-    return groups
+        groups.append(singles[k:k + 2])
+    return [sum(n * (3 if own else 4) for n, own in g) / 4 for g in groups]
 
 
 def tc_num_groups(nant):
