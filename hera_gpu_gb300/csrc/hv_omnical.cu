@@ -25,9 +25,9 @@
 // needed.  The sums over each antenna's and each unique baseline's
 // baselines are gathers over a fixed incidence list (CSR), each segment
 // summed by a fixed group of lanes in a fixed order, so the result does not
-// depend on scheduling and repeats bit for bit.  In float32, arrays of 17 to
-// 256 antennas whose baselines are distinct antenna pairs take a kernel of
-// their own (omnical_dense_kernel).
+// depend on scheduling and repeats bit for bit.  In float32, most arrays
+// of 31 to 256 antennas whose baselines are distinct antenna pairs take a kernel
+// of their own (omnical_dense_kernel).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -74,7 +74,7 @@ struct OmParams {
   const uint2* bl;        // [nbls] (i | j << 16, k)
   const int* seg_off;     // [npanels][nants + nubls + 1] into seg_ent
   const uint32_t* seg_ent;// baseline within its panel | (conjugate << 31)
-  const int* seg_ord;     // [npanels][nants + nubls] segments, longest first
+  const int* seg_ord;     // float64: [npanels][nants + nubls] segments, longest first
   const typename Cx<R>::T* data;  // [ndata][nbls]
   const R* wgts;                  // [ndata][nbls]
   typename Cx<R>::T* gains;       // [ndata][nants], in/out
@@ -143,11 +143,12 @@ __device__ void block_sum3(R& a, R& b, R& c, R* red) {
 // For every segment s of the incidence list: a group of G lanes sums
 // val(entry) over the segment's entries (lane l takes entries l, l + G, ...,
 // kGU at a time, added in that order; then a butterfly over the group) and
-// lane 0 of the group calls out(s, sum).  The groups take the segments in the
-// order ord, by falling length, so that those of a warp are about as long.  The
-// loop over segments is uniform across the block, so every lane takes part in
-// every shuffle.
-template <int kGU, typename V, typename Val, typename Out>
+// lane 0 of the group calls out(s, sum).  With kOrd (float64) the groups take
+// the segments in the order ord, by falling length, so that those of a warp are
+// about as long; in float32 the look-up cost 5% and gained nothing.  The loop
+// over segments is uniform across the block, so every lane takes part in every
+// shuffle.
+template <bool kOrd, int kGU, typename V, typename Val, typename Out>
 __device__ __forceinline__ void seg_gather(const int* __restrict__ off,
                                            const uint32_t* __restrict__ ent,
                                            const int* __restrict__ ord, int nseg, int G, Val val,
@@ -157,7 +158,7 @@ __device__ __forceinline__ void seg_gather(const int* __restrict__ off,
   const int gid = warp * per_warp + lane / G, gl = lane & (G - 1);
   for (int base = 0; base < nseg; base += ngroups) {
     const bool has = base + gid < nseg;
-    const int s = has ? __ldg(ord + base + gid) : 0;
+    const int s = kOrd && has ? __ldg(ord + base + gid) : base + gid;
     V acc = V{};
     if (has) {
       const int e1 = __ldg(off + s + 1);
@@ -342,7 +343,7 @@ __global__ void __launch_bounds__(kOmMaxThreads, OM_MINB) omnical_kernel(const O
               dw[b] = mag2(model(sol, nants, e)) * wgt[b0 + b];
           }
           __syncthreads();
-          seg_gather<Unroll<R>::gather, RealV<R>>(
+          seg_gather<sizeof(R) == 8, Unroll<R>::gather, RealV<R>>(
               p.seg_off + (size_t)pn * (nseg + 1), p.seg_ent,
               p.seg_ord + (size_t)pn * nseg, nseg, p.group,
               [&](uint32_t e) { return RealV<R>{dw[e & 0x7fffffffu]}; },
@@ -404,7 +405,7 @@ __global__ void __launch_bounds__(kOmMaxThreads, OM_MINB) omnical_kernel(const O
         }
         __syncthreads();
         const bool last = pn == np - 1;
-        seg_gather<Unroll<R>::gather, CplxV<R>>(
+        seg_gather<sizeof(R) == 8, Unroll<R>::gather, CplxV<R>>(
             p.seg_off + (size_t)pn * (nseg + 1), p.seg_ent,
             p.seg_ord + (size_t)pn * nseg, nseg, p.group,
             [&](uint32_t e) {
@@ -497,9 +498,15 @@ __global__ void __launch_bounds__(kOmMaxThreads, OM_MINB) omnical_kernel(const O
 // (81%: gathers and updates at the unique baselines' scattered places).
 // Measured on GB300, 12 iterations of 2000 problems, general kernel and this
 // one: 180 antennas 3.70 and 2.48 ms, 128 antennas 2.84 and 1.64 ms, 54
-// antennas 0.44 and 0.36 ms; 12 antennas (4000 problems) 94 and 103 us, so it
-// starts at kDenseMinAnts.
-constexpr int kDenseMinAnts = 17, kDenseMaxAnts = 256;
+// antennas 0.44 and 0.36 ms.  Smaller arrays stay with the general kernel (4000
+// problems of 20 antennas 148 and 165 us, 28 antennas 237 and 237, 31 antennas
+// 335 and 292), and so do arrays of 65 to 79, whose few warps a problem are
+// slower while a call has few problems (70 antennas: 4000 problems 1127 and
+// 1092 us, 600 problems 140 and 145, 100 problems 84 and 93; 80 antennas 1372
+// and 1245, 166 and 165, 98 and 100).  The number of problems must not decide: a
+// problem gives the same result alone or among others.
+constexpr int kDenseMinAnts = 31, kDenseMaxAnts = 256;
+constexpr int kDenseGap0 = 65, kDenseGap1 = 79;
 constexpr int kDenseThreads = 256;
 constexpr uint32_t kNoPair = 0x7fffu;  // slot without a baseline (256 antennas: < 32640 pairs)
 
@@ -816,12 +823,13 @@ struct DensePlan {
 // Rows of up to 128 antennas take half a warp: fewer idle lanes at the row's
 // end (54 antennas: 77% busy, 61% with whole warps).
 bool make_dense_plan(const uint32_t* ggu, int nbls, int nants, int nubls, DensePlan* pl) {
-  if (nants < kDenseMinAnts || nants > kDenseMaxAnts || nbls < 1 || nubls < 1 || nubls > 65535 ||
+  if (nants < kDenseMinAnts || nants > kDenseMaxAnts ||
+      (nants >= kDenseGap0 && nants <= kDenseGap1) || nbls < 1 || nubls < 1 || nubls > 65535 ||
       nbls > nants * (nants - 1) / 2)
     return false;
   pl->gl = nants <= 128 ? 16 : 32;
   const int need = (nants + pl->gl - 1) / pl->gl;
-  pl->nb = pl->gl == 32 ? (need <= 6 ? 6 : 8) : need <= 2 ? 2 : need <= 4 ? 4 : 8;
+  pl->nb = pl->gl == 32 ? (need <= 6 ? 6 : 8) : need <= 2 ? 2 : need <= 4 ? 4 : need <= 6 ? 6 : 8;
   // a few rows a group: small arrays take few warps, so that more problems
   // share an SM
   const int gw = 32 / pl->gl;
@@ -864,6 +872,7 @@ DenseFn dense_kernel(int gl, int nb) {
   if (gl == 32) return nb == 6 ? omnical_dense_kernel<32, 6> : omnical_dense_kernel<32, 8>;
   return nb == 2   ? omnical_dense_kernel<16, 2>
          : nb == 4 ? omnical_dense_kernel<16, 4>
+         : nb == 6 ? omnical_dense_kernel<16, 6>
                    : omnical_dense_kernel<16, 8>;
 }
 
@@ -960,12 +969,12 @@ int check_indices(hv_context* ctx, const uint32_t* ggu, int nbls, int nants, int
 // antenna a, the panel's baselines with i == a (as is) and j == a
 // (conjugated); for unique baseline k, those with k; entries hold the
 // baseline's index within its panel.
-void build_csr(const uint32_t* ggu, int nbls, int nants, int nubls, int panel, int npanels,
+void build_csr(const uint32_t* ggu, int nbls, int nants, int nubls, int panel, int npanels, bool order,
                std::vector<uint2>& bl, std::vector<int>& off, std::vector<uint32_t>& ent) {
   const int nseg = nants + nubls;
   bl.resize(nbls);
-  // the panels' offsets, then each panel's segments by falling length
-  off.assign((size_t)npanels * (2 * nseg + 1), 0);
+  // the panels' offsets, then (order) each panel's segments by falling length
+  off.assign((size_t)npanels * ((order ? 2 : 1) * nseg + 1), 0);
   ent.resize((size_t)3 * nbls);
   size_t base = 0;
   for (int pn = 0; pn < npanels; ++pn) {
@@ -979,9 +988,11 @@ void build_csr(const uint32_t* ggu, int nbls, int nants, int nubls, int panel, i
     }
     o[0] = (int)base;
     for (int s = 0; s < nseg; ++s) o[s + 1] = o[s] + cnt[s + 1];
-    int* ord = off.data() + (size_t)npanels * (nseg + 1) + (size_t)pn * nseg;
-    std::iota(ord, ord + nseg, 0);
-    std::stable_sort(ord, ord + nseg, [&](int x, int y) { return cnt[x + 1] > cnt[y + 1]; });
+    if (order) {
+      int* ord = off.data() + (size_t)npanels * (nseg + 1) + (size_t)pn * nseg;
+      std::iota(ord, ord + nseg, 0);
+      std::stable_sort(ord, ord + nseg, [&](int x, int y) { return cnt[x + 1] > cnt[y + 1]; });
+    }
     std::vector<int> pos(o, o + nseg);
     for (int b = b0; b < b1; ++b) {
       const uint32_t i = ggu[3 * b], j = ggu[3 * b + 1], k = ggu[3 * b + 2];
@@ -1089,7 +1100,7 @@ int run_typed(hv_context* ctx, const uint32_t* ggu, int nbls, void* d_gains, int
   std::vector<uint2> bl;
   std::vector<int> off;
   std::vector<uint32_t> ent;
-  build_csr(ggu, nbls, nants, nubls, pl.panel, pl.npanels, bl, off, ent);
+  build_csr(ggu, nbls, nants, nubls, pl.panel, pl.npanels, sizeof(R) == 8, bl, off, ent);
   const int nsm = std::max(1, hv_context_num_sms(ctx));
   const int grid = std::max(1, std::min(ndata, pl.blocks_per_sm * nsm));
   const size_t n_bl = sizeof(uint2) * bl.size(), n_off = sizeof(int) * off.size(),

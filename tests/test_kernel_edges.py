@@ -191,14 +191,15 @@ def test_median_strips(ks):
     assert np.isnan(inner).all()
 
 
-# omnical in float32: the antenna-matrix kernel (17 to 256 antennas, distinct
-# pairs) at the edges of its rows and column chunks, with pairs in both orders,
+# omnical in float32: the antenna-matrix kernel (31 to 64 and 80 to 256 antennas,
+# distinct pairs) at the edges of its rows and column chunks, with pairs in both orders,
 # baselines in any order and some missing; and layouts it must leave to the
-# general kernel (16 and 257 antennas, a pair twice, one unique baseline for
-# all).  A dozen iterations: float32 rounding (6e-8 a step and term) stays far
+# general kernel (fewer, 65 to 79 and 257 antennas, a pair twice, one unique
+# baseline for all).  A dozen iterations: float32 rounding (6e-8 a step and term) stays far
 # below 1e-5 of the largest gain, and no problem is near a stop.
 @gpu
-@pytest.mark.parametrize("nants", [16, 17, 31, 32, 33, 64, 65, 128, 129, 192, 193, 256, 257])
+@pytest.mark.parametrize("nants", [16, 17, 30, 31, 32, 33, 64, 65, 79, 80, 96, 97, 128, 129, 192,
+                                   193, 256, 257])
 @pytest.mark.parametrize("kind", ["plain", "shuffled", "twice", "one"])
 def test_omnical_layouts(nants, kind):
     from hera_gpu_gb300 import omnical
