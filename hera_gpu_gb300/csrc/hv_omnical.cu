@@ -86,6 +86,7 @@ struct OmParams {
   float gstep;
   int maxiter, check_every, check_after;
   int group;       // lanes per segment in the gathers (1, 2, 4, 8, 16 or 32)
+  int sum_threads; // threads whose order the sums over the block follow (>= blockDim.x)
   int* counter;    // next problem
 };
 
@@ -134,6 +135,38 @@ __device__ void block_sum3(R& a, R& b, R& c, R* red) {
   b = red[32];
   c = red[64];
   for (int w = 1; w < nw; ++w) {
+    a += red[w];
+    b += red[32 + w];
+    c += red[64 + w];
+  }
+}
+
+// The same for the values that part(v, a, b, c) gives for each of nv threads (a
+// multiple of 32, at least blockDim.x): a CTA of fewer threads takes several
+// each, in the order in which nv threads would be added.
+template <typename R, typename Part>
+__device__ __forceinline__ void block_sum3_of(int nv, Part part, R& a, R& b, R& c, R* red) {
+  __syncthreads();  // red may still be read from the last call
+  for (int v = threadIdx.x; v < nv; v += blockDim.x) {
+    a = b = c = 0;
+    part(v, a, b, c);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      a += __shfl_xor_sync(0xffffffffu, a, o);
+      b += __shfl_xor_sync(0xffffffffu, b, o);
+      c += __shfl_xor_sync(0xffffffffu, c, o);
+    }
+    if ((v & 31) == 0) {
+      red[v >> 5] = a;
+      red[32 + (v >> 5)] = b;
+      red[64 + (v >> 5)] = c;
+    }
+  }
+  __syncthreads();
+  a = red[0];
+  b = red[32];
+  c = red[64];
+  for (int w = 1; w < nv >> 5; ++w) {
     a += red[w];
     b += red[32 + w];
     c += red[64 + w];
@@ -202,20 +235,20 @@ template <typename R> struct Unroll {
   static constexpr int gather = sizeof(R) == 4 ? OM_GATHER_F : OM_GATHER_D;  // seg_gather
 };
 
-// sum_b |data_b - model_b|^2 w_b over this thread's baselines (calc_chisq,
-// redcal.py:97-114)
+// sum_b |data_b - model_b|^2 w_b over the baselines of thread tid of nt
+// (calc_chisq, redcal.py:97-114)
 template <typename R, typename C>
 __device__ __forceinline__ R chisq_part(const C* sol, int nants, const uint2* __restrict__ bl,
-                                        const C* data, const R* wgt, int nbls) {
+                                        const C* data, const R* wgt, int nbls, int tid, int nt) {
   constexpr int U = Unroll<R>::n;
   R acc = 0;
-  for (int b0 = threadIdx.x; b0 < nbls; b0 += U * blockDim.x) {
+  for (int b0 = tid; b0 < nbls; b0 += U * nt) {
     uint2 e[U];
     C x[U];
     R w[U];
 #pragma unroll
     for (int q = 0; q < U; ++q) {
-      const int b = b0 + q * blockDim.x;
+      const int b = b0 + q * nt;
       if (b < nbls) {
         e[q] = bl[b];
         x[q] = data[b];
@@ -224,7 +257,7 @@ __device__ __forceinline__ R chisq_part(const C* sol, int nants, const uint2* __
     }
 #pragma unroll
     for (int q = 0; q < U; ++q) {
-      if (b0 + q * blockDim.x < nbls) {
+      if (b0 + q * nt < nbls) {
         const C m = model(sol, nants, e[q]);
         const R dx = x[q].x - m.x, dy = x[q].y - m.y;
         acc += (dx * dx + dy * dy) * w[q];
@@ -260,8 +293,8 @@ __device__ __forceinline__ R chisq_part(const C* sol, int nants, const uint2* __
 // the weights come from the factors' magnitudes (3 instead of 11), and gain /
 // weight is divided when the weights are formed.  12 iterations of 1000 problems
 // of 54 antennas: 1.72 ms without, 1.52 with data and w kept apart and the
-// segments gathered in their own order, 1.43 now; 200 of 180 antennas 5.05, 4.42
-// and 4.37 ms.  It takes 8 bytes more of shared memory a segment; problems that
+// segments gathered in their own order, 1.35 now; 200 of 180 antennas 5.05, 4.42
+// and 4.07 ms.  It takes 8 bytes more of shared memory a segment; problems that
 // only fit without it go without.
 template <typename R, bool kDataShared, bool kFactored>
 __global__ void __launch_bounds__(kOmMaxThreads, OM_MINB) omnical_kernel(const OmParams<R> p) {
@@ -285,7 +318,7 @@ __global__ void __launch_bounds__(kOmMaxThreads, OM_MINB) omnical_kernel(const O
   R* const sw = reinterpret_cast<R*>(sdata + nbls);
   __shared__ int s_prob;
 
-  const int tid = threadIdx.x, nt = blockDim.x;
+  const int tid = threadIdx.x, nt = blockDim.x, nv = p.sum_threads;
   const R one_m = (R)(1.0f - p.gstep);  // formed in float, as the reference
   const R gs = (R)p.gstep;
   const uint2* __restrict__ bl = p.bl;
@@ -319,8 +352,10 @@ __global__ void __launch_bounds__(kOmMaxThreads, OM_MINB) omnical_kernel(const O
     C *sol = solA, *nsol = solB;
 
     // chi^2 of the starting solution (redcal.py:566-577)
-    R chisq = chisq_part(sol, nants, bl, cdata, wgt, nbls), z1 = 0, z2 = 0;
-    block_sum3(chisq, z1, z2, red);
+    R chisq, z1, z2;
+    block_sum3_of<R>(nv, [&](int v, R& x, R&, R&) {
+      x = chisq_part<R>(sol, nants, bl, cdata, wgt, nbls, v, nv);
+    }, chisq, z1, z2, red);
     R conv = 0;
     uint32_t iters = 0;
 
@@ -443,14 +478,16 @@ __global__ void __launch_bounds__(kOmMaxThreads, OM_MINB) omnical_kernel(const O
       }
       // convergence and chi^2 of the stepped solution (calc_conv,
       // calc_chisq, update_active)
-      R nchisq = chisq_part(nsol, nants, bl, cdata, wgt, nbls), csum = 0, cwgt = 0;
-      for (int s = tid; s < nseg; s += nt) {
-        const C x = nsol[s], y = sol[s];
-        const R dx = x.x - y.x, dy = x.y - y.y;
-        csum += dx * dx + dy * dy;
-        cwgt += mag2(x);
-      }
-      block_sum3(nchisq, csum, cwgt, red);
+      R nchisq, csum, cwgt;
+      block_sum3_of<R>(nv, [&](int v, R& x2, R& cs, R& cw) {
+        x2 = chisq_part<R>(nsol, nants, bl, cdata, wgt, nbls, v, nv);
+        for (int s = v; s < nseg; s += nv) {
+          const C x = nsol[s], y = sol[s];
+          const R dx = x.x - y.x, dy = x.y - y.y;
+          cs += dx * dx + dy * dy;
+          cw += mag2(x);
+        }
+      }, nchisq, csum, cwgt, red);
       conv = sqrt(csum / cwgt);
       if (conv < p.conv_crit || nchisq > chisq) break;
       chisq = nchisq;
@@ -877,7 +914,7 @@ DenseFn dense_kernel(int gl, int nb) {
 }
 
 struct Plan {
-  int threads = 64, group = 1, blocks_per_sm = 1, panel = 0, npanels = 1;
+  int threads = 64, sum_threads = 64, group = 1, blocks_per_sm = 1, panel = 0, npanels = 1;
   bool data_shared = false, factored = false;
   size_t smem = 0;
 };
@@ -915,36 +952,44 @@ int make_plan(int nants, int nubls, int nbls, bool factored, int max_threads, Pl
     pl.smem = fixed + sizeof(C) * (size_t)pl.panel;
   }
   pl.blocks_per_sm = std::max(1, per_sm(pl.smem));
+  pl.sum_threads = pl.threads;
   // lanes per segment, a power of two <= 32, from the mean segment length
   // of a panel: float32 (latency-bound) about its square root; float64
   // (bound by the FP64 pipe, where each level of the butterfly over the
-  // lanes costs adds) 2 from a length of 22 on (a CTA of at most 256 threads,
-  // whose lanes are soon all taken: 26), 4 from four times that.  Measured, one
-  // and two lanes: 54 antennas (28.2, 256 threads) 1.38 and 1.27 ms, 45 (23.0)
-  // 1.29 and 1.36, 180 (22.8, 512 threads) 4.36 and 4.08; two and four lanes:
-  // 61 (32.5, 256) 1.32 and 1.44, 135 (34.2, 512) 2.22 and 2.39.
+  // lanes costs adds) 2 from a length of 22 on (26 where data and weights are
+  // in shared memory), 4 from four times that.  Measured, one and two lanes: 54
+  // antennas (28.2, 256 threads) 1.38 and 1.27 ms, 45 (23.0) 1.29 and 1.36, 180
+  // (22.8, panels) 4.36 and 4.08; two and four lanes: 61 (32.5) 1.32 and 1.44,
+  // 135 (34.2, panels) 2.22 and 2.39.
   const double mean = nseg ? 3.0 * pl.panel / nseg : 1.0;
   int g = 1;
   if (sizeof(R) == 4)
     while (g < 32 && 4.0 * g * g <= mean) g *= 2;
   else
-    while (g < 32 && (pl.threads > 256 ? 22.0 : 26.0) * g * g <= mean) g *= 2;
+    while (g < 32 && (pl.data_shared ? 26.0 : 22.0) * g * g <= mean) g *= 2;
   pl.group = g;
   *out = pl;
   return HV_OK;
 }
 
-// The plan of a call.  Float64 takes CTAs of 256 threads where all baselines or
-// half of them fit in shared memory: more problems an SM, whose barriers and
-// serial sums overlap.  Measured, 512 and 256 threads: 37 antennas 1.09 and 0.96
-// ms, 70 (two CTAs of either) 1.26 and 1.16, 90 (one panel and two) 1.95 and
-// 1.93; 100 (one panel and three) 1.80 and 2.02, 180 4.36 and 7.16.
+// The plan of a call.  Float64 problems whose data and weights are in shared
+// memory take CTAs of 256 threads where a call has more than two problems an
+// SM: more of them share it, and their barriers and serial sums overlap (54
+// antennas, 1000 problems of 12 iterations: 1.43 and 1.35 ms; 37 antennas, 1500:
+// 1.15 and 1.02), while few problems end sooner with 512 threads each (77
+// antennas, 15 problems: 0.50 and 0.40 ms of 256 and 512).  Both
+// sum in the same order, so that a problem gives the same result alone or among
+// others.
 template <typename R>
-int choose_plan(int nants, int nubls, int nbls, bool factored, Plan* out) {
-  if (sizeof(R) == 8 && make_plan<R>(nants, nubls, nbls, factored, 256, out) == HV_OK &&
-      out->npanels <= 2)
-    return HV_OK;
-  return make_plan<R>(nants, nubls, nbls, factored, kOmMaxThreads, out);
+int choose_plan(int nants, int nubls, int nbls, bool factored, int ndata, int num_sms, Plan* out) {
+  const int r = make_plan<R>(nants, nubls, nbls, factored, kOmMaxThreads, out);
+  Plan few;
+  if (sizeof(R) == 8 && r == HV_OK && out->data_shared && ndata > 2 * num_sms &&
+      make_plan<R>(nants, nubls, nbls, factored, 256, &few) == HV_OK && few.data_shared) {
+    few.sum_threads = out->threads;
+    *out = few;
+  }
+  return r;
 }
 
 int fail(hv_context* ctx, int code, const char* msg) {
@@ -1094,14 +1139,14 @@ int run_typed(hv_context* ctx, const uint32_t* ggu, int nbls, void* d_gains, int
                        d_conv, st);
   }
   Plan pl;
-  if ((sizeof(R) == 4 || choose_plan<R>(nants, nubls, nbls, true, &pl) != HV_OK) &&
-      choose_plan<R>(nants, nubls, nbls, false, &pl) != HV_OK)
+  const int nsm = std::max(1, hv_context_num_sms(ctx));
+  if ((sizeof(R) == 4 || choose_plan<R>(nants, nubls, nbls, true, ndata, nsm, &pl) != HV_OK) &&
+      choose_plan<R>(nants, nubls, nbls, false, ndata, nsm, &pl) != HV_OK)
     return fail(ctx, HV_ERR_ARG, "omnical: too many antennas and unique baselines for one CTA");
   std::vector<uint2> bl;
   std::vector<int> off;
   std::vector<uint32_t> ent;
   build_csr(ggu, nbls, nants, nubls, pl.panel, pl.npanels, sizeof(R) == 8, bl, off, ent);
-  const int nsm = std::max(1, hv_context_num_sms(ctx));
   const int grid = std::max(1, std::min(ndata, pl.blocks_per_sm * nsm));
   const size_t n_bl = sizeof(uint2) * bl.size(), n_off = sizeof(int) * off.size(),
                n_ent = sizeof(uint32_t) * ent.size();
@@ -1162,6 +1207,7 @@ int run_typed(hv_context* ctx, const uint32_t* ggu, int nbls, void* d_gains, int
     p.check_every = check_every;
     p.check_after = check_after;
     p.group = pl.group;
+    p.sum_threads = pl.sum_threads;
     p.counter = reinterpret_cast<int*>(b8 + o_cnt);
     constexpr bool kF = sizeof(R) == 8;
     if (pl.factored)

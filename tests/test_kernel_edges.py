@@ -263,6 +263,26 @@ def test_omnical_float64_layouts(nants):
     np.testing.assert_array_equal(got["iters"], ref["iters"])
 
 
+# a float64 problem gives the same bits in a call of many problems (CTAs of 256
+# threads) as alone (up to 512)
+@gpu
+@pytest.mark.parametrize("nants", [37, 54, 70])
+def test_omnical_float64_alone_and_among_many(nants):
+    from hera_gpu_gb300 import omnical
+    ggu, nubls = synth.hex_redundant_layout(nants)
+    a = [np.concatenate([x] * 110) for x in
+         synth.redundant_data(ggu, nubls, 3, seed=nants, noise=0.05)]
+    many = omnical(ggu, *[x.astype(t) for x, t in zip(a, (np.complex128, np.complex128,
+                                                          np.complex128, np.float64))],
+                   1e-10, 12, precision=2)
+    one = omnical(ggu, *[x[:3].astype(t) for x, t in zip(a, (np.complex128, np.complex128,
+                                                             np.complex128, np.float64))],
+                  1e-10, 12, precision=2)
+    for x in ("gains", "ubls", "chisq", "iters", "conv"):
+        np.testing.assert_array_equal(many[x][-3:], one[x])
+        np.testing.assert_array_equal(many[x][:3], one[x])
+
+
 # antenna blocks of the fused forms (32, 64, 96 and 128 rows; one to five
 # blocks), at their edges
 @gpu
