@@ -20,25 +20,34 @@
 //   * class sums go to 64-bit integers in global memory (two neighbouring
 //     classes a word, added with integer reductions: exact and independent of
 //     order), and are converted once, smallest class first, in FP64.
-// The result is deterministic, and its distance from an exact evaluation is
-// set by the rounding of U (the phases themselves are formed in integers):
-// relative Frobenius errors against 113-bit arithmetic of 3.6e-15 at 16
+// The result is deterministic.  What the rounding to 59 bits and the dropped
+// classes lose is relative to the two antennas' largest components, M_a M_b:
+// about 2^-59 sqrt(n) M_a M_b over n sources.  An FP64 sum loses 2^-53 of its
+// partial sums instead, which are small where two antennas are bright on
+// different sources.  So the two amplitudes' overlap is formed along with the
+// class sums, and a slice with a pair of antennas whose overlap is too small for
+// the digits to be at least as exact as the FP64 sum takes the SIMT product
+// (kOverlapMin).  Elsewhere the distance from an exact evaluation is set by the
+// rounding of U (the phases themselves are formed in integers): relative
+// Frobenius errors against 113-bit arithmetic of 3.6e-15 at 16
 // antennas x 1000 sources (SIMT product 4.0e-15), 5.5e-15 at 40 x 2000
 // (6.9e-15), and 2.2e-16 on a 2.5 m array, where the phases are exact enough to
 // show the product (1.1e-15).
 //
 // Measured on GB300, one slice of 350 antennas x 50k sources above the horizon
-// (ncu): phasors 0.33 ms, digits 0.25 ms, class sums 0.72 ms (0.63 of a call of
-// more slices), conversion 0.02 ms; with SIMT 1.30 ms and 32.8 ms.  A call of 3
-// such slices 102.6 -> 3.74 ms.
+// (ncu): phasors 0.33 ms, digits 0.26 ms, class sums and overlaps 0.74 ms,
+// conversion 0.02 ms; with SIMT 1.30 ms and 32.8 ms.  A call of 3 such slices
+// 102.6 -> 3.87 ms (3.73 without the overlaps).
 //
-// Slices whose phasors are not finite, or whose antenna scales leave
-// [2^-400, 2^400], are flagged on the device and take the SIMT product of
-// hv_plain.cu from the same phasors.
+// Slices whose phasors are not finite, whose antenna scales leave
+// [2^-400, 2^400], or with a pair of antennas of too little overlap are flagged
+// on the device and take the SIMT product of hv_plain.cu from the same phasors.
 //
 //   gen64      phasors in FP64 to HBM, and the largest component per antenna
 //   digits64   phasors -> digit tiles, in the layout the MMAs read
-//   mma64      class sums (TMA bulk copies, tcgen05, integer reductions)
+//   mma64      class sums and overlaps (TMA bulk copies, tcgen05, integer
+//              reductions)
+//   overlap64  flags the slices with a pair of too little overlap
 //   final64    class sums (or the SIMT chunks of a flagged slice) -> output
 #include <algorithm>
 
@@ -270,13 +279,44 @@ __device__ __forceinline__ long long scaled_int(double v, int field) {
   return (b >> 63) ? -(long long)x : (long long)x;
 }
 
+// Overlap of antennas a and b over the sources of a window: sum_s w_a w_b with
+// the weights w = 256 (m / 2^E)^2, m the larger component of the phasor and 2^E
+// the power of two above the antenna's largest, rounded down to 4 significant
+// bits (exact in E4M3).  It is 2^16 P^2 for the FP64 sum's typical partial sum P
+// in units of 2^(E_a + E_b), where that sum rounds by about 2^-54.3 P sqrt(min(n,
+// kPlainChunk)) and the digits by 2^-59.4 sqrt(n) (root mean squares of rounding
+// errors spread evenly): the digits are the more exact from 2^5.8 = 56 on for n up
+// to kPlainChunk, and in proportion to n beyond.  Arrays of Airy or random beams
+// over 150 to 100k sources lie at 5 to 600 times this limit.
+constexpr int kOverlapMin = 64;
+// A chunk's sum is capped here: exact in FP32 below, 256 chunks fit in 32 bits,
+// and the limit never exceeds 1024.
+constexpr float kOverlapCap = 1048576.f;
+
+// Where a slice's weights start in its digits.
+__device__ __forceinline__ size_t weight_tiles(const F64Dims& d) {
+  return (size_t)(d.Np / 128) * d.nks * (kPlanes * kTile);
+}
+// A component (its high word) in units of 2^-15 of the scale, rounded down.
+__device__ __forceinline__ uint32_t top15(int hi, int field) {
+  const int ex = (hi >> 20) & 0x7ff;
+  return ex > field - 16 ? (uint32_t)((hi & 0xfffff) | 0x100000) >> (6 + field - ex) : 0u;
+}
+// E4M3 code of the weight of m units.
+__device__ __forceinline__ uint32_t weight_code(uint32_t m) {
+  const uint32_t w = m * m >> 22;
+  const int e = 31 - __clz(w | 1u);
+  return w ? (uint32_t)((e + 7) << 3) | ((w << 3 >> e) & 7u) : 0u;
+}
+
 // Digit tiles: [slice][antenna block][source step of 32][plane][4096], a plane
 // tile in the K-major core-matrix layout the MMAs read without a swizzle (8
 // antennas x 16 sources a 128-byte core matrix; the two along the sources
 // adjacent, then the next 8 antennas), so that every group of planes of a
 // step is one contiguous bulk copy.  One block makes a step: thread (antenna,
-// half of the step, component) 16 sources.  Bound by HBM (16 B read, 24 B
-// written a phasor).
+// half of the step, component) 16 sources, and the weights of 8 of them, whose
+// tiles lie behind the digits, [antenna block][source step][4096].  Bound by HBM
+// (16 B read, 25 B written a phasor).
 __global__ void __launch_bounds__(512)
 digits64_kernel(const F64Dims d, const double2* __restrict__ v,
                 const uint32_t* __restrict__ rowmax, uint8_t* __restrict__ dig,
@@ -326,13 +366,28 @@ digits64_kernel(const F64Dims d, const double2* __restrict__ v,
       }
     }
   }
-  uint8_t* out = dig + (size_t)z * d.dig_stride +
-                 ((size_t)blk * d.nks + ks) * (size_t)(kPlanes * kTile) + ri * kTile +
-                 (row >> 3) * 256 + half * 128 + (row & 7) * 16;
+  const size_t tile = (size_t)blk * d.nks + ks;
+  const int at = (row >> 3) * 256 + half * 128 + (row & 7) * 16;
+  uint8_t* zd = dig + (size_t)z * d.dig_stride;
+  uint8_t* out = zd + tile * (kPlanes * kTile) + ri * kTile + at;
 #pragma unroll
   for (int k = 0; k < kDig; ++k)
     *reinterpret_cast<uint4*>(out + (size_t)k * 2 * kTile) =
         make_uint4(w[k][0], w[k][1], w[k][2], w[k][3]);
+  // the weights of the thread's half of the 16 sources, from both components
+  // (their high words, read again: with them the loop above took 83 registers,
+  // one block an SM instead of two)
+  uint32_t wt[2] = {0, 0};
+#pragma unroll
+  for (int e = 0; e < 8; ++e) {
+    const int s = ks * 32 + half * 16 + ri * 8 + e;
+    if (rm != 0 && ok && s < n) {
+      const int4 h = *reinterpret_cast<const int4*>(src - ri + 2 * (size_t)s * d.Np);
+      wt[e >> 2] |= weight_code(max(top15(h.y, field), top15(h.w, field))) << (8 * (e & 3));
+    }
+  }
+  *reinterpret_cast<uint2*>(zd + weight_tiles(d) + tile * kTile + at + 8 * ri) =
+      make_uint2(wt[0], wt[1]);
 }
 
 // --------------------------------------------------------------- mma64 ----
@@ -350,13 +405,17 @@ digits64_kernel(const F64Dims d, const double2* __restrict__ v,
 // two digits 2 k and 2 k + 1 (the even classes 4 k and 4 k + 2, words 2 k and
 // 2 k + 1), and the conversion takes (S + S^H) / 2: 42 digit pairs instead
 // of 78, and the digits are read once.  Three blocks: 0.93 -> 0.86 ms a slice.
-constexpr int kUnits = 9;
-__constant__ int8_t kUnit[kUnits][3] = {{5, 0, 5}, {5, 6, 11}, {2, 0, 5}, {4, 0, 4}, {4, 5, 9},
+//
+// The last unit of a pair of blocks sums the overlaps, one product of the weights
+// a step; its stages take as many steps as fit.
+constexpr int kDigUnits = 9, kUnits = kDigUnits + 1;
+__constant__ int8_t kUnit[kDigUnits][3] = {{5, 0, 5}, {5, 6, 11}, {2, 0, 5}, {4, 0, 4}, {4, 5, 9},
                                         {3, 0, 3}, {3, 4, 7},  {1, 0, 3}, {0, 0, 1}};
 // {g, 0} or {k, 1} of a block with itself
-__constant__ int8_t kOwnUnit[kUnits][2] = {{5, 0}, {4, 0}, {3, 0}, {2, 0}, {1, 0},
+__constant__ int8_t kOwnUnit[kDigUnits][2] = {{5, 0}, {4, 0}, {3, 0}, {2, 0}, {1, 0},
                                            {0, 1}, {1, 1}, {2, 1}, {0, 0}};
 constexpr int kMaxA = 6, kMaxB = 7;        // digits a unit needs of A and of B
+constexpr int kOverSteps = 2 * kMaxA;      // steps of weights a stage holds
 constexpr int kStageBytes = (kMaxA + kMaxB) * 2 * kTile;
 constexpr int kStages = 2;
 constexpr int kMmaSmem = kStages * kStageBytes + 128;
@@ -411,10 +470,12 @@ mma64_kernel(const F64Dims d, const uint8_t* __restrict__ dig, const int* __rest
   for (const int nb = d.Np / 128; J >= nb - I; ++I) J -= nb - I;
   J += I;
   // digits of A and of B
-  const bool own = I == J, same = own && kOwnUnit[unit][1];
-  const int g = own ? kOwnUnit[unit][0] : kUnit[unit][0];
-  const int i0 = same ? 2 * g : own ? 0 : kUnit[unit][1];
-  const int i1 = same ? 2 * g + 1 : own ? g : kUnit[unit][2];
+  const bool over = unit == kDigUnits;
+  const int du = over ? 0 : unit;
+  const bool own = I == J, same = own && (over || kOwnUnit[du][1]);
+  const int g = own ? kOwnUnit[du][0] : kUnit[du][0];
+  const int i0 = same ? 2 * g : own ? 0 : kUnit[du][1];
+  const int i1 = same ? 2 * g + 1 : own ? g : kUnit[du][2];
   const int j0 = same ? i0 : own ? g + 1 : max(0, 2 * g - i1);
   const int j1 = same ? i1 : 2 * g + 1 - i0;
   const uint32_t base = smem_u32(smem);
@@ -446,19 +507,23 @@ mma64_kernel(const F64Dims d, const uint8_t* __restrict__ dig, const int* __rest
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *holder;
-  const int nsteps = k1 - k0;
+  // pipeline steps: one source step, or kOverSteps of them
+  const int nsteps = over ? ceil_div(k1 - k0, kOverSteps) : k1 - k0;
   if (warp == 0 && lane == 0) {
     // producer: the unit's A planes and B planes of each step, contiguous
-    const size_t step_bytes = (size_t)kPlanes * kTile;
-    const uint8_t* zd = dig + (size_t)z * d.dig_stride;
-    const uint8_t* pa = zd + ((size_t)I * d.nks + k0) * step_bytes + (size_t)i0 * 2 * kTile;
-    const uint8_t* pb = zd + ((size_t)J * d.nks + k0) * step_bytes + (size_t)j0 * 2 * kTile;
-    const uint32_t na = (uint32_t)(i1 - i0 + 1) * 2 * kTile, nb = (uint32_t)(j1 - j0 + 1) * 2 * kTile;
+    const size_t step_bytes = (size_t)(over ? kOverSteps : kPlanes) * kTile;
+    const uint8_t* zd = dig + (size_t)z * d.dig_stride + (over ? weight_tiles(d) : 0);
+    const size_t block = (size_t)d.nks * (over ? 1 : kPlanes) * kTile;
+    const size_t first = (size_t)k0 * (over ? 1 : kPlanes) * kTile;
+    const uint8_t* pa = zd + I * block + first + (over ? 0 : i0 * 2 * kTile);
+    const uint8_t* pb = zd + J * block + first + (over ? 0 : j0 * 2 * kTile);
+    uint32_t na = (uint32_t)(i1 - i0 + 1) * 2 * kTile, nb = (uint32_t)(j1 - j0 + 1) * 2 * kTile;
     int k = 0;
     for (; k < nsteps; ++k, pa += step_bytes, pb += step_bytes) {
       const int s = k % kStages;
       if (!wait1(empty(s), ((k / kStages) & 1) ^ 1, abort_flag, err, wait_ns)) break;
       const uint32_t st = base + (uint32_t)s * kStageBytes;
+      if (over) na = nb = (uint32_t)min(kOverSteps, k1 - k0 - k * kOverSteps) * kTile;
       mbar_expect_tx(full(s), same ? na : na + nb);
       bulk_load(st, pa, na, full(s));
       if (!same) bulk_load(st + kMaxA * 2 * kTile, pb, nb, full(s));
@@ -476,8 +541,11 @@ mma64_kernel(const F64Dims d, const uint8_t* __restrict__ dig, const int* __rest
       const uint32_t a0 = plain_desc_lo(st);
       const uint32_t b0 = same ? a0 : plain_desc_lo(st + kMaxA * 2 * kTile);
       constexpr uint32_t kP = kTile >> 4;  // descriptor units of a plane
+      if (over)
+        for (int t = 0; t < min(kOverSteps, k1 - k0 - k * kOverSteps); ++t)
+          mma64(tmem, a0 + t * kP, b0 + t * kP, idp, k > 0 || t > 0);
 #pragma unroll 1
-      for (int q = 0; q < 2; ++q) {
+      for (int q = 0; q < (over ? 0 : 2); ++q) {
         const uint32_t dre = tmem + 256u * q, dim = dre + 128u;
         uint32_t acc = k > 0;
         for (int i = i0; i <= i1; ++i) {
@@ -509,11 +577,21 @@ mma64_kernel(const F64Dims d, const uint8_t* __restrict__ dig, const int* __rest
     unsigned long long* w = reinterpret_cast<unsigned long long*>(W) + (size_t)z * d.w_stride +
                             (size_t)(2 * (same ? 2 * g : g) + ri) * plane +
                             (size_t)J * 128 * d.Np + a;
+    uint32_t* wo = reinterpret_cast<uint32_t*>(W + (size_t)z * d.w_stride + 2 * kGroups * plane) +
+                   (size_t)J * 128 * d.Np + a;
     const uint32_t tq = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)ri * 128u;
     const long long weight = own ? 2 : 1;
     const bool no_hi = own && !same && g == 0;  // (no pair i < j in class 0)
 #pragma unroll 1
-    for (int c = 0; c < 128; c += 32) {
+    for (int c = 0; c < (over ? ri ? 0 : 128 : 0); c += 32) {
+      float x[32];
+      tmem_ld32(tq + c, x);
+#pragma unroll
+      for (int k = 0; k < 32; ++k)
+        atomicAdd(wo + (size_t)(c + k) * d.Np, (uint32_t)fminf(x[k], kOverlapCap));
+    }
+#pragma unroll 1
+    for (int c = over ? 128 : 0; c < 128; c += 32) {
       float hi[32], lo[32];
       tmem_ld32(tq + c, hi);
       tmem_ld32(tq + 256u + c, lo);
@@ -537,6 +615,28 @@ mma64_kernel(const F64Dims d, const uint8_t* __restrict__ dig, const int* __rest
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512)
                  : "memory");
   }
+}
+
+// ----------------------------------------------------------- overlap64 ----
+// Flags the slices with a pair of antennas, neither of zeros, whose overlap is
+// below the limit.
+__global__ void __launch_bounds__(256)
+overlap64_kernel(const F64Dims d, const long long* __restrict__ W,
+                 const uint32_t* __restrict__ rowmax, int* __restrict__ flags) {
+  const int z = blockIdx.y, n = window_count(d, z);
+  const unsigned long long limit = (unsigned long long)kOverlapMin * max(n, kPlainChunk);
+  const uint32_t* rm = rowmax + (size_t)z * d.Np;
+  const uint32_t* o = reinterpret_cast<const uint32_t*>(W + (size_t)z * d.w_stride +
+                                                        (size_t)2 * kGroups * d.Np * d.Np);
+  const int b = blockIdx.x * 8 + (threadIdx.x >> 5);
+  if (n == 0 || b >= d.nant || rm[b] == 0) return;
+  bool low = false;
+#pragma unroll 4
+  for (int a = threadIdx.x & 31; a <= b; a += 32) {
+    const unsigned long long x = o[(size_t)b * d.Np + a];
+    low |= rm[a] != 0 & x * kPlainChunk < limit;
+  }
+  if (low) atomicOr(flags + z, 1);
 }
 
 // ------------------------------------------------------------- final64 ----
@@ -635,11 +735,13 @@ final64_kernel(const F64Dims d, const long long* __restrict__ W,
 
 size_t f64_digit_bytes(int Np, int S) {
   // a flagged slice keeps its SIMT chunk sums here
-  const size_t dig = (size_t)kPlanes * (Np / 128) * (size_t)ceil_div(S, 32) * kTile;
+  const size_t dig = (size_t)(kPlanes + 1) * (Np / 128) * (size_t)ceil_div(S, 32) * kTile;
   const size_t part = sizeof(double) * 2 * (size_t)Np * Np * ceil_div(S, kPlainChunk);
   return std::max(dig, part);
 }
-size_t f64_word_bytes(int Np) { return sizeof(long long) * 2 * kGroups * (size_t)Np * Np; }
+size_t f64_word_bytes(int Np) {
+  return (sizeof(long long) * 2 * kGroups + sizeof(uint32_t)) * (size_t)Np * Np;
+}
 size_t f64_table_bytes() { return sizeof(longlong2) * kTable; }
 
 cudaError_t launch_f64_table(void* table, cudaStream_t st) {
@@ -673,7 +775,7 @@ cudaError_t launch_f64_product(const F64Dims& d, int nz, const void* v, const ui
   // item's start and its reductions take as long as some 20 steps (200
   // antennas x 50k sources 550 us a call at 12 items an SM, 499 at 4, 500 at
   // 3); at least 8 steps
-  const long long units = (long long)kUnits * npairs * nz;
+  const long long units = (long long)kDigUnits * npairs * nz;
   const long long per_sm = (units * std::max(1, d.nks / 2) + num_sms - 1) / num_sms;
   const int steps = (int)std::min<long long>(kMaxChunkSteps, std::max<long long>(8, per_sm / 4));
   const int nchunks = ceil_div(d.nks, steps);
@@ -681,6 +783,9 @@ cudaError_t launch_f64_product(const F64Dims& d, int nz, const void* v, const ui
   mma64_kernel<<<items, kMmaThreads, kMmaSmem, st>>>(
       d, static_cast<const uint8_t*>(dig), flags, W, npairs, nchunks, steps, err,
       wait_ns ? wait_ns : 10000000000ull);
+  e = cudaGetLastError();
+  if (e != cudaSuccess) return e;
+  overlap64_kernel<<<dim3(ceil_div(d.nant, 8), nz), 256, 0, st>>>(d, W, rowmax, flags);
   return cudaGetLastError();
 }
 

@@ -56,9 +56,10 @@ typedef enum {
   HV_METHOD_AUTO = 0,     /* tensor-core form for precision 1, FP64 for 2      */
   HV_METHOD_PLAIN = 1,    /* the reference's method: phasors to HBM, then a
                              Hermitian product: FP32 SIMT (precision 1); FP64
-                             (precision 2) formed exactly from scaled integers
-                             on the FP8 tensor cores, or FP64 SIMT where that
-                             does not apply                                    */
+                             (precision 2) formed from scaled integers on the
+                             FP8 tensor cores, or FP64 SIMT for slices where
+                             that would be less exact (antennas that are
+                             bright on different sources) or does not apply    */
   HV_METHOD_TC_BF16 = 2,  /* fused: phasors generated in shared memory, split
                              BF16 tcgen05 products, FP32 accumulation in TMEM  */
   HV_METHOD_TC_FP16 = 3   /* fused, FP16 hi products and E4M3 (FP8) cross
