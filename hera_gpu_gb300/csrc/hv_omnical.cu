@@ -570,6 +570,33 @@ size_t dense_smem(int nants, int nubls, int groups) {
          sizeof(float) * (2 * nseg + 96) + 16;
 }
 
+// Sum of the n partial sums part(i), each cleared after it was read (clear(i)):
+// four running sums, added pairwise at the end, since one running sum's error
+// grows with its 16 or 32 additions (gains of 53 antennas after 12 iterations
+// 9.7e-8 from 64 bits, 7.8e-8 this way and in the general kernel).
+template <typename V, typename Part, typename Clear>
+__device__ __forceinline__ V sum_parts(int n, Part part, Clear clear) {
+  V a[4] = {V{}, V{}, V{}, V{}};
+  int i = 0;
+#pragma unroll 1
+  for (; i + 4 <= n; i += 4) {
+    V x[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) x[q] = part(i + q);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      clear(i + q);
+      a[q] = a[q] + x[q];
+    }
+  }
+#pragma unroll 1
+  for (; i < n; ++i) {
+    a[0] = a[0] + part(i);
+    clear(i);
+  }
+  return (a[0] + a[1]) + (a[2] + a[3]);
+}
+
 template <int GL, int NB>
 __global__ void __launch_bounds__(kDenseThreads, NB <= 6 ? 3 : 2)
 omnical_dense_kernel(const DenseParams p) {
@@ -719,16 +746,17 @@ omnical_dense_kernel(const DenseParams p) {
           if (cb * GL + gl < nants) colsum[grp * nants + cb * GL + gl].x = col[cb];
         __syncthreads();
         for (int s = tid; s < nseg; s += nt) {
-          R v = 0;
+          R v;
           if (s < nants) {
-            v = s ? rowsum[s].x : R(0);
-            for (int g = 0; g < ngroups; ++g) v += colsum[g * nants + s].x;
+            v = sum_parts<RealV<R>>(
+                    ngroups, [&](int g) { return RealV<R>{colsum[g * nants + s].x}; },
+                    [](int) {}).v;
+            if (s) v += rowsum[s].x;
           } else {
-            for (int c = 0; c < 2 * ngroups; ++c) {
-              C& u = ucopy[c * nubls + (s - nants)];
-              v += u.x;
-              u.x = 0;
-            }
+            C* const u = ucopy + (s - nants);
+            v = sum_parts<RealV<R>>(
+                    2 * ngroups, [&](int c) { return RealV<R>{u[c * nubls].x}; },
+                    [&](int c) { u[c * nubls].x = 0; }).v;
           }
           gw[s] = v;
         }
@@ -783,21 +811,25 @@ omnical_dense_kernel(const DenseParams p) {
       __syncthreads();
       const bool rebase = (it + 1) % p.check_every == 1;
       for (int s = tid; s < nseg; s += nt) {
-        C v{};
+        CplxV<R> v;
         if (s < nants) {
-          if (s) v = rowsum[s];
-          for (int g = 0; g < ngroups; ++g) {
-            const C t = colsum[g * nants + s];
-            v.x += t.x;
-            v.y += t.y;
-          }
+          v = sum_parts<CplxV<R>>(
+              ngroups,
+              [&](int g) {
+                const C t = colsum[g * nants + s];
+                return CplxV<R>{t.x, t.y};
+              },
+              [](int) {});
+          if (s) v = v + CplxV<R>{rowsum[s].x, rowsum[s].y};
         } else {
-          for (int c = 0; c < 2 * ngroups; ++c) {
-            C& u = ucopy[c * nubls + (s - nants)];
-            v.x += u.x;
-            v.y += u.y;
-            u = C{};
-          }
+          C* const u = ucopy + (s - nants);
+          v = sum_parts<CplxV<R>>(
+              2 * ngroups,
+              [&](int c) {
+                const C t = u[c * nubls];
+                return CplxV<R>{t.x, t.y};
+              },
+              [&](int c) { u[c * nubls] = C{}; });
         }
         C f;
         f.x = one_m + gs * v.x / gw[s];
