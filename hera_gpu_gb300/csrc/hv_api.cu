@@ -30,6 +30,7 @@ namespace {
 struct DevBuf {
   void* p = nullptr;
   size_t cap = 0;
+  uint64_t call = 0;  // the last call that used it
 };
 struct HostBuf {
   void* p = nullptr;
@@ -51,6 +52,7 @@ struct hv_context {
   cudaEvent_t joined = nullptr;
   size_t budget = 0;  // 0 = unlimited
   size_t held = 0;
+  uint64_t call = 0;  // visibility calls so far
   std::string err;
   uint64_t launches = 0;
   int* d_err = nullptr;  // device-side error flag (bounded waits)
@@ -69,9 +71,7 @@ struct hv_context {
   // workspace
   DevBuf freqs, beamT, ucoef, rec, counts, blkcounts, v, partial, tcgroups;
   DevBuf umax, sortkv, crd_sorted, I_sorted, tctable, pixmax, sbound;
-  // tensor-core FP64 product: given back when another path finds no room
-  DevBuf f64_v, f64_digits, f64_words, f64_small;
-  bool f64_running = false;
+  DevBuf f64_v, f64_digits, f64_words, f64_small;  // tensor-core FP64 product
   HostBuf tctable_h;  // page-locked staging of the fused kernel's simulation table
   // page-locked staging of small host-API calls: the error flag (the first
   // kStageHead bytes), then the inputs or the output; at most kStageBytes
@@ -129,20 +129,41 @@ void release(hv_context* ctx, DevBuf& b) {
   b.cap = 0;
 }
 
-// Gives the FP64 product's workspace back (unless it is in use); false if
-// there was none.  The device is idle: ensure() has waited for it.
-bool release_f64(hv_context* ctx) {
-  if (ctx->f64_running) return false;
+template <typename F>
+void each_buffer(hv_context* ctx, F f) {
+  for (DevBuf* b : {&ctx->in_antpos, &ctx->in_eq2tops, &ctx->in_crd, &ctx->in_I, &ctx->in_bm,
+                    &ctx->out_vis, &ctx->freqs, &ctx->beamT, &ctx->ucoef, &ctx->rec, &ctx->counts,
+                    &ctx->blkcounts, &ctx->v, &ctx->partial, &ctx->tcgroups, &ctx->umax,
+                    &ctx->sortkv, &ctx->crd_sorted, &ctx->I_sorted, &ctx->tctable, &ctx->pixmax,
+                    &ctx->sbound, &ctx->f64_v, &ctx->f64_digits, &ctx->f64_words,
+                    &ctx->f64_small})
+    f(*b);
+}
+
+// Workspace that earlier calls have left and the present one has not used: it
+// is kept for the next call of its kind, but never stands against a call that
+// finds no room.  What a call is given so does not depend on the calls before it.
+bool idle(const hv_context* ctx, const DevBuf& b) { return b.p && b.call != ctx->call; }
+size_t idle_bytes(hv_context* ctx) {
+  size_t n = 0;
+  each_buffer(ctx, [&](DevBuf& b) { n += idle(ctx, b) ? b.cap : 0; });
+  return n;
+}
+// Gives the idle workspace back; false if there was none.  The device must have
+// been waited for.
+bool release_idle(hv_context* ctx) {
   bool any = false;
-  for (DevBuf* b : {&ctx->f64_v, &ctx->f64_digits, &ctx->f64_words, &ctx->f64_small}) {
-    any = any || b->p;
-    release(ctx, *b);
-  }
+  each_buffer(ctx, [&](DevBuf& b) {
+    if (!idle(ctx, b)) return;
+    release(ctx, b);
+    any = true;
+  });
   return any;
 }
 
 int ensure(hv_context* ctx, DevBuf& b, size_t bytes) {
   if (bytes == 0) bytes = 256;
+  b.call = ctx->call;
   if (b.cap >= bytes) return HV_OK;
   // the old buffer may still be read by queued work (on any stream)
   HV_CK(cudaDeviceSynchronize());
@@ -154,12 +175,12 @@ int ensure(hv_context* ctx, DevBuf& b, size_t bytes) {
   }
   size_t want = bytes + bytes / 8;  // slack against regrowth
   if (ctx->budget && ctx->held + want > ctx->budget) want = bytes;
-  if (ctx->budget && ctx->held + want > ctx->budget) release_f64(ctx);
+  if (ctx->budget && ctx->held + want > ctx->budget) release_idle(ctx);
   if (ctx->budget && ctx->held + want > ctx->budget)
     return fail(ctx, HV_ERR_OOM, "workspace of %zu bytes exceeds the HBM budget (%zu held of %zu)",
                 want, ctx->held, ctx->budget);
   cudaError_t e = cudaMalloc(&b.p, want);
-  if (e == cudaErrorMemoryAllocation && release_f64(ctx)) {
+  if (e == cudaErrorMemoryAllocation && release_idle(ctx)) {
     cudaGetLastError();
     e = cudaMalloc(&b.p, want);
   }
@@ -175,12 +196,31 @@ int ensure(hv_context* ctx, DevBuf& b, size_t bytes) {
 
 // Whether buffers can grow to the wanted sizes, ensure()'s slack included,
 // within the budget: asked before any of them grows, since one grown for more
-// work than fits would leave less room for the others.
-bool fits(const hv_context* ctx, const std::pair<DevBuf*, size_t>* want, size_t n) {
-  size_t grow = 0;
-  for (size_t i = 0; i < n; ++i)
-    grow += want[i].second > want[i].first->cap ? want[i].second - want[i].first->cap : 0;
-  return !ctx->budget || ctx->held + grow + grow / 8 + 256 * n <= ctx->budget;
+// work than fits would leave less room for the others.  Buffers that an earlier
+// call has grown beyond these sizes are given back where that makes the room; the
+// present call must not have used them yet.
+bool fits(hv_context* ctx, const std::pair<DevBuf*, size_t>* want, size_t n) {
+  auto slack = [](size_t bytes) { return bytes + bytes / 8 + 256; };
+  auto room = [&] {
+    size_t old = 0, grown = 0;
+    for (size_t i = 0; i < n; ++i) {
+      want[i].first->call = ctx->call;
+      if (want[i].second <= want[i].first->cap) continue;
+      old += want[i].first->cap;
+      grown += slack(want[i].second);
+    }
+    if (grown == 0) return true;
+    return !ctx->budget || ctx->held - idle_bytes(ctx) - old + grown <= ctx->budget;
+  };
+  if (room()) return true;
+  bool larger = false;
+  for (size_t i = 0; i < n; ++i) {
+    if (want[i].first->cap <= slack(want[i].second)) continue;
+    if (!larger) cudaDeviceSynchronize();
+    release(ctx, *want[i].first);
+    larger = true;
+  }
+  return larger && room();
 }
 
 // Page-locked host buffer that stays valid for the copies queued from it.
@@ -264,15 +304,11 @@ int run_f64(hv_context* ctx, const double* eq2tops, const double* crd_eq, const 
   long long nz = std::max<long long>(1, std::min<long long>(
       std::min<long long>(32768, (long long)ntimes * nfreq), (long long)(kF64Cap / per)));
   int ntb = 0, nfb = 0;
-  struct Running {
-    hv_context* c;
-    ~Running() { c->f64_running = false; }
-  } running{ctx};
   for (;; nz /= 2) {
-    ctx->f64_running = nz > 0;
     if (nz == 0) {
-      cudaDeviceSynchronize();
-      release_f64(ctx);
+      // the SIMT product takes what was found of the room
+      for (DevBuf* b : {&ctx->f64_v, &ctx->f64_digits, &ctx->f64_words, &ctx->f64_small})
+        b->call = 0;
       return -1;
     }
     nfb = (int)std::min<long long>(nfreq, nz);
@@ -709,13 +745,7 @@ int hv_destroy(hv_context* ctx) {
   if (!ctx) return HV_OK;
   cudaSetDevice(ctx->device);
   if (ctx->stream) cudaStreamSynchronize(ctx->stream);
-  DevBuf* bufs[] = {&ctx->in_antpos, &ctx->in_eq2tops, &ctx->in_crd, &ctx->in_I, &ctx->in_bm,
-                    &ctx->out_vis, &ctx->freqs, &ctx->beamT, &ctx->ucoef, &ctx->rec,
-                    &ctx->counts, &ctx->blkcounts, &ctx->v, &ctx->partial, &ctx->tcgroups,
-                    &ctx->umax, &ctx->sortkv, &ctx->crd_sorted, &ctx->I_sorted, &ctx->tctable,
-                    &ctx->pixmax, &ctx->sbound, &ctx->f64_v, &ctx->f64_digits,
-                    &ctx->f64_words, &ctx->f64_small};
-  for (DevBuf* b : bufs) release(ctx, *b);
+  each_buffer(ctx, [&](DevBuf& b) { release(ctx, b); });
   if (ctx->tctable_h.p) cudaFreeHost(ctx->tctable_h.p);
   if (ctx->stage_h.p) cudaFreeHost(ctx->stage_h.p);
   for (auto& hp : ctx->host_pool) cudaFreeHost(hp.first);
@@ -758,6 +788,7 @@ int hv_vis_multifreq_device(hv_context* ctx, int precision, int method, const vo
     return fail(ctx, HV_ERR_ARG, "null array argument");
   HV_CK(cudaSetDevice(ctx->device));
   cudaStream_t st = stream ? static_cast<cudaStream_t>(stream) : ctx->stream;
+  ++ctx->call;
   r = dispatch_device(ctx, precision, method, d_antpos, nant, freqs, nfreq, d_eq2tops, ntimes,
                       d_crd_eq, d_I_sky, nsrc, d_bm_cubes, beam_px, d_vis_out, st);
   if (r != HV_OK || st == ctx->stream) return r;
@@ -785,6 +816,7 @@ int hv_vis_multifreq(hv_context* ctx, int precision, int method, const void* ant
     return fail(ctx, HV_ERR_ARG, "null array argument");
   HV_CK(cudaSetDevice(ctx->device));
   cudaStream_t st = ctx->stream;
+  ++ctx->call;
   const size_t rs = precision == 1 ? 4 : 8;
   const size_t b_antpos = rs * nant * 3, b_e2t = rs * (size_t)ntimes * 9,
                b_crd = rs * 3 * (size_t)nsrc, b_I = rs * (size_t)nsrc,

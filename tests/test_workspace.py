@@ -1,0 +1,64 @@
+"""The contexts' workspace under a budget and on a full device, without a GPU
+(fake_gpu.py): what a call gets does not depend on the calls before it."""
+import pytest
+
+import fake_gpu
+
+GB = 1 << 30
+
+
+@pytest.fixture(scope="module")
+def library(tmp_path_factory):
+    return fake_gpu.build_library(tmp_path_factory.mktemp("fake"))
+
+
+@pytest.fixture
+def gpu(library):
+    g = fake_gpu.FakeGpu(library, 280 * GB)
+    yield g
+    g.close()
+
+
+# shapes of the calls: precision, method, antennas, sources, times, frequencies
+FP32 = (1, "tc", 350, 200_000, 20)
+PLAIN = (1, "plain", 350, 100_000, 8)
+FP64 = (2, "auto", 350, 100_000, 3)
+SIZES = {"tc": FP32, "plain": PLAIN, "fp64": FP64}
+
+
+# every form after every other one, within a budget that holds each alone: the
+# same launches as in a fresh context
+@pytest.mark.parametrize("budget", [1 * GB, 2 * GB, 5 * GB])
+@pytest.mark.parametrize("first", list(SIZES))
+@pytest.mark.parametrize("then", list(SIZES))
+def test_a_call_does_not_depend_on_the_one_before(gpu, first, then, budget):
+    fresh = gpu.context(budget)
+    alone = gpu.call(fresh, *SIZES[then])
+    want = fake_gpu.kernels(gpu.log())
+    used = gpu.context(budget)
+    gpu.call(used, *SIZES[first])
+    gpu.log()
+    assert gpu.call(used, *SIZES[then]) == alone
+    assert fake_gpu.kernels(gpu.log()) == want
+
+
+# an FP64 call keeps the digit form after a large call in FP32 that fills the budget
+def test_fp64_product_after_a_large_fp32_call(gpu):
+    ctx = gpu.context(2 * GB)
+    assert gpu.call(ctx, *FP32) == 0
+    gpu.log()
+    assert gpu.call(ctx, 2, "auto", 350, 40_000, 1) == 0
+    log = gpu.log()
+    assert fake_gpu.launched(log, "mma64_kernel") and not fake_gpu.launched(log, "herk_plain_f64")
+
+
+# calls that fit as they are allocate, free and wait for nothing
+@pytest.mark.parametrize("kind,budget", [("tc", 0), ("tc", 2 * GB), ("plain", 0), ("plain", 1 * GB),
+                                         ("plain", 2 * GB), ("fp64", 0), ("fp64", 1 * GB),
+                                         ("fp64", 2 * GB), ("fp64", 5 * GB)])
+def test_a_repeated_call_keeps_its_workspace(gpu, kind, budget):
+    ctx = gpu.context(budget)
+    assert gpu.call(ctx, *SIZES[kind]) == 0
+    gpu.log()
+    gpu.call(ctx, *SIZES[kind])
+    assert not [op for op, _, _ in gpu.log() if op in ("malloc", "free", "sync", "hostalloc")]
