@@ -31,6 +31,7 @@ struct DevBuf {
   void* p = nullptr;
   size_t cap = 0;
   uint64_t call = 0;  // the last call that used it
+  bool kept = false;  // in a captured graph
 };
 struct HostBuf {
   void* p = nullptr;
@@ -53,6 +54,7 @@ struct hv_context {
   size_t budget = 0;  // 0 = unlimited
   size_t held = 0;
   uint64_t call = 0;  // visibility calls so far
+  bool capturing = false;  // the present one is being captured into a graph
   std::string err;
   uint64_t launches = 0;
   int* d_err = nullptr;  // device-side error flag (bounded waits)
@@ -143,7 +145,10 @@ void each_buffer(hv_context* ctx, F f) {
 // Workspace that earlier calls have left and the present one has not used: it
 // is kept for the next call of its kind, but never stands against a call that
 // finds no room.  What a call is given so does not depend on the calls before it.
-bool idle(const hv_context* ctx, const DevBuf& b) { return b.p && b.call != ctx->call; }
+// (A captured graph reads its workspace again whenever it is launched.)
+bool idle(const hv_context* ctx, const DevBuf& b) {
+  return b.p && !b.kept && b.call != ctx->call;
+}
 size_t idle_bytes(hv_context* ctx) {
   size_t n = 0;
   each_buffer(ctx, [&](DevBuf& b) { n += idle(ctx, b) ? b.cap : 0; });
@@ -164,6 +169,7 @@ bool release_idle(hv_context* ctx) {
 int ensure(hv_context* ctx, DevBuf& b, size_t bytes) {
   if (bytes == 0) bytes = 256;
   b.call = ctx->call;
+  b.kept = b.kept || ctx->capturing;
   if (b.cap >= bytes) return HV_OK;
   // the old buffer may still be read by queued work (on any stream)
   HV_CK(cudaDeviceSynchronize());
@@ -198,7 +204,8 @@ int ensure(hv_context* ctx, DevBuf& b, size_t bytes) {
 // within the budget: asked before any of them grows, since one grown for more
 // work than fits would leave less room for the others.  Buffers that an earlier
 // call has grown beyond these sizes are given back where that makes the room; the
-// present call must not have used them yet.
+// present call must not have used them yet.  None can grow while the call is being
+// captured: it runs in the workspace of the calls before it.
 bool fits(hv_context* ctx, const std::pair<DevBuf*, size_t>* want, size_t n) {
   auto slack = [](size_t bytes) { return bytes + bytes / 8 + 256; };
   auto room = [&] {
@@ -210,12 +217,13 @@ bool fits(hv_context* ctx, const std::pair<DevBuf*, size_t>* want, size_t n) {
       grown += slack(want[i].second);
     }
     if (grown == 0) return true;
+    if (ctx->capturing) return false;
     return !ctx->budget || ctx->held - idle_bytes(ctx) - old + grown <= ctx->budget;
   };
   if (room()) return true;
   bool larger = false;
-  for (size_t i = 0; i < n; ++i) {
-    if (want[i].first->cap <= slack(want[i].second)) continue;
+  for (size_t i = 0; i < n && !ctx->capturing; ++i) {
+    if (want[i].first->kept || want[i].first->cap <= slack(want[i].second)) continue;
     if (!larger) cudaDeviceSynchronize();
     release(ctx, *want[i].first);
     larger = true;
@@ -788,16 +796,17 @@ int hv_vis_multifreq_device(hv_context* ctx, int precision, int method, const vo
     return fail(ctx, HV_ERR_ARG, "null array argument");
   HV_CK(cudaSetDevice(ctx->device));
   cudaStream_t st = stream ? static_cast<cudaStream_t>(stream) : ctx->stream;
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  HV_CK(cudaStreamIsCapturing(st, &cap));
   ++ctx->call;
+  ctx->capturing = cap != cudaStreamCaptureStatusNone;
   r = dispatch_device(ctx, precision, method, d_antpos, nant, freqs, nfreq, d_eq2tops, ntimes,
                       d_crd_eq, d_I_sky, nsrc, d_bm_cubes, beam_px, d_vis_out, st);
   if (r != HV_OK || st == ctx->stream) return r;
   // the context's stream follows the call's work (not while the caller's
   // stream is being captured: that would pull the context's stream into the
   // capture), so that hv_sync waits for it and reads its error flag after it
-  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-  HV_CK(cudaStreamIsCapturing(st, &cap));
-  if (cap == cudaStreamCaptureStatusNone) {
+  if (!ctx->capturing) {
     HV_CK(cudaEventRecord(ctx->joined, st));
     HV_CK(cudaStreamWaitEvent(ctx->stream, ctx->joined, 0));
   }
@@ -817,6 +826,7 @@ int hv_vis_multifreq(hv_context* ctx, int precision, int method, const void* ant
   HV_CK(cudaSetDevice(ctx->device));
   cudaStream_t st = ctx->stream;
   ++ctx->call;
+  ctx->capturing = false;
   const size_t rs = precision == 1 ? 4 : 8;
   const size_t b_antpos = rs * nant * 3, b_e2t = rs * (size_t)ntimes * 9,
                b_crd = rs * 3 * (size_t)nsrc, b_I = rs * (size_t)nsrc,

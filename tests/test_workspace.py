@@ -62,3 +62,36 @@ def test_a_repeated_call_keeps_its_workspace(gpu, kind, budget):
     gpu.log()
     gpu.call(ctx, *SIZES[kind])
     assert not [op for op, _, _ in gpu.log() if op in ("malloc", "free", "sync", "hostalloc")]
+
+
+# a call whose workspace the one before it has laid out can be captured, also
+# where a budget leaves room for few slices a launch, or none of the digit form
+@pytest.mark.parametrize("kind", list(SIZES))
+@pytest.mark.parametrize("budget", [0] + [(1 << 30) + (k << 26) for k in range(0, 32, 3)])
+def test_a_repeated_call_can_be_captured(gpu, kind, budget):
+    ctx = gpu.context(budget)
+    if gpu.call(ctx, *SIZES[kind], stream=77) != 0:
+        return      # a budget below the form's least
+    want = fake_gpu.kernels(gpu.log())
+    gpu.lib.fake_capture(77)
+    assert gpu.call(ctx, *SIZES[kind], stream=77) == 0
+    gpu.lib.fake_capture(None)
+    log = gpu.log()
+    assert fake_gpu.kernels(log) == want
+    assert not [op for op, _, _ in log if op.startswith("refused") or op in ("malloc", "free")]
+
+
+# the FP64 workspace of a captured graph is not given back to a call without room
+def test_the_workspace_of_a_captured_call_stays(gpu):
+    freed = []
+    for captured in (False, True):
+        ctx = gpu.context(2 * GB)
+        assert gpu.call(ctx, *FP64, stream=77) == 0
+        if captured:
+            gpu.lib.fake_capture(77)
+            assert gpu.call(ctx, *FP64, stream=77) == 0
+            gpu.lib.fake_capture(None)
+        gpu.log()
+        gpu.call(ctx, *FP32)
+        freed.append(len([op for op, _, _ in gpu.log() if op == "free"]))
+    assert freed[1] <= freed[0] - 4
