@@ -424,16 +424,29 @@ int run_device(hv_context* ctx, int method, const R* antpos, int nant, const dou
       HV_ENSURE(ctx->tcgroups, gbytes);
       HV_CK(cudaMemcpyAsync(ctx->tcgroups.p, host.data(), gbytes, cudaMemcpyHostToDevice, st));
       // batch of times per launch, bounded by the partial-sum and record caps
-      int ntb = ntimes, chunk = 0, flush = 0;
+      // (a small call's shorter chunks make up to 16 times the partial sums:
+      // without the room for them it takes the regular ones)
+      int ntb = 0, chunk = 0, flush = 0;
       size_t slice_floats = 0;
-      for (;;) {
-        chunk = tc_chunk_sources(S1, ntb, nfreq, ngroups, tc_block_rows(nant, form), ctx->num_sms,
-                                 &flush);
-        slice_floats = tc_partial_floats(Np, S1, 1, chunk);
-        const size_t pbytes = sizeof(float) * slice_floats * (size_t)ntb * nfreq;
-        const size_t rbytes = sizeof(Rec) * (size_t)ntb * (((size_t)S1 + 31) / 32 * 32);
-        if (ntb == 1 || (pbytes <= kTcPartialCap && rbytes <= kTcRecCap)) break;
-        ntb = (ntb + 1) / 2;
+      for (bool spread = true;; spread = false) {
+        size_t pbytes = 0, rbytes = 0;
+        for (ntb = ntimes;; ntb = (ntb + 1) / 2) {
+          chunk = tc_chunk_sources(S1, ntb, nfreq, ngroups, tc_block_rows(nant, form),
+                                   ctx->num_sms, spread, &flush);
+          slice_floats = tc_partial_floats(Np, S1, 1, chunk);
+          pbytes = sizeof(float) * slice_floats * (size_t)ntb * nfreq;
+          rbytes = sizeof(Rec) * (size_t)ntb * (((size_t)S1 + 31) / 32 * 32);
+          if (ntb == 1 || (pbytes <= kTcPartialCap && rbytes <= kTcRecCap)) break;
+        }
+        const std::pair<DevBuf*, size_t> want[] = {
+            {&ctx->partial, pbytes},
+            {&ctx->rec, rbytes},
+            {&ctx->blkcounts, sizeof(int) * (size_t)prep_blocks(nsrc) * ntb},
+            {&ctx->umax, sizeof(float) * (size_t)ntimes * nfreq},
+            {&ctx->sortkv, sizeof(unsigned long long) * (size_t)nsrc},
+            {&ctx->crd_sorted, sizeof(float) * 3 * (size_t)nsrc},
+            {&ctx->I_sorted, sizeof(float) * (size_t)nsrc}};
+        if (!spread || fits(ctx, want, std::size(want))) break;
       }
       HV_ENSURE(ctx->partial, sizeof(float) * slice_floats * (size_t)ntb * nfreq);
       const size_t rec_stride = ((size_t)S1 + 31) / 32 * 32;  // whole stages per time

@@ -275,8 +275,10 @@ cudaError_t launch_tc_batch(const TcSimDesc* sims, int nsims, const void* rec, l
                             int num_sms, cudaStream_t st, unsigned long long wait_ns = 0,
                             int stall = 0, TcShare* share = nullptr);
 size_t tc_partial_floats(int Np, int nsrc, int nslices, int chunk);
+// Sources per split-K chunk, and per accumulator flush.  spread: calls too small to
+// fill the GPU may take chunks of fewer than 1024 sources.
 int tc_chunk_sources(int nsrc, int ntimes, int nfreq, int ngroups, int block_rows, int num_sms,
-                     int* flush);
+                     bool spread, int* flush);
 size_t tc_group_table_bytes(int nant);
 int tc_fill_group_table(int nant, int form, void* host_buf);
 int tc_max_slots(int nant);

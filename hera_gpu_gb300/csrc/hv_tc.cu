@@ -1472,7 +1472,7 @@ int tc_fill_group_table(int nant, int form, void* host_buf) {
 }
 
 int tc_chunk_sources(int nsrc, int ntimes, int nfreq, int ngroups, int block_rows, int num_sms,
-                     int* flush) {
+                     bool spread, int* flush) {
   // Sources an accumulator sums before it is flushed: as many as give about 40
   // runs a cluster (or CTA), 1024 to TC_FLUSH_SOURCES, in whole stages (the
   // error grows with the run; about half the catalogue is above the horizon).
@@ -1523,7 +1523,7 @@ int tc_chunk_sources(int nsrc, int ntimes, int nfreq, int ngroups, int block_row
     const long long items = slices * units * ((up + x - 1) / x);
     return (items + workers - 1) / workers * (std::min(x, up) + fixed);
   };
-  if (c == 1024 && nslices * units * ((up + c - 1) / c) < workers) {
+  if (spread && c == 1024 && nslices * units * ((up + c - 1) / c) < workers) {
     long long best = c;
     for (long long x = c - 32; x >= 64; x -= 32)
       if (span(x, ntimes) < span(best, ntimes)) best = x;

@@ -95,3 +95,26 @@ def test_the_workspace_of_a_captured_call_stays(gpu):
         gpu.call(ctx, *FP32)
         freed.append(len([op for op, _, _ in gpu.log() if op == "free"]))
     assert freed[1] <= freed[0] - 4
+
+
+# small calls fit the budgets that hold one partial sum a 1024 sources and slice
+# beside their other workspace (3 % above the least)
+@pytest.mark.parametrize("shape,mb", [((1, "tc", 16, 1000, 10), 2.57), ((1, "tc", 64, 3000, 4), 2.96),
+                                      ((1, "tc", 350, 3000, 5), 20.8), ((1, "tc", 140, 2000, 8), 10.6),
+                                      ((1, "tc", 200, 20_000, 1), 14.8),
+                                      ((1, "tc_fp16", 100, 8000, 5), 8.41)])
+def test_small_calls_under_a_budget(gpu, shape, mb):
+    assert gpu.call(gpu.context(int(mb * 1e6)), *shape, px=31) == 0
+
+
+# with the room for them they take their shorter chunks, whatever ran before
+def test_small_calls_keep_their_chunks(gpu):
+    def partial_sums(ctx):      # the largest allocation
+        gpu.log()
+        assert gpu.call(ctx, 1, "tc", 16, 1000, 10, px=31) == 0
+        return max(a for op, a, _ in gpu.log() if op == "malloc")
+    fresh = partial_sums(gpu.context())
+    assert fresh > 8 * partial_sums(gpu.context(3 << 20))
+    used = gpu.context(40 << 20)
+    assert gpu.call(used, 1, "plain", 128, 30_000, 1, px=31) == 0
+    assert partial_sums(used) >= fresh * 8 // 9
