@@ -668,6 +668,15 @@ void hv_context_set_error(hv_context* ctx, const char* msg) { ctx->err = msg; }
 void hv_context_add_launches(hv_context* ctx, uint64_t n) { ctx->launches += n; }
 int hv_context_num_sms(hv_context* ctx) { return ctx->num_sms; }
 
+cudaError_t hv_context_malloc(hv_context* ctx, void** p, size_t bytes, cudaStream_t st) {
+  cudaError_t e = cudaMallocAsync(p, bytes, st);
+  if (e != cudaErrorMemoryAllocation) return e;
+  ++ctx->call;  // no call is using the workspace but for work still queued
+  cudaGetLastError();
+  if (cudaDeviceSynchronize() != cudaSuccess || !release_idle(ctx)) return e;
+  return cudaMallocAsync(p, bytes, st);
+}
+
 void* hv_context_host_take(hv_context* ctx, size_t bytes, size_t* cap) {
   // the smallest pooled block that fits, else a new one
   size_t best = ctx->host_pool.size();
@@ -960,7 +969,7 @@ int hv_profile_read(hv_context* ctx, double* ms, uint64_t* launches) {
 int hv_device_alloc(hv_context* ctx, size_t bytes, void** ptr) {
   if (!ctx || !ptr) return HV_ERR_ARG;
   HV_CK(cudaSetDevice(ctx->device));
-  cudaError_t e = cudaMallocAsync(ptr, bytes ? bytes : 1, ctx->stream);
+  cudaError_t e = hv_context_malloc(ctx, ptr, bytes ? bytes : 1, ctx->stream);
   if (e != cudaSuccess) {
     cudaGetLastError();
     return fail(ctx, HV_ERR_OOM, "cudaMallocAsync(%zu) failed: %s", bytes, cudaGetErrorString(e));

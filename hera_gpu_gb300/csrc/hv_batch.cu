@@ -277,9 +277,11 @@ int allocate(hv_batch* b) {
     hv_context_host_give(b->ctx, b->host, b->host_cap);
     b->host = nullptr;
   }
-  HB_CK(cudaMallocAsync(&b->arena, std::max<size_t>(b->arena_bytes, 256), st));
-  HB_CK(cudaMallocAsync(&b->rec, sizeof(hv::SrcRec32) * (size_t)std::max<long long>(b->rec_rows, 1), st));
-  HB_CK(cudaMallocAsync(&b->table, hv::tc_sim_table_bytes((int)(b->sims.size() + b->classes.size())), st));
+  HB_CK(hv_context_malloc(b->ctx, &b->arena, std::max<size_t>(b->arena_bytes, 256), st));
+  HB_CK(hv_context_malloc(b->ctx, &b->rec,
+                          sizeof(hv::SrcRec32) * (size_t)std::max<long long>(b->rec_rows, 1), st));
+  HB_CK(hv_context_malloc(b->ctx, &b->table,
+                          hv::tc_sim_table_bytes((int)(b->sims.size() + b->classes.size())), st));
   if (!b->host) {
     b->host = hv_context_host_take(b->ctx, std::max<size_t>(b->host_bytes, 256), &b->host_cap);
     if (!b->host) return bfail(b, HV_ERR_OOM, "page-locked host block of %zu bytes", b->host_bytes);
@@ -420,8 +422,8 @@ int hv_batch_create(hv_context* ctx, const hv_sim* sims, int nsims, unsigned fla
   do {
     if (cudaGetDevice(&b->device) != cudaSuccess) { r = HV_ERR_CUDA; break; }
     b->num_sms = hv_context_num_sms(ctx);
-    if (cudaMallocAsync(reinterpret_cast<void**>(&b->d_err), 8 + 8 * (size_t)nsims,
-                        hv_context_stream(ctx)) != cudaSuccess) { r = HV_ERR_OOM; break; }
+    if (hv_context_malloc(ctx, reinterpret_cast<void**>(&b->d_err), 8 + 8 * (size_t)nsims,
+                          hv_context_stream(ctx)) != cudaSuccess) { r = HV_ERR_OOM; break; }
     cudaMemsetAsync(b->d_err, 0, 8 + 8 * (size_t)nsims, hv_context_stream(ctx));
     b->d_claim = reinterpret_cast<unsigned long long*>(b->d_err + 2);
     std::map<int, int> class_of;  // cluster size (0 = no cluster) -> class

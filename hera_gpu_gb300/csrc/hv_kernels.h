@@ -291,6 +291,9 @@ cudaStream_t hv_context_stream(hv_context* ctx);
 void hv_context_set_error(hv_context* ctx, const char* msg);
 void hv_context_add_launches(hv_context* ctx, uint64_t n);
 int hv_context_num_sms(hv_context* ctx);
+// cudaMallocAsync; a request that finds no room is made once more after the
+// context's workspace has been given back.
+cudaError_t hv_context_malloc(hv_context* ctx, void** p, size_t bytes, cudaStream_t st);
 // Page-locked host block of at least `bytes` (its size in *cap) from the
 // context's pool of returned blocks, or newly allocated; nullptr on failure.
 void* hv_context_host_take(hv_context* ctx, size_t bytes, size_t* cap);

@@ -571,8 +571,8 @@ int hv_median_filter(hv_context* ctx, const float* in, float* out, int nimg, int
   if (!in || !out) return HV_ERR_ARG;
   cudaStream_t st = hv_context_stream(ctx);
   void *d_in = nullptr, *d_out = nullptr;
-  if (cudaMallocAsync(&d_in, bytes, st) != cudaSuccess ||
-      cudaMallocAsync(&d_out, bytes, st) != cudaSuccess) {
+  if (hv_context_malloc(ctx, &d_in, bytes, st) != cudaSuccess ||
+      hv_context_malloc(ctx, &d_out, bytes, st) != cudaSuccess) {
     cudaGetLastError();
     if (d_in) cudaFreeAsync(d_in, st);
     hv_context_set_error(ctx, "median filter: device allocation failed");

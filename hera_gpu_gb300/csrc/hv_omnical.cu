@@ -1110,7 +1110,7 @@ int run_dense(hv_context* ctx, const DensePlan& dp, int nbls, void* d_gains, int
   const size_t n_off = sizeof(int) * dp.row_off.size(), n_slot = sizeof(uint32_t) * dp.slots.size();
   const size_t o_slot = (n_off + 255) & ~size_t(255), o_cnt = (o_slot + n_slot + 255) & ~size_t(255);
   void* buf = nullptr;
-  if (cudaMallocAsync(&buf, o_cnt + 256, st) != cudaSuccess) {
+  if (hv_context_malloc(ctx, &buf, o_cnt + 256, st) != cudaSuccess) {
     cudaGetLastError();
     return fail(ctx, HV_ERR_OOM, "omnical: device allocation failed");
   }
@@ -1187,7 +1187,7 @@ int run_typed(hv_context* ctx, const uint32_t* ggu, int nbls, void* d_gains, int
   const size_t o_cnt = (o_ent + n_ent + 255) & ~size_t(255);
   const size_t total = o_cnt + 256;
   void* buf = nullptr;
-  if (cudaMallocAsync(&buf, total, st) != cudaSuccess) {
+  if (hv_context_malloc(ctx, &buf, total, st) != cudaSuccess) {
     cudaGetLastError();
     return fail(ctx, HV_ERR_OOM, "omnical: device allocation failed");
   }
@@ -1317,7 +1317,7 @@ int hv_omnical(hv_context* ctx, int precision, const uint32_t* ggu, int nbls, vo
   }
   cudaStream_t st = hv_context_stream(ctx);
   void* buf = nullptr;
-  if (cudaMallocAsync(&buf, tot, st) != cudaSuccess) {
+  if (hv_context_malloc(ctx, &buf, tot, st) != cudaSuccess) {
     cudaGetLastError();
     return fail(ctx, HV_ERR_OOM, "omnical: device allocation failed");
   }

@@ -1,8 +1,12 @@
 """The contexts' workspace under a budget and on a full device, without a GPU
 (fake_gpu.py): what a call gets does not depend on the calls before it."""
+import ctypes
+
+import numpy as np
 import pytest
 
 import fake_gpu
+from hera_gpu_gb300 import synth
 
 GB = 1 << 30
 
@@ -118,3 +122,34 @@ def test_small_calls_keep_their_chunks(gpu):
     used = gpu.context(40 << 20)
     assert gpu.call(used, 1, "plain", 128, 30_000, 1, px=31) == 0
     assert partial_sums(used) >= fresh * 8 // 9
+
+
+# batches, Omnical, the median filter and device allocations on a device that the
+# workspace of an FP64 call has filled
+@pytest.mark.parametrize("kind", ["batch", "omnical", "omnical dense", "median", "alloc"])
+def test_other_allocations_find_the_workspaces_room(gpu, kind):
+    gpu.reset(6 * GB)
+    ctx = gpu.context()
+    assert gpu.call(ctx, 2, "auto", 350, 60_000, 20) == 0
+    left = 6 * GB - gpu.lib.fake_used()
+    assert left < 2 * GB        # less than the requests below
+    lib = gpu.lib
+    if kind == "alloc":
+        p = ctypes.c_void_p()
+        assert lib.hv_device_alloc(ctx, 3 * GB, ctypes.byref(p)) == 0
+    elif kind == "median":
+        img = np.zeros((1, 20_000, 16_000), dtype=np.float32)
+        assert lib.hv_median_filter(ctx, img.ctypes.data, img.ctypes.data, 1, *img.shape[1:], 3, 3) == 0
+    elif kind == "batch":
+        assert gpu.batch(ctx, [(350, 60_000, 60, 16)])[0] == 0
+    else:
+        nants = 100 if kind == "omnical dense" else 20
+        ggu, nubls = synth.hex_redundant_layout(nants)
+        ggu = np.ascontiguousarray(ggu, dtype=np.uint32)
+        n = int(2.2 * GB) // (len(ggu) * 12)
+        a = [np.zeros((n, k), dtype=np.complex64) for k in (nants, nubls, len(ggu))]
+        w, out = np.zeros((n, len(ggu)), dtype=np.float32), np.zeros((3, n), dtype=np.float32)
+        assert lib.hv_omnical(ctx, 1, ggu.ctypes.data, len(ggu), a[0].ctypes.data, nants,
+                              a[1].ctypes.data, nubls, a[2].ctypes.data, w.ctypes.data, n, 1e-10, 4,
+                              4, 1, 0.3, out[0].ctypes.data, out[1].ctypes.data,
+                              out[2].ctypes.data) == 0
