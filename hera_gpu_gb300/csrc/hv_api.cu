@@ -201,8 +201,9 @@ int ensure(hv_context* ctx, DevBuf& b, size_t bytes) {
 }
 
 // Whether buffers can grow to the wanted sizes, ensure()'s slack included,
-// within the budget: asked before any of them grows, since one grown for more
-// work than fits would leave less room for the others.  Buffers that an earlier
+// within the budget and on the device: asked before any of them grows, since one
+// grown for more work than fits would leave less room for the others, and a failed
+// attempt costs a free, a wait and an allocation in every call.  Buffers that an earlier
 // call has grown beyond these sizes are given back where that makes the room; the
 // present call must not have used them yet.  None can grow while the call is being
 // captured: it runs in the workspace of the calls before it.
@@ -218,7 +219,11 @@ bool fits(hv_context* ctx, const std::pair<DevBuf*, size_t>* want, size_t n) {
     }
     if (grown == 0) return true;
     if (ctx->capturing) return false;
-    return !ctx->budget || ctx->held - idle_bytes(ctx) - old + grown <= ctx->budget;
+    const size_t spare = idle_bytes(ctx) + old;
+    if (ctx->budget && ctx->held - spare + grown > ctx->budget) return false;
+    // (allocations come in pieces of 2 MB)
+    size_t free = 0, total = 0;
+    return cudaMemGetInfo(&free, &total) != cudaSuccess || grown + (n << 21) <= free + spare;
   };
   if (room()) return true;
   bool larger = false;

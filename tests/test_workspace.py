@@ -68,6 +68,19 @@ def test_a_repeated_call_keeps_its_workspace(gpu, kind, budget):
     assert not [op for op, _, _ in gpu.log() if op in ("malloc", "free", "sync", "hostalloc")]
 
 
+# nor do they on a device that has room for few slices a launch, or none of the
+# digit form
+@pytest.mark.parametrize("kind,gb", [("plain", 0.9), ("plain", 1.5), ("plain", 2.2), ("fp64", 0.9),
+                                     ("fp64", 1.5), ("fp64", 2.9), ("tc", 2.0)])
+def test_a_repeated_call_on_a_small_device(gpu, kind, gb):
+    gpu.reset(int(gb * GB))
+    ctx = gpu.context()
+    assert gpu.call(ctx, *SIZES[kind]) == 0
+    gpu.log()
+    gpu.call(ctx, *SIZES[kind])
+    assert not [op for op, _, _ in gpu.log() if op.split()[0] in ("malloc", "free", "sync")]
+
+
 # a call whose workspace the one before it has laid out can be captured, also
 # where a budget leaves room for few slices a launch, or none of the digit form
 @pytest.mark.parametrize("kind", list(SIZES))
