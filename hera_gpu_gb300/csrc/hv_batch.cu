@@ -315,9 +315,14 @@ int enqueue(hv_batch* b, cudaStream_t st, int timed_class = -1) {
   // small ones fill the tail.  The classes run on up to three streams: a
   // persistent launch fills the GPU, so the next class starts on the SMs that
   // its tail leaves instead of after it (12 simulations in 6 classes 18.0 ->
-  // 16.75 ms).
+  // 16.75 ms).  Profiled, they run one after the other, so that each one's events
+  // time it alone.
   const TcShare* aux = hv_context_share(b->ctx);
-  const bool fork = timed_class < 0 && b->classes.size() > 1;
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  const bool prof = timed_class < 0 && hv_context_profiling(b->ctx) &&
+                    cudaStreamIsCapturing(st, &cs) == cudaSuccess &&
+                    cs == cudaStreamCaptureStatusNone;
+  const bool fork = timed_class < 0 && !prof && b->classes.size() > 1;
   if (fork) {
     HB_CK(cudaEventRecord(aux->fork, st));
     HB_CK(cudaStreamWaitEvent(aux->hi, aux->fork, 0));
@@ -358,10 +363,6 @@ int enqueue(hv_batch* b, cudaStream_t st, int timed_class = -1) {
     if (!d.empty() && (timed_class < 0 || timed_class == (int)c)) {
       const cudaStream_t cst = !fork || c % 3 == 0 ? st : c % 3 == 1 ? aux->hi : aux->lo;
       cudaEvent_t e0 = nullptr, e1 = nullptr;
-      cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-      const bool prof = timed_class < 0 && hv_context_profiling(b->ctx) &&
-                        cudaStreamIsCapturing(st, &cs) == cudaSuccess &&
-                        cs == cudaStreamCaptureStatusNone;
       if (prof) {
         HB_CK(cudaEventCreate(&e0));
         HB_CK(cudaEventCreate(&e1));
