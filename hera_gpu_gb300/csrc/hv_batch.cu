@@ -329,7 +329,7 @@ int enqueue(hv_batch* b, cudaStream_t st, int timed_class = -1) {
     HB_CK(cudaStreamWaitEvent(aux->lo, aux->fork, 0));
   }
   size_t toff = 0;
-  for (size_t c = 0; c < b->classes.size(); ++c) {
+  auto launch_class = [&](size_t c) -> int {
     std::vector<int> order = b->classes[c];
     std::stable_sort(order.begin(), order.end(), [&](int x, int y) {
       const SimPlan &sx = b->sims[x], &sy = b->sims[y];
@@ -383,12 +383,19 @@ int enqueue(hv_batch* b, cudaStream_t st, int timed_class = -1) {
       ++nl;
     }
     toff += tc_sim_table_bytes((int)d.size());
-  }
-  if (fork) {
-    HB_CK(cudaEventRecord(aux->join_hi, aux->hi));
-    HB_CK(cudaEventRecord(aux->join_lo, aux->lo));
-    HB_CK(cudaStreamWaitEvent(st, aux->join_hi, 0));
-    HB_CK(cudaStreamWaitEvent(st, aux->join_lo, 0));
+    return HV_OK;
+  };
+  int r = HV_OK;
+  for (size_t c = 0; c < b->classes.size() && r == HV_OK; ++c) r = launch_class(c);
+  // also after a failure: what was launched on the other streams comes before
+  // anything that the caller queues on st, the release of the arena above all
+  if (fork || r != HV_OK) {
+    cudaError_t e = cudaEventRecord(aux->join_hi, aux->hi);
+    if (e == cudaSuccess) e = cudaStreamWaitEvent(st, aux->join_hi, 0);
+    if (e == cudaSuccess) e = cudaEventRecord(aux->join_lo, aux->lo);
+    if (e == cudaSuccess) e = cudaStreamWaitEvent(st, aux->join_lo, 0);
+    if (r != HV_OK) return r;
+    HB_CK(e);
   }
   if (timed_class < 0) {
     HB_CK(launch_reduce_batch(sims, n, pre, b->totals, st));

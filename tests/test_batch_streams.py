@@ -51,3 +51,24 @@ def fused_launch(gpu, batch):
     gpu.log()
     assert gpu.lib.hv_batch_launch(batch, None) == 0
     return fused(gpu.log())
+
+
+# a launch that fails between the fork and the join: what the other streams were
+# given is waited for before the arena is given back on the batch's stream
+@pytest.mark.parametrize("after", [1, 2, 3, 4])
+def test_a_failed_class_joins_its_streams(gpu, after):
+    ctx = gpu.context()
+    rc, batch = gpu.batch(ctx, SIMS)
+    assert rc == 0
+    gpu.log()
+    gpu.lib.fake_fail(b"tc_vis_kernel", after)
+    assert gpu.lib.hv_batch_launch(batch, None) != 0
+    gpu.lib.hv_batch_destroy(batch)
+    log = gpu.log()
+    freed = next(i for i, (op, _, _) in enumerate(log) if op == "freeasync")
+    own = log[freed][1]
+    last = {s: i for i, s in fused(log[:freed]) if s != own}
+    assert last
+    for stream, i in last.items():
+        joined = [e for j, (op, e, s) in enumerate(log[:freed]) if j > i and op == "record" and s == stream]
+        assert any(op == "wait" and s == own and e in joined for op, s, e in log[i:freed])
