@@ -108,8 +108,8 @@ int fail(hv_context* c, int code, const char* fmt, ...) {
     ctx->launches += (n);      \
   } while (0)
 
-// A launch of a visibility-product kernel, bracketed by events when profiling.
-#define HV_LAUNCH_TIMED(call, st)                                   \
+// The n launches of a visibility product, bracketed by events when profiling.
+#define HV_LAUNCH_TIMED(n, call, st)                                \
   do {                                                              \
     cudaEvent_t e0_ = nullptr, e1_ = nullptr;                       \
     if (ctx->profiling) {                                           \
@@ -117,7 +117,7 @@ int fail(hv_context* c, int code, const char* fmt, ...) {
       HV_CK(cudaEventCreate(&e1_));                                 \
       HV_CK(cudaEventRecord(e0_, (st)));                            \
     }                                                               \
-    HV_LAUNCH(1, call);                                             \
+    HV_LAUNCH(n, call);                                             \
     if (ctx->profiling) {                                           \
       HV_CK(cudaEventRecord(e1_, (st)));                            \
       ctx->prof_events.emplace_back(e0_, e1_);                      \
@@ -374,11 +374,11 @@ int run_f64(hv_context* ctx, const double* eq2tops, const double* crd_eq, const 
         HV_CK(cudaMemsetAsync(words, 0, b_w * n, st));
         HV_LAUNCH(1, launch_f64_phasors(d, n, ctx->rec.p, (size_t)S1, U, beam, P, small,
                                         ctx->f64_v.p, rowmax, st));
-        // digits and class sums; the SIMT product of the flagged slices
-        HV_LAUNCH_TIMED(launch_f64_product(d, n, ctx->f64_v.p, rowmax, ctx->f64_digits.p, flags,
+        // digits, class sums and overlaps; the SIMT product of the flagged slices
+        HV_LAUNCH_TIMED(3, launch_f64_product(d, n, ctx->f64_v.p, rowmax, ctx->f64_digits.p, flags,
                                            words, ctx->num_sms, ctx->d_err, ctx->wait_ns, st),
                         st);
-        HV_LAUNCH(2, launch_herk_flagged(d, n, ctx->f64_v.p, flags,
+        HV_LAUNCH(1, launch_herk_flagged(d, n, ctx->f64_v.p, flags,
                                          static_cast<double*>(ctx->f64_digits.p),
                                          b_dig / sizeof(double), st));
         HV_LAUNCH(1, launch_f64_final(d, n, words, rowmax, flags, ctx->f64_digits.p, t0, f0,
@@ -537,7 +537,7 @@ int run_device(hv_context* ctx, int method, const R* antpos, int nant, const dou
         HV_ENSURE(ctx->tctable, tc_sim_table_bytes(1));
         HV_HOST_ENSURE(ctx->tctable_h, tc_sim_table_bytes(1));
         if (nsrc > 0)
-          HV_LAUNCH_TIMED(launch_tc_batch(&L, 1, ctx->rec.p, (long long)nt * rec_stride,
+          HV_LAUNCH_TIMED(1, launch_tc_batch(&L, 1, ctx->rec.p, (long long)nt * rec_stride,
                                           ctx->tctable.p, ctx->tctable_h.p, ctx->d_err,
                                           ctx->d_claim, ctx->num_sms, st, ctx->wait_ns,
                                           ctx->stall, &ctx->share),
@@ -603,7 +603,7 @@ int run_device(hv_context* ctx, int method, const R* antpos, int nant, const dou
                        d, n, ctx->rec.p, nsrc,
                        static_cast<const U*>(ctx->ucoef.p) + ((size_t)t0 * nfreq + f0) * Np,
                        beamT + (size_t)f0 * PP * Np, P, ctx->v.p, st));
-      HV_LAUNCH_TIMED(launch_herk_plain<R>(d, n, ctx->v.p, nsrc, static_cast<R*>(ctx->partial.p),
+      HV_LAUNCH_TIMED(1, launch_herk_plain<R>(d, n, ctx->v.p, nsrc, static_cast<R*>(ctx->partial.p),
                                            st),
                       st);
       HV_LAUNCH(1, launch_reduce<R>(static_cast<R*>(ctx->partial.p), d.p_stride, counts + t0, nt,

@@ -166,3 +166,14 @@ def test_other_allocations_find_the_workspaces_room(gpu, kind):
                               a[1].ctypes.data, nubls, a[2].ctypes.data, w.ctypes.data, n, 1e-10, 4,
                               4, 1, 0.3, out[0].ctypes.data, out[1].ctypes.data,
                               out[2].ctypes.data) == 0
+
+
+# hv_launch_count counts the launches that were made
+@pytest.mark.parametrize("shape", [*SIZES.values(), (1, "tc", 350, 3000, 5), (1, "tc", 16, 9000, 2),
+                                   (1, "tc_fp16", 200, 5000, 3), (1, "tc", 20, 0, 2),
+                                   (2, "auto", 30, 2000, 2), (2, "auto", 2100, 500, 1)])
+def test_launches_are_counted(gpu, shape):
+    ctx = gpu.context()
+    before = gpu.lib.hv_launch_count(ctx)
+    assert gpu.call(ctx, *shape) == 0
+    assert gpu.lib.hv_launch_count(ctx) - before == len(fake_gpu.kernels(gpu.log()))
