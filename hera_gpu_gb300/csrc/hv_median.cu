@@ -519,7 +519,6 @@ int launch(hv_context* ctx, const float* d_in, float* d_out, int nimg, int rows,
   static bool configured = false;
   if (!configured) {
     for (const void* k : {reinterpret_cast<const void*>(median_filter_kernel<0>),
-                          reinterpret_cast<const void*>(median_filter_kernel<1>),
                           reinterpret_cast<const void*>(median_filter_kernel<5>),
                           reinterpret_cast<const void*>(median_filter_kernel<13>),
                           reinterpret_cast<const void*>(median_filter_kernel<25>),
@@ -533,8 +532,7 @@ int launch(hv_context* ctx, const float* d_in, float* d_out, int nimg, int rows,
   const dim3 block(kMfCols, kMfRows);
   const int n = k0 * k1;  // the register form needs n / 2 + 1 <= K
   if (launch_strips(d_in, d_out, nimg, rows, cols, k0, k1, st)) {
-  } else if (n <= 1) median_filter_kernel<1><<<grid, block, smem, st>>>(d_in, d_out, rows, cols, k0, k1);
-  else if (n <= 9) median_filter_kernel<5><<<grid, block, smem, st>>>(d_in, d_out, rows, cols, k0, k1);
+  } else if (n <= 9) median_filter_kernel<5><<<grid, block, smem, st>>>(d_in, d_out, rows, cols, k0, k1);
   else if (n <= 25) median_filter_kernel<13><<<grid, block, smem, st>>>(d_in, d_out, rows, cols, k0, k1);
   else if (n <= 49) median_filter_kernel<25><<<grid, block, smem, st>>>(d_in, d_out, rows, cols, k0, k1);
   else if (n <= 81) median_filter_kernel<41><<<grid, block, smem, st>>>(d_in, d_out, rows, cols, k0, k1);

@@ -911,6 +911,5 @@ template cudaError_t launch_ucoef<double>(const double*, int, int, const double*
 template cudaError_t launch_prep<float>(const float*, const float*, int, const float*, int, int, int, int*, void*, int*, cudaStream_t);
 template cudaError_t launch_prep_strided<float>(const float*, const float*, int, const float*, int, int, int, int*, void*, size_t, int*, cudaStream_t);
 template cudaError_t launch_prep_strided<double>(const double*, const double*, int, const double*, int, int, int, int*, void*, size_t, int*, cudaStream_t);
-template cudaError_t launch_prep<double>(const double*, const double*, int, const double*, int, int, int, int*, void*, int*, cudaStream_t);
 
 }  // namespace hv
