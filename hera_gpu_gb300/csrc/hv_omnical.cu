@@ -509,12 +509,13 @@ __global__ void __launch_bounds__(kOmMaxThreads, OM_MINB) omnical_kernel(const O
 // Arrays whose baselines are antenna pairs, each pair at most once (the usual
 // case), seen as the lower triangle of the antenna matrix: a group of GL lanes
 // takes a row r, lane l its columns l, l + GL, ... below r, the same ones in
-// every row.  The column antennas' factors and sums so stay in registers, the
-// row antenna's factor is one broadcast, its sum a register until the row's
-// butterfly, and a baseline costs one gather (its unique baseline's factor)
-// and one read-modify-write (its sum) in shared memory.  The general kernel
-// below gathers six solution values, stores d and reads it back three times
-// through incidence lists, a panel of baselines at a time.
+// every row.  The column antennas' sums so stay in registers, the row antenna's
+// factor is one broadcast, its sum a register until the row's butterfly, and a
+// baseline costs the column antenna's factor (read again in every row, consecutive
+// lanes at consecutive places), one gather (its unique baseline's factor) and one
+// read-modify-write (its sum) in shared memory.  The general kernel above gathers
+// six solution values, stores d and reads it back three times through incidence
+// lists, a panel of baselines at a time.
 //
 // Sums of unique baselines: every group has two private copies (one for pairs
 // stored as (row, column), one for (column, row)), added up in a fixed order
@@ -535,15 +536,31 @@ __global__ void __launch_bounds__(kOmMaxThreads, OM_MINB) omnical_kernel(const O
 // (81%: gathers and updates at the unique baselines' scattered places).
 // Measured on GB300, 12 iterations of 2000 problems, general kernel and this
 // one: 180 antennas 3.70 and 2.48 ms, 128 antennas 2.84 and 1.64 ms, 54
-// antennas 0.44 and 0.36 ms.  Smaller arrays stay with the general kernel (4000
-// problems of 20 antennas 148 and 165 us, 28 antennas 237 and 237, 31 antennas
-// 335 and 292), and so do arrays of 65 to 79, whose few warps a problem are
-// slower while a call has few problems (70 antennas: 4000 problems 1127 and
-// 1092 us, 600 problems 140 and 145, 100 problems 84 and 93; 80 antennas 1372
-// and 1245, 166 and 165, 98 and 100).  The number of problems must not decide: a
-// problem gives the same result alone or among others.
+// antennas 0.44 and 0.36 ms.
+//
+// It is taken where it is not slower than the general kernel, be the problems few
+// or many: their number must not decide, since a problem gives the same result
+// alone or among others.  Measured over 10 to 2000 problems (time over the
+// general kernel's, few and many problems):
+//  * smaller arrays stay with the general kernel (4000 problems of 20 antennas
+//    148 and 165 us, 28 antennas 237 and 237, 31 antennas 335 and 292), and so do
+//    arrays of 65 to 87, whose few warps a problem are slower while a call has few
+//    problems (70 antennas 1.11 and 0.97, 80 1.02 and 0.91, 84 1.18 and 0.95; 88
+//    0.96 and 0.81);
+//  * the two copies of the unique baselines' sums a group are cleared and added
+//    up in every iteration, which counts for arrays of up to 64 antennas: they may
+//    have kDenseCopies sums for a pair of antennas, a full hexagon has 1.9 to 2.8
+//    (54 antennas: 3.3 sums 0.98 and 0.84, 4.4 1.15 and 0.96; 62: 2.9 sums 0.93
+//    and 0.85, 3.8 1.06 and 0.86);
+//  * the copies also fill the shared memory.  One CTA an SM is enough for 108 to
+//    128 antennas, whose general kernel takes long rows (128 antennas, 723 unique
+//    baselines: 0.74 and 0.78), and from 225 on (225: 0.68 and 1.02), elsewhere
+//    two are needed (96 antennas: 277 unique baselines, two CTAs, 0.85 and 0.79;
+//    370, one, 0.71 and 1.05; 150: 568, two, 0.93 and 0.87; 852, one, 0.75 and
+//    1.22).
 constexpr int kDenseMinAnts = 31, kDenseMaxAnts = 256;
-constexpr int kDenseGap0 = 65, kDenseGap1 = 79;
+constexpr int kDenseGap0 = 65, kDenseGap1 = 87;
+constexpr double kDenseCopies = 3.5;
 constexpr int kDenseThreads = 256;
 constexpr uint32_t kNoPair = 0x7fffu;  // slot without a baseline (256 antennas: < 32640 pairs)
 
@@ -904,7 +921,12 @@ bool make_dense_plan(const uint32_t* ggu, int nbls, int nants, int nubls, DenseP
   const int gw = 32 / pl->gl;
   const int warps = std::max(1, std::min(kDenseThreads / 32, (nants + 3 * gw - 1) / (3 * gw)));
   pl->threads = 32 * warps;
-  if (dense_smem(nants, nubls, warps * gw) > (size_t)kOmSmemLimit) return false;
+  const size_t smem = dense_smem(nants, nubls, warps * gw);
+  if (smem > (size_t)kOmSmemLimit) return false;
+  if (nants <= 64 ? 2.0 * warps * gw * nubls > kDenseCopies * (nants * (nants - 1) / 2)
+                  : (nants < 108 || (nants > 128 && nants < 225)) &&
+                        2 * (smem + 1024) > (size_t)(228 * 1024))
+    return false;
   // rows padded to whole chunks of the longest row of their warp's groups
   pl->row_off.resize(nants);
   int n = 0;
