@@ -123,30 +123,42 @@ def sources_up(w, t):
     return int(np.count_nonzero(z > 0))
 
 
-def tc_chunk(nsrc, nslices, ngroups, num_sms):
+def tc_block_rows(nant, method):
+    """Rows of the fused kernel's antenna blocks (hv_tc.cu tc_block_rows): as
+    few blocks of at most 128 as there can be, evenly filled in split BF16."""
+    if method != "tc":
+        return 128
+    nb = -(-nant // 128)
+    return -(--(-nant // nb) // 32) * 32
+
+
+def tc_chunk(nsrc, nslices, nant, method, num_sms):
     """Split-K chunk the library picks (hv_tc.cu tc_chunk_sources) where the
     items fill the GPU."""
-    up = max(nsrc // 2, 1)
-    nrun = max(1, -(-40 * num_sms // (nslices * ngroups)))
-    run = min((max(1024, -(-up // nrun)) + 16) // 32 * 32, 2048)
+    up, ngroups = max(nsrc // 2, 1), tc_num_groups(nant, method)
+    start = 64 + 2 * tc_block_rows(nant, method)
+    nspan = max(1, -(-40 * num_sms // (nslices * ngroups)))
+    span = -(-min(32768, max(1024, -(-up // nspan))) // 32) * 32
+    run = min(2048, -(-(span // -(-span // 2080)) // 32) * 32)
     return min(range(run, 32769, run),
-               key=lambda c: min(nslices, 1 << 20) * ngroups * (up + 320 * -(-up // c))
-               + num_sms * (min(c, up) + 320))
+               key=lambda c: min(nslices, 1 << 20) * ngroups * (up + start * -(-up // c))
+               + num_sms * (min(c, up) + start))
 
 
-def tc_groups(nant):
+def tc_groups(nant, method):
     """The fused kernel's block-pair groups (hv_tc.cu make_groups): per group
     the columns of its four MMAs a product, as multiples of one.  Pairs (I, J),
     (I, J + 1) share row block I; the pairs left over at the end of a row,
     (I, nb - 1), are taken as (nb - 1, I) and paired in ascending I.  A block
     with itself takes three of the four MMAs."""
-    nb = (nant + 127) // 128
-    ncols = [(min(128, nant - 128 * b) + 15) // 16 * 16 for b in range(nb)]
+    rows = tc_block_rows(nant, method)
+    nb = -(-nant // rows)
+    ncols = [(min(rows, nant - rows * b) + 15) // 16 * 16 for b in range(nb)]
     groups, singles = [], []
     for I in range(nb):
         J = I
         while J + 1 < nb:
-            groups.append([(128, I == J), (ncols[J + 1], False)])
+            groups.append([(rows, I == J), (ncols[J + 1], False)])
             J += 2
         if J < nb:
             singles.append((ncols[I], I == nb - 1))
@@ -155,8 +167,8 @@ def tc_groups(nant):
     return [sum(n * (3 if own else 4) for n, own in g) / 4 for g in groups]
 
 
-def tc_num_groups(nant):
-    return len(tc_groups(nant))
+def tc_num_groups(nant, method):
+    return len(tc_groups(nant, method))
 
 
 # ------------------------------------------------------------------- clocks --
@@ -487,12 +499,12 @@ def run_ours(args):
         kern_s = r["kern_ms"] / 1e3
         if method in ("tc", "tc_fp16"):
             ks, mmas = (16, 12) if method == "tc" else (32, 16)
-            chunk = tc_chunk(S, T_PER_STEP * F, tc_num_groups(N), num_sms)
+            chunk = tc_chunk(S, T_PER_STEP * F, N, method, num_sms)
             stages = sum(sum(math.ceil(min(chunk, su - k0) / ks) for k0 in range(0, su, chunk))
                          for su in s_up) * F
             # tensor-pipe work in units of an M128 K16 BF16 MMA (an FP8 MMA
             # of K = 32 takes the same time)
-            hw_flops = stages * mmas * 2 * 128 * 16 * sum(tc_groups(N))
+            hw_flops = stages * mmas * 2 * 128 * 16 * sum(tc_groups(N, method))
             peak = peaks.get("bf16_tflops_sustained", peaks.get("bf16_tflops"))
             traffic_unit = TC_DRAM_BYTES_PER_UNIT.get(method)
             units = sum(s_up) * F
@@ -506,7 +518,7 @@ def run_ours(args):
                     "peak_kind": f"bf16 dense sustained ({peak_src})",
                     "algorithmic": "4 N (N+1) S_up flops per slice (Hermitian upper triangle); "
                                    "hw_* counts the issued MMAs in BF16 M128 K16 equivalents "
-                                   + ("(3 split-BF16 products, 128-blocks)" if method == "tc" else
+                                   + ("(3 split-BF16 products, blocks of 32 to 128 rows)" if method == "tc" else
                                       "(FP16 hi product + 2 FP8 cross products, 128-blocks)")}
         peak = 152 * 128 * 2 * 1.92e9 / 1e12
         return {"bound": "fp32-simt", "achieved": herk_flops / kern_s / 1e12, "peak": peak,

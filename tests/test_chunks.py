@@ -1,11 +1,18 @@
 """The split of the fused kernel's sources and antennas, from the library's own
 host code (fake_gpu.py)."""
 import ctypes
+import os
 import random
+import sys
 
 import pytest
 
 import fake_gpu
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+sys.path.insert(0, ROOT)
+
+import bench  # noqa: E402
 
 SMS = 152
 
@@ -48,3 +55,12 @@ def test_accumulator_runs_are_no_longer_than_flushes_of_spans(lib):
         mean = [sum(k * k for k in x) / up for x in (pieces, runs)]
         assert mean[1] <= 1.03 * mean[0], (nsrc, ntimes, nfreq, nant)
 
+
+# the benchmark's account of the issued MMAs restates both
+@pytest.mark.parametrize("method,form", [("tc", 0), ("tc_fp16", 1)])
+def test_the_benchmark_restates_the_split(lib, method, form):
+    for nsrc, ntimes, nfreq, nant in shapes(1000):
+        assert bench.tc_num_groups(nant, method) == lib._ZN2hv13tc_num_groupsEi(nant)
+        assert bench.tc_block_rows(nant, method) == lib._ZN2hv13tc_block_rowsEii(nant, form)
+        got = bench.tc_chunk(nsrc, ntimes * nfreq, nant, method, SMS)
+        assert got == chunk_and_run(lib, nsrc, ntimes, nfreq, nant, form, spread=False)[0]
