@@ -27,12 +27,11 @@ __device__ __forceinline__ double2 make_phasor(const SrcRec64& r, const Ucoef64&
   return phasor64(r, u, A);
 }
 
-// A warp generates kGenSpan sources for 32 antennas, whose coefficients stay in
+// A warp generates `span` sources for 32 antennas, whose coefficients stay in
 // its registers.  Slice z of the launch: time z / nf, frequency z % nf.
-constexpr int kGenSpan = 64;
 template <typename R>
 __global__ void __launch_bounds__(256)
-gen_phasors_kernel(const PlainDims d, const typename Traits<R>::Rec* __restrict__ rec,
+gen_phasors_kernel(const PlainDims d, int span, const typename Traits<R>::Rec* __restrict__ rec,
                    const typename Traits<R>::U* __restrict__ U, const R* __restrict__ beamT,
                    int PP, int dx, int dy, typename Traits<R>::C* __restrict__ v) {
   using C = typename Traits<R>::C;
@@ -40,14 +39,14 @@ gen_phasors_kernel(const PlainDims d, const typename Traits<R>::Rec* __restrict_
   const int n = d.counts[tl];
   const int groups = d.Np / 32;
   const long long job = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
-  const long long s0 = job / groups * kGenSpan;
+  const long long s0 = job / groups * span;
   if (s0 >= n) return;
   const int a = (int)(job % groups) * 32 + (threadIdx.x & 31);
   const typename Traits<R>::U u = U[((size_t)tl * d.u_nf + f) * d.Np + a];
   const R* beam = beamT + (size_t)f * PP * d.Np;
   rec += (size_t)tl * d.rec_stride;
   v += (size_t)z * d.v_stride + a;
-  const int s1 = (int)min((long long)n, s0 + kGenSpan);
+  const int s1 = (int)min((long long)n, s0 + span);
 #pragma unroll 2
   for (int s = (int)s0; s < s1; ++s) {
     C val;
@@ -60,13 +59,23 @@ gen_phasors_kernel(const PlainDims d, const typename Traits<R>::Rec* __restrict_
   }
 }
 
+// Sources a warp takes at most; fewer while that leaves fewer warps than fill the
+// GPU twice (half the sources are above the horizon; groups of padding hardly
+// count), since they come one after the other: 4 antennas x 100 sources 66 us at
+// 64, 5 at one; 350 x 20000 47 us at 64, 21 at 8, more again at 4.
+constexpr int kGenSpan = 64, kGenFill = 2 * 152 * 64;
+
 template <typename R>
 cudaError_t launch_gen_phasors(const PlainDims& d, int nz, const void* rec, int nsrc_max,
                                const void* U, const R* beamT, int P, void* v, cudaStream_t st) {
   const int dx = P > 1 ? 1 : 0, dy = P > 1 ? P : 0;
-  const long long jobs = (long long)ceil_div(std::max(nsrc_max, 1), kGenSpan) * (d.Np / 32);
-  gen_phasors_kernel<R><<<dim3((unsigned)((jobs + 7) / 8), nz), 256, 0, st>>>(
-      d, reinterpret_cast<const typename Traits<R>::Rec*>(rec),
+  const int nsrc = std::max(nsrc_max, 1);
+  auto jobs = [&](int span) { return (long long)ceil_div(nsrc, span) * (d.Np / 32); };
+  int span = kGenSpan;
+  while (span > 1 && (long long)ceil_div(nsrc, span) * ceil_div(d.nant, 32) * nz < kGenFill)
+    span /= 2;
+  gen_phasors_kernel<R><<<dim3((unsigned)((jobs(span) + 7) / 8), nz), 256, 0, st>>>(
+      d, span, reinterpret_cast<const typename Traits<R>::Rec*>(rec),
       reinterpret_cast<const typename Traits<R>::U*>(U), beamT, P * P, dx, dy,
       reinterpret_cast<typename Traits<R>::C*>(v));
   return cudaGetLastError();

@@ -44,7 +44,8 @@ class FakeGpu:
         self.lib.fake_reset(capacity)
 
     def log(self):
-        """Lines since the last call: (operation, first value, second value)."""
+        """Lines since the last call: (operation, first value, second value); of a
+        launch the stream and the blocks."""
         n = self.lib.fake_log(None, 0) + 1
         buf = ctypes.create_string_buffer(n)
         self.lib.fake_log(buf, n)

@@ -65,13 +65,13 @@ void give_back(void* p) {
   blocks.erase(it);
 }
 
-cudaError_t launch(const void* f, cudaStream_t st) {
+cudaError_t launch(const void* f, dim3 g, cudaStream_t st) {
   const std::string& name = kernels[f];
   if (!fail_name.empty() && name.find(fail_name) != std::string::npos && fail_after-- == 0) {
     note(("launch fails " + name).c_str(), st);
     return result(cudaErrorLaunchOutOfResources);
   }
-  note(("launch " + name).c_str(), st);
+  note(("launch " + name).c_str(), st, (void*)((size_t)g.x * g.y * g.z));
   return cudaSuccess;
 }
 
@@ -138,11 +138,11 @@ cudaError_t __cudaGetKernel(cudaKernel_t* k, const void* f) {
   *k = reinterpret_cast<cudaKernel_t>(const_cast<void*>(f));
   return cudaSuccess;
 }
-cudaError_t __cudaLaunchKernel(cudaKernel_t k, dim3, dim3, void**, size_t, cudaStream_t st) {
-  return launch(k, st);
+cudaError_t __cudaLaunchKernel(cudaKernel_t k, dim3 g, dim3, void**, size_t, cudaStream_t st) {
+  return launch(k, g, st);
 }
 cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t* c, const void* f, void**) {
-  return launch(f, c->stream);
+  return launch(f, c->gridDim, c->stream);
 }
 
 // --------------------------------------------------------------- device --
