@@ -91,12 +91,14 @@ __device__ __forceinline__ void decode_upper(int t, int nb, int& I, int& J) {
   J = I + t;
 }
 
-// FP64: one tile of a chunk, 4 x 4 outputs a thread; bound by the FP64 pipe
-// (2 FMA a clock and SM).
-__device__ __forceinline__ void herk_tile(const double2* __restrict__ v, int n, int Np,
-                                          double* __restrict__ partial) {
-  using R = double;
-  using C = double2;
+// One tile of a chunk, 4 x 4 outputs a thread.  FP64: bound by the FP64 pipe (2 FMA
+// a clock and SM).  FP32: each stage of 16 sources is summed from zero, as in
+// herk_plain_kernel, whose bits it gives; for launches of few blocks.
+template <typename R>
+__device__ __forceinline__ void herk_tile(const typename Traits<R>::C* __restrict__ v, int n,
+                                          int Np, R* __restrict__ partial) {
+  using C = typename Traits<R>::C;
+  constexpr bool kTwoLevel = sizeof(R) == 4;
   const int s0 = blockIdx.y * kPlainChunk;
   if (s0 >= n) return;
   const int s1 = min(s0 + kPlainChunk, n);
@@ -136,6 +138,14 @@ __device__ __forceinline__ void herk_tile(const double2* __restrict__ v, int n, 
     }
     __syncthreads();
     if (s + kHK < s1) gload(s + kHK);
+    R st_re[4][4], st_im[4][4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        st_re[i][j] = kTwoLevel ? R(0) : acc_re[i][j];
+        st_im[i][j] = kTwoLevel ? R(0) : acc_im[i][j];
+      }
 #pragma unroll
     for (int k = 0; k < kHK; ++k) {
       C a[4], b[4];
@@ -148,10 +158,17 @@ __device__ __forceinline__ void herk_tile(const double2* __restrict__ v, int n, 
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
           // v_a conj(v_b) = (ar br + ai bi) + i (ai br - ar bi)
-          acc_re[i][j] = fma(a[i].x, b[j].x, fma(a[i].y, b[j].y, acc_re[i][j]));
-          acc_im[i][j] = fma(a[i].y, b[j].x, fma(-a[i].x, b[j].y, acc_im[i][j]));
+          st_re[i][j] = fma(a[i].x, b[j].x, fma(a[i].y, b[j].y, st_re[i][j]));
+          st_im[i][j] = fma(a[i].y, b[j].x, fma(-a[i].x, b[j].y, st_im[i][j]));
         }
     }
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        acc_re[i][j] = kTwoLevel ? acc_re[i][j] + st_re[i][j] : st_re[i][j];
+        acc_im[i][j] = kTwoLevel ? acc_im[i][j] + st_im[i][j] : st_im[i][j];
+      }
     __syncthreads();
   }
   R* pre = partial + (size_t)blockIdx.y * 2 * Np * Np;
@@ -284,12 +301,13 @@ herk_plain_kernel(const PlainDims d, const float2* __restrict__ v_base,
   }
 }
 
+template <typename R>
 __global__ void __launch_bounds__(256)
-herk_plain_f64_kernel(const PlainDims d, const double2* __restrict__ v,
-                      double* __restrict__ partial) {
+herk_tile_kernel(const PlainDims d, const typename Traits<R>::C* __restrict__ v,
+                 R* __restrict__ partial) {
   const int z = blockIdx.z;
-  herk_tile(v + (size_t)z * d.v_stride, d.counts[z / d.nf], d.Np,
-            partial + (size_t)z * d.p_stride);
+  herk_tile<R>(v + (size_t)z * d.v_stride, d.counts[z / d.nf], d.Np,
+               partial + (size_t)z * d.p_stride);
 }
 
 __global__ void __launch_bounds__(256)
@@ -299,7 +317,7 @@ herk_flagged_kernel(const F64Dims d, const double2* __restrict__ v,
   const int z = blockIdx.z;
   if (!flags[z]) return;
   const int n = max(0, min(d.counts[z / d.nf] - d.s0, d.S));
-  herk_tile(v + (size_t)z * d.v_stride, n, d.Np, partial + (size_t)z * partial_stride);
+  herk_tile<double>(v + (size_t)z * d.v_stride, n, d.Np, partial + (size_t)z * partial_stride);
 }
 
 cudaError_t launch_herk_flagged(const F64Dims& d, int nz, const void* v, const int* flags,
@@ -311,15 +329,33 @@ cudaError_t launch_herk_flagged(const F64Dims& d, int nz, const void* v, const i
   return cudaGetLastError();
 }
 
+// FP32 launches whose blocks with sources (about half of the catalogue's chunks)
+// are on the SMs at once, two each, take herk_tile, and launches of one or two
+// slices that fill the SMs about twice: a packed block alone on its SM, or one of
+// two, ends later (350 antennas x 20k sources x 4 slices 1058 us a call, packed,
+// and 963; 512 x 8000 x 8 1050 and 964; 350 x 100k x 2 2024 and 1908), while a
+// last wave that is half empty costs it less (700 x 5000 x 5 950 and 1104), and
+// launches of more waves are even or faster packed.
+constexpr int kHerkWave = 2 * 152;
+bool herk_few(int tiles, int nsrc_max, int nz) {
+  const long long blocks = (long long)tiles * ceil_div((nsrc_max + 1) / 2, kPlainChunk) * nz;
+  return blocks <= kHerkWave ||
+         (nz <= 2 && blocks > kHerkWave * 17 / 10 && blocks <= 2 * kHerkWave);
+}
+
 template <typename R>
 cudaError_t launch_herk_plain(const PlainDims& d, int nz, const void* v, int nsrc_max, R* partial,
                               cudaStream_t st) {
   const int nb = d.Np / kHT;
   const dim3 grid(nb * (nb + 1) / 2, ceil_div(std::max(nsrc_max, 1), kPlainChunk), nz);
-  if constexpr (sizeof(R) == 4)
-    herk_plain_kernel<<<grid, 256, 0, st>>>(d, static_cast<const float2*>(v), partial);
-  else
-    herk_plain_f64_kernel<<<grid, 256, 0, st>>>(d, static_cast<const double2*>(v), partial);
+  if constexpr (sizeof(R) == 4) {
+    if (!herk_few(grid.x, nsrc_max, nz)) {
+      herk_plain_kernel<<<grid, 256, 0, st>>>(d, static_cast<const float2*>(v), partial);
+      return cudaGetLastError();
+    }
+  }
+  herk_tile_kernel<R><<<grid, 256, 0, st>>>(d, static_cast<const typename Traits<R>::C*>(v),
+                                            partial);
   return cudaGetLastError();
 }
 

@@ -34,7 +34,18 @@ def test_phasors_of_many_sources(fake):
     assert 8 * sum(blocks(fake.log(), "gen_phasors")) <= 1.01 * 100_000 / 64 * 12 * 5
 
 
-# every span gives the same bits: a call of many slices and its
+# blocks that are on the SMs at once (two each) take the kernel that ends sooner
+@pytest.mark.parametrize("nant,nsrc,ntimes,few", [
+    (16, 1000, 1, True), (350, 20_000, 1, True), (350, 20_000, 4, True), (350, 100_000, 1, True),
+    (350, 100_000, 2, True), (350, 100_000, 5, False), (700, 5000, 5, False), (512, 8000, 8, True)])
+def test_products_of_few_blocks(fake, nant, nsrc, ntimes, few):
+    assert fake.call(fake.context(), 1, "plain", nant, nsrc, ntimes) == 0
+    log = fake.log()
+    assert bool(blocks(log, "herk_tile_kernel")) == few
+    assert bool(blocks(log, "herk_plain_kernel")) != few
+
+
+# both kernels and every span give the same bits: a call of many slices and its
 # single slices; a chunk of 4096 sources and a rest, stages of 16 and a rest
 @gpu
 @pytest.mark.parametrize("nant,nsrc", [(5, 9001), (130, 9001), (70, 300)])
