@@ -292,12 +292,11 @@ constexpr size_t kTcRecCap = size_t(4) << 30;
 constexpr size_t kPlainCap = size_t(2) << 30;
 
 // FP64 product on the tensor cores (hv_f64.cu) for every slice; HV_OK, an
-// error, or -1: the SIMT product is to be used (arrays whose class sums would
-// not fit, or no room for the workspace within the budget or on the device).
-// Measured at 350 antennas x 100k sources x 3 times: SIMT 102.7 ms a call;
-// at 25 antennas x 1008 sources x 35 times SIMT 75 ms (few tiles a slice, one
-// slice at a time).
-constexpr int kF64MaxNp = 2048;             // 96 bytes of class sums an element: 400 MB
+// error, or -1: the SIMT product is to be used (larger arrays, or no room for the
+// workspace within the budget or on the device).  Measured at 350 antennas x 100k
+// sources x 3 times: SIMT 102.7 ms a call, 3.87 here; at 25 antennas x 1008
+// sources x 35 times 75 ms (one slice at a time) and 0.29.
+constexpr int kF64MaxNp = 2048;             // a slice of 65536 sources takes 5.9 GB there
 constexpr int kF64Window = 65536;           // sources per window (40 bytes a phasor)
 constexpr size_t kF64Cap = size_t(4) << 30; // workspace of the slices of one launch
 

@@ -532,8 +532,8 @@ __global__ void __launch_bounds__(kOmMaxThreads, OM_MINB) omnical_kernel(const O
 // copies costs more than the gathers (54 antennas, 1000 problems, 12
 // iterations: 2.1 ms, general kernel 1.7 ms).
 //
-// Bound by issue slots (67% busy at 180 antennas) and the shared-memory pipe
-// (81%: gathers and updates at the unique baselines' scattered places).
+// Bound by issue slots (68% busy at 180 antennas) and the shared-memory pipe
+// (79%: gathers and updates at the unique baselines' scattered places).
 // Measured on GB300, 12 iterations of 2000 problems, general kernel and this
 // one: 180 antennas 3.70 and 2.48 ms, 128 antennas 2.84 and 1.64 ms, 54
 // antennas 0.44 and 0.36 ms.

@@ -1653,10 +1653,10 @@ cudaError_t launch_form(const TcSimDesc* sims, int nsims, const void* rec, long 
   p.rows = tc_block_rows(sims[0].nant, kForm);
   const int slot = p.rows * TC_ROW_BYTES;
   const int per_stage = TILES * p.max_slots * slot;
-  // records and the barrier block (barriers, item ring, TMEM holder);
+  // records and the barrier block (barriers, item ring, TMEM holder), or the rows
+  // past the last tile's block that the row operand is read with, which lie behind
+  // that tile, if they are more
   constexpr int TC_NREC = TcForm<kForm>::NREC;
-  // and, behind the last tile, the rows past its block that the row operand
-  // is read with
   const int fixed = std::max(TC_NREC * KS * 32 + 8 * (2 * TC_NREC + 3 * TC_MAX_STAGES + 3 + 3 * TC_ITEM_RING) + 8,
                              TC_ROWS * TC_ROW_BYTES - slot);
   const int max_stages = std::min(kForm == 0 ? TC_MAX_STAGES : TC_STAGES,

@@ -74,7 +74,11 @@ typedef struct hv_context hv_context;
 int hv_version(void);
 
 /* Open a context on CUDA device `device`; `hbm_budget_bytes` caps the
- * workspace the context may hold (0 = no cap).  Replaces the import-time
+ * workspace the context may hold (0 = no cap: up to 6 GB of partial sums and 4
+ * GB of source records for the fused forms, 2 GB for the plain form, 4 GB for
+ * FP64, as large as the calls made ask for; it is kept for the next call of its
+ * kind until hv_destroy, and given back to a call, batch or allocation of this
+ * context that finds no room).  Replaces the import-time
  * pycuda.autoinit context of the reference (vis.py:1). */
 int hv_create(hv_context** ctx, int device, size_t hbm_budget_bytes);
 int hv_destroy(hv_context* ctx);
@@ -108,7 +112,8 @@ int hv_vis_multifreq(hv_context* ctx, int precision, int method,
  * hv_sync() before reading `d_vis_out` on another stream or the host (the
  * context's stream is made to wait for the call's work on `stream`, unless
  * `stream` is being captured into a graph; then synchronise `stream`
- * itself). */
+ * itself).  A call to be captured must have been made once before, and the graph
+ * uses the context's workspace: a larger call on this context replaces it. */
 int hv_vis_multifreq_device(hv_context* ctx, int precision, int method,
                             const void* d_antpos, int nant,
                             const double* freqs, int nfreq,
@@ -121,11 +126,13 @@ int hv_vis_multifreq_device(hv_context* ctx, int precision, int method,
  * (e.g. HV_ERR_TIMEOUT from a bounded wait). */
 int hv_sync(hv_context* ctx);
 
-/* Device timing of the visibility-product kernels (the fused tensor-core
- * kernel, or the SIMT Hermitian product of the plain form): with profiling
- * on, every launch of them is bracketed by CUDA events on the stream it runs
- * on.  hv_profile_read() synchronises, returns the summed milliseconds and
- * launch count since the previous read, and clears them. */
+/* Device timing of the visibility products (the fused tensor-core kernel, the
+ * plain form's Hermitian product, or the digits and class sums of FP64): with
+ * profiling on, every one is bracketed by CUDA events on the stream it runs on.
+ * A batch that is not a graph then runs its size classes one after the other,
+ * each timed alone.  hv_profile_read() synchronises, returns the summed
+ * milliseconds and the number of products since the previous read, and clears
+ * them. */
 int hv_set_profiling(hv_context* ctx, int enable);
 int hv_profile_read(hv_context* ctx, double* ms, uint64_t* launches);
 
