@@ -400,14 +400,14 @@ def load_peaks():
 # fused-kernel launch, measured once with ncu (dram__bytes_read.sum +
 # dram__bytes_write.sum of the launch on 350 antennas x 1,048,576 sources x
 # 16 channels x 4 LSTs, which under ncu computes all 33,517,808 units:
-# split BF16 2.367 GB, FP16 + FP8 2.615 GB): the bench cannot read DRAM
+# split BF16 2.087 GB, FP16 + FP8 2.199 GB): the bench cannot read DRAM
 # counters itself, so the figure is carried here and scaled by the units
-# each timed launch processed.  That launch uses split-K chunks of 16384
+# each timed launch processed.  That launch uses split-K chunks of 14336
 # sources; the 64-channel benchmark call uses chunks of 32768, with half
 # as many partial sums to write, so for it the figure is an upper bound
 # (a full-size capture of these counters takes several ncu passes, more
 # than a capture of that size may).
-TC_DRAM_BYTES_PER_UNIT = {"tc": 70.619, "tc_fp16": 78.013}
+TC_DRAM_BYTES_PER_UNIT = {"tc": 62.277, "tc_fp16": 65.603}
 
 
 def run_leg(fn, *a):
