@@ -289,9 +289,9 @@ __device__ __forceinline__ long long scaled_int(double v, int field) {
 // to kPlainChunk, and in proportion to n beyond.  Arrays of Airy or random beams
 // over 150 to 100k sources lie at 5 to 600 times this limit.
 constexpr int kOverlapMin = 64;
-// A chunk's sum is capped here: exact in FP32 below, 256 chunks fit in 32 bits,
-// and the limit never exceeds 1024.
-constexpr float kOverlapCap = 1048576.f;
+// Sums are capped here to fit in 32 bits.  They are exact in FP32 up to 2^24, and
+// the limit never exceeds 1024.
+constexpr float kOverlapCap = 1073741824.f;
 
 // Where a slice's weights start in its digits.
 __device__ __forceinline__ size_t weight_tiles(const F64Dims& d) {
@@ -407,7 +407,8 @@ digits64_kernel(const F64Dims d, const double2* __restrict__ v,
 // of 78, and the digits are read once.  Three blocks: 0.93 -> 0.86 ms a slice.
 //
 // The last unit of a pair of blocks sums the overlaps, one product of the weights
-// a step; its stages take as many steps as fit.
+// a step, over the whole window (the first chunk's item, plain stores); its stages
+// take as many steps as fit.
 constexpr int kDigUnits = 9, kUnits = kDigUnits + 1;
 __constant__ int8_t kUnit[kDigUnits][3] = {{5, 0, 5}, {5, 6, 11}, {2, 0, 5}, {4, 0, 4}, {4, 5, 9},
                                         {3, 0, 3}, {3, 4, 7},  {1, 0, 3}, {0, 0, 1}};
@@ -464,13 +465,13 @@ mma64_kernel(const F64Dims d, const uint8_t* __restrict__ dig, const int* __rest
   const int pair = blockIdx.x % npairs, unit = blockIdx.x / npairs % kUnits;
   const int cz = blockIdx.x / (npairs * kUnits), chunk = cz % nchunks, z = cz / nchunks;
   const int steps = ceil_div(window_count(d, z), 32);
-  const int k0 = chunk * chunk_steps, k1 = min(steps, k0 + chunk_steps);
-  if (k0 >= k1 || flags[z]) return;
+  const bool over = unit == kDigUnits;
+  const int k0 = chunk * chunk_steps, k1 = over ? steps : min(steps, k0 + chunk_steps);
+  if (k0 >= k1 || flags[z] || (over && chunk)) return;
   int I = 0, J = pair;
   for (const int nb = d.Np / 128; J >= nb - I; ++I) J -= nb - I;
   J += I;
   // digits of A and of B
-  const bool over = unit == kDigUnits;
   const int du = over ? 0 : unit;
   const bool own = I == J, same = own && (over || kOwnUnit[du][1]);
   const int g = own ? kOwnUnit[du][0] : kUnit[du][0];
@@ -588,7 +589,7 @@ mma64_kernel(const F64Dims d, const uint8_t* __restrict__ dig, const int* __rest
       tmem_ld32(tq + c, x);
 #pragma unroll
       for (int k = 0; k < 32; ++k)
-        atomicAdd(wo + (size_t)(c + k) * d.Np, (uint32_t)fminf(x[k], kOverlapCap));
+        wo[(size_t)(c + k) * d.Np] = (uint32_t)fminf(x[k], kOverlapCap);
     }
 #pragma unroll 1
     for (int c = over ? 128 : 0; c < 128; c += 32) {
